@@ -7,7 +7,8 @@ library is an error, never a silent fallback.
 
 All functions take an ``rng`` handle (:class:`StepRNG`) rather than a raw seed: the CPU path reads
 ``rng.seed`` (a Python int), the kernels read the seed from device memory (``rng.dev``), which keeps
-a captured CUDA graph valid when the seed changes every step.
+a captured CUDA graph valid when the seed changes every step.  ``**packed`` (``tmap=`` a TokenMap, kernels only) says that
+the activation rows are packed tokens.
 """
 from __future__ import annotations
 
@@ -40,17 +41,18 @@ def _is_cuda(t: torch.Tensor) -> bool:
 
 
 # ----------------------------------------------------------------------------- encoder ops
-def embed_ln_fwd(ids, word, pos, gamma, beta, eps, S, p, rng, stream, out, mean, rstd):
+def embed_ln_fwd(ids, word, pos, gamma, beta, eps, S, p, rng, stream, out, mean, rstd, **packed):
     if _is_cuda(out):
-        return _cuda().embed_ln_fwd(ids, word, pos, gamma, beta, eps, S, p, rng, stream, out, mean, rstd)
+        return _cuda().embed_ln_fwd(ids, word, pos, gamma, beta, eps, S, p, rng, stream, out, mean, rstd, **packed)
     y, m, r = ref.embed_ln_fwd(ids, word, pos, gamma, beta, eps, S, p, rng.seed, stream, out.dtype)
     out.copy_(y); mean.copy_(m); rstd.copy_(r)
 
 
-def embed_ln_bwd(dy, ids, word, pos, gamma, mean, rstd, S, p, rng, stream, pad_id, dword, dpos, dgamma, dbeta):
+def embed_ln_bwd(dy, ids, word, pos, gamma, mean, rstd, S, p, rng, stream, pad_id, dword, dpos, dgamma, dbeta,
+                 **packed):
     if _is_cuda(dy):
         return _cuda().embed_ln_bwd(dy, ids, word, pos, gamma, mean, rstd, S, p, rng, stream, pad_id,
-                                    dword, dpos, dgamma, dbeta)
+                                    dword, dpos, dgamma, dbeta, **packed)
     ref.embed_ln_bwd(dy, ids, word, pos, gamma, mean, rstd, S, p, rng.seed, stream, pad_id, dword, dpos, dgamma, dbeta)
 
 
@@ -64,19 +66,19 @@ def attention_workspace(b, S, nh, device, dtype, ds=None):
     return ws
 
 
-def attention_fwd(qkv, bqkv, mask, nh, p, rng, stream, ctx_out, ws):
+def attention_fwd(qkv, bqkv, mask, nh, p, rng, stream, ctx_out, ws, **packed):
     b = mask.shape[0]
     if _is_cuda(qkv):
-        return _cuda().attention_fwd(qkv, bqkv, mask, nh, p, rng, stream, ctx_out, ws)
+        return _cuda().attention_fwd(qkv, bqkv, mask, nh, p, rng, stream, ctx_out, ws, **packed)
     ctx, probs = ref.attention_fwd(qkv, bqkv, mask, nh, p, rng.seed, stream)
     ctx_out.copy_(ctx)
     ws["probs"][:b].copy_(probs)
 
 
-def attention_bwd(dctx, qkv, bqkv, mask, nh, p, rng, stream, ws, dqkv_out, dbqkv_out):
+def attention_bwd(dctx, qkv, bqkv, mask, nh, p, rng, stream, ws, dqkv_out, dbqkv_out, **packed):
     b = mask.shape[0]
     if _is_cuda(qkv):
-        return _cuda().attention_bwd(dctx, qkv, bqkv, mask, nh, p, rng, stream, ws, dqkv_out, dbqkv_out)
+        return _cuda().attention_bwd(dctx, qkv, bqkv, mask, nh, p, rng, stream, ws, dqkv_out, dbqkv_out, **packed)
     d = ref.attention_bwd(dctx, qkv, bqkv, mask, ws["probs"][:b], nh, p, rng.seed, stream)
     dqkv_out.copy_(d)
     ref.colsum(d, dbqkv_out)
@@ -91,11 +93,11 @@ def bias_dropout_add_ln_fwd(x, bias, resid, gamma, beta, eps, p, rng, stream, y_
 
 
 def bias_dropout_add_ln_bwd(dy, pre, gamma, mean, rstd, p, rng, stream, dgamma, dbeta, dbias,
-                            dpre_out, dbranch_out):
+                            dpre_out, dbranch_out, **packed):
     """Returns ``(d_pre, d_branch)``; with ``p == 0`` both are the same tensor (``dpre_out``)."""
     if _is_cuda(dy):
         return _cuda().bias_dropout_add_ln_bwd(dy, pre, gamma, mean, rstd, p, rng, stream,
-                                               dgamma, dbeta, dbias, dpre_out, dbranch_out)
+                                               dgamma, dbeta, dbias, dpre_out, dbranch_out, **packed)
     d_pre, d_branch = ref.bias_dropout_add_ln_bwd(dy, pre, gamma, mean, rstd, p, rng.seed, stream,
                                                   dgamma, dbeta, dbias)
     dpre_out.copy_(d_pre)
@@ -117,15 +119,15 @@ def bias_gelu_bwd(da, x, bias, dbias, dx_out):
     dx_out.copy_(ref.bias_gelu_bwd(da, x, bias, dbias))
 
 
-def pool_fwd(h, mask, mode, out):
+def pool_fwd(h, mask, mode, out, **packed):
     if _is_cuda(h):
-        return _cuda().pool_fwd(h, mask, mode, out)
+        return _cuda().pool_fwd(h, mask, mode, out, **packed)
     out.copy_(ref.pool_fwd(h, mask, mode))
 
 
-def pool_bwd(de, mask, mode, S, dh_out):
+def pool_bwd(de, mask, mode, S, dh_out, **packed):
     if _is_cuda(de):
-        return _cuda().pool_bwd(de, mask, mode, S, dh_out)
+        return _cuda().pool_bwd(de, mask, mode, S, dh_out, **packed)
     dh_out.copy_(ref.pool_bwd(de, mask, mode, S, dh_out.dtype))
 
 

@@ -17,12 +17,35 @@
 // Reference behaviour: the attention of the HF DistilBERT layers that main.py:225-262 wraps.
 #include <type_traits>
 #include "common.cuh"
+#include "token_map.cuh"
 
 namespace rb {
 namespace amma {
 
 constexpr int HD = 64;
 constexpr int RP = HD + 8;   // operand row pitch (elements): 144 B keeps the 8 rows of an ldmatrix on distinct banks
+
+// Where the tokens of a sequence live: packed rows (token_map.cuh) or, with slot == nullptr, the padded [b, S] layout.
+// Dropped tokens are masked keys that no kept query can see and queries nobody reads: they are neither loaded nor
+// written, and tiles of 8 keys or 16 queries behind a sequence's last kept token are skipped.
+struct Tok {
+  const int* slot;   // [b * S] row of a token or -1
+  const int* len;    // [b] last kept position + 1
+  const int* meta;   // row counts
+};
+__device__ __forceinline__ int seq_len(const Tok& tk, int b, int S) { return tk.slot != nullptr ? __ldcg(tk.len + b) : S; }
+__device__ __forceinline__ int seq_row(const Tok& tk, int b, int S, int s) {
+  return tk.slot != nullptr ? __ldcg(tk.slot + (size_t)b * S + s) : b * S + s;
+}
+// The zero rows behind the last packed token (rows of no sequence): columns [c0, c0 + HD) of each, by the CTAs of the
+// last sequence.
+template <typename T>
+__device__ __forceinline__ void clear_zero_rows(const Tok& tk, T* out, int ld, int c0, int width) {
+  const int lo = __ldcg(tk.meta + TOK_VALID), hi = __ldcg(tk.meta + TOK_ROWS);
+  const int per = width / 8;
+  for (int i = threadIdx.x; i < (hi - lo) * per; i += blockDim.x)
+    *reinterpret_cast<uint4*>(out + (size_t)(lo + i / per) * ld + c0 + (i % per) * 8) = make_uint4(0u, 0u, 0u, 0u);
+}
 
 template <typename T> struct Pack;
 template <> struct Pack<__nv_bfloat16> {
@@ -80,15 +103,17 @@ __device__ __forceinline__ float quad_max(float v) {
 }
 
 // acc[j] (j = 8-wide tile of columns) += A(16 rows r0.. of `a`, all HD columns) * B^T, B = SP rows of `bsm`:
-// the shape of Q K^T and of dO V^T.  Both operands are [row][RP] tiles.
+// the shape of Q K^T and of dO V^T.  Both operands are [row][RP] tiles; only the first `lim` rows of B exist (in all
+// of these routines lim is a multiple of 16 and the same in every lane).
 template <typename T, int SP>
-__device__ __forceinline__ void rows_times_transposed(float (&acc)[SP / 8][4], const T* a, const T* bsm, int r0, int lane) {
+__device__ __forceinline__ void rows_times_transposed(float (&acc)[SP / 8][4], const T* a, const T* bsm, int r0, int lane, int lim) {
   uint32_t af[HD / 16][4];
 #pragma unroll
   for (int kk = 0; kk < HD / 16; ++kk)
     ldsm4(af[kk], a + (r0 + (lane & 7) + ((lane >> 3) & 1) * 8) * RP + kk * 16 + (lane >> 4) * 8);
 #pragma unroll
   for (int j = 0; j < SP / 8; ++j) {
+    if (8 * j >= lim) continue;
 #pragma unroll
     for (int kk = 0; kk < HD / 16; kk += 2) {
       uint32_t bf[4];   // {b0, b1} of k-step kk, {b0, b1} of k-step kk + 1
@@ -102,9 +127,10 @@ __device__ __forceinline__ void rows_times_transposed(float (&acc)[SP / 8][4], c
 // out[jd] (jd = 8-wide tile of the HD columns) += A * B for a 16 x SP A held as packed fragments
 // (afr[kq] = the 16 x 16 block of columns 16 kq..) and B = the SP rows of the [row][RP] tile `bsm`.
 template <typename T, int SP>
-__device__ __forceinline__ void frag_times_rows(float (&out)[HD / 8][4], const uint32_t (&afr)[SP / 16][4], const T* bsm, int lane) {
+__device__ __forceinline__ void frag_times_rows(float (&out)[HD / 8][4], const uint32_t (&afr)[SP / 16][4], const T* bsm, int lane, int lim) {
 #pragma unroll
   for (int kq = 0; kq < SP / 16; ++kq) {
+    if (16 * kq >= lim) continue;
 #pragma unroll
     for (int jd = 0; jd < HD / 8; jd += 2) {
       uint32_t bf[4];   // {b0, b1} of column tile jd, {b0, b1} of column tile jd + 1
@@ -118,9 +144,10 @@ __device__ __forceinline__ void frag_times_rows(float (&out)[HD / 8][4], const u
 // out[jd] += A^T * B where A is the [SP][PP] tile `asm_` (rows = reduction index) restricted to its 16 columns
 // c0.., and B = the SP rows of the [row][RP] tile `bsm`: the shape of dS^T Q and of P~^T dO.
 template <typename T, int SP>
-__device__ __forceinline__ void transposed_times_rows(float (&out)[HD / 8][4], const T* asm_, int PP, int c0, const T* bsm, int lane) {
+__device__ __forceinline__ void transposed_times_rows(float (&out)[HD / 8][4], const T* asm_, int PP, int c0, const T* bsm, int lane, int lim) {
 #pragma unroll
   for (int kq = 0; kq < SP / 16; ++kq) {
+    if (16 * kq >= lim) continue;
     uint32_t af[4];
     const int mi = lane >> 3;
     ldsm4_t(af, asm_ + (16 * kq + (lane & 7) + (mi >> 1) * 8) * PP + c0 + (mi & 1) * 8);
@@ -134,19 +161,20 @@ __device__ __forceinline__ void transposed_times_rows(float (&out)[HD / 8][4], c
   }
 }
 
-// Writes the warp's 16 x HD accumulator tile (rows row0.. of the sequence) to global rows of stride ld and,
+// Writes the warp's 16 x HD accumulator tile to the global rows row_lo / row_hi (this lane's two rows; negative: none)
+// of stride ld and,
 // when col_sums != nullptr, adds the column sums of the rounded values to col_sums[0..HD) in shared memory.
 template <typename T>
-__device__ __forceinline__ void write_rows(const float (&out)[HD / 8][4], T* dst, int ld, int row0, int S, int lane,
+__device__ __forceinline__ void write_rows(const float (&out)[HD / 8][4], T* dst, int ld, int row_lo, int row_hi, int lane,
                                            float* col_sums) {
   const int g = lane >> 2, t = lane & 3;
-  const bool v0 = row0 + g < S, v1 = row0 + g + 8 < S;
+  const bool v0 = row_lo >= 0, v1 = row_hi >= 0;
 #pragma unroll
   for (int jd = 0; jd < HD / 8; ++jd) {
     const uint32_t lo = Pack<T>::pack(out[jd][0], out[jd][1]);
     const uint32_t hi = Pack<T>::pack(out[jd][2], out[jd][3]);
-    if (v0) *reinterpret_cast<uint32_t*>(dst + (size_t)g * ld + 8 * jd + 2 * t) = lo;
-    if (v1) *reinterpret_cast<uint32_t*>(dst + (size_t)(g + 8) * ld + 8 * jd + 2 * t) = hi;
+    if (v0) *reinterpret_cast<uint32_t*>(dst + (size_t)row_lo * ld + 8 * jd + 2 * t) = lo;
+    if (v1) *reinterpret_cast<uint32_t*>(dst + (size_t)row_hi * ld + 8 * jd + 2 * t) = hi;
     if (col_sums != nullptr) {
       const float2 a = Pack<T>::unpack(lo), b = Pack<T>::unpack(hi);
       float s0 = (v0 ? a.x : 0.f) + (v1 ? b.x : 0.f);
@@ -164,22 +192,29 @@ __device__ __forceinline__ void write_rows(const float (&out)[HD / 8][4], T* dst
   }
 }
 
-// Stages (q + bq, k + bk, v + bv [, dO]) of one (batch, head) as [SP][RP] tiles; rows >= S are zero.
+// Stages (q + bq, k + bk, v + bv [, dO]) of one (batch, head) as [SP][RP] tiles; rows of tokens that do not
+// exist are zero, rows >= lim are left alone.
 // The CTA has SP * 2 threads and the tiles SP * 8 segments of 8 columns, so a thread owns the same 8 columns of
 // four rows: all of its global loads are issued before the first one is used.
 template <typename T, int SP, bool WITH_DO>
 __device__ __forceinline__ void stage_operands(const T* __restrict__ qkv, const T* __restrict__ bqkv, const T* __restrict__ dctx,
-                                               T* sQ, T* sK, T* sV, T* sDO, int b, int h, int S, int H) {
+                                               T* sQ, T* sK, T* sV, T* sDO, const Tok& tk, int b, int h, int S, int H, int len,
+                                               int lim) {
   constexpr int ROWS_PER_PASS = SP * 2 / 8;
   const int d = (threadIdx.x & 7) * 8, s0 = threadIdx.x >> 3;
   Raw8<T> rq[4], rk[4], rv[4], rg[4];
+  int row[4];
 #pragma unroll
   for (int it = 0; it < 4; ++it) {
     const int s = s0 + it * ROWS_PER_PASS;
-    if (s < S) {
-      const size_t base = (size_t)(b * S + s) * 3 * H + h * HD + d;
+    row[it] = s < len ? seq_row(tk, b, S, s) : -1;
+  }
+#pragma unroll
+  for (int it = 0; it < 4; ++it) {
+    if (row[it] >= 0) {
+      const size_t base = (size_t)row[it] * 3 * H + h * HD + d;
       rq[it] = load_raw8(qkv + base); rk[it] = load_raw8(qkv + base + H); rv[it] = load_raw8(qkv + base + 2 * H);
-      if constexpr (WITH_DO) rg[it] = load_raw8(dctx + (size_t)(b * S + s) * H + h * HD + d);
+      if constexpr (WITH_DO) rg[it] = load_raw8(dctx + (size_t)row[it] * H + h * HD + d);
     }
   }
   float bq[8], bk[8], bv[8];
@@ -187,8 +222,9 @@ __device__ __forceinline__ void stage_operands(const T* __restrict__ qkv, const 
 #pragma unroll
   for (int it = 0; it < 4; ++it) {
     const int s = s0 + it * ROWS_PER_PASS;
+    if (s >= lim) continue;
     float q[8], k[8], v[8];
-    if (s < S) {
+    if (row[it] >= 0) {
       unpack8(rq[it], q); unpack8(rk[it], k); unpack8(rv[it], v);
 #pragma unroll
       for (int j = 0; j < 8; ++j) { q[j] += bq[j]; k[j] += bk[j]; v[j] += bv[j]; }
@@ -205,32 +241,41 @@ __device__ __forceinline__ void stage_operands(const T* __restrict__ qkv, const 
 template <typename T, int SP>
 __global__ void __launch_bounds__(SP * 2, SP == 128 ? 2 : 1) attention_fwd_mma_kernel(
     const T* __restrict__ qkv, const T* __restrict__ bqkv, const int* __restrict__ mask, T* __restrict__ ctx,
-    T* __restrict__ probs, int S, int H, int nh, float p, const int* __restrict__ seed_ptr, uint32_t stream) {
+    T* __restrict__ probs, int S, int H, int nh, float p, const int* __restrict__ seed_ptr, uint32_t stream, const Tok tk) {
   rb::grid_dep_wait();        // launched with launch_pdl: nothing above touches global memory
   rb::grid_dep_launch();      // the kernel that follows may start its set-up; it waits for this grid before reading
   extern __shared__ __align__(128) uint8_t sm_raw[];
   T* sQ = reinterpret_cast<T*>(sm_raw);
   T* sK = sQ + SP * RP;
   T* sV = sK + SP * RP;
-  uint8_t* sCode = reinterpret_cast<uint8_t*>(sV + SP * RP);   // per key: 0 = beyond S, 1 = attend, 2 = masked
+  int* sRow = reinterpret_cast<int*>(sV + SP * RP);            // row of each token, -1 = none
+  uint8_t* sCode = reinterpret_cast<uint8_t*>(sRow + SP);      // per key: 0 = no such token, 1 = attend, 2 = masked
   const int h = blockIdx.x, b = blockIdx.y;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int g = lane >> 2, t = lane & 3;
   const uint32_t seed = p > 0.f ? (uint32_t)(*seed_ptr) : 0u;
   const float inv_keep = p > 0.f ? 1.f / (1.f - p) : 1.f;
   const float scale = rsqrtf((float)HD);
-  for (int j = threadIdx.x; j < SP; j += blockDim.x) sCode[j] = j < S ? (mask[b * S + j] != 0 ? 1 : 2) : 0;
-  stage_operands<T, SP, false>(qkv, bqkv, nullptr, sQ, sK, sV, nullptr, b, h, S, H);
+  const int len = seq_len(tk, b, S), lim = (len + 15) & ~15;
+  for (int j = threadIdx.x; j < SP; j += blockDim.x) {
+    const int row = j < len ? seq_row(tk, b, S, j) : -1;
+    sRow[j] = row;
+    sCode[j] = row >= 0 ? (mask[b * S + j] != 0 ? 1 : 2) : 0;
+  }
+  stage_operands<T, SP, false>(qkv, bqkv, nullptr, sQ, sK, sV, nullptr, tk, b, h, S, H, len, lim);
+  if (tk.slot != nullptr && b == (int)gridDim.y - 1) clear_zero_rows<T>(tk, ctx, H, h * HD, HD);
   __syncthreads();
   const int r0 = warp * 16;
+  if (r0 >= lim) return;
   float acc[SP / 8][4];
 #pragma unroll
   for (int j = 0; j < SP / 8; ++j) { acc[j][0] = 0.f; acc[j][1] = 0.f; acc[j][2] = 0.f; acc[j][3] = 0.f; }
-  rows_times_transposed<T, SP>(acc, sQ, sK, r0, lane);
+  rows_times_transposed<T, SP>(acc, sQ, sK, r0, lane, lim);
   // softmax of rows r0 + g (elements 0, 1 of each tile) and r0 + g + 8 (elements 2, 3)
   float mx0 = -1e30f, mx1 = -1e30f;
 #pragma unroll
   for (int j = 0; j < SP / 8; ++j) {
+    if (8 * j >= lim) continue;
 #pragma unroll
     for (int e = 0; e < 2; ++e) {
       const bool on = sCode[8 * j + 2 * t + e] == 1;
@@ -244,6 +289,7 @@ __global__ void __launch_bounds__(SP * 2, SP == 128 ? 2 : 1) attention_fwd_mma_k
   float sum0 = 0.f, sum1 = 0.f;
 #pragma unroll
   for (int j = 0; j < SP / 8; ++j) {
+    if (8 * j >= lim) continue;
 #pragma unroll
     for (int e = 0; e < 2; ++e) {
       const bool in_range = sCode[8 * j + 2 * t + e] != 0;
@@ -255,17 +301,19 @@ __global__ void __launch_bounds__(SP * 2, SP == 128 ? 2 : 1) attention_fwd_mma_k
   }
   sum0 = quad_sum(sum0); sum1 = quad_sum(sum1);
   const int i0 = r0 + g, i1 = r0 + g + 8;
-  const float inv0 = i0 < S ? 1.f / sum0 : 0.f, inv1 = i1 < S ? 1.f / sum1 : 0.f;
+  const int row0 = sRow[i0], row1 = sRow[i1];
+  const float inv0 = row0 >= 0 ? 1.f / sum0 : 0.f, inv1 = row1 >= 0 ? 1.f / sum1 : 0.f;
   const size_t prow0 = ((size_t)(b * nh + h) * S + i0) * S, prow1 = ((size_t)(b * nh + h) * S + i1) * S;
   const bool pair_store = (S & 1) == 0;   // then every (row, even column) element is 4-byte aligned
   uint32_t pf[SP / 16][4];                // P~ as the A operand of O = P~ V
 #pragma unroll
   for (int j = 0; j < SP / 8; ++j) {
+    if (8 * j >= lim) continue;
     const int c = 8 * j + 2 * t;
     // the stored probabilities are the rounded ones, as in the unfused op
     const uint32_t u0 = Pack<T>::pack(acc[j][0] * inv0, acc[j][1] * inv0);
     const uint32_t u1 = Pack<T>::pack(acc[j][2] * inv1, acc[j][3] * inv1);
-    if (i0 < S) {
+    if (row0 >= 0) {
       if (pair_store) { if (c < S) *reinterpret_cast<uint32_t*>(probs + prow0 + c) = u0; }
       else {
         const T* e = reinterpret_cast<const T*>(&u0);
@@ -273,7 +321,7 @@ __global__ void __launch_bounds__(SP * 2, SP == 128 ? 2 : 1) attention_fwd_mma_k
         if (c + 1 < S) probs[prow0 + c + 1] = e[1];
       }
     }
-    if (i1 < S) {
+    if (row1 >= 0) {
       if (pair_store) { if (c < S) *reinterpret_cast<uint32_t*>(probs + prow1 + c) = u1; }
       else {
         const T* e = reinterpret_cast<const T*>(&u1);
@@ -295,15 +343,15 @@ __global__ void __launch_bounds__(SP * 2, SP == 128 ? 2 : 1) attention_fwd_mma_k
   float out[HD / 8][4];
 #pragma unroll
   for (int jd = 0; jd < HD / 8; ++jd) { out[jd][0] = 0.f; out[jd][1] = 0.f; out[jd][2] = 0.f; out[jd][3] = 0.f; }
-  frag_times_rows<T, SP>(out, pf, sV, lane);
-  write_rows<T>(out, ctx + (size_t)(b * S + r0) * H + h * HD, H, r0, S, lane, nullptr);
+  frag_times_rows<T, SP>(out, pf, sV, lane, lim);
+  write_rows<T>(out, ctx + h * HD, H, row0, row1, lane, nullptr);
 }
 
 template <typename T, int SP>
 __global__ void __launch_bounds__(SP * 2) attention_bwd_mma_kernel(
     const T* __restrict__ dctx, const T* __restrict__ qkv, const T* __restrict__ bqkv, const T* __restrict__ probs,
     T* __restrict__ dqkv, int S, int H, int nh, float p, const int* __restrict__ seed_ptr, uint32_t stream,
-    float* __restrict__ bias_acc) {
+    float* __restrict__ bias_acc, const Tok tk) {
   rb::grid_dep_wait();
   rb::grid_dep_launch();
   extern __shared__ __align__(128) uint8_t sm_raw[];
@@ -315,6 +363,7 @@ __global__ void __launch_bounds__(SP * 2) attention_bwd_mma_kernel(
   T* sDS = sDO + SP * RP;      // [query][key] dS
   T* sW = sDS + SP * PP;       // [query][key] dropped-out probabilities P~
   float* sBias = reinterpret_cast<float*>(sW + SP * PP);   // [3][HD] column sums of dQ, dK, dV
+  int* sRow = reinterpret_cast<int*>(sBias + 3 * HD);      // row of each token, -1 = none
   const int h = blockIdx.x, b = blockIdx.y;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int g = lane >> 2, t = lane & 3;
@@ -323,15 +372,20 @@ __global__ void __launch_bounds__(SP * 2) attention_bwd_mma_kernel(
   const float scale = rsqrtf((float)HD);
   if (bias_acc != nullptr)
     for (int i = threadIdx.x; i < 3 * HD; i += blockDim.x) sBias[i] = 0.f;
-  stage_operands<T, SP, true>(qkv, bqkv, dctx, sQ, sK, sV, sDO, b, h, S, H);
+  const int len = seq_len(tk, b, S), lim = (len + 15) & ~15;
+  for (int j = threadIdx.x; j < SP; j += blockDim.x) sRow[j] = j < len ? seq_row(tk, b, S, j) : -1;
+  stage_operands<T, SP, true>(qkv, bqkv, dctx, sQ, sK, sV, sDO, tk, b, h, S, H, len, lim);
+  if (tk.slot != nullptr && b == (int)gridDim.y - 1)
+    for (int w = 0; w < 3; ++w) clear_zero_rows<T>(tk, dqkv, 3 * H, w * H + h * HD, HD);
   __syncthreads();
   const int r0 = warp * 16;
-  {
+  const int row0 = sRow[r0 + g], row1 = sRow[r0 + g + 8];
+  if (r0 < lim) {
     // dP for this warp's 16 query rows, then dS and P~ in registers
     float acc[SP / 8][4];
 #pragma unroll
     for (int j = 0; j < SP / 8; ++j) { acc[j][0] = 0.f; acc[j][1] = 0.f; acc[j][2] = 0.f; acc[j][3] = 0.f; }
-    rows_times_transposed<T, SP>(acc, sDO, sV, r0, lane);
+    rows_times_transposed<T, SP>(acc, sDO, sV, r0, lane, lim);
     const int i0 = r0 + g, i1 = r0 + g + 8;
     const size_t prow0 = ((size_t)(b * nh + h) * S + i0) * S, prow1 = ((size_t)(b * nh + h) * S + i1) * S;
     const bool pair_load = (S & 1) == 0;
@@ -339,13 +393,14 @@ __global__ void __launch_bounds__(SP * 2) attention_bwd_mma_kernel(
     float dot0 = 0.f, dot1 = 0.f;
 #pragma unroll
     for (int j = 0; j < SP / 8; ++j) {
+      if (8 * j >= lim) continue;
       const int c = 8 * j + 2 * t;
       float2 pr0 = make_float2(0.f, 0.f), pr1 = make_float2(0.f, 0.f);
-      if (i0 < S && c < S) {
+      if (row0 >= 0 && c < S) {
         if (pair_load) pr0 = Pack<T>::unpack(*reinterpret_cast<const uint32_t*>(probs + prow0 + c));
         else { pr0.x = to_f(probs[prow0 + c]); if (c + 1 < S) pr0.y = to_f(probs[prow0 + c + 1]); }
       }
-      if (i1 < S && c < S) {
+      if (row1 >= 0 && c < S) {
         if (pair_load) pr1 = Pack<T>::unpack(*reinterpret_cast<const uint32_t*>(probs + prow1 + c));
         else { pr1.x = to_f(probs[prow1 + c]); if (c + 1 < S) pr1.y = to_f(probs[prow1 + c + 1]); }
       }
@@ -371,6 +426,7 @@ __global__ void __launch_bounds__(SP * 2) attention_bwd_mma_kernel(
     uint32_t dsf[SP / 16][4];   // dS as the A operand of dQ = dS K
 #pragma unroll
     for (int j = 0; j < SP / 8; ++j) {
+      if (8 * j >= lim) continue;
       const int c = 8 * j + 2 * t;
       const float2 pr0 = Pack<T>::unpack(wf[j][0]), pr1 = Pack<T>::unpack(wf[j][1]);
       const uint32_t d0 = Pack<T>::pack(pr0.x * (acc[j][0] - dot0) * scale, pr0.y * (acc[j][1] - dot0) * scale);
@@ -383,23 +439,23 @@ __global__ void __launch_bounds__(SP * 2) attention_bwd_mma_kernel(
     float out[HD / 8][4];
 #pragma unroll
     for (int jd = 0; jd < HD / 8; ++jd) { out[jd][0] = 0.f; out[jd][1] = 0.f; out[jd][2] = 0.f; out[jd][3] = 0.f; }
-    frag_times_rows<T, SP>(out, dsf, sK, lane);
-    write_rows<T>(out, dqkv + (size_t)(b * S + r0) * 3 * H + h * HD, 3 * H, r0, S, lane,
+    frag_times_rows<T, SP>(out, dsf, sK, lane, lim);
+    write_rows<T>(out, dqkv + h * HD, 3 * H, row0, row1, lane,
                   bias_acc != nullptr ? sBias : nullptr);
   }
   __syncthreads();
   // this warp's 16 key rows of dK = dS^T Q and dV = P~^T dO
-  {
+  if (r0 < lim) {
     float out[HD / 8][4];
 #pragma unroll
     for (int jd = 0; jd < HD / 8; ++jd) { out[jd][0] = 0.f; out[jd][1] = 0.f; out[jd][2] = 0.f; out[jd][3] = 0.f; }
-    transposed_times_rows<T, SP>(out, sDS, PP, r0, sQ, lane);
-    write_rows<T>(out, dqkv + (size_t)(b * S + r0) * 3 * H + H + h * HD, 3 * H, r0, S, lane,
+    transposed_times_rows<T, SP>(out, sDS, PP, r0, sQ, lane, lim);
+    write_rows<T>(out, dqkv + H + h * HD, 3 * H, row0, row1, lane,
                   bias_acc != nullptr ? sBias + HD : nullptr);
 #pragma unroll
     for (int jd = 0; jd < HD / 8; ++jd) { out[jd][0] = 0.f; out[jd][1] = 0.f; out[jd][2] = 0.f; out[jd][3] = 0.f; }
-    transposed_times_rows<T, SP>(out, sW, PP, r0, sDO, lane);
-    write_rows<T>(out, dqkv + (size_t)(b * S + r0) * 3 * H + 2 * H + h * HD, 3 * H, r0, S, lane,
+    transposed_times_rows<T, SP>(out, sW, PP, r0, sDO, lane, lim);
+    write_rows<T>(out, dqkv + 2 * H + h * HD, 3 * H, row0, row1, lane,
                   bias_acc != nullptr ? sBias + 2 * HD : nullptr);
   }
   if (bias_acc != nullptr) {
@@ -412,31 +468,32 @@ __global__ void __launch_bounds__(SP * 2) attention_bwd_mma_kernel(
   }
 }
 
-template <int SP> constexpr size_t fwd_smem(size_t esz) { return (size_t)3 * SP * RP * esz + SP; }
+template <int SP> constexpr size_t fwd_smem(size_t esz) { return (size_t)3 * SP * RP * esz + SP * sizeof(int) + SP; }
 template <int SP> constexpr size_t bwd_smem(size_t esz) {
-  return (size_t)4 * SP * RP * esz + (size_t)2 * SP * (SP + 8) * esz + 3 * HD * sizeof(float);
+  return (size_t)4 * SP * RP * esz + (size_t)2 * SP * (SP + 8) * esz + 3 * HD * sizeof(float) + SP * sizeof(int);
 }
 
 template <typename T, int SP>
 static int launch_fwd(const void* qkv, const void* bqkv, const int* mask, void* ctx, void* probs, int b, int S, int H,
-                      int nh, float p, const int* seed, unsigned stream_id, cudaStream_t st) {
+                      int nh, float p, const int* seed, unsigned stream_id, const Tok& tk, cudaStream_t st) {
   auto k = attention_fwd_mma_kernel<T, SP>;
   constexpr size_t smem = fwd_smem<SP>(sizeof(T));
   if (smem > 48 * 1024 &&
       cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return -5;
-  rb::launch_pdl(k, dim3(nh, b), dim3(SP * 2), smem, st, (const T*)qkv, (const T*)bqkv, mask, (T*)ctx, (T*)probs, S, H, nh, p, seed, stream_id);
+  rb::launch_pdl(k, dim3(nh, b), dim3(SP * 2), smem, st, (const T*)qkv, (const T*)bqkv, mask, (T*)ctx, (T*)probs, S, H, nh, p, seed, stream_id, tk);
   return 0;
 }
 
 template <typename T, int SP>
 static int launch_bwd(const void* dctx, const void* qkv, const void* bqkv, const void* probs, void* dqkv, int b, int S,
-                      int H, int nh, float p, const int* seed, unsigned stream_id, float* bias_acc, cudaStream_t st) {
+                      int H, int nh, float p, const int* seed, unsigned stream_id, float* bias_acc, const Tok& tk,
+                      cudaStream_t st) {
   auto k = attention_bwd_mma_kernel<T, SP>;
   constexpr size_t smem = bwd_smem<SP>(sizeof(T));
   if (smem > 48 * 1024 &&
       cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return -5;
   rb::launch_pdl(k, dim3(nh, b), dim3(SP * 2), smem, st, (const T*)dctx, (const T*)qkv, (const T*)bqkv, (const T*)probs,
-                 (T*)dqkv, S, H, nh, p, seed, stream_id, bias_acc);
+                 (T*)dqkv, S, H, nh, p, seed, stream_id, bias_acc, tk);
   return 0;
 }
 
@@ -454,15 +511,16 @@ constexpr int QB = 64;     // rows owned by a CTA
 constexpr int KBLK = 128;  // rows of the other dimension per step
 constexpr int PPK = QB + 8;
 
-// rows first.. of a [*, ld] matrix (pointer already at this (batch, head)'s first column) -> [n_tile][RP] tile
+// tokens first.. of sequence b from a [*, ld] matrix (pointer already at this head's first column) -> [n_tile][RP] tile
 template <typename T>
 __device__ __forceinline__ void stage_block(T* dst, const T* __restrict__ src, size_t ld, const T* __restrict__ bias,
-                                            int first, int n_tile, int S) {
+                                            int first, int n_tile, const Tok& tk, int b, int S, int len) {
   for (int i = threadIdx.x; i < n_tile * (HD / 8); i += blockDim.x) {
     const int s = i >> 3, d = (i & 7) * 8;
     float v[8];
-    if (first + s < S) {
-      load8(src + (size_t)(first + s) * ld + d, v);
+    const int row = first + s < len ? seq_row(tk, b, S, first + s) : -1;
+    if (row >= 0) {
+      load8(src + (size_t)row * ld + d, v);
       if (bias != nullptr) {
         float bb[8];
         load8(bias + d, bb);
@@ -502,7 +560,7 @@ __device__ __forceinline__ void store_pair(T* __restrict__ base, size_t idx, uin
 template <typename T>
 __global__ void __launch_bounds__(128) attention_fwd_long_kernel(
     const T* __restrict__ qkv, const T* __restrict__ bqkv, const int* __restrict__ mask, T* __restrict__ ctx,
-    T* __restrict__ probs, int S, int H, int nh, float p, const int* __restrict__ seed_ptr, uint32_t stream) {
+    T* __restrict__ probs, int S, int H, int nh, float p, const int* __restrict__ seed_ptr, uint32_t stream, const Tok tk) {
   extern __shared__ __align__(128) uint8_t sm_raw[];
   T* sQ = reinterpret_cast<T*>(sm_raw);
   T* sK = sQ + QB * RP;
@@ -514,27 +572,32 @@ __global__ void __launch_bounds__(128) attention_fwd_long_kernel(
   const uint32_t seed = p > 0.f ? (uint32_t)(*seed_ptr) : 0u;
   const float inv_keep = p > 0.f ? 1.f / (1.f - p) : 1.f;
   const float scale = rsqrtf((float)HD);
-  const T* base = qkv + (size_t)b * S * 3 * H + h * HD;
-  stage_block<T>(sQ, base, (size_t)3 * H, bqkv + h * HD, q0, QB, S);
+  const T* base = qkv + h * HD;
+  if (tk.slot != nullptr && b == (int)gridDim.y - 1 && q0 == 0) clear_zero_rows<T>(tk, ctx, H, h * HD, HD);
+  const int len = seq_len(tk, b, S), lim = (len + 15) & ~15;
+  if (q0 >= len) return;
+  stage_block<T>(sQ, base, (size_t)3 * H, bqkv + h * HD, q0, QB, tk, b, S, len);
   const int r0 = warp * 16;
   const int i0 = q0 + r0 + g, i1 = i0 + 8;
-  const int nkb = (S + KBLK - 1) / KBLK;
+  const int row0 = i0 < len ? seq_row(tk, b, S, i0) : -1, row1 = i1 < len ? seq_row(tk, b, S, i1) : -1;
+  const int nkb = (len + KBLK - 1) / KBLK;
   float m0 = -1e30f, m1 = -1e30f, l0 = 0.f, l1 = 0.f;
   for (int kb = 0; kb < nkb; ++kb) {
     __syncthreads();
-    stage_block<T>(sK, base + H, (size_t)3 * H, bqkv + H + h * HD, kb * KBLK, KBLK, S);
+    stage_block<T>(sK, base + H, (size_t)3 * H, bqkv + H + h * HD, kb * KBLK, KBLK, tk, b, S, len);
     for (int j = threadIdx.x; j < KBLK; j += blockDim.x) {
       const int key = kb * KBLK + j;
-      sCode[j] = key < S ? (mask[b * S + key] != 0 ? 1 : 2) : 0;
+      sCode[j] = key < len && seq_row(tk, b, S, key) >= 0 ? (mask[b * S + key] != 0 ? 1 : 2) : 0;
     }
     __syncthreads();
     float acc[KBLK / 8][4];
 #pragma unroll
     for (int j = 0; j < KBLK / 8; ++j) { acc[j][0] = 0.f; acc[j][1] = 0.f; acc[j][2] = 0.f; acc[j][3] = 0.f; }
-    rows_times_transposed<T, KBLK>(acc, sQ, sK, r0, lane);
+    rows_times_transposed<T, KBLK>(acc, sQ, sK, r0, lane, lim - kb * KBLK);
     float bm0 = -1e30f, bm1 = -1e30f;
 #pragma unroll
     for (int j = 0; j < KBLK / 8; ++j) {
+      if (kb * KBLK + 8 * j >= lim) continue;
 #pragma unroll
       for (int e = 0; e < 2; ++e) {
         const int code = sCode[8 * j + 2 * t + e];
@@ -547,6 +610,7 @@ __global__ void __launch_bounds__(128) attention_fwd_long_kernel(
     float s0 = 0.f, s1 = 0.f;
 #pragma unroll
     for (int j = 0; j < KBLK / 8; ++j) {
+      if (kb * KBLK + 8 * j >= lim) continue;
 #pragma unroll
       for (int e = 0; e < 2; ++e) {
         if (sCode[8 * j + 2 * t + e] != 0) { s0 += __expf(acc[j][e] - n0); s1 += __expf(acc[j][2 + e] - n1); }
@@ -557,7 +621,7 @@ __global__ void __launch_bounds__(128) attention_fwd_long_kernel(
     m0 = n0; m1 = n1;
   }
   l0 = quad_sum(l0); l1 = quad_sum(l1);
-  const float inv0 = i0 < S ? 1.f / l0 : 0.f, inv1 = i1 < S ? 1.f / l1 : 0.f;
+  const float inv0 = row0 >= 0 ? 1.f / l0 : 0.f, inv1 = row1 >= 0 ? 1.f / l1 : 0.f;
   const size_t prow0 = ((size_t)(b * nh + h) * S + i0) * S, prow1 = ((size_t)(b * nh + h) * S + i1) * S;
   const bool pair = (S & 1) == 0;
   float out[HD / 8][4];
@@ -565,20 +629,21 @@ __global__ void __launch_bounds__(128) attention_fwd_long_kernel(
   for (int jd = 0; jd < HD / 8; ++jd) { out[jd][0] = 0.f; out[jd][1] = 0.f; out[jd][2] = 0.f; out[jd][3] = 0.f; }
   for (int kb = 0; kb < nkb; ++kb) {
     __syncthreads();
-    stage_block<T>(sK, base + H, (size_t)3 * H, bqkv + H + h * HD, kb * KBLK, KBLK, S);
-    stage_block<T>(sV, base + 2 * H, (size_t)3 * H, bqkv + 2 * H + h * HD, kb * KBLK, KBLK, S);
+    stage_block<T>(sK, base + H, (size_t)3 * H, bqkv + H + h * HD, kb * KBLK, KBLK, tk, b, S, len);
+    stage_block<T>(sV, base + 2 * H, (size_t)3 * H, bqkv + 2 * H + h * HD, kb * KBLK, KBLK, tk, b, S, len);
     for (int j = threadIdx.x; j < KBLK; j += blockDim.x) {
       const int key = kb * KBLK + j;
-      sCode[j] = key < S ? (mask[b * S + key] != 0 ? 1 : 2) : 0;
+      sCode[j] = key < len && seq_row(tk, b, S, key) >= 0 ? (mask[b * S + key] != 0 ? 1 : 2) : 0;
     }
     __syncthreads();
     float acc[KBLK / 8][4];
 #pragma unroll
     for (int j = 0; j < KBLK / 8; ++j) { acc[j][0] = 0.f; acc[j][1] = 0.f; acc[j][2] = 0.f; acc[j][3] = 0.f; }
-    rows_times_transposed<T, KBLK>(acc, sQ, sK, r0, lane);
+    rows_times_transposed<T, KBLK>(acc, sQ, sK, r0, lane, lim - kb * KBLK);
     uint32_t pf[KBLK / 16][4];
 #pragma unroll
     for (int j = 0; j < KBLK / 8; ++j) {
+      if (kb * KBLK + 8 * j >= lim) continue;
       const int c = 8 * j + 2 * t, key = kb * KBLK + c;
       float e00, e01, e10, e11;
       {
@@ -589,8 +654,8 @@ __global__ void __launch_bounds__(128) attention_fwd_long_kernel(
         e11 = c1 != 0 ? __expf((c1 == 1 ? acc[j][3] * scale : -1e30f) - m1) * inv1 : 0.f;
       }
       const uint32_t u0 = Pack<T>::pack(e00, e01), u1 = Pack<T>::pack(e10, e11);
-      store_pair<T>(probs, prow0 + key, u0, i0 < S && key < S, key + 1 < S, pair);
-      store_pair<T>(probs, prow1 + key, u1, i1 < S && key < S, key + 1 < S, pair);
+      store_pair<T>(probs, prow0 + key, u0, row0 >= 0 && key < S, key + 1 < S, pair);
+      store_pair<T>(probs, prow1 + key, u1, row1 >= 0 && key < S, key + 1 < S, pair);
       float2 q0v = Pack<T>::unpack(u0), q1v = Pack<T>::unpack(u1);
       if (p > 0.f) {
         q0v.x = keep(seed, stream, (uint32_t)(prow0 + key), p) ? q0v.x * inv_keep : 0.f;
@@ -601,16 +666,16 @@ __global__ void __launch_bounds__(128) attention_fwd_long_kernel(
       pf[j >> 1][(j & 1) * 2 + 0] = Pack<T>::pack(q0v.x, q0v.y);
       pf[j >> 1][(j & 1) * 2 + 1] = Pack<T>::pack(q1v.x, q1v.y);
     }
-    frag_times_rows<T, KBLK>(out, pf, sV, lane);
+    frag_times_rows<T, KBLK>(out, pf, sV, lane, lim - kb * KBLK);
   }
-  write_rows<T>(out, ctx + (size_t)(b * S + q0 + r0) * H + h * HD, H, q0 + r0, S, lane, nullptr);
+  write_rows<T>(out, ctx + h * HD, H, row0, row1, lane, nullptr);
 }
 
 template <typename T>
 __global__ void __launch_bounds__(128) attention_bwd_long_dq_kernel(
     const T* __restrict__ dctx, const T* __restrict__ qkv, const T* __restrict__ bqkv, const T* __restrict__ probs,
     T* __restrict__ ds_ws, T* __restrict__ dqkv, int S, int H, int nh, float p, const int* __restrict__ seed_ptr,
-    uint32_t stream, float* __restrict__ bias_acc) {
+    uint32_t stream, float* __restrict__ bias_acc, const Tok tk) {
   extern __shared__ __align__(128) uint8_t sm_raw[];
   T* sDO = reinterpret_cast<T*>(sm_raw);
   T* sK = sDO + QB * RP;
@@ -622,13 +687,17 @@ __global__ void __launch_bounds__(128) attention_bwd_long_dq_kernel(
   const uint32_t seed = p > 0.f ? (uint32_t)(*seed_ptr) : 0u;
   const float inv_keep = p > 0.f ? 1.f / (1.f - p) : 1.f;
   const float scale = rsqrtf((float)HD);
-  const T* base = qkv + (size_t)b * S * 3 * H + h * HD;
+  const T* base = qkv + h * HD;
+  if (tk.slot != nullptr && b == (int)gridDim.y - 1 && q0 == 0) clear_zero_rows<T>(tk, dqkv, 3 * H, h * HD, HD);
+  const int len = seq_len(tk, b, S), lim = (len + 15) & ~15;
+  if (q0 >= len) return;
   if (bias_acc != nullptr)
     for (int i = threadIdx.x; i < HD; i += blockDim.x) sBias[i] = 0.f;
-  stage_block<T>(sDO, dctx + (size_t)b * S * H + h * HD, (size_t)H, nullptr, q0, QB, S);
+  stage_block<T>(sDO, dctx + h * HD, (size_t)H, nullptr, q0, QB, tk, b, S, len);
   const int r0 = warp * 16;
   const int i0 = q0 + r0 + g, i1 = i0 + 8;
-  const int nkb = (S + KBLK - 1) / KBLK;
+  const int row0 = i0 < len ? seq_row(tk, b, S, i0) : -1, row1 = i1 < len ? seq_row(tk, b, S, i1) : -1;
+  const int nkb = (len + KBLK - 1) / KBLK;
   const size_t prow0 = ((size_t)(b * nh + h) * S + i0) * S, prow1 = ((size_t)(b * nh + h) * S + i1) * S;
   const bool pair = (S & 1) == 0;
   float dot0 = 0.f, dot1 = 0.f;
@@ -638,20 +707,21 @@ __global__ void __launch_bounds__(128) attention_bwd_long_dq_kernel(
   for (int pass = 0; pass < 2; ++pass) {
     for (int kb = 0; kb < nkb; ++kb) {
       __syncthreads();
-      stage_block<T>(sV, base + 2 * H, (size_t)3 * H, bqkv + 2 * H + h * HD, kb * KBLK, KBLK, S);
-      if (pass == 1) stage_block<T>(sK, base + H, (size_t)3 * H, bqkv + H + h * HD, kb * KBLK, KBLK, S);
+      stage_block<T>(sV, base + 2 * H, (size_t)3 * H, bqkv + 2 * H + h * HD, kb * KBLK, KBLK, tk, b, S, len);
+      if (pass == 1) stage_block<T>(sK, base + H, (size_t)3 * H, bqkv + H + h * HD, kb * KBLK, KBLK, tk, b, S, len);
       __syncthreads();
       float acc[KBLK / 8][4];
 #pragma unroll
       for (int j = 0; j < KBLK / 8; ++j) { acc[j][0] = 0.f; acc[j][1] = 0.f; acc[j][2] = 0.f; acc[j][3] = 0.f; }
-      rows_times_transposed<T, KBLK>(acc, sDO, sV, r0, lane);
+      rows_times_transposed<T, KBLK>(acc, sDO, sV, r0, lane, lim - kb * KBLK);
       uint32_t dsf[KBLK / 16][4];
 #pragma unroll
       for (int j = 0; j < KBLK / 8; ++j) {
+        if (kb * KBLK + 8 * j >= lim) continue;
         const int key = kb * KBLK + 8 * j + 2 * t;
         const bool k0 = key < S, k1 = key + 1 < S;
-        const float2 pr0 = load_pair<T>(probs, prow0 + key, i0 < S && k0, k1, pair);
-        const float2 pr1 = load_pair<T>(probs, prow1 + key, i1 < S && k0, k1, pair);
+        const float2 pr0 = load_pair<T>(probs, prow0 + key, row0 >= 0 && k0, k1, pair);
+        const float2 pr1 = load_pair<T>(probs, prow1 + key, row1 >= 0 && k0, k1, pair);
         float m00 = 1.f, m01 = 1.f, m10 = 1.f, m11 = 1.f;
         if (p > 0.f) {
           m00 = keep(seed, stream, (uint32_t)(prow0 + key), p) ? inv_keep : 0.f;
@@ -666,17 +736,17 @@ __global__ void __launch_bounds__(128) attention_bwd_long_dq_kernel(
         } else {
           const uint32_t d0 = Pack<T>::pack(pr0.x * (a00 - dot0) * scale, pr0.y * (a01 - dot0) * scale);
           const uint32_t d1 = Pack<T>::pack(pr1.x * (a10 - dot1) * scale, pr1.y * (a11 - dot1) * scale);
-          store_pair<T>(ds_ws, prow0 + key, d0, i0 < S && k0, k1, pair);
-          store_pair<T>(ds_ws, prow1 + key, d1, i1 < S && k0, k1, pair);
+          store_pair<T>(ds_ws, prow0 + key, d0, row0 >= 0 && k0, k1, pair);
+          store_pair<T>(ds_ws, prow1 + key, d1, row1 >= 0 && k0, k1, pair);
           dsf[j >> 1][(j & 1) * 2 + 0] = d0;
           dsf[j >> 1][(j & 1) * 2 + 1] = d1;
         }
       }
-      if (pass == 1) frag_times_rows<T, KBLK>(out, dsf, sK, lane);
+      if (pass == 1) frag_times_rows<T, KBLK>(out, dsf, sK, lane, lim - kb * KBLK);
     }
     if (pass == 0) { dot0 = quad_sum(dot0); dot1 = quad_sum(dot1); }
   }
-  write_rows<T>(out, dqkv + (size_t)(b * S + q0 + r0) * 3 * H + h * HD, 3 * H, q0 + r0, S, lane,
+  write_rows<T>(out, dqkv + h * HD, 3 * H, row0, row1, lane,
                 bias_acc != nullptr ? sBias : nullptr);
   if (bias_acc != nullptr) {
     __syncthreads();
@@ -690,7 +760,7 @@ template <typename T>
 __global__ void __launch_bounds__(128) attention_bwd_long_dkv_kernel(
     const T* __restrict__ dctx, const T* __restrict__ qkv, const T* __restrict__ bqkv, const T* __restrict__ probs,
     const T* __restrict__ ds_ws, T* __restrict__ dqkv, int S, int H, int nh, float p, const int* __restrict__ seed_ptr,
-    uint32_t stream, float* __restrict__ bias_acc) {
+    uint32_t stream, float* __restrict__ bias_acc, const Tok tk) {
   extern __shared__ __align__(128) uint8_t sm_raw[];
   T* sDS = reinterpret_cast<T*>(sm_raw);      // [query of the block][key of this CTA]
   T* sW = sDS + KBLK * PPK;
@@ -701,11 +771,17 @@ __global__ void __launch_bounds__(128) attention_bwd_long_dkv_kernel(
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const uint32_t seed = p > 0.f ? (uint32_t)(*seed_ptr) : 0u;
   const float inv_keep = p > 0.f ? 1.f / (1.f - p) : 1.f;
-  const T* base = qkv + (size_t)b * S * 3 * H + h * HD;
+  const T* base = qkv + h * HD;
+  if (tk.slot != nullptr && b == (int)gridDim.y - 1 && key0 == 0) {
+    clear_zero_rows<T>(tk, dqkv, 3 * H, H + h * HD, HD);
+    clear_zero_rows<T>(tk, dqkv, 3 * H, 2 * H + h * HD, HD);
+  }
+  const int len = seq_len(tk, b, S), lim = (len + 15) & ~15;
+  if (key0 >= len) return;
   if (bias_acc != nullptr)
     for (int i = threadIdx.x; i < 2 * HD; i += blockDim.x) sBias[i] = 0.f;
   const bool vec = (S & 7) == 0;     // then every 8-key segment starts 16-byte aligned and lies inside the row
-  const int nqb = (S + KBLK - 1) / KBLK;
+  const int nqb = (len + KBLK - 1) / KBLK;
   float outK[HD / 8][4], outV[HD / 8][4];
 #pragma unroll
   for (int jd = 0; jd < HD / 8; ++jd) {
@@ -714,15 +790,16 @@ __global__ void __launch_bounds__(128) attention_bwd_long_dkv_kernel(
   }
   for (int qb = 0; qb < nqb; ++qb) {
     __syncthreads();
-    stage_block<T>(sQ, base, (size_t)3 * H, bqkv + h * HD, qb * KBLK, KBLK, S);
-    stage_block<T>(sDO, dctx + (size_t)b * S * H + h * HD, (size_t)H, nullptr, qb * KBLK, KBLK, S);
+    stage_block<T>(sQ, base, (size_t)3 * H, bqkv + h * HD, qb * KBLK, KBLK, tk, b, S, len);
+    stage_block<T>(sDO, dctx + h * HD, (size_t)H, nullptr, qb * KBLK, KBLK, tk, b, S, len);
     for (int i = threadIdx.x; i < KBLK * (QB / 8); i += blockDim.x) {
       const int qr = i >> 3, kc = (i & 7) * 8;
       const int q = qb * KBLK + qr, key = key0 + kc;
       float dsv[8], wv[8];
 #pragma unroll
       for (int j = 0; j < 8; ++j) { dsv[j] = 0.f; wv[j] = 0.f; }
-      if (q < S && key < S) {
+      // rows of tokens that do not exist were never written; keys >= lim were not written either
+      if (q < len && key < lim && key < S && seq_row(tk, b, S, q) >= 0) {
         const size_t idx = ((size_t)(b * nh + h) * S + q) * S + key;
         if (vec) {
           load8(ds_ws + idx, dsv);
@@ -740,13 +817,14 @@ __global__ void __launch_bounds__(128) attention_bwd_long_dkv_kernel(
       store8(sW + qr * PPK + kc, wv);
     }
     __syncthreads();
-    transposed_times_rows<T, KBLK>(outK, sDS, PPK, warp * 16, sQ, lane);
-    transposed_times_rows<T, KBLK>(outV, sW, PPK, warp * 16, sDO, lane);
+    transposed_times_rows<T, KBLK>(outK, sDS, PPK, warp * 16, sQ, lane, lim - qb * KBLK);
+    transposed_times_rows<T, KBLK>(outV, sW, PPK, warp * 16, sDO, lane, lim - qb * KBLK);
   }
-  const int k0 = key0 + warp * 16;
-  write_rows<T>(outK, dqkv + (size_t)(b * S + k0) * 3 * H + H + h * HD, 3 * H, k0, S, lane,
+  const int k0 = key0 + warp * 16 + (lane >> 2);
+  const int row0 = k0 < len ? seq_row(tk, b, S, k0) : -1, row1 = k0 + 8 < len ? seq_row(tk, b, S, k0 + 8) : -1;
+  write_rows<T>(outK, dqkv + H + h * HD, 3 * H, row0, row1, lane,
                 bias_acc != nullptr ? sBias : nullptr);
-  write_rows<T>(outV, dqkv + (size_t)(b * S + k0) * 3 * H + 2 * H + h * HD, 3 * H, k0, S, lane,
+  write_rows<T>(outV, dqkv + 2 * H + h * HD, 3 * H, row0, row1, lane,
                 bias_acc != nullptr ? sBias + HD : nullptr);
   if (bias_acc != nullptr) {
     __syncthreads();
@@ -765,19 +843,19 @@ constexpr size_t dkv_long_smem(size_t esz) {
 
 template <typename T>
 static int launch_fwd_long(const void* qkv, const void* bqkv, const int* mask, void* ctx, void* probs, int b, int S, int H,
-                           int nh, float p, const int* seed, unsigned stream_id, cudaStream_t st) {
+                           int nh, float p, const int* seed, unsigned stream_id, const Tok& tk, cudaStream_t st) {
   auto k = attention_fwd_long_kernel<T>;
   constexpr size_t smem = fwd_long_smem(sizeof(T));
   if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return -5;
   k<<<dim3(nh, b, (S + QB - 1) / QB), 128, smem, st>>>((const T*)qkv, (const T*)bqkv, mask, (T*)ctx, (T*)probs, S, H, nh, p,
-                                                        seed, stream_id);
+                                                        seed, stream_id, tk);
   return 0;
 }
 
 template <typename T>
 static int launch_bwd_long(const void* dctx, const void* qkv, const void* bqkv, const void* probs, void* ds_ws, void* dqkv,
                            int b, int S, int H, int nh, float p, const int* seed, unsigned stream_id, float* bias_acc,
-                           cudaStream_t st) {
+                           const Tok& tk, cudaStream_t st) {
   auto kq = attention_bwd_long_dq_kernel<T>;
   auto kkv = attention_bwd_long_dkv_kernel<T>;
   constexpr size_t sq = dq_long_smem(sizeof(T)), skv = dkv_long_smem(sizeof(T));
@@ -785,9 +863,9 @@ static int launch_bwd_long(const void* dctx, const void* qkv, const void* bqkv, 
   if (cudaFuncSetAttribute(kkv, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)skv) != cudaSuccess) return -5;
   const dim3 grid(nh, b, (S + QB - 1) / QB);
   kq<<<grid, 128, sq, st>>>((const T*)dctx, (const T*)qkv, (const T*)bqkv, (const T*)probs, (T*)ds_ws, (T*)dqkv, S, H, nh, p,
-                            seed, stream_id, bias_acc);
+                            seed, stream_id, bias_acc, tk);
   kkv<<<grid, 128, skv, st>>>((const T*)dctx, (const T*)qkv, (const T*)bqkv, (const T*)probs, (const T*)ds_ws, (T*)dqkv, S,
-                              H, nh, p, seed, stream_id, bias_acc);
+                              H, nh, p, seed, stream_id, bias_acc, tk);
   return 0;
 }
 
@@ -797,13 +875,15 @@ static int launch_bwd_long(const void* dctx, const void* qkv, const void* bqkv, 
 using namespace rb;
 
 // dtype: 1 = bf16, 2 = fp16.  Requires H / nh == 64, 1 <= S <= 128, H % 8 == 0; returns -4 otherwise (callers
-// then use the attention_tc.cu entry points, which also cover head dim 32).
+// then use the attention_tc.cu entry points, which also cover head dim 32).  tok_slot / tok_len / tok_meta
+// (all or none): packed tokens, see token_map.cuh.
 RB_API int rb_attention_fwd_mma(int dtype, const void* qkv, const void* bqkv, const int* mask, void* ctx, void* probs,
                                 int b, int S, int H, int nh, float p, const int* seed, unsigned stream_id,
-                                cudaStream_t st) {
+                                const int* tok_slot, const int* tok_len, const int* tok_meta, cudaStream_t st) {
   if (S > 128 || S < 1 || H % nh || H % 8 || H / nh != amma::HD || (dtype != RB_BF16 && dtype != RB_F16)) return -4;
+  const amma::Tok tk{tok_slot, tok_len, tok_meta};
   int rc;
-#define RB_FWD(T, SP) amma::launch_fwd<T, SP>(qkv, bqkv, mask, ctx, probs, b, S, H, nh, p, seed, stream_id, st)
+#define RB_FWD(T, SP) amma::launch_fwd<T, SP>(qkv, bqkv, mask, ctx, probs, b, S, H, nh, p, seed, stream_id, tk, st)
   if (dtype == RB_BF16) rc = S <= 32 ? RB_FWD(__nv_bfloat16, 32) : S <= 64 ? RB_FWD(__nv_bfloat16, 64) : RB_FWD(__nv_bfloat16, 128);
   else rc = S <= 32 ? RB_FWD(__half, 32) : S <= 64 ? RB_FWD(__half, 64) : RB_FWD(__half, 128);
 #undef RB_FWD
@@ -816,10 +896,12 @@ RB_API int rb_attention_fwd_mma(int dtype, const void* qkv, const void* bqkv, co
 // accumulated there so that no separate pass over dqkv is needed.
 RB_API int rb_attention_bwd_mma(int dtype, const void* dctx, const void* qkv, const void* bqkv, const void* probs,
                                 void* dqkv, int b, int S, int H, int nh, float p, const int* seed, unsigned stream_id,
-                                float* bias_acc, cudaStream_t st) {
+                                float* bias_acc, const int* tok_slot, const int* tok_len, const int* tok_meta,
+                                cudaStream_t st) {
   if (S > 128 || S < 1 || H % nh || H % 8 || H / nh != amma::HD || (dtype != RB_BF16 && dtype != RB_F16)) return -4;
+  const amma::Tok tk{tok_slot, tok_len, tok_meta};
   int rc;
-#define RB_BWD(T, SP) amma::launch_bwd<T, SP>(dctx, qkv, bqkv, probs, dqkv, b, S, H, nh, p, seed, stream_id, bias_acc, st)
+#define RB_BWD(T, SP) amma::launch_bwd<T, SP>(dctx, qkv, bqkv, probs, dqkv, b, S, H, nh, p, seed, stream_id, bias_acc, tk, st)
   if (dtype == RB_BF16) rc = S <= 32 ? RB_BWD(__nv_bfloat16, 32) : S <= 64 ? RB_BWD(__nv_bfloat16, 64) : RB_BWD(__nv_bfloat16, 128);
   else rc = S <= 32 ? RB_BWD(__half, 32) : S <= 64 ? RB_BWD(__half, 64) : RB_BWD(__half, 128);
 #undef RB_BWD
@@ -837,11 +919,12 @@ static bool long_args_ok(int dtype, int b, int S, int H, int nh) {
 
 RB_API int rb_attention_fwd_long(int dtype, const void* qkv, const void* bqkv, const int* mask, void* ctx, void* probs,
                                  int b, int S, int H, int nh, float p, const int* seed, unsigned stream_id,
-                                 cudaStream_t st) {
+                                 const int* tok_slot, const int* tok_len, const int* tok_meta, cudaStream_t st) {
   if (!long_args_ok(dtype, b, S, H, nh)) return -4;
+  const amma::Tok tk{tok_slot, tok_len, tok_meta};
   const int rc = dtype == RB_BF16
-                     ? amma::launch_fwd_long<__nv_bfloat16>(qkv, bqkv, mask, ctx, probs, b, S, H, nh, p, seed, stream_id, st)
-                     : amma::launch_fwd_long<__half>(qkv, bqkv, mask, ctx, probs, b, S, H, nh, p, seed, stream_id, st);
+                     ? amma::launch_fwd_long<__nv_bfloat16>(qkv, bqkv, mask, ctx, probs, b, S, H, nh, p, seed, stream_id, tk, st)
+                     : amma::launch_fwd_long<__half>(qkv, bqkv, mask, ctx, probs, b, S, H, nh, p, seed, stream_id, tk, st);
   if (rc) return rc;
   RB_LAUNCH_CHECK();
   return 0;
@@ -849,13 +932,15 @@ RB_API int rb_attention_fwd_long(int dtype, const void* qkv, const void* bqkv, c
 
 RB_API int rb_attention_bwd_long(int dtype, const void* dctx, const void* qkv, const void* bqkv, const void* probs,
                                  void* ds_ws, void* dqkv, int b, int S, int H, int nh, float p, const int* seed,
-                                 unsigned stream_id, float* bias_acc, cudaStream_t st) {
+                                 unsigned stream_id, float* bias_acc, const int* tok_slot, const int* tok_len, const int* tok_meta,
+                                cudaStream_t st) {
   if (!long_args_ok(dtype, b, S, H, nh) || ds_ws == nullptr) return -4;
+  const amma::Tok tk{tok_slot, tok_len, tok_meta};
   const int rc = dtype == RB_BF16
                      ? amma::launch_bwd_long<__nv_bfloat16>(dctx, qkv, bqkv, probs, ds_ws, dqkv, b, S, H, nh, p, seed,
-                                                            stream_id, bias_acc, st)
+                                                            stream_id, bias_acc, tk, st)
                      : amma::launch_bwd_long<__half>(dctx, qkv, bqkv, probs, ds_ws, dqkv, b, S, H, nh, p, seed, stream_id,
-                                                     bias_acc, st);
+                                                     bias_acc, tk, st);
   if (rc) return rc;
   RB_LAUNCH_CHECK();
   return 0;

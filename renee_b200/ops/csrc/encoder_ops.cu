@@ -12,6 +12,7 @@
 // and converted by the last block to finish, which also re-zeroes the accumulator for the next call.
 #include <cstdio>
 #include "common.cuh"
+#include "token_map.cuh"
 
 namespace rb {
 
@@ -164,15 +165,100 @@ __global__ void __launch_bounds__(128) bias_dropout_add_ln_fwd_kernel(
   if (lane == 0) { mean[row] = mu; rstd[row] = rs; }
 }
 
+// Per-sequence counts of the token map and their prefix sum.  A group of G = min(32, S rounded up to a power of two)
+// lanes reads one mask row, 32 / G rows per warp; the last CTA to finish scans the B counts (one contiguous run per
+// thread).  Latency-bound: a few dependent loads and two block scans, whatever the batch.
+__global__ void __launch_bounds__(1024) token_map_kernel(const int* __restrict__ mask, int B, int S, int G,
+                                                         int* __restrict__ off, int* __restrict__ len,
+                                                         int* __restrict__ cnt, int* __restrict__ meta) {
+  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+  const int per_warp = 32 / G, lig = lane % G, grp = lane / G;
+  const unsigned gmask = (G == 32 ? 0xffffffffu : (1u << G) - 1u);
+  for (int b0 = (blockIdx.x * 32 + wib) * per_warp; b0 < B; b0 += gridDim.x * 32 * per_warp) {
+    const int b = b0 + grp;
+    int n = 0, last = -1, first = 0;
+    for (int s0 = 0; s0 < S; s0 += G) {                       // the same trip count in every lane
+      const int s = s0 + lig;
+      const bool on = b < B && s < S && mask[(size_t)b * S + s] != 0;
+      const unsigned bits = (__ballot_sync(0xffffffffu, on) >> (grp * G)) & gmask;
+      n += __popc(bits);
+      if (bits) last = s0 + 31 - __clz(bits);
+      if (s0 == 0) first = bits & 1u;
+    }
+    if (lig == 0 && b < B) {
+      off[b] = n == 0 ? S : n + (first ? 0 : 1);
+      len[b] = n == 0 ? S : max(last + 1, 1);
+      cnt[b] = n;
+    }
+  }
+  __shared__ int s_last;
+  __shared__ int s_part[32];
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) s_last = atomicAdd(meta + TOK_COUNTER, 1) == (int)gridDim.x - 1;
+  __syncthreads();
+  if (!s_last) return;
+  __threadfence();
+  const int per = (B + 1023) / 1024, lo = min(B, (int)threadIdx.x * per), hi = min(B, lo + per);
+  int sum = 0;
+  for (int b = lo; b < hi; ++b) sum += __ldcg(off + b);
+  int inc = sum;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) { const int v = __shfl_up_sync(0xffffffffu, inc, o); if (lane >= o) inc += v; }
+  if (lane == 31) s_part[wib] = inc;
+  __syncthreads();
+  if (wib == 0) {
+    int v = s_part[lane];
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) { const int u = __shfl_up_sync(0xffffffffu, v, o); if (lane >= o) v += u; }
+    s_part[lane] = v;
+  }
+  __syncthreads();
+  int run = inc - sum + (wib > 0 ? s_part[wib - 1] : 0);
+  for (int b = lo; b < hi; ++b) { const int c = __ldcg(off + b); off[b] = run; run += c; }
+  if (threadIdx.x == 0) {
+    const int total = s_part[31];
+    meta[TOK_VALID] = total;
+    meta[TOK_ROWS] = min(B * S, (total + TOK_ALIGN - 1) / TOK_ALIGN * TOK_ALIGN);
+    meta[TOK_COUNTER] = 0;
+  }
+}
+
+// With a token map (meta != nullptr): the warp of padded token `row` works out its packed row from the sequence's offset
+// and mask row, records the pair in tok / slot, and writes there; warps of dropped tokens only record -1, and up to
+// TOK_ALIGN - 1 warps past the last token fill the zero rows.
 template <typename T, int NV>
 __global__ void __launch_bounds__(128) embed_ln_fwd_kernel(
     const int* __restrict__ ids, const T* __restrict__ word, const T* __restrict__ pos,
     const T* __restrict__ gamma, const T* __restrict__ beta, T* __restrict__ y,
     float* __restrict__ mean, float* __restrict__ rstd, int rows, int H, int S, float eps, float p,
-    const int* __restrict__ seed_ptr, uint32_t stream) {
+    const int* __restrict__ seed_ptr, uint32_t stream, const int* __restrict__ mask, const int* __restrict__ meta,
+    const int* __restrict__ off, const int* __restrict__ cnt, int* __restrict__ tok, int* __restrict__ slot) {
   grid_dep_launch();
   const int lane = threadIdx.x & 31;
   const int row = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  int out = row;                                              // row of y, mean and rstd
+  if (meta != nullptr) {
+    if (row >= rows) {
+      out = meta[TOK_VALID] + (row - rows);
+      if (out >= meta[TOK_ROWS]) return;
+      const float zero[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+      for (int col = lane * 8; col < H; col += 256) store8(y + (size_t)out * H + col, zero);
+      if (lane == 0) { mean[out] = 0.f; rstd[out] = 0.f; tok[out] = -1; }
+      return;
+    }
+    const int b = row / S, s = row - b * S;
+    const bool all = cnt[b] == 0;
+    int before = 0;
+    for (int s0 = 0; s0 <= s; s0 += 32) {                     // kept tokens of the row up to and including s
+      const int q = s0 + lane;
+      before += __popc(__ballot_sync(0xffffffffu, q <= s && (q == 0 || all || mask[(size_t)b * S + q] != 0)));
+    }
+    const bool kept = s == 0 || all || mask[row] != 0;
+    out = kept ? off[b] + before - 1 : -1;
+    if (lane == 0) { slot[row] = out; if (kept) tok[out] = row; }
+    if (!kept) return;
+  }
   if (row >= rows) return;
   const uint32_t seed = p > 0.f ? (uint32_t)(*seed_ptr) : 0u;
   const float inv_keep = p > 0.f ? 1.f / (1.f - p) : 1.f;
@@ -218,10 +304,10 @@ __global__ void __launch_bounds__(128) embed_ln_fwd_kernel(
         if (p > 0.f) t = keep(seed, stream, (uint32_t)(row * H + col + j), p) ? t * inv_keep : 0.f;
         o[j] = t;
       }
-      store8(y + (size_t)row * H + col, o);
+      store8(y + (size_t)out * H + col, o);
     }
   }
-  if (lane == 0) { mean[row] = mu; rstd[row] = rs; }
+  if (lane == 0) { mean[out] = mu; rstd[out] = rs; }
 }
 
 // ------------------------------------------------------------------------------------ LN backward
@@ -247,9 +333,12 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 4 ? 6 : (WARPS == 8 ? 2 :
     T* __restrict__ d_pre, T* __restrict__ d_branch, T* __restrict__ dword, T* __restrict__ dpos,
     float* __restrict__ acc, unsigned* __restrict__ counter, T* __restrict__ dgamma, T* __restrict__ dbeta,
     T* __restrict__ dbias, int rows, int H, int S, int pad_id, float p, const int* __restrict__ seed_ptr,
-    uint32_t stream) {
+    uint32_t stream, const int* __restrict__ tok_meta, const int* __restrict__ tok) {
+  // packed tokens (token_map.cuh): EMBED walks the padded layout and tok is its slot array (dropped tokens are skipped);
+  // otherwise the rows are the packed ones and tok numbers their dropout counters
   grid_dep_wait();            // launched with launch_pdl: nothing above touches global memory
   grid_dep_launch();
+  if (!EMBED && tok_meta != nullptr) rows = __ldcg(tok_meta + TOK_ROWS);
   extern __shared__ __align__(16) float sm[];  // [warps][3][H]
   const int lane = threadIdx.x & 31;
   const int wib = threadIdx.x >> 5;
@@ -270,13 +359,16 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 4 ? 6 : (WARPS == 8 ? 2 :
     const int col = (lane + 32 * i) * 8;
     if (col < H) gam[i] = load_raw8<T>(gamma + col);
   }
-  for (int row = warp; row < rows; row += total_warps) {
+  for (int row0 = warp; row0 < rows; row0 += total_warps) {
+    const int row = EMBED && tok != nullptr ? __ldcg(tok + row0) : row0;       // row of the stored activations
+    if (EMBED && row < 0) continue;
+    const int crow = !EMBED && tok != nullptr && p > 0.f ? __ldcg(tok + row0) : row0;   // row of the dropout counters
     const float mu = mean[row], rs = rstd[row];
     // dy and the LN input stay packed across the two warp reductions
     Raw8<T> rd[NV], rx[NV], rb[NV];
     float s1 = 0.f, s2 = 0.f;
     int id = 0;
-    if (EMBED) id = ids[row];
+    if (EMBED) id = ids[row0];
 #pragma unroll
     for (int i = 0; i < NV; ++i) {
       const int col = (lane + 32 * i) * 8;
@@ -284,7 +376,7 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 4 ? 6 : (WARPS == 8 ? 2 :
         rd[i] = load_raw8<T>(dy + (size_t)row * H + col);
         if (EMBED) {
           rx[i] = load_raw8<T>(word + (size_t)id * H + col);
-          rb[i] = load_raw8<T>(pos + (size_t)(row % S) * H + col);
+          rb[i] = load_raw8<T>(pos + (size_t)(row0 % S) * H + col);
         } else {
           rx[i] = load_raw8<T>(pre + (size_t)row * H + col);
         }
@@ -304,7 +396,7 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 4 ? 6 : (WARPS == 8 ? 2 :
 #pragma unroll
           for (int j = 0; j < 8; ++j) {
             x[j] += b[j];
-            if (p > 0.f) d[j] = keep(seed, stream, (uint32_t)(row * H + col + j), p) ? d[j] * inv_keep : 0.f;
+            if (p > 0.f) d[j] = keep(seed, stream, (uint32_t)(crow * H + col + j), p) ? d[j] * inv_keep : 0.f;
           }
         }
 #pragma unroll
@@ -335,7 +427,7 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 4 ? 6 : (WARPS == 8 ? 2 :
 #pragma unroll
           for (int j = 0; j < 8; ++j) {
             x[j] += b[j];
-            if (p > 0.f) d[j] = keep(seed, stream, (uint32_t)(row * H + col + j), p) ? d[j] * inv_keep : 0.f;
+            if (p > 0.f) d[j] = keep(seed, stream, (uint32_t)(crow * H + col + j), p) ? d[j] * inv_keep : 0.f;
           }
         }
 #pragma unroll
@@ -352,7 +444,7 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 4 ? 6 : (WARPS == 8 ? 2 :
           if (p > 0.f) {
 #pragma unroll
             for (int j = 0; j < 8; ++j)
-              db[j] = round_through<T>(keep(seed, stream, (uint32_t)(row * H + col + j), p) ? dx[j] * inv_keep : 0.f);
+              db[j] = round_through<T>(keep(seed, stream, (uint32_t)(crow * H + col + j), p) ? dx[j] * inv_keep : 0.f);
             store8(d_branch + (size_t)row * H + col, db);
           } else {
 #pragma unroll
@@ -484,23 +576,23 @@ __global__ void __launch_bounds__(128) colsum_kernel(const T* __restrict__ x, fl
 }
 
 // ------------------------------------------------------------------------------------ pooling
-// grid = b, block covers H/8 vectors
+// grid = b, block covers H/8 vectors.  Packed tokens: slot gives the row of a token (CLS and attended ones are kept).
 template <typename T>
 __global__ void pool_fwd_kernel(const T* __restrict__ h, const int* __restrict__ mask, float* __restrict__ out,
-                                int S, int H, int cls) {
+                                int S, int H, int cls, const int* __restrict__ slot) {
   const int b = blockIdx.x;
   for (int col = threadIdx.x * 8; col < H; col += blockDim.x * 8) {
     float acc[8];
 #pragma unroll
     for (int j = 0; j < 8; ++j) acc[j] = 0.f;
     if (cls) {
-      load8(h + (size_t)b * S * H + col, acc);
+      load8(h + (size_t)(slot != nullptr ? slot[b * S] : b * S) * H + col, acc);
     } else {
       float cnt = 0.f;
       for (int s = 0; s < S; ++s) {
         if (mask[b * S + s] != 0) {
           float a[8];
-          load8(h + ((size_t)b * S + s) * H + col, a);
+          load8(h + (size_t)(slot != nullptr ? slot[b * S + s] : b * S + s) * H + col, a);
 #pragma unroll
           for (int j = 0; j < 8; ++j) acc[j] += a[j];
           cnt += 1.f;
@@ -514,25 +606,32 @@ __global__ void pool_fwd_kernel(const T* __restrict__ h, const int* __restrict__
   }
 }
 
-// grid = b*S rows
+// grid = b*S rows.  Packed tokens: rows past the packed ones do nothing, the zero rows (tok < 0) get zeros.
 template <typename T>
 __global__ void pool_bwd_kernel(const float* __restrict__ de, const int* __restrict__ mask, T* __restrict__ dh,
-                                int S, int H, int cls) {
+                                int S, int H, int cls, const int* __restrict__ tok_meta, const int* __restrict__ tok,
+                                const int* __restrict__ tok_cnt) {
   const int row = blockIdx.x;
-  const int b = row / S, s = row % S;
+  if (tok_meta != nullptr && row >= tok_meta[TOK_ROWS]) return;
+  const int src = tok_meta != nullptr ? tok[row] : row;
+  const int b = src < 0 ? 0 : src / S, s = src - b * S;
   float w;
-  if (cls) {
+  if (src < 0) {
+    w = 0.f;
+  } else if (cls) {
     w = (s == 0) ? 1.f : 0.f;
   } else {
     float cnt = 0.f;
-    for (int t = 0; t < S; ++t) cnt += mask[b * S + t] != 0 ? 1.f : 0.f;
-    w = mask[b * S + s] != 0 ? 1.f / fmaxf(cnt, 1e-9f) : 0.f;
+    if (tok_cnt != nullptr) cnt = (float)tok_cnt[b];
+    else
+      for (int t = 0; t < S; ++t) cnt += mask[b * S + t] != 0 ? 1.f : 0.f;
+    w = mask[src] != 0 ? 1.f / fmaxf(cnt, 1e-9f) : 0.f;
   }
   for (int col = threadIdx.x * 8; col < H; col += blockDim.x * 8) {
     float a[8];
     load8(de + (size_t)b * H + col, a);
 #pragma unroll
-    for (int j = 0; j < 8; ++j) a[j] *= w;
+    for (int j = 0; j < 8; ++j) a[j] = w == 0.f ? 0.f : a[j] * w;
     store8(dh + (size_t)row * H + col, a);
   }
 }
@@ -587,12 +686,26 @@ RB_API int rb_bias_dropout_add_ln_fwd(int dtype, const void* x, const void* bias
 
 RB_API int rb_embed_ln_fwd(int dtype, const int* ids, const void* word, const void* pos, const void* gamma,
                            const void* beta, void* y, float* mean, float* rstd, int rows, int H, int S, float eps,
-                           float p, const int* seed, unsigned stream_id, cudaStream_t st) {
+                           float p, const int* seed, unsigned stream_id, const int* mask, const int* tok_meta,
+                           const int* tok_off, const int* tok_cnt, int* tok, int* tok_slot, cudaStream_t st) {
   if (H % 8) return -3;
-  const int blocks = (rows + 3) / 4;
+  const int blocks = (rows + (tok_meta != nullptr ? TOK_ALIGN : 0) + 3) / 4;
   DISPATCH_T(dtype, DISPATCH_NV(H, (embed_ln_fwd_kernel<T, NV><<<blocks, 128, 0, st>>>(
       ids, (const T*)word, (const T*)pos, (const T*)gamma, (const T*)beta, (T*)y, mean, rstd, rows, H, S, eps, p,
-      seed, stream_id))));
+      seed, stream_id, mask, tok_meta, tok_off, tok_cnt, tok, tok_slot))));
+  RB_LAUNCH_CHECK();
+  return 0;
+}
+
+// Counts, lengths and packed offsets of the B sequences of a [B, S] mask (token_map.cuh); tok and slot are filled by
+// rb_embed_ln_fwd.  meta's counter word must be 0 on entry and is left 0.
+RB_API int rb_token_map(const int* mask, int B, int S, int* off, int* len, int* cnt, int* meta, cudaStream_t st) {
+  if (B < 1 || S < 1 || (long long)B * S > (1LL << 30)) return -3;
+  int G = 1;
+  while (G < 32 && G < S) G <<= 1;
+  int blocks = (B + 32 * (32 / G) - 1) / (32 * (32 / G));
+  if (blocks > sm_count()) blocks = sm_count();
+  token_map_kernel<<<blocks, 1024, 0, st>>>(mask, B, S, G, off, len, cnt, meta);
   RB_LAUNCH_CHECK();
   return 0;
 }
@@ -617,14 +730,14 @@ template <int WARPS>
 static int launch_ln_bwd(int dtype, const void* dy, const void* pre, const void* gamma, const float* mean,
                          const float* rstd, void* d_pre, void* d_branch, float* acc, unsigned* counter, void* dgamma,
                          void* dbeta, void* dbias, int rows, int H, float p, const int* seed, unsigned stream_id,
-                         cudaStream_t st) {
+                         const int* tok_meta, const int* tok, cudaStream_t st) {
   const int blocks = ln_bwd_blocks(rows, 1, false, WARPS);
   const size_t smem = (size_t)WARPS * 3 * (size_t)H * sizeof(float);
   DISPATCH_T(dtype, DISPATCH_NV(H, (cudaFuncSetAttribute(ln_bwd_kernel<T, NV, false, WARPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
                                     launch_pdl(ln_bwd_kernel<T, NV, false, WARPS>, dim3(blocks), dim3(WARPS * 32), smem, st,
       (const T*)dy, (const T*)pre, (const int*)nullptr, (const T*)nullptr, (const T*)nullptr, (const T*)gamma, mean, rstd,
       (T*)d_pre, (T*)d_branch, (T*)nullptr, (T*)nullptr, acc, counter, (T*)dgamma, (T*)dbeta, (T*)dbias, rows, H, 1, 0, p,
-      seed, stream_id))));
+      seed, stream_id, tok_meta, tok))));
   RB_LAUNCH_CHECK();
   return 0;
 }
@@ -632,19 +745,19 @@ static int launch_ln_bwd(int dtype, const void* dy, const void* pre, const void*
 RB_API int rb_bias_dropout_add_ln_bwd(int dtype, const void* dy, const void* pre, const void* gamma, const float* mean,
                                       const float* rstd, void* d_pre, void* d_branch, float* acc, unsigned* counter,
                                       void* dgamma, void* dbeta, void* dbias, int rows, int H, float p, const int* seed,
-                                      unsigned stream_id, cudaStream_t st) {
+                                      unsigned stream_id, const int* tok_meta, const int* tok, cudaStream_t st) {
   if (H % 8) return -3;
   int w = g_ln_bwd_warps;
   while (w > 4 && (size_t)w * 3 * H * sizeof(float) > 200 * 1024) w >>= 1;     // the per-warp column sums must fit
-  if (w == 16) return launch_ln_bwd<16>(dtype, dy, pre, gamma, mean, rstd, d_pre, d_branch, acc, counter, dgamma, dbeta, dbias, rows, H, p, seed, stream_id, st);
-  if (w == 8) return launch_ln_bwd<8>(dtype, dy, pre, gamma, mean, rstd, d_pre, d_branch, acc, counter, dgamma, dbeta, dbias, rows, H, p, seed, stream_id, st);
-  return launch_ln_bwd<4>(dtype, dy, pre, gamma, mean, rstd, d_pre, d_branch, acc, counter, dgamma, dbeta, dbias, rows, H, p, seed, stream_id, st);
+  if (w == 16) return launch_ln_bwd<16>(dtype, dy, pre, gamma, mean, rstd, d_pre, d_branch, acc, counter, dgamma, dbeta, dbias, rows, H, p, seed, stream_id, tok_meta, tok, st);
+  if (w == 8) return launch_ln_bwd<8>(dtype, dy, pre, gamma, mean, rstd, d_pre, d_branch, acc, counter, dgamma, dbeta, dbias, rows, H, p, seed, stream_id, tok_meta, tok, st);
+  return launch_ln_bwd<4>(dtype, dy, pre, gamma, mean, rstd, d_pre, d_branch, acc, counter, dgamma, dbeta, dbias, rows, H, p, seed, stream_id, tok_meta, tok, st);
 }
 
 RB_API int rb_embed_ln_bwd(int dtype, const void* dy, const int* ids, const void* word, const void* pos,
                            const void* gamma, const float* mean, const float* rstd, void* dword, void* dpos,
                            float* acc, unsigned* counter, void* dgamma, void* dbeta, int rows, int H, int S, int pad_id,
-                           float p, const int* seed, unsigned stream_id, cudaStream_t st) {
+                           float p, const int* seed, unsigned stream_id, const int* tok_slot, cudaStream_t st) {
   if (H % 8) return -3;
   const int blocks = ln_bwd_blocks(rows, S, true);
   const size_t smem = 4 * 3 * (size_t)H * sizeof(float);
@@ -652,7 +765,7 @@ RB_API int rb_embed_ln_bwd(int dtype, const void* dy, const int* ids, const void
                                     launch_pdl(ln_bwd_kernel<T, NV, true>, dim3(blocks), dim3(128), smem, st,
       (const T*)dy, (const T*)nullptr, ids, (const T*)word, (const T*)pos, (const T*)gamma, mean, rstd, (T*)nullptr,
       (T*)nullptr, (T*)dword, (T*)dpos, acc, counter, (T*)dgamma, (T*)dbeta, (T*)nullptr, rows, H, S, pad_id, p, seed,
-      stream_id))));
+      stream_id, (const int*)nullptr, tok_slot))));
   RB_LAUNCH_CHECK();
   return 0;
 }
@@ -697,17 +810,17 @@ RB_API int rb_colsum(int dtype, const void* x, float* acc, unsigned* counter, vo
 }
 
 RB_API int rb_pool_fwd(int dtype, const void* h, const int* mask, float* out, int b, int S, int H, int cls,
-                       cudaStream_t st) {
+                       const int* tok_slot, cudaStream_t st) {
   if (H % 8) return -3;
-  DISPATCH_T(dtype, (pool_fwd_kernel<T><<<b, 128, 0, st>>>((const T*)h, mask, out, S, H, cls)));
+  DISPATCH_T(dtype, (pool_fwd_kernel<T><<<b, 128, 0, st>>>((const T*)h, mask, out, S, H, cls, tok_slot)));
   RB_LAUNCH_CHECK();
   return 0;
 }
 
 RB_API int rb_pool_bwd(int dtype, const float* de, const int* mask, void* dh, int b, int S, int H, int cls,
-                       cudaStream_t st) {
+                       const int* tok_meta, const int* tok, const int* tok_cnt, cudaStream_t st) {
   if (H % 8) return -3;
-  DISPATCH_T(dtype, (pool_bwd_kernel<T><<<b * S, 128, 0, st>>>(de, mask, (T*)dh, S, H, cls)));
+  DISPATCH_T(dtype, (pool_bwd_kernel<T><<<b * S, 128, 0, st>>>(de, mask, (T*)dh, S, H, cls, tok_meta, tok, tok_cnt)));
   RB_LAUNCH_CHECK();
   return 0;
 }

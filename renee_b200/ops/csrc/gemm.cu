@@ -46,6 +46,7 @@
 // Every wait is bounded (tc.cuh): a protocol error ends with a status word, never with a hang.
 #include <type_traits>
 #include "peer.cuh"
+#include "token_map.cuh"
 
 namespace rb {
 namespace eg {
@@ -105,6 +106,9 @@ struct Params {
   // DW_SGD (classifier weights): momentum, weight decay, rounding mode; the row stride numbers the elements for the
   // rounding hash; the learning rate and the seed come from hp
   float mo, wd; int stochastic_round; int ldW;
+  // Packed tokens (token_map.cuh): M (layouts NT, NN) or K (TN) counts token rows, and the number that exists is only
+  // known on the device; tok numbers the dropout counters of packed rows
+  const int* tok_meta; const int* tok;
   int* status;
 };
 
@@ -171,7 +175,6 @@ enc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
   const uint32_t rank = NCTA == 2 ? tc::cluster_ctarank() : 0u;
   const int unit = NCTA == 2 ? (int)(blockIdx.x >> 1) : (int)blockIdx.x;          // which persistent worker
   const int n_units = NCTA == 2 ? (int)(gridDim.x >> 1) : (int)gridDim.x;
-  const int n_items = p.n_m_tiles * p.n_n_tiles * p.splits;
   const int b_rows = p.BN / NCTA;                                                 // B rows (N index) this CTA loads
   const int STAGE = A_BYTES + b_rows * BK * 2;                                    // 24, 32 or 48 KB
   const int STAGES = min(MAX_STAGES, RING / STAGE);
@@ -202,6 +205,20 @@ enc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
   // everything above touched no global memory: it may have run under the tail of the previous kernel
   grid_dep_wait();
   grid_dep_launch();
+  // extents of this launch: the host's, or with packed tokens the device's row count (every thread reads the same word)
+  int M = p.M, n_m_tiles = p.n_m_tiles, kb_total = p.kb_total, kb_per_split = p.kb_per_split, splits = p.splits;
+  if (p.tok_meta != nullptr) {
+    const int rows = __ldcg(p.tok_meta + TOK_ROWS);
+    if (LAYOUT == L_TN) {
+      kb_total = (rows + BK - 1) / BK;
+      kb_per_split = (kb_total + splits - 1) / splits;
+      splits = (kb_total + kb_per_split - 1) / kb_per_split;       // no split is empty
+    } else {
+      M = rows;
+      n_m_tiles = (rows + BM * NCTA - 1) / (BM * NCTA);
+    }
+  }
+  const int n_items = n_m_tiles * p.n_n_tiles * splits;
 
   if (warp == 0 && lane == 0) {
     // ---------------- TMA producer: one continuous stream of (item, k block) stages
@@ -216,10 +233,10 @@ enc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
       asm volatile("fence.proxy.async;" ::: "memory");
     }
     for (int item = unit; item < n_items && !aborted; item += n_units) {
-      const int tile = item / p.splits, split = item - tile * p.splits;
+      const int tile = item / splits, split = item - tile * splits;
       const int m0 = (tile / p.n_n_tiles) * (BM * NCTA) + (int)rank * BM;
       const int n0 = (tile % p.n_n_tiles) * p.BN + (int)rank * b_rows;
-      const int kb0 = split * p.kb_per_split, kb1 = min(p.kb_total, kb0 + p.kb_per_split);
+      const int kb0 = split * kb_per_split, kb1 = min(kb_total, kb0 + kb_per_split);
       for (int kb = kb0; kb < kb1; ++kb, s = (s + 1 == STAGES ? 0 : s + 1), ph ^= (s == 0 ? 1u : 0u)) {
         if (!tc::mbar_wait(empty_bar + s, ph ^ 1, aborted, p.status, tc::SITE_EMPTY, kb)) break;
         uint8_t* sA = smem + s * STAGE;
@@ -261,8 +278,8 @@ enc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
     int s = 0, t_local = 0;
     uint32_t ph = 0;
     for (int item = unit; item < n_items && !aborted; item += n_units, ++t_local) {
-      const int tile = item / p.splits, split = item - tile * p.splits;
-      const int kb0 = split * p.kb_per_split, kb1 = min(p.kb_total, kb0 + p.kb_per_split);
+      const int tile = item / splits, split = item - tile * splits;
+      const int kb0 = split * kb_per_split, kb1 = min(kb_total, kb0 + kb_per_split);
       const int buf = t_local & 1;
       const uint32_t use = (uint32_t)(t_local >> 1);
       if (!tc::mbar_wait(tmem_empty_bar + buf, (use & 1) ^ 1, aborted, p.status, tc::SITE_TMEM_EMPTY, item)) break;
@@ -313,13 +330,13 @@ enc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
     float loss = 0.f;                                     // SIGMOID_POS: this thread's share of sum softplus(z)
     const int slot = ((int)blockIdx.x * EGROUPS + g) * 8;
     for (int item = unit; item < n_items; item += n_units, ++t_local) {
-      const int tile = item / p.splits;
+      const int tile = item / splits;
       if (EPI == E_TOPK) {
         const int mt = tile / p.n_n_tiles;
         if (mt != cur_m) {
           if (cur_m >= 0) {
             const int frow = cur_m * (BM * NCTA) + (int)rank * BM + r;
-            if (frow < p.M && u_active) {
+            if (frow < M && u_active) {
 #pragma unroll
               for (int k = 0; k < 8; ++k) {
                 p.cand_val[(size_t)frow * p.cand_ld + slot + k] = tv[k];
@@ -345,6 +362,9 @@ enc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
         tc::tma_load_2d(pan, &tmR, my_in_bar, n0 + g_col, m0);
         if (EPI == E_DW_SGD) tc::tma_load_2d(pan2, &tmF, my_in_bar, n0 + g_col, m0);
       }
+      // dropout counters number the padded layout's rows; the word is fetched while the main loop still runs
+      int drop_row = row;
+      if (EPI == E_BIAS_DROPOUT_RESID && p.tok != nullptr && row < M) drop_row = __ldcg(p.tok + row);
       if (!tc::mbar_wait(tmem_full_bar + buf, use & 1, aborted, p.status, tc::SITE_TMEM_FULL, item)) *s_abort = 1;
       asm volatile("bar.sync 1, %0;" ::"n"(EPI_THREADS) : "memory");
       if (*s_abort) break;                                   // the same answer in every epilogue warp
@@ -376,7 +396,7 @@ enc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
 #pragma unroll
                 for (int j = 0; j < 8; ++j) o[j] = a[j];
               } else if (EPI == E_SIGMOID_POS) {
-                if (p.loss_acc != nullptr && row < p.M) {
+                if (p.loss_acc != nullptr && row < M) {
                   // sampled loss (dl_base.py:579-583): softplus of every logit here; minus the logits at the positives
                   // by a separate small kernel
 #pragma unroll
@@ -408,7 +428,7 @@ enc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
 #pragma unroll
                 for (int j = 0; j < 8; ++j) {
                   float t = a[j] + b[j];
-                  if (p.p > 0.f) t = keep(seed, p.stream, (uint32_t)(row * p.N + c + j), p.p) ? t * inv_keep : 0.f;
+                  if (p.p > 0.f) t = keep(seed, p.stream, (uint32_t)(drop_row * p.N + c + j), p.p) ? t * inv_keep : 0.f;
                   o[j] = res[j] + t;
                 }
               } else if (EPI == E_ADD) {
@@ -432,13 +452,13 @@ enc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
                   o[j] = p.stochastic_round ? sr_round<T>(nw, mix32(sr_seed, 0x5152u, e + j)) : nw;
                 }
                 *slot2 = pack8<T>(mm);
-              } else {   // E_GELU_BWD: rows past M read F = 0 and a zero accumulator, so they add nothing to the sums
+              } else {   // E_GELU_BWD
                 float f[8];
                 unpack8<T>(*slot, f);
 #pragma unroll
                 for (int j = 0; j < 8; ++j) {
                   o[j] = round_through<T>(a[j] * gelu_grad_f(f[j]));
-                  a[j] = o[j];
+                  a[j] = row < M ? o[j] : 0.f;               // rows past the packed tokens hold what an earlier pass left
                 }
               }
               *slot = pack8<T>(o);
@@ -456,7 +476,7 @@ enc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
             asm volatile("bar.sync %0, 128;" ::"r"(bar_id) : "memory");      // every row of the panel is written
             const int nnz = *p.nnz_ptr;
             const int lab_lo = p.label0 + m0;
-            const int lab_hi = p.label0 + min(m0 + BM, p.M);
+            const int lab_hi = p.label0 + min(m0 + BM, M);
             int lo = 0, hi = nnz;
             while (lo < hi) { const int mid = (lo + hi) >> 1; if (p.pos_labels[mid] < lab_lo) lo = mid + 1; else hi = mid; }
             const int e0 = lo;
@@ -526,7 +546,7 @@ enc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
           float v[32];
           tc::tmem_ld32(tdx + c0, v);
           const int col0 = n0 + g * ucols + c0;
-          if (row < p.M) {
+          if (row < M) {
             float* d = p.dX + (size_t)row * p.ldX + col0;
 #pragma unroll
             for (int j4 = 0; j4 < 8; ++j4)
@@ -542,8 +562,8 @@ enc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
           tc::tmem_ld32(tsk + c0, v);
           const int c_in_tile = g * ucols + c0;
           const int col0 = n0 + c_in_tile;
-          if (row < p.M) {
-            if (p.splits == 1) {
+          if (row < M) {
+            if (splits == 1) {
 #pragma unroll
               for (int j8 = 0; j8 < 4; ++j8)
                 if (col0 + 8 * j8 < p.N)
@@ -563,13 +583,13 @@ enc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
       if (lane == 0) {
         if (NCTA == 2) tc::mbar_arrive_leader(tmem_empty_bar + buf); else tc::mbar_arrive(tmem_empty_bar + buf);
       }
-      if (EPI == E_SPLITK && p.splits > 1) {
+      if (EPI == E_SPLITK && splits > 1) {
         // split-K fix-up: the CTA that adds the last partial of its half of a tile converts the sum and re-zeroes
         // the scratch (each CTA of a pair counts its own half)
         unsigned* cnt = p.sk_counters + (size_t)tile * NCTA + rank;
         __threadfence();
         asm volatile("bar.sync 1, %0;" ::"n"(EPI_THREADS) : "memory");
-        if (threadIdx.x == 64) *s_last = (atomicAdd(cnt, 1u) == (unsigned)(p.splits - 1)) ? 1 : 0;
+        if (threadIdx.x == 64) *s_last = (atomicAdd(cnt, 1u) == (unsigned)(splits - 1)) ? 1 : 0;
         asm volatile("bar.sync 1, %0;" ::"n"(EPI_THREADS) : "memory");
         if (*s_last) {
           // this CTA's 128 x BN block of the tile's scratch is contiguous: walk it with coalesced 16-byte accesses,
@@ -594,7 +614,7 @@ enc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
                 __stcg(blk + i4, make_float4(0.f, 0.f, 0.f, 0.f));
                 const int rr = i4 / bn4, cc = (i4 - rr * bn4) * 4;
                 const int grow = m0 + rr, gcol = n0 + cc;
-                if (grow < p.M && gcol < p.N) {
+                if (grow < M && gcol < p.N) {
                   uint2 o;
                   T* e = reinterpret_cast<T*>(&o);
                   e[0] = from_f<T>(x[u].x); e[1] = from_f<T>(x[u].y); e[2] = from_f<T>(x[u].z); e[3] = from_f<T>(x[u].w);
@@ -628,7 +648,7 @@ enc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
     }
     if (EPI == E_TOPK && cur_m >= 0 && u_active) {
       const int frow = cur_m * (BM * NCTA) + (int)rank * BM + r;
-      if (frow < p.M) {
+      if (frow < M) {
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
           p.cand_val[(size_t)frow * p.cand_ld + slot + k] = tv[k];
@@ -658,12 +678,12 @@ template <typename T, int NV>
 __global__ void __launch_bounds__(128) ln_fwd_kernel(const T* __restrict__ pre, const T* __restrict__ gamma,
                                                      const T* __restrict__ beta, T* __restrict__ y,
                                                      float* __restrict__ mean, float* __restrict__ rstd, int rows, int H,
-                                                     float eps) {
+                                                     float eps, const int* __restrict__ tok_meta) {
   grid_dep_wait();            // launched with launch_pdl: nothing above touches global memory
   grid_dep_launch();          // the kernel that follows may start its set-up now; it waits for this grid before reading
   const int lane = threadIdx.x & 31;
   const int row = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  if (row >= rows) return;
+  if (row >= (tok_meta != nullptr ? __ldcg(tok_meta + TOK_ROWS) : rows)) return;
   float v[NV][8];
   float sum = 0.f;
 #pragma unroll
@@ -847,11 +867,14 @@ RB_API int rb_enc_gemm_plan(int layout, int epi, int M, int N, int K, int bn_for
 //   R [M, ldr]: residual (BIAS_DROPOUT_RESID, ADD) or stored pre-activation (GELU_BWD); F [M, ldf]: pre-activation
 //   output (BIAS_GELU).  Layout TN with more than one K-split needs sk_scratch / sk_counters of the sizes
 //   rb_enc_gemm_plan reports (zero on entry, left zero).  bn_forced / ncta_forced: 0 = choose.
+//   tok_meta / tok (nullable): packed tokens (token_map.cuh).  M (NT, NN) or K (TN) is then the capacity in rows and the
+//   kernel takes the row count from tok_meta; plan_rows (0 = the capacity) is the count to plan tiles and splits for.
 // Returns 0, or -3 for an unsupported shape (the caller then uses the library GEMM).
 RB_API int rb_enc_gemm(int dtype, int layout, int epi, const void* A, const void* B, void* C, int M, int N, int K, int lda,
                        int ldb, int ldc, const void* bias, const void* R, int ldr, void* F, int ldf, float p_drop,
                        const int* seed, unsigned stream_id, float* colacc, int col_tot, int col_off, float* sk_scratch,
-                       unsigned* sk_counters, int bn_forced, int ncta_forced, int* status, cudaStream_t st) {
+                       unsigned* sk_counters, int bn_forced, int ncta_forced, const int* tok_meta, const int* tok,
+                       int plan_rows, int* status, cudaStream_t st) {
   if (dtype != RB_BF16 && dtype != RB_F16) return -1;
   if (M < 1 || N < 1 || K < 1 || N % 8 || lda % 8 || ldb % 8 || ldc % 8 || ldr % 8 || ldf % 8) return -3;
   if (layout == L_TN && M % 8) return -3;
@@ -860,7 +883,9 @@ RB_API int rb_enc_gemm(int dtype, int layout, int epi, const void* A, const void
   if (epi == E_BIAS_GELU && F == nullptr) return -3;
   if (epi == E_BIAS_DROPOUT_RESID && p_drop > 0.f && seed == nullptr) return -3;
   const bool bf16 = dtype == RB_BF16;
-  const Plan pl = make_plan(layout, epi, M, N, K, bn_forced, ncta_forced);
+  const bool tn = layout == L_TN;
+  const int pr = plan_rows > 0 ? plan_rows : (tn ? K : M);
+  const Plan pl = make_plan(layout, epi, tn ? M : pr, N, tn ? pr : K, bn_forced, ncta_forced);
   const int BN = pl.bn, b_rows = BN / pl.ncta;
   Maps m;
   int rc;
@@ -888,6 +913,7 @@ RB_API int rb_enc_gemm(int dtype, int layout, int epi, const void* A, const void
   p.p = p_drop; p.seed = seed; p.stream = stream_id;
   p.colacc = colacc; p.col_tot = col_tot; p.col_off = col_off;
   p.sk_scratch = sk_scratch; p.sk_counters = sk_counters; p.status = status;
+  p.tok_meta = tok_meta; p.tok = tok;
   const int n_items = p.n_m_tiles * p.n_n_tiles * p.splits;
   int max_units = sm_count() / pl.ncta;
   if (g_max_units > 0 && g_max_units < max_units) max_units = g_max_units;
@@ -1048,13 +1074,13 @@ RB_API int rb_xfc_dw_sgd_v2(const void* Gt, int ldG, const void* X, int B, void*
   }
 
 RB_API int rb_ln_fwd(int dtype, const void* pre, const void* gamma, const void* beta, void* y, float* mean, float* rstd,
-                     int rows, int H, float eps, cudaStream_t st) {
+                     int rows, int H, float eps, const int* tok_meta, cudaStream_t st) {
   if (H % 8 || rows < 1) return -3;
   const int blocks = (rows + 3) / 4;
   switch (dtype) {
-    case RB_F32: { using T = float; EG_DISPATCH_NV(H, (launch_pdl(ln_fwd_kernel<T, NV>, dim3(blocks), dim3(128), 0, st, (const T*)pre, (const T*)gamma, (const T*)beta, (T*)y, mean, rstd, rows, H, eps))); break; }
-    case RB_BF16: { using T = __nv_bfloat16; EG_DISPATCH_NV(H, (launch_pdl(ln_fwd_kernel<T, NV>, dim3(blocks), dim3(128), 0, st, (const T*)pre, (const T*)gamma, (const T*)beta, (T*)y, mean, rstd, rows, H, eps))); break; }
-    case RB_F16: { using T = __half; EG_DISPATCH_NV(H, (launch_pdl(ln_fwd_kernel<T, NV>, dim3(blocks), dim3(128), 0, st, (const T*)pre, (const T*)gamma, (const T*)beta, (T*)y, mean, rstd, rows, H, eps))); break; }
+    case RB_F32: { using T = float; EG_DISPATCH_NV(H, (launch_pdl(ln_fwd_kernel<T, NV>, dim3(blocks), dim3(128), 0, st, (const T*)pre, (const T*)gamma, (const T*)beta, (T*)y, mean, rstd, rows, H, eps, tok_meta))); break; }
+    case RB_BF16: { using T = __nv_bfloat16; EG_DISPATCH_NV(H, (launch_pdl(ln_fwd_kernel<T, NV>, dim3(blocks), dim3(128), 0, st, (const T*)pre, (const T*)gamma, (const T*)beta, (T*)y, mean, rstd, rows, H, eps, tok_meta))); break; }
+    case RB_F16: { using T = __half; EG_DISPATCH_NV(H, (launch_pdl(ln_fwd_kernel<T, NV>, dim3(blocks), dim3(128), 0, st, (const T*)pre, (const T*)gamma, (const T*)beta, (T*)y, mean, rstd, rows, H, eps, tok_meta))); break; }
     default: return -1;
   }
   RB_LAUNCH_CHECK();

@@ -187,21 +187,51 @@ def _acc_for(outs, width, default_counter):
     return ws.colacc, default_counter(ws)
 
 
+# ----------------------------------------------------------------------------- packed tokens
+class TokenMap:
+    """Packed rows of a padded ``[b, S]`` batch (``csrc/token_map.cuh``): the encoder's activations hold only attended
+    tokens, first tokens and wholly masked sequences.  ``update(mask)`` counts on the device (no host synchronisation);
+    ``embed_ln_fwd`` then fills ``tok`` and ``slot``.  ``rows_hint`` is the caller's estimate of the row count, used to
+    plan tiles only; 0 = plan for the padded count."""
+
+    def __init__(self, b: int, S: int, device):
+        z = lambda n: torch.zeros(n, dtype=torch.int32, device=device)
+        self.tok, self.slot = z(b * S), z(b * S)
+        self.off, self.len, self.cnt, self.meta = z(b), z(b), z(b), z(4)
+        self.rows_hint = 0
+
+    def update(self, mask) -> None:
+        b, S = mask.shape
+        _call("rb_token_map", _p(mask), _I(b), _I(S), _p(self.off), _p(self.len), _p(self.cnt), _p(self.meta), _stream())
+
+
+def _tok(tmap, *names):
+    return [_p(None if tmap is None else getattr(tmap, n)) for n in names]
+
+
 # ----------------------------------------------------------------------------- encoder ops
-def embed_ln_fwd(ids, word, pos, gamma, beta, eps, S, p, rng, stream, out, mean, rstd):
+def embed_ln_fwd(ids, word, pos, gamma, beta, eps, S, p, rng, stream, out, mean, rstd, mask=None, tmap=None):
     T, H = out.shape
     _call("rb_embed_ln_fwd", _I(DT[out.dtype]), _p(ids), _p(word), _p(pos), _p(gamma), _p(beta), _p(out), _p(mean),
-          _p(rstd), _I(T), _I(H), _I(S), _F(eps), _F(p), _p(rng.dev), _U(stream), _stream())
+          _p(rstd), _I(T), _I(H), _I(S), _F(eps), _F(p), _p(rng.dev), _U(stream), _p(mask),
+          *_tok(tmap, "meta", "off", "cnt", "tok", "slot"), _stream())
 
 
-def embed_ln_bwd(dy, ids, word, pos, gamma, mean, rstd, S, p, rng, stream, pad_id, dword, dpos, dgamma, dbeta):
+def embed_ln_bwd(dy, ids, word, pos, gamma, mean, rstd, S, p, rng, stream, pad_id, dword, dpos, dgamma, dbeta, tmap=None):
     T, H = dy.shape
     acc, counter = _acc_for([dgamma, dbeta], H, lambda ws: ws.counters)
     dword.zero_()
     dpos.zero_()
     _call("rb_embed_ln_bwd", _I(DT[dy.dtype]), _p(dy), _p(ids), _p(word), _p(pos), _p(gamma), _p(mean), _p(rstd),
           _p(dword), _p(dpos), _p(acc), _p(counter), _p(dgamma), _p(dbeta), _I(T), _I(H), _I(S), _I(pad_id),
-          _F(p), _p(rng.dev), _U(stream), _stream())
+          _F(p), _p(rng.dev), _U(stream), *_tok(tmap, "slot"), _stream())
+
+
+def attention_packs(dtype, S: int, H: int, nh: int) -> bool:
+    """Whether the attention kernels that serve this shape understand packed tokens (those of attention_mma.cu do)."""
+    if dtype == torch.float32 or H // nh != 64 or os.environ.get("RENEE_B200_ATTENTION", "") == "tiles":
+        return False
+    return S <= 128 or (S <= 512 and os.environ.get("RENEE_B200_ATTENTION_LONG", "") != "0")
 
 
 def _attention_fits(qkv, S: int, H: int, nh: int) -> bool:
@@ -233,12 +263,12 @@ def _seed_tensor(rng):
     return rng.dev.to(torch.int64).reshape(-1)[0] & 0xFFFFFFFF
 
 
-def attention_fwd(qkv, bqkv, mask, nh, p, rng, stream, ctx_out, ws):
+def attention_fwd(qkv, bqkv, mask, nh, p, rng, stream, ctx_out, ws, tmap=None):
     b, S = mask.shape
     H = ctx_out.shape[1]
     if _attention_long(qkv, S, H, nh, ws):
         _call("rb_attention_fwd_long", _I(DT[qkv.dtype]), _p(qkv), _p(bqkv), _p(mask), _p(ctx_out), _p(ws["probs"]),
-              _I(b), _I(S), _I(H), _I(nh), _F(p), _p(rng.dev), _U(stream), _stream())
+              _I(b), _I(S), _I(H), _I(nh), _F(p), _p(rng.dev), _U(stream), *_tok(tmap, "slot", "len", "meta"), _stream())
         return
     if not _attention_fits(qkv, S, H, nh):
         from . import reference as ref
@@ -246,18 +276,20 @@ def attention_fwd(qkv, bqkv, mask, nh, p, rng, stream, ctx_out, ws):
         ctx_out.copy_(ctx)
         ws["probs"][:b].copy_(probs)
         return
-    _call("rb_attention_fwd" if qkv.dtype == torch.float32 else _attention_entry("fwd", H, nh), _I(DT[qkv.dtype]),
-          _p(qkv), _p(bqkv), _p(mask), _p(ctx_out), _p(ws["probs"]), _I(b), _I(S),
-          _I(H), _I(nh), _F(p), _p(rng.dev), _U(stream), _stream())
+    entry = "rb_attention_fwd" if qkv.dtype == torch.float32 else _attention_entry("fwd", H, nh)
+    _call(entry, _I(DT[qkv.dtype]), _p(qkv), _p(bqkv), _p(mask), _p(ctx_out), _p(ws["probs"]), _I(b), _I(S),
+          _I(H), _I(nh), _F(p), _p(rng.dev), _U(stream),
+          *(_tok(tmap, "slot", "len", "meta") if entry.endswith("_mma") else ()), _stream())
 
 
-def attention_bwd(dctx, qkv, bqkv, mask, nh, p, rng, stream, ws, dqkv_out, dbqkv_out):
+def attention_bwd(dctx, qkv, bqkv, mask, nh, p, rng, stream, ws, dqkv_out, dbqkv_out, tmap=None):
     b, S = mask.shape
     H = dctx.shape[1]
     if _attention_long(qkv, S, H, nh, ws):
         acc = _DEFER.slot([dbqkv_out], 3 * H) if _DEFER is not None else None
         _call("rb_attention_bwd_long", _I(DT[qkv.dtype]), _p(dctx), _p(qkv), _p(bqkv), _p(ws["probs"]), _p(ws["ds"]),
-              _p(dqkv_out), _I(b), _I(S), _I(H), _I(nh), _F(p), _p(rng.dev), _U(stream), _p(acc), _stream(), launches=2)
+              _p(dqkv_out), _I(b), _I(S), _I(H), _I(nh), _F(p), _p(rng.dev), _U(stream), _p(acc),
+              *_tok(tmap, "slot", "len", "meta"), _stream(), launches=2)
         if acc is None:
             colsum(dqkv_out, dbqkv_out)
         return
@@ -274,8 +306,10 @@ def attention_bwd(dctx, qkv, bqkv, mask, nh, p, rng, stream, ws, dqkv_out, dbqkv
         return
     # with a deferred-columns plan active the kernel also accumulates the q/k/v bias gradients
     acc = _DEFER.slot([dbqkv_out], 3 * H) if _DEFER is not None else None
-    _call(_attention_entry("bwd", H, nh), _I(DT[qkv.dtype]), _p(dctx), _p(qkv), _p(bqkv), _p(ws["probs"]), _p(dqkv_out), _I(b),
-          _I(S), _I(H), _I(nh), _F(p), _p(rng.dev), _U(stream), _p(acc), _stream())
+    entry = _attention_entry("bwd", H, nh)
+    _call(entry, _I(DT[qkv.dtype]), _p(dctx), _p(qkv), _p(bqkv), _p(ws["probs"]), _p(dqkv_out), _I(b),
+          _I(S), _I(H), _I(nh), _F(p), _p(rng.dev), _U(stream), _p(acc),
+          *(_tok(tmap, "slot", "len", "meta") if entry.endswith("_mma") else ()), _stream())
     if acc is None:
         colsum(dqkv_out, dbqkv_out)
 
@@ -286,12 +320,13 @@ def bias_dropout_add_ln_fwd(x, bias, resid, gamma, beta, eps, p, rng, stream, y_
           _p(pre_out), _p(mean), _p(rstd), _I(T), _I(H), _F(eps), _F(p), _p(rng.dev), _U(stream), _stream())
 
 
-def bias_dropout_add_ln_bwd(dy, pre, gamma, mean, rstd, p, rng, stream, dgamma, dbeta, dbias, dpre_out, dbranch_out):
+def bias_dropout_add_ln_bwd(dy, pre, gamma, mean, rstd, p, rng, stream, dgamma, dbeta, dbias, dpre_out, dbranch_out,
+                            tmap=None):
     T, H = dy.shape
     acc, counter = _acc_for([dgamma, dbeta, dbias], H, lambda ws: ws.counters)
     _call("rb_bias_dropout_add_ln_bwd", _I(DT[dy.dtype]), _p(dy), _p(pre), _p(gamma), _p(mean), _p(rstd), _p(dpre_out),
           _p(dbranch_out if p > 0 else None), _p(acc), _p(counter), _p(dgamma), _p(dbeta), _p(dbias),
-          _I(T), _I(H), _F(p), _p(rng.dev), _U(stream), _stream())
+          _I(T), _I(H), _F(p), _p(rng.dev), _U(stream), *_tok(tmap, "meta", "tok"), _stream())
     return (dpre_out, dbranch_out) if p > 0 else (dpre_out, dpre_out)
 
 
@@ -339,8 +374,9 @@ def enc_gemm_supported(t: torch.Tensor, *dims: int) -> bool:
 
 
 def _enc_gemm(layout, epi, A, B, C, M, N, K, bias=None, R=None, F=None, p=0.0, rng=None, stream=0, colacc=None,
-              col_tot=0, col_off=0, bn=0, ncta=0):
+              col_tot=0, col_off=0, bn=0, ncta=0, tmap=None):
     dev = C.device
+    hint = 0 if tmap is None else tmap.rows_hint
     ws = workspace(dev)
     sk_buf, sk_cnt = None, None
     if not bn:
@@ -349,7 +385,7 @@ def _enc_gemm(layout, epi, A, B, C, M, N, K, bias=None, R=None, F=None, p=0.0, r
         ncta = int(os.environ.get("RENEE_B200_GEMM_NCTA", "0"))
     if layout == L_TN:
         ncta_o, bn_o, sp_o, words_o, floats_o = _I(0), _I(0), _I(0), _I(0), _LL(0)
-        lib().rb_enc_gemm_plan(_I(layout), _I(epi), _I(M), _I(N), _I(K), _I(bn), _I(ncta), _c.byref(ncta_o), _c.byref(bn_o),
+        lib().rb_enc_gemm_plan(_I(layout), _I(epi), _I(M), _I(N), _I(hint or K), _I(bn), _I(ncta), _c.byref(ncta_o), _c.byref(bn_o),
                                _c.byref(sp_o), _c.byref(floats_o), _c.byref(words_o))
         if sp_o.value > 1:
             key = dev.index if dev.index is not None else torch.cuda.current_device()
@@ -357,10 +393,12 @@ def _enc_gemm(layout, epi, A, B, C, M, N, K, bias=None, R=None, F=None, p=0.0, r
     _call("rb_enc_gemm", _I(DT[C.dtype]), _I(layout), _I(epi), _p(A), _p(B), _p(C), _I(M), _I(N), _I(K),
           _I(A.stride(0)), _I(B.stride(0)), _I(C.stride(0)), _p(bias), _p(R), _I(R.stride(0) if R is not None else 0),
           _p(F), _I(F.stride(0) if F is not None else 0), _F(p), _p(rng.dev if rng is not None else None), _U(stream),
-          _p(colacc), _I(col_tot), _I(col_off), _p(sk_buf), _p(sk_cnt), _I(bn), _I(ncta), _p(ws.status), _stream())
+          _p(colacc), _I(col_tot), _I(col_off), _p(sk_buf), _p(sk_cnt), _I(bn), _I(ncta),
+          *_tok(tmap, "meta", "tok"), _I(hint), _p(ws.status), _stream())
 
 
-def linear_fwd(x, W, out, epi="store", bias=None, resid=None, pre_out=None, p=0.0, rng=None, stream=0, bn=0, ncta=0):
+def linear_fwd(x, W, out, epi="store", bias=None, resid=None, pre_out=None, p=0.0, rng=None, stream=0, bn=0, ncta=0,
+               tmap=None):
     """``out = epilogue(x @ W.T)`` for ``x [T, K]``, ``W [N, K]`` (an ``nn.Linear`` weight):
 
     * ``store``: the product;
@@ -368,15 +406,16 @@ def linear_fwd(x, W, out, epi="store", bias=None, resid=None, pre_out=None, p=0.
     * ``bias_dropout_resid``: ``out = resid + dropout(x W^T + bias)`` — the input of the following LayerNorm.
 
     ``bn`` / ``ncta`` force the N tile (64, 128, 256) and the tile shape (1: one CTA per 128-row tile, 2: a CTA
-    pair per 256-row tile); 0 lets the library choose."""
+    pair per 256-row tile); 0 lets the library choose.  With a token map the rows of ``x`` are packed tokens."""
     T, K = x.shape
     N = W.shape[0]
     code = {"store": E_STORE, "bias_gelu": E_BIAS_GELU, "bias_dropout_resid": E_BIAS_DROPOUT_RESID}[epi]
-    _enc_gemm(L_NT, code, x, W, out, T, N, K, bias=bias, R=resid, F=pre_out, p=p, rng=rng, stream=stream, bn=bn, ncta=ncta)
+    _enc_gemm(L_NT, code, x, W, out, T, N, K, bias=bias, R=resid, F=pre_out, p=p, rng=rng, stream=stream, bn=bn, ncta=ncta,
+              tmap=tmap)
     return out
 
 
-def linear_dgrad(dy, W, out, epi="store", resid=None, pre=None, dbias=None, bn=0, ncta=0):
+def linear_dgrad(dy, W, out, epi="store", resid=None, pre=None, dbias=None, bn=0, ncta=0, tmap=None):
     """``out = epilogue(dy @ W)`` for ``dy [T, N]``, ``W [N, K]``:
 
     * ``store``: the product;  ``add``: product ``+ resid`` (the residual branch's gradient);
@@ -386,28 +425,28 @@ def linear_dgrad(dy, W, out, epi="store", resid=None, pre=None, dbias=None, bn=0
     K = W.shape[1]
     code = {"store": E_STORE, "add": E_ADD, "gelu_bwd": E_GELU_BWD}[epi]
     if code != E_GELU_BWD or dbias is None:
-        _enc_gemm(L_NN, code, dy, W, out, T, K, N, R=resid if code == E_ADD else pre, bn=bn, ncta=ncta)
+        _enc_gemm(L_NN, code, dy, W, out, T, K, N, R=resid if code == E_ADD else pre, bn=bn, ncta=ncta, tmap=tmap)
         return out
     plan = _DEFER if _DEFER is not None else DeferredColumns(out.device, out.dtype)
     acc = plan.slot([dbias], K)
-    _enc_gemm(L_NN, code, dy, W, out, T, K, N, R=pre, colacc=acc, col_tot=K, col_off=0, bn=bn, ncta=ncta)
+    _enc_gemm(L_NN, code, dy, W, out, T, K, N, R=pre, colacc=acc, col_tot=K, col_off=0, bn=bn, ncta=ncta, tmap=tmap)
     if _DEFER is None:
         plan.finalize()
     return out
 
 
-def linear_wgrad(dy, x, dW, bn=0, ncta=0):
+def linear_wgrad(dy, x, dW, bn=0, ncta=0, tmap=None):
     """``dW = dy.T @ x`` for ``dy [T, N]``, ``x [T, K]``, ``dW [N, K]`` (split over T, reduced in fp32)."""
     T, N = dy.shape
     K = x.shape[1]
-    _enc_gemm(L_TN, E_SPLITK, dy, x, dW, N, K, T, bn=bn, ncta=ncta)
+    _enc_gemm(L_TN, E_SPLITK, dy, x, dW, N, K, T, bn=bn, ncta=ncta, tmap=tmap)
     return dW
 
 
-def ln_fwd(pre, gamma, beta, eps, y_out, mean, rstd):
+def ln_fwd(pre, gamma, beta, eps, y_out, mean, rstd, tmap=None):
     T, H = pre.shape
     _call("rb_ln_fwd", _I(DT[pre.dtype]), _p(pre), _p(gamma), _p(beta), _p(y_out), _p(mean), _p(rstd), _I(T), _I(H),
-          _F(eps), _stream())
+          _F(eps), *_tok(tmap, "meta"), _stream())
 
 
 def colsum(x, out):
@@ -417,16 +456,16 @@ def colsum(x, out):
     return out
 
 
-def pool_fwd(h, mask, mode, out):
+def pool_fwd(h, mask, mode, out, tmap=None):
     b, S, H = h.shape
     _call("rb_pool_fwd", _I(DT[h.dtype]), _p(h), _p(mask), _p(out), _I(b), _I(S), _I(H), _I(1 if mode == "cls" else 0),
-          _stream())
+          *_tok(tmap, "slot"), _stream())
 
 
-def pool_bwd(de, mask, mode, S, dh_out):
+def pool_bwd(de, mask, mode, S, dh_out, tmap=None):
     b, H = de.shape
     _call("rb_pool_bwd", _I(DT[dh_out.dtype]), _p(de), _p(mask), _p(dh_out), _I(b), _I(S), _I(H),
-          _I(1 if mode == "cls" else 0), _stream())
+          _I(1 if mode == "cls" else 0), *_tok(tmap, "meta", "tok", "cnt"), _stream())
 
 
 def dropout_cast_fwd(e, p, rng, stream, out):

@@ -183,6 +183,7 @@ class XCTrainer:
         dev = self.device
         b, S = cfg.batch_size + 1, cfg.maxlen
         self.max_nnz = 0
+        self._rows_hints: dict = {}
         self.buf = dict(
             ids=guard.zeros(b, S, dtype=torch.int32, device=dev, name="step.ids"),
             mask=guard.zeros(b, S, dtype=torch.int32, device=dev, name="step.mask"),
@@ -232,6 +233,14 @@ class XCTrainer:
             batch.uploaded()            # the loader may refill the batch's staging buffers once these copies are done
         return b, nnz
 
+    def _hint_rows(self, batch: XCBatch) -> None:
+        """Tells the encoder how many tokens batches of this shape hold, once per shape (the GEMM tiles are planned for it;
+        the count that is computed with comes from the mask on the device)."""
+        shape = tuple(batch.attention_mask.shape)
+        if shape not in self._rows_hints:
+            self._rows_hints[shape] = 0 if batch.attention_mask.is_cuda else int(torch.count_nonzero(batch.attention_mask))
+        self.encoder.rows_hint = self._rows_hints[shape]
+
     def h2d_bytes(self, batch: XCBatch) -> int:
         return int(batch.input_ids.numel() * 4 + batch.attention_mask.numel() * 4 + batch.pos_rows.numel() * 8
                    + HP.HOST_SLOTS * 4)
@@ -240,6 +249,7 @@ class XCTrainer:
         """Host→device part of a step: this step's hyper-parameters (32 bytes) and inputs."""
         self._set_hparams()
         b, nnz = self._upload(batch)
+        self._hint_rows(batch)
         want_loss = (not self.cfg.noloss) and (self.count % LOSS_SAMPLE_FREQ == 0)
         self._staged = (b, batch.batch_size, nnz, want_loss)
 
@@ -542,6 +552,7 @@ class XCTrainer:
         b = batch.input_ids.shape[0]
         ids = batch.input_ids.to(dev, non_blocking=True)
         mask = batch.attention_mask.to(dev, non_blocking=True)
+        self._hint_rows(batch)
         emb = self.encoder.forward(ids, mask, self.step_rng, train=False)
         return emb.to(self.xfc.dtype)
 
