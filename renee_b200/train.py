@@ -42,6 +42,7 @@ from .utils.timing import nvtx_range
 from .utils.sharding import LabelSharding
 
 LOSS_SAMPLE_FREQ = 100   # dl_base.py:144
+EMBED_GRAPHS = 4         # batch shapes whose evaluation pass is kept as a CUDA graph
 _S_CLS_DROPOUT = 5
 
 
@@ -149,6 +150,8 @@ class XCTrainer:
         self._graphs: dict = {}
         self._graph_warm: dict = {}
         self._graph_generation = -1
+        self._embed_graphs: dict = {}
+        self._embed_generation = -1
         self._pending_loss = None
         self._side_stream = None
         self._aborted = False
@@ -550,11 +553,47 @@ class XCTrainer:
             self.model.train()
             return e
         b = batch.input_ids.shape[0]
+        self._hint_rows(batch)
+        if dev.type == "cuda" and self.cfg.cuda_graph and self.act_dtype != torch.float32:
+            return self._embed_graphed(batch)
         ids = batch.input_ids.to(dev, non_blocking=True)
         mask = batch.attention_mask.to(dev, non_blocking=True)
         self._hint_rows(batch)
         emb = self.encoder.forward(ids, mask, self.step_rng, train=False)
         return emb.to(self.xfc.dtype)
+
+    def _embed_graphed(self, batch: XCBatch) -> torch.Tensor:
+        """The evaluation encoder from a CUDA graph: some 45 launches take the host 1.1 ms to issue and the GPU 0.7 ms to
+        run (256 x 32 tokens, DistilBERT).  The first batch of a shape runs eagerly, the second captures; at most
+        ``EMBED_GRAPHS`` shapes are kept (a last partial batch has its own), further ones stay eager."""
+        enc, shape = self.encoder, tuple(batch.input_ids.shape)
+        if self._embed_generation != enc.generation:
+            self._embed_graphs = {}                              # the encoder re-allocated its activations
+            self._embed_generation = enc.generation
+        st = self._embed_graphs.get(shape)
+        if st is None and len(self._embed_graphs) < EMBED_GRAPHS:
+            st = dict(ids=torch.empty(shape, dtype=torch.int32, device=self.device),
+                      mask=torch.empty(shape, dtype=torch.int32, device=self.device), graph=None, emb=None, seen=0)
+        if st is None:
+            ids = batch.input_ids.to(self.device, torch.int32, non_blocking=True)
+            mask = batch.attention_mask.to(self.device, torch.int32, non_blocking=True)
+            return enc.forward(ids, mask, self.step_rng, train=False).to(self.xfc.dtype, copy=True)
+        st["ids"].copy_(batch.input_ids, non_blocking=True)
+        st["mask"].copy_(batch.attention_mask, non_blocking=True)
+        if st["graph"] is None and st["seen"] == 0:
+            st["seen"], st["emb"] = 1, enc.forward(st["ids"], st["mask"], self.step_rng, train=False)
+            if self._embed_generation != enc.generation:         # this pass allocated the activations
+                self._embed_graphs, self._embed_generation = {}, enc.generation
+            self._embed_graphs[shape] = st
+        else:
+            if st["graph"] is None:
+                torch.cuda.synchronize()
+                graph = torch.cuda.CUDAGraph()
+                with torch.cuda.graph(graph, capture_error_mode="thread_local"):
+                    st["emb"] = enc.forward(st["ids"], st["mask"], self.step_rng, train=False)
+                st["graph"] = graph
+            st["graph"].replay()
+        return st["emb"].to(self.xfc.dtype, copy=True)           # the embedding buffer belongs to the encoder
 
     def local_topk(self, X: torch.Tensor, k: int):
         if self.cfg.default_impl:

@@ -85,3 +85,29 @@ def test_packed_equals_padded(S, b, kind, pooling, dt, hint):
         tol = 2.0 ** -7 * y.abs() + (3e-2 if name.startswith("embeddings") else 1e-4) * scale
         assert bool(((x - y).abs() <= tol).all()), (name, float((x - y).abs().max()), scale)
 
+
+def test_embed_eval_graph_equals_the_eager_pass():
+    """Several shapes, new batches of a shape after its capture, more shapes than graphs are kept, weights changed in between."""
+    from types import SimpleNamespace
+
+    from renee_b200.models.encoder import EncoderConfig
+    from renee_b200.parallel.dist import DistContext
+    from renee_b200.train import EMBED_GRAPHS, TrainConfig, XCTrainer
+    from renee_b200.utils.sharding import shard_labels
+    dev = torch.device("cuda", 0)
+    enc = EncoderConfig(dim=128, n_layers=2, n_heads=2, hidden_dim=256, vocab_size=500)
+    cfg = TrainConfig(batch_size=40, epochs=1, maxlen=24, pooling="mean", fp16xfc=True, noloss=True)
+    tr = XCTrainer(cfg, enc, shard_labels(512, 1), DistContext(device=dev), steps_per_epoch=4)
+    gen = torch.Generator().manual_seed(5)
+    kept = []
+    for rep in range(4):
+        for b in list(range(40, 40 - EMBED_GRAPHS - 2, -1)):
+            mask = _mask("prefix", b, 24, gen).cpu()
+            ids = torch.randint(5, 500, (b, 24), generator=gen, dtype=torch.int32) * mask
+            got = tr.embed_eval(SimpleNamespace(input_ids=ids, attention_mask=mask))
+            kept.append((got, got.clone()))
+            want = tr.encoder.forward(ids.cuda(), mask.cuda(), tr.step_rng, train=False).to(got.dtype)
+            assert torch.equal(got, want)
+        tr.encoder.p16.mul_(1.01)
+    assert len(tr._embed_graphs) == EMBED_GRAPHS and all(g["graph"] is not None for g in tr._embed_graphs.values())
+    assert all(torch.equal(a, c) for a, c in kept)         # a result is not overwritten by later batches
