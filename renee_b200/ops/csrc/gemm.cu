@@ -22,8 +22,10 @@
 //                                   m = mo m + (acc + wd w), w -= lr m (stochastic rounding optional) in shared memory,
 //                                   both tiles leave by TMA; dW = Gt X is never stored (parity: dl_base.py:623-633, 343-344)
 //              TOPK                 nothing is stored: every epilogue thread keeps the 8 largest entries of its row
-//                                   over all the tiles its CTA visits and writes them as candidates at the end
-//                                   (prediction: X W^T is never materialised; parity: dl_base.py:745-756)
+//                                   over all the tiles its CTA visits and writes them as candidates at the end; topk.cu
+//                                   reduces the candidates to the k best and recomputes the labels of a thread that
+//                                   may have dropped one (prediction: X W^T is never materialised; parity:
+//                                   dl_base.py:745-756)
 //
 // Structure.  Persistent CTAs walk the work items (tile x K-split).  576 threads: warp 0 TMA producer, warp 1
 // TMEM owner + MMA issuer, warps 2..17 epilogue (four groups of four warps, one TMEM lane quarter per warp, one
@@ -47,6 +49,7 @@
 #include <type_traits>
 #include "peer.cuh"
 #include "token_map.cuh"
+#include "topk.cuh"
 
 namespace rb {
 namespace eg {
@@ -95,7 +98,7 @@ struct Params {
   float p; const int* seed; uint32_t stream;        // dropout      BIAS_DROPOUT_RESID
   float* colacc; int col_tot; int col_off;          // GELU_BWD: replicas of [col_tot] floats, this vector at col_off
   float* sk_scratch; unsigned* sk_counters;         // SPLITK: [tiles][128 NCTA x BN] fp32 (zero between launches), [tiles]
-  float* cand_val; int* cand_idx; int cand_ld;      // TOPK: [M, cand_ld] candidates, 8 per (CTA, epilogue group)
+  float* cand_val; int* cand_idx; int cand_ld;      // TOPK: [M, cand_ld] candidates, 8 per (unit, epilogue group)
   // SIGMOID_POS (classifier logits + gradient): label-sorted positives, label id of row 0, all-gather flags to wait for
   const int* pos_rows; const int* pos_labels; const int* nnz_ptr; int label0;
   const uint32_t* wait_flags; int wait_n; const uint32_t* step_ptr;
@@ -144,6 +147,14 @@ __device__ __forceinline__ float warp_colsum32(float (&v)[32], int lane) {
 
 // Byte offset of the 16-byte chunk `chunk` (8 columns) of row r inside a 128-byte-swizzled panel.
 __device__ __forceinline__ uint32_t panel_off(int r, int chunk) { return (uint32_t)r * 128u + (uint32_t)((chunk ^ (r & 7)) << 4); }
+
+// (M tile, N tile) of an item's tile.  TOPK walks two M tiles side by side: the units of even number take one, the
+// others the other, so that the (much larger) N operand is read from HBM once per pair of M tiles instead of once per M
+// tile, and a unit still stays with one M tile until its N tiles are done (topk.cuh has the same numbering).
+template <int EPI> __device__ __forceinline__ void tile_coords(int tile, int n_m, int n_n, int& mt, int& nt) {
+  if (EPI == E_TOPK) topk_tile(tile, n_m, n_n, mt, nt);
+  else { mt = tile / n_n; nt = tile - mt * n_n; }
+}
 
 template <typename T, int LAYOUT, int EPI, int NCTA>
 __global__ void __launch_bounds__(THREADS, 1)
@@ -234,8 +245,10 @@ enc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
     }
     for (int item = unit; item < n_items && !aborted; item += n_units) {
       const int tile = item / splits, split = item - tile * splits;
-      const int m0 = (tile / p.n_n_tiles) * (BM * NCTA) + (int)rank * BM;
-      const int n0 = (tile % p.n_n_tiles) * p.BN + (int)rank * b_rows;
+      int mt, nt;
+      tile_coords<EPI>(tile, n_m_tiles, p.n_n_tiles, mt, nt);
+      const int m0 = mt * (BM * NCTA) + (int)rank * BM;
+      const int n0 = nt * p.BN + (int)rank * b_rows;
       const int kb0 = split * kb_per_split, kb1 = min(kb_total, kb0 + kb_per_split);
       for (int kb = kb0; kb < kb1; ++kb, s = (s + 1 == STAGES ? 0 : s + 1), ph ^= (s == 0 ? 1u : 0u)) {
         if (!tc::mbar_wait(empty_bar + s, ph ^ 1, aborted, p.status, tc::SITE_EMPTY, kb)) break;
@@ -327,30 +340,28 @@ enc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
     float tv[8];
     int ti[8];
     int cur_m = -1;
+    const auto topk_flush = [&]() {                       // the list of this unit and column group for row block cur_m
+      const int frow = cur_m * (BM * NCTA) + (int)rank * BM + r;
+      if (cur_m < 0 || frow >= M || !u_active) return;
+      const size_t at = (size_t)frow * p.cand_ld + (size_t)(unit * EGROUPS + g) * 8;
+      float4* cv = reinterpret_cast<float4*>(p.cand_val + at);
+      int4* ci = reinterpret_cast<int4*>(p.cand_idx + at);
+      cv[0] = make_float4(tv[0], tv[1], tv[2], tv[3]); cv[1] = make_float4(tv[4], tv[5], tv[6], tv[7]);
+      ci[0] = make_int4(ti[0], ti[1], ti[2], ti[3]); ci[1] = make_int4(ti[4], ti[5], ti[6], ti[7]);
+    };
     float loss = 0.f;                                     // SIGMOID_POS: this thread's share of sum softplus(z)
-    const int slot = ((int)blockIdx.x * EGROUPS + g) * 8;
     for (int item = unit; item < n_items; item += n_units, ++t_local) {
       const int tile = item / splits;
-      if (EPI == E_TOPK) {
-        const int mt = tile / p.n_n_tiles;
-        if (mt != cur_m) {
-          if (cur_m >= 0) {
-            const int frow = cur_m * (BM * NCTA) + (int)rank * BM + r;
-            if (frow < M && u_active) {
+      int mt, nt;
+      tile_coords<EPI>(tile, n_m_tiles, p.n_n_tiles, mt, nt);
+      if (EPI == E_TOPK && mt != cur_m) {
+        topk_flush();
 #pragma unroll
-              for (int k = 0; k < 8; ++k) {
-                p.cand_val[(size_t)frow * p.cand_ld + slot + k] = tv[k];
-                p.cand_idx[(size_t)frow * p.cand_ld + slot + k] = ti[k];
-              }
-            }
-          }
-#pragma unroll
-          for (int k = 0; k < 8; ++k) { tv[k] = -3.0e38f; ti[k] = 0; }
-          cur_m = mt;
-        }
+        for (int k = 0; k < 8; ++k) { tv[k] = -INFINITY; ti[k] = -1; }
+        cur_m = mt;
       }
-      const int m0 = (tile / p.n_n_tiles) * (BM * NCTA) + (int)rank * BM;
-      const int n0 = (tile % p.n_n_tiles) * p.BN;
+      const int m0 = mt * (BM * NCTA) + (int)rank * BM;
+      const int n0 = nt * p.BN;
       const int row = m0 + r;
       const int buf = t_local & 1;
       const uint32_t use = (uint32_t)(t_local >> 1);
@@ -522,16 +533,28 @@ enc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
             float v[32];
             tc::tmem_ld32(ttk + cc, v);
             const int c0 = n0 + g * ucols + cc;
+            // Most fragments hold nothing for any of the warp's rows once the lists are warm: one maximum over the 32
+            // values decides.  A NaN must pass the test (it ranks above every number), hence max.NaN.
+            float m8[8];
 #pragma unroll
-            for (int j = 0; j < 32; ++j) {
-              const float x = v[j];
-              if (x > tv[7] && c0 + j < p.N) {           // strict: of equal values the lower column stays
-                tv[7] = x; ti[7] = c0 + j;
+            for (int q = 0; q < 8; ++q) m8[q] = max_nan(max_nan(v[4 * q], v[4 * q + 1]), max_nan(v[4 * q + 2], v[4 * q + 3]));
+            const float top = max_nan(max_nan(max_nan(m8[0], m8[1]), max_nan(m8[2], m8[3])),
+                                      max_nan(max_nan(m8[4], m8[5]), max_nan(m8[6], m8[7])));
+            if (top <= tv[7]) continue;
 #pragma unroll
-                for (int k = 7; k > 0; --k) {
-                  if (tv[k] > tv[k - 1]) {
-                    const float a = tv[k]; tv[k] = tv[k - 1]; tv[k - 1] = a;
-                    const int b = ti[k]; ti[k] = ti[k - 1]; ti[k - 1] = b;
+            for (int q = 0; q < 8; ++q) {
+              if (m8[q] <= tv[7]) continue;
+#pragma unroll
+              for (int j = 4 * q; j < 4 * q + 4; ++j) {
+                const float x = topk_store_value(v[j]);
+                if (x > tv[7] && c0 + j < p.N) {         // strict: of equal values the lower column stays
+                  tv[7] = x; ti[7] = c0 + j;
+#pragma unroll
+                  for (int k = 7; k > 0; --k) {
+                    if (tv[k] > tv[k - 1]) {
+                      const float a = tv[k]; tv[k] = tv[k - 1]; tv[k - 1] = a;
+                      const int b = ti[k]; ti[k] = ti[k - 1]; ti[k - 1] = b;
+                    }
                   }
                 }
               }
@@ -646,16 +669,7 @@ enc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
         }
       }
     }
-    if (EPI == E_TOPK && cur_m >= 0 && u_active) {
-      const int frow = cur_m * (BM * NCTA) + (int)rank * BM + r;
-      if (frow < M) {
-#pragma unroll
-        for (int k = 0; k < 8; ++k) {
-          p.cand_val[(size_t)frow * p.cand_ld + slot + k] = tv[k];
-          p.cand_idx[(size_t)frow * p.cand_ld + slot + k] = ti[k];
-        }
-      }
-    }
+    if (EPI == E_TOPK) topk_flush();
   }
   tc::tc_fence_before();
   __syncthreads();
@@ -927,17 +941,33 @@ RB_API int rb_enc_gemm(int dtype, int layout, int epi, const void* A, const void
   return 0;
 }
 
-// Prediction: candidates for the top-k (k <= 8) of every row of X W^T without materialising the product.
-//   X [B, ldx >= D], W [Ls, ldw >= D] (16-bit, same dtype); cand_val / cand_idx [B, cand_ld] with
-//   cand_ld >= rb_xfc_topk8_width(): every (CTA, epilogue group) writes the 8 best (value, column of W) it met in
-//   the row into its own 8 entries; entries nobody writes must have been pre-filled with -inf by the caller.
-// The k best of a row's candidates are the k best of the row (k <= 8).
-RB_API int rb_xfc_topk8_width(void) { return sm_count() * EGROUPS * 8; }
+// Units of a TOPK launch.  An even number as soon as a unit gets several items: two M tiles are walked side by side and
+// a unit must stay with one of them (topk.cuh).
+static int topk_units(const Plan& pl, int n_m, int n_n) {
+  const int max_units = sm_count() / pl.ncta;
+  const long n_items = (long)n_m * n_n;
+  return n_items <= max_units ? (int)n_items : (max_units > 1 ? max_units & ~1 : 1);
+}
 
-RB_API int rb_xfc_topk8(int dtype, const void* X, const void* W, int B, int Ls, int D, int ldx, int ldw, float* cand_val,
-                        int* cand_idx, int cand_ld, int* status, cudaStream_t st) {
+// Layout of the candidates that rb_xfc_topk_candidates leaves for (B, Ls, D): out[0] CTAs per tile, [1] N tile,
+// [2] units, [3] N tiles, [4] M tiles, [5] floats (and ints) per row.
+RB_API int rb_xfc_topk_plan(int B, int Ls, int D, int* out) {
+  if (B < 1 || Ls < 1 || D < 1) return -3;
+  const Plan pl = make_plan(L_NT, E_TOPK, B, Ls, D, 0, 0);
+  const int n_m = (B + BM * pl.ncta - 1) / (BM * pl.ncta), n_n = (Ls + pl.bn - 1) / pl.bn;
+  const int units = topk_units(pl, n_m, n_n);
+  out[0] = pl.ncta; out[1] = pl.bn; out[2] = units; out[3] = n_n; out[4] = n_m; out[5] = units * EGROUPS * 8;
+  return 0;
+}
+
+// Prediction: candidates for the k largest entries of every row of X W^T without materialising the product.
+//   X [B, ldx >= D], W [Ls, ldw >= D] (16-bit, same dtype); cand_val / cand_idx [B, rb_xfc_topk_plan's row length]:
+// every (unit, epilogue group) writes the 8 best (value, column of W) that it met in a row, in descending order, value
+// -inf and column -1 where it met fewer.  topk.cu turns them into the k best.
+RB_API int rb_xfc_topk_candidates(int dtype, const void* X, const void* W, int B, int Ls, int D, int ldx, int ldw,
+                                  float* cand_val, int* cand_idx, int* status, cudaStream_t st) {
   if (dtype != RB_BF16 && dtype != RB_F16) return -1;
-  if (B < 1 || Ls < 1 || D < 1 || ldx % 8 || ldw % 8 || cand_ld < rb_xfc_topk8_width()) return -3;
+  if (B < 1 || Ls < 1 || D < 1 || ldx % 8 || ldw % 8) return -3;
   const bool bf16 = dtype == RB_BF16;
   const Plan pl = make_plan(L_NT, E_TOPK, B, Ls, D, 0, 0);
   const int BN = pl.bn, b_rows = BN / pl.ncta;
@@ -951,10 +981,8 @@ RB_API int rb_xfc_topk8(int dtype, const void* X, const void* W, int B, int Ls, 
   p.M = B; p.N = Ls; p.BN = BN;
   p.n_m_tiles = (B + BM * pl.ncta - 1) / (BM * pl.ncta); p.n_n_tiles = (Ls + BN - 1) / BN;
   p.kb_total = (D + BK - 1) / BK; p.splits = 1; p.kb_per_split = p.kb_total;
-  p.cand_val = cand_val; p.cand_idx = cand_idx; p.cand_ld = cand_ld; p.status = status;
-  const long n_items = (long)p.n_m_tiles * p.n_n_tiles;
-  const int max_units = sm_count() / pl.ncta;
-  const int units = n_items < max_units ? (int)n_items : max_units;
+  const int units = topk_units(pl, p.n_m_tiles, p.n_n_tiles);
+  p.cand_val = cand_val; p.cand_idx = cand_idx; p.cand_ld = units * EGROUPS * 8; p.status = status;
   rc = pl.ncta == 2
            ? (bf16 ? dispatch_enc_gemm<__nv_bfloat16, 2>(L_NT, E_TOPK, m, p, units, st) : dispatch_enc_gemm<__half, 2>(L_NT, E_TOPK, m, p, units, st))
            : (bf16 ? dispatch_enc_gemm<__nv_bfloat16, 1>(L_NT, E_TOPK, m, p, units, st) : dispatch_enc_gemm<__half, 1>(L_NT, E_TOPK, m, p, units, st));

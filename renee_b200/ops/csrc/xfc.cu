@@ -17,6 +17,7 @@
 // Structure of every kernel: 192 threads; warp 0 = TMA producer, warp 1 = TMEM owner + MMA issuer,
 // warps 2..5 = epilogue (one TMEM lane quarter each).  4-stage smem ring, 128x{<=256}x64 tiles,
 // UMMA 128xNx16.  All waits are bounded (see tc.cuh).
+#include "topk.cuh"
 #include "peer.cuh"
 
 namespace rb {
@@ -625,11 +626,6 @@ xfc_dw_sgd_tma_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
 // 8-bit histogram passes find the k-th largest key exactly, the fifth collects every element above it
 // plus as many ties as needed.  Output is unordered (the cross-chunk / cross-rank merge sorts k items).
 // Replaces torch.topk / the K passes of torch.max + index_put_ of the reference (dl_base.py:745-756).
-__device__ __forceinline__ uint32_t order_key(float x) {
-  const uint32_t u = __float_as_uint(x);
-  return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
-}
-
 __global__ void __launch_bounds__(256) topk_rows_kernel(const float* __restrict__ Z, int ldZ, int n, int k, int label0,
                                                         float* __restrict__ out_val, int* __restrict__ out_idx) {
   __shared__ unsigned hist[256];

@@ -643,34 +643,37 @@ def topk_rows(Z, n, k, label0, out_val, out_idx):
 
 
 def xfc_topk8(W, X, k):
-    """Top-k (k <= 8) of every row of ``X Wᵀ`` with the selection fused into the GEMM epilogue: each epilogue
-    thread of the persistent tcgen05 GEMM keeps the 8 best entries of its row over all label tiles its CTA
-    visits, so the ``[B, Ls]`` logits are never written; the few thousand candidates per row are then reduced by
-    the row-selection kernel.  Returns ``(values [B, k] fp32 descending, label ids [B, k] int64)``."""
+    """Top-k of every row of ``X Wᵀ`` with the selection fused into the GEMM epilogue: each epilogue thread of the
+    persistent tcgen05 GEMM keeps the 8 best entries of its row over all label tiles its CTA visits, so the ``[B, Ls]``
+    logits are never written; one CTA per row then reduces the candidates and recomputes the few lists that may have
+    dropped one of the k best (``csrc/topk.cu``; exact for every ``k <= rb_topk_max_k()``).  Returns ``(values [B, k] fp32
+    descending, label ids [B, k] int64)``."""
     B, D = X.shape
     Ls = W.shape[0]
-    width = int(lib().rb_xfc_topk8_width())
-    cv = torch.full((B, width), -3.0e38, dtype=torch.float32, device=X.device)
-    ci = torch.zeros(B, width, dtype=torch.int32, device=X.device)
-    ws = workspace(X.device)
-    _call("rb_xfc_topk8", _I(DT[X.dtype]), _p(X), _p(W), _I(B), _I(Ls), _I(D), _I(X.stride(0)), _I(W.stride(0)), _p(cv),
-          _p(ci), _I(width), _p(ws.status), _stream())
+    plan = (_I * 6)()
+    rc = lib().rb_xfc_topk_plan(_I(B), _I(Ls), _I(D), plan)
+    if rc != 0:
+        raise KernelError(f"rb_xfc_topk_plan failed with code {rc}")
+    cv = torch.empty(B, plan[5], dtype=torch.float32, device=X.device)
+    ci = torch.empty(B, plan[5], dtype=torch.int32, device=X.device)
     vals = torch.empty(B, k, dtype=torch.float32, device=X.device)
-    pos = torch.empty(B, k, dtype=torch.int32, device=X.device)
-    topk_rows(cv, width, k, 0, vals, pos)
-    idx = torch.gather(ci, 1, pos.long())
-    v, order = torch.sort(vals, dim=1, descending=True)
-    return v, torch.gather(idx, 1, order).long()
+    idx = torch.empty(B, k, dtype=torch.int64, device=X.device)
+    ws = workspace(X.device)
+    _call("rb_xfc_topk_candidates", _I(DT[X.dtype]), _p(X), _p(W), _I(B), _I(Ls), _I(D), _I(X.stride(0)), _I(W.stride(0)),
+          _p(cv), _p(ci), _p(ws.status), _stream())
+    _call("rb_topk_select", _I(DT[X.dtype]), _p(cv), _p(ci), plan, _p(X), _p(W), _I(B), _I(Ls), _I(D), _I(X.stride(0)),
+          _I(W.stride(0)), _I(k), _p(vals), _p(idx), _stream())
+    return vals, idx
 
 
 def xfc_topk(xfc, X, k):
-    """Local top-k of ``X Wᵀ`` over this rank's shard.  ``k <= 8`` (evaluation during training uses 5): fused into
-    the GEMM epilogue (:func:`xfc_topk8`).  Larger ``k`` (100 for the final evaluation): per label chunk, the tcgen05
+    """Local top-k of ``X Wᵀ`` over this rank's shard.  Up to ``rb_topk_max_k()`` (256; evaluation uses 5 during training
+    and 100 at the end): fused into the GEMM epilogue (:func:`xfc_topk8`).  Larger ``k``: per label chunk, the tcgen05
     logits GEMM writes fp32 logits batch-major into an L2-sized buffer and a radix-select kernel extracts each
     row's k best; the per-chunk candidates (k each) are merged at the end."""
     B, D = X.shape
     k_eff = min(k, xfc.Ls)
-    if k_eff <= 8 and D % 64 == 0 and os.environ.get("RENEE_B200_FUSED_TOPK", "1") != "0":
+    if 0 < k_eff <= lib().rb_topk_max_k() and B > 0 and D % 64 == 0 and os.environ.get("RENEE_B200_FUSED_TOPK", "1") != "0":
         return xfc_topk8(xfc.W, X, k_eff)
     chunk = min(xfc.chunk, max(128, (32 << 20) // (4 * B) // 128 * 128))
     ldZ = (min(chunk, xfc.Ls) + 7) // 8 * 8
