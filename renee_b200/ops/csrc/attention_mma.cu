@@ -1,5 +1,6 @@
-// Register-resident self-attention forward/backward for 16-bit activations, head dim 64, S <= 512
-// (one CTA per (batch, head) up to 128 tokens; blocked kernels, further down, for 129..512).
+// Register-resident self-attention forward/backward for 16-bit activations, head dim 64 (S <= 512) or 32 (S <= 128):
+// one CTA per (batch, head) up to 256 tokens, with score rows in registers up to 64 (forward: 128) and key blocks beyond;
+// streaming kernels, further down, for 257..512.
 // Same fusion and interface as attention_tc.cu (bias add, scale, key-padding mask, softmax, counter-based
 // attention dropout, head split/merge addressing, q/k/v bias gradients), organised so that the score
 // matrix never touches shared memory:
@@ -105,8 +106,9 @@ __device__ __forceinline__ float quad_max(float v) {
 // acc[j] (j = 8-wide tile of columns) += A(16 rows r0.. of `a`, all HD columns) * B^T, B = SP rows of `bsm`:
 // the shape of Q K^T and of dO V^T.  Both operands are [row][RP] tiles; only the first `lim` rows of B exist (in all
 // of these routines lim is a multiple of 16 and the same in every lane).
-template <typename T, int SP>
+template <typename T, int SP, int HD = amma::HD>
 __device__ __forceinline__ void rows_times_transposed(float (&acc)[SP / 8][4], const T* a, const T* bsm, int r0, int lane, int lim) {
+  constexpr int RP = HD + 8;
   uint32_t af[HD / 16][4];
 #pragma unroll
   for (int kk = 0; kk < HD / 16; ++kk)
@@ -126,8 +128,9 @@ __device__ __forceinline__ void rows_times_transposed(float (&acc)[SP / 8][4], c
 
 // out[jd] (jd = 8-wide tile of the HD columns) += A * B for a 16 x SP A held as packed fragments
 // (afr[kq] = the 16 x 16 block of columns 16 kq..) and B = the SP rows of the [row][RP] tile `bsm`.
-template <typename T, int SP>
+template <typename T, int SP, int HD = amma::HD>
 __device__ __forceinline__ void frag_times_rows(float (&out)[HD / 8][4], const uint32_t (&afr)[SP / 16][4], const T* bsm, int lane, int lim) {
+  constexpr int RP = HD + 8;
 #pragma unroll
   for (int kq = 0; kq < SP / 16; ++kq) {
     if (16 * kq >= lim) continue;
@@ -142,9 +145,10 @@ __device__ __forceinline__ void frag_times_rows(float (&out)[HD / 8][4], const u
 }
 
 // out[jd] += A^T * B where A is the [SP][PP] tile `asm_` (rows = reduction index) restricted to its 16 columns
-// c0.., and B = the SP rows of the [row][RP] tile `bsm`: the shape of dS^T Q and of P~^T dO.
-template <typename T, int SP>
-__device__ __forceinline__ void transposed_times_rows(float (&out)[HD / 8][4], const T* asm_, int PP, int c0, const T* bsm, int lane, int lim) {
+// c0.., and B = the SP rows of the [row][RP] tile `bsm` (its first 8 NJ columns): the shape of dS^T Q and of P~^T dO.
+template <typename T, int SP, int HD = amma::HD, int NJ = HD / 8>
+__device__ __forceinline__ void transposed_times_rows(float (&out)[NJ][4], const T* asm_, int PP, int c0, const T* bsm, int lane, int lim) {
+  constexpr int RP = HD + 8;
 #pragma unroll
   for (int kq = 0; kq < SP / 16; ++kq) {
     if (16 * kq >= lim) continue;
@@ -152,7 +156,7 @@ __device__ __forceinline__ void transposed_times_rows(float (&out)[HD / 8][4], c
     const int mi = lane >> 3;
     ldsm4_t(af, asm_ + (16 * kq + (lane & 7) + (mi >> 1) * 8) * PP + c0 + (mi & 1) * 8);
 #pragma unroll
-    for (int jd = 0; jd < HD / 8; jd += 2) {
+    for (int jd = 0; jd < NJ; jd += 2) {
       uint32_t bf[4];
       ldsm4_t(bf, bsm + (16 * kq + (lane & 7) + ((lane >> 3) & 1) * 8) * RP + 8 * jd + (lane >> 4) * 8);
       mma16816<T>(out[jd], af, bf[0], bf[1]);
@@ -161,16 +165,16 @@ __device__ __forceinline__ void transposed_times_rows(float (&out)[HD / 8][4], c
   }
 }
 
-// Writes the warp's 16 x HD accumulator tile to the global rows row_lo / row_hi (this lane's two rows; negative: none)
+// Writes the warp's 16 x 8 NJ accumulator tile to the global rows row_lo / row_hi (this lane's two rows; negative: none)
 // of stride ld and,
-// when col_sums != nullptr, adds the column sums of the rounded values to col_sums[0..HD) in shared memory.
-template <typename T>
-__device__ __forceinline__ void write_rows(const float (&out)[HD / 8][4], T* dst, int ld, int row_lo, int row_hi, int lane,
+// when col_sums != nullptr, adds the column sums of the rounded values to col_sums[0..8 NJ) in shared memory.
+template <typename T, int NJ>
+__device__ __forceinline__ void write_rows(const float (&out)[NJ][4], T* dst, int ld, int row_lo, int row_hi, int lane,
                                            float* col_sums) {
   const int g = lane >> 2, t = lane & 3;
   const bool v0 = row_lo >= 0, v1 = row_hi >= 0;
 #pragma unroll
-  for (int jd = 0; jd < HD / 8; ++jd) {
+  for (int jd = 0; jd < NJ; ++jd) {
     const uint32_t lo = Pack<T>::pack(out[jd][0], out[jd][1]);
     const uint32_t hi = Pack<T>::pack(out[jd][2], out[jd][3]);
     if (v0) *reinterpret_cast<uint32_t*>(dst + (size_t)row_lo * ld + 8 * jd + 2 * t) = lo;
@@ -194,23 +198,23 @@ __device__ __forceinline__ void write_rows(const float (&out)[HD / 8][4], T* dst
 
 // Stages (q + bq, k + bk, v + bv [, dO]) of one (batch, head) as [SP][RP] tiles; rows of tokens that do not
 // exist are zero, rows >= lim are left alone.
-// The CTA has SP * 2 threads and the tiles SP * 8 segments of 8 columns, so a thread owns the same 8 columns of
-// four rows: all of its global loads are issued before the first one is used.
-template <typename T, int SP, bool WITH_DO>
+// The CTA has SP * 2 threads and the tiles SP * HD / 8 segments of 8 columns, so a thread owns the same 8 columns of
+// HD / 16 rows: all of its global loads are issued before the first one is used.
+template <typename T, int SP, int HD, bool WITH_DO>
 __device__ __forceinline__ void stage_operands(const T* __restrict__ qkv, const T* __restrict__ bqkv, const T* __restrict__ dctx,
                                                T* sQ, T* sK, T* sV, T* sDO, const Tok& tk, int b, int h, int S, int H, int len,
                                                int lim) {
-  constexpr int ROWS_PER_PASS = SP * 2 / 8;
-  const int d = (threadIdx.x & 7) * 8, s0 = threadIdx.x >> 3;
-  Raw8<T> rq[4], rk[4], rv[4], rg[4];
-  int row[4];
+  constexpr int RP = HD + 8, SEGS = HD / 8, ROWS_PER_PASS = SP * 2 / SEGS, NIT = HD / 16;
+  const int d = (threadIdx.x % SEGS) * 8, s0 = threadIdx.x / SEGS;
+  Raw8<T> rq[NIT], rk[NIT], rv[NIT], rg[NIT];
+  int row[NIT];
 #pragma unroll
-  for (int it = 0; it < 4; ++it) {
+  for (int it = 0; it < NIT; ++it) {
     const int s = s0 + it * ROWS_PER_PASS;
     row[it] = s < len ? seq_row(tk, b, S, s) : -1;
   }
 #pragma unroll
-  for (int it = 0; it < 4; ++it) {
+  for (int it = 0; it < NIT; ++it) {
     if (row[it] >= 0) {
       const size_t base = (size_t)row[it] * 3 * H + h * HD + d;
       rq[it] = load_raw8(qkv + base); rk[it] = load_raw8(qkv + base + H); rv[it] = load_raw8(qkv + base + 2 * H);
@@ -220,7 +224,7 @@ __device__ __forceinline__ void stage_operands(const T* __restrict__ qkv, const 
   float bq[8], bk[8], bv[8];
   load8(bqkv + h * HD + d, bq); load8(bqkv + H + h * HD + d, bk); load8(bqkv + 2 * H + h * HD + d, bv);
 #pragma unroll
-  for (int it = 0; it < 4; ++it) {
+  for (int it = 0; it < NIT; ++it) {
     const int s = s0 + it * ROWS_PER_PASS;
     if (s >= lim) continue;
     float q[8], k[8], v[8];
@@ -238,13 +242,14 @@ __device__ __forceinline__ void stage_operands(const T* __restrict__ qkv, const 
   }
 }
 
-template <typename T, int SP>
+template <typename T, int SP, int HD>
 __global__ void __launch_bounds__(SP * 2, SP == 128 ? 2 : 1) attention_fwd_mma_kernel(
     const T* __restrict__ qkv, const T* __restrict__ bqkv, const int* __restrict__ mask, T* __restrict__ ctx,
-    T* __restrict__ probs, int S, int H, int nh, float p, const int* __restrict__ seed_ptr, uint32_t stream, const Tok tk) {
+    T* __restrict__ probs, int S, int H, int nh, float p, const int* __restrict__ seed_ptr, uint32_t stream, const Tok tk, int len_lo) {
   rb::grid_dep_wait();        // launched with launch_pdl: nothing above touches global memory
   rb::grid_dep_launch();      // the kernel that follows may start its set-up; it waits for this grid before reading
   extern __shared__ __align__(128) uint8_t sm_raw[];
+  constexpr int RP = HD + 8;
   T* sQ = reinterpret_cast<T*>(sm_raw);
   T* sK = sQ + SP * RP;
   T* sV = sK + SP * RP;
@@ -256,21 +261,22 @@ __global__ void __launch_bounds__(SP * 2, SP == 128 ? 2 : 1) attention_fwd_mma_k
   const uint32_t seed = p > 0.f ? (uint32_t)(*seed_ptr) : 0u;
   const float inv_keep = p > 0.f ? 1.f / (1.f - p) : 1.f;
   const float scale = rsqrtf((float)HD);
+  if (tk.slot != nullptr && b == (int)gridDim.y - 1) clear_zero_rows<T>(tk, ctx, H, h * HD, HD);
   const int len = seq_len(tk, b, S), lim = (len + 15) & ~15;
+  if (len > SP || len <= len_lo) return;       // another launch serves this length
   for (int j = threadIdx.x; j < SP; j += blockDim.x) {
     const int row = j < len ? seq_row(tk, b, S, j) : -1;
     sRow[j] = row;
     sCode[j] = row >= 0 ? (mask[b * S + j] != 0 ? 1 : 2) : 0;
   }
-  stage_operands<T, SP, false>(qkv, bqkv, nullptr, sQ, sK, sV, nullptr, tk, b, h, S, H, len, lim);
-  if (tk.slot != nullptr && b == (int)gridDim.y - 1) clear_zero_rows<T>(tk, ctx, H, h * HD, HD);
+  stage_operands<T, SP, HD, false>(qkv, bqkv, nullptr, sQ, sK, sV, nullptr, tk, b, h, S, H, len, lim);
   __syncthreads();
   const int r0 = warp * 16;
   if (r0 >= lim) return;
   float acc[SP / 8][4];
 #pragma unroll
   for (int j = 0; j < SP / 8; ++j) { acc[j][0] = 0.f; acc[j][1] = 0.f; acc[j][2] = 0.f; acc[j][3] = 0.f; }
-  rows_times_transposed<T, SP>(acc, sQ, sK, r0, lane, lim);
+  rows_times_transposed<T, SP, HD>(acc, sQ, sK, r0, lane, lim);
   // softmax of rows r0 + g (elements 0, 1 of each tile) and r0 + g + 8 (elements 2, 3)
   float mx0 = -1e30f, mx1 = -1e30f;
 #pragma unroll
@@ -343,18 +349,19 @@ __global__ void __launch_bounds__(SP * 2, SP == 128 ? 2 : 1) attention_fwd_mma_k
   float out[HD / 8][4];
 #pragma unroll
   for (int jd = 0; jd < HD / 8; ++jd) { out[jd][0] = 0.f; out[jd][1] = 0.f; out[jd][2] = 0.f; out[jd][3] = 0.f; }
-  frag_times_rows<T, SP>(out, pf, sV, lane, lim);
+  frag_times_rows<T, SP, HD>(out, pf, sV, lane, lim);
   write_rows<T>(out, ctx + h * HD, H, row0, row1, lane, nullptr);
 }
 
-template <typename T, int SP>
+template <typename T, int SP, int HD>
 __global__ void __launch_bounds__(SP * 2) attention_bwd_mma_kernel(
     const T* __restrict__ dctx, const T* __restrict__ qkv, const T* __restrict__ bqkv, const T* __restrict__ probs,
     T* __restrict__ dqkv, int S, int H, int nh, float p, const int* __restrict__ seed_ptr, uint32_t stream,
-    float* __restrict__ bias_acc, const Tok tk) {
+    float* __restrict__ bias_acc, const Tok tk, int len_lo) {
   rb::grid_dep_wait();
   rb::grid_dep_launch();
   extern __shared__ __align__(128) uint8_t sm_raw[];
+  constexpr int RP = HD + 8;
   constexpr int PP = SP + 8;   // 4-byte fragment stores of a quad group land on distinct banks
   T* sQ = reinterpret_cast<T*>(sm_raw);
   T* sK = sQ + SP * RP;
@@ -372,11 +379,12 @@ __global__ void __launch_bounds__(SP * 2) attention_bwd_mma_kernel(
   const float scale = rsqrtf((float)HD);
   if (bias_acc != nullptr)
     for (int i = threadIdx.x; i < 3 * HD; i += blockDim.x) sBias[i] = 0.f;
-  const int len = seq_len(tk, b, S), lim = (len + 15) & ~15;
-  for (int j = threadIdx.x; j < SP; j += blockDim.x) sRow[j] = j < len ? seq_row(tk, b, S, j) : -1;
-  stage_operands<T, SP, true>(qkv, bqkv, dctx, sQ, sK, sV, sDO, tk, b, h, S, H, len, lim);
   if (tk.slot != nullptr && b == (int)gridDim.y - 1)
     for (int w = 0; w < 3; ++w) clear_zero_rows<T>(tk, dqkv, 3 * H, w * H + h * HD, HD);
+  const int len = seq_len(tk, b, S), lim = (len + 15) & ~15;
+  if (len > SP || len <= len_lo) return;       // another launch serves this length
+  for (int j = threadIdx.x; j < SP; j += blockDim.x) sRow[j] = j < len ? seq_row(tk, b, S, j) : -1;
+  stage_operands<T, SP, HD, true>(qkv, bqkv, dctx, sQ, sK, sV, sDO, tk, b, h, S, H, len, lim);
   __syncthreads();
   const int r0 = warp * 16;
   const int row0 = sRow[r0 + g], row1 = sRow[r0 + g + 8];
@@ -385,7 +393,7 @@ __global__ void __launch_bounds__(SP * 2) attention_bwd_mma_kernel(
     float acc[SP / 8][4];
 #pragma unroll
     for (int j = 0; j < SP / 8; ++j) { acc[j][0] = 0.f; acc[j][1] = 0.f; acc[j][2] = 0.f; acc[j][3] = 0.f; }
-    rows_times_transposed<T, SP>(acc, sDO, sV, r0, lane, lim);
+    rows_times_transposed<T, SP, HD>(acc, sDO, sV, r0, lane, lim);
     const int i0 = r0 + g, i1 = r0 + g + 8;
     const size_t prow0 = ((size_t)(b * nh + h) * S + i0) * S, prow1 = ((size_t)(b * nh + h) * S + i1) * S;
     const bool pair_load = (S & 1) == 0;
@@ -439,7 +447,7 @@ __global__ void __launch_bounds__(SP * 2) attention_bwd_mma_kernel(
     float out[HD / 8][4];
 #pragma unroll
     for (int jd = 0; jd < HD / 8; ++jd) { out[jd][0] = 0.f; out[jd][1] = 0.f; out[jd][2] = 0.f; out[jd][3] = 0.f; }
-    frag_times_rows<T, SP>(out, dsf, sK, lane, lim);
+    frag_times_rows<T, SP, HD>(out, dsf, sK, lane, lim);
     write_rows<T>(out, dqkv + h * HD, 3 * H, row0, row1, lane,
                   bias_acc != nullptr ? sBias : nullptr);
   }
@@ -449,12 +457,12 @@ __global__ void __launch_bounds__(SP * 2) attention_bwd_mma_kernel(
     float out[HD / 8][4];
 #pragma unroll
     for (int jd = 0; jd < HD / 8; ++jd) { out[jd][0] = 0.f; out[jd][1] = 0.f; out[jd][2] = 0.f; out[jd][3] = 0.f; }
-    transposed_times_rows<T, SP>(out, sDS, PP, r0, sQ, lane, lim);
+    transposed_times_rows<T, SP, HD>(out, sDS, PP, r0, sQ, lane, lim);
     write_rows<T>(out, dqkv + H + h * HD, 3 * H, row0, row1, lane,
                   bias_acc != nullptr ? sBias + HD : nullptr);
 #pragma unroll
     for (int jd = 0; jd < HD / 8; ++jd) { out[jd][0] = 0.f; out[jd][1] = 0.f; out[jd][2] = 0.f; out[jd][3] = 0.f; }
-    transposed_times_rows<T, SP>(out, sW, PP, r0, sDO, lane, lim);
+    transposed_times_rows<T, SP, HD>(out, sW, PP, r0, sDO, lane, lim);
     write_rows<T>(out, dqkv + 2 * H + h * HD, 3 * H, row0, row1, lane,
                   bias_acc != nullptr ? sBias + 2 * HD : nullptr);
   }
@@ -468,37 +476,343 @@ __global__ void __launch_bounds__(SP * 2) attention_bwd_mma_kernel(
   }
 }
 
-template <int SP> constexpr size_t fwd_smem(size_t esz) { return (size_t)3 * SP * RP * esz + SP * sizeof(int) + SP; }
-template <int SP> constexpr size_t bwd_smem(size_t esz) {
-  return (size_t)4 * SP * RP * esz + (size_t)2 * SP * (SP + 8) * esz + 3 * HD * sizeof(float) + SP * sizeof(int);
+
+// two consecutive elements idx, idx + 1 of a [.., S] row; ok0 / ok1 say which exist; `pair` = 4-byte access allowed
+template <typename T>
+__device__ __forceinline__ float2 load_pair(const T* __restrict__ base, size_t idx, bool ok0, bool ok1, bool pair) {
+  float2 r = make_float2(0.f, 0.f);
+  if (ok0) {
+    if (pair) r = Pack<T>::unpack(*reinterpret_cast<const uint32_t*>(base + idx));
+    else { r.x = to_f(base[idx]); if (ok1) r.y = to_f(base[idx + 1]); }
+  }
+  return r;
+}
+template <typename T>
+__device__ __forceinline__ void store_pair(T* __restrict__ base, size_t idx, uint32_t u, bool ok0, bool ok1, bool pair) {
+  if (ok0) {
+    if (pair) *reinterpret_cast<uint32_t*>(base + idx) = u;
+    else {
+      const T* e = reinterpret_cast<const T*>(&u);
+      base[idx] = e[0];
+      if (ok1) base[idx + 1] = e[1];
+    }
+  }
 }
 
-template <typename T, int SP>
+// ------------------------------------------------------------------------------------ sequences of 65..256 tokens
+// One CTA of SP / 16 warps per (batch, head), SP = 128 or 256, operands staged once.  What keeps the scores in
+// registers at 32..64 tokens does not scale: a warp's 16 x SP score rows and, in the backward, two [SP][SP] tiles in
+// shared memory allowed one CTA of 8 warps per SM at 128 tokens and forced two streaming kernels beyond.  So both passes
+// walk the keys in blocks of KB = 64 over the resident operands: 128 registers per thread, and the dS and P~ tiles shrink
+// to [SP][KB] (112 KB per CTA at SP = 128: two per SM; 218 KB at SP = 256).
+// Measured inside the 64 x 256 training step (12 heads, lengths 64..256): streaming kernels 520 (forward) + 842 (dQ) +
+// 304 us (dK, dV) per layer padded; now, packed, 120 and 264 us.  Step 11.36 (packed, streaming kernels) -> 7.50 ms.
+//   forward   pass 1: running row maximum and sum; pass 2: probabilities (stored for the backward), dropout, O += P~ V
+//   backward  pass 1: row sums of dP * P, keeping the dropout decisions as one bit each; pass 2, per key block: dS and P~
+//             to shared memory, dQ += dS K, then the block's dK = dS^T Q and dV = P~^T dO, spread over all warps.
+constexpr int KB = 64;
+
+template <typename T, int SP, int HD>
+__global__ void __launch_bounds__(SP * 2, SP == 128 ? 2 : 1) attention_fwd_blk_kernel(
+    const T* __restrict__ qkv, const T* __restrict__ bqkv, const int* __restrict__ mask, T* __restrict__ ctx,
+    T* __restrict__ probs, int S, int H, int nh, float p, const int* __restrict__ seed_ptr, uint32_t stream, const Tok tk,
+    int len_lo) {
+  rb::grid_dep_wait();
+  rb::grid_dep_launch();
+  extern __shared__ __align__(128) uint8_t sm_raw[];
+  constexpr int RP = HD + 8;
+  T* sQ = reinterpret_cast<T*>(sm_raw);
+  T* sK = sQ + SP * RP;
+  T* sV = sK + SP * RP;
+  int* sRow = reinterpret_cast<int*>(sV + SP * RP);
+  uint8_t* sCode = reinterpret_cast<uint8_t*>(sRow + SP);      // per key: 0 = no such token, 1 = attend, 2 = masked
+  const int h = blockIdx.x, b = blockIdx.y;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int g = lane >> 2, t = lane & 3;
+  const uint32_t seed = p > 0.f ? (uint32_t)(*seed_ptr) : 0u;
+  const float inv_keep = p > 0.f ? 1.f / (1.f - p) : 1.f;
+  const float scale = rsqrtf((float)HD);
+  if (tk.slot != nullptr && b == (int)gridDim.y - 1) clear_zero_rows<T>(tk, ctx, H, h * HD, HD);
+  const int len = seq_len(tk, b, S), lim = (len + 15) & ~15;
+  if (len > SP || len <= len_lo) return;
+  for (int j = threadIdx.x; j < SP; j += blockDim.x) {
+    const int row = j < len ? seq_row(tk, b, S, j) : -1;
+    sRow[j] = row;
+    sCode[j] = row >= 0 ? (mask[b * S + j] != 0 ? 1 : 2) : 0;
+  }
+  stage_operands<T, SP, HD, false>(qkv, bqkv, nullptr, sQ, sK, sV, nullptr, tk, b, h, S, H, len, lim);
+  __syncthreads();
+  const int r0 = warp * 16;
+  if (r0 >= lim) return;
+  float m0 = -1e30f, m1 = -1e30f, l0 = 0.f, l1 = 0.f;
+#pragma unroll 1
+  for (int k0 = 0; k0 < lim; k0 += KB) {
+    float acc[KB / 8][4];
+#pragma unroll
+    for (int j = 0; j < KB / 8; ++j) { acc[j][0] = 0.f; acc[j][1] = 0.f; acc[j][2] = 0.f; acc[j][3] = 0.f; }
+    rows_times_transposed<T, KB, HD>(acc, sQ, sK + k0 * RP, r0, lane, lim - k0);
+    float b0 = -1e30f, b1 = -1e30f;
+#pragma unroll
+    for (int j = 0; j < KB / 8; ++j) {
+      if (k0 + 8 * j >= lim) continue;
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const bool on = sCode[k0 + 8 * j + 2 * t + e] == 1;
+        acc[j][e] = on ? acc[j][e] * scale : -1e30f;
+        acc[j][2 + e] = on ? acc[j][2 + e] * scale : -1e30f;
+        b0 = fmaxf(b0, acc[j][e]);
+        b1 = fmaxf(b1, acc[j][2 + e]);
+      }
+    }
+    const float n0 = fmaxf(m0, quad_max(b0)), n1 = fmaxf(m1, quad_max(b1));
+    float s0 = 0.f, s1 = 0.f;
+#pragma unroll
+    for (int j = 0; j < KB / 8; ++j) {
+      if (k0 + 8 * j >= lim) continue;
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        if (sCode[k0 + 8 * j + 2 * t + e] != 0) { s0 += __expf(acc[j][e] - n0); s1 += __expf(acc[j][2 + e] - n1); }
+      }
+    }
+    l0 = l0 * __expf(m0 - n0) + s0;
+    l1 = l1 * __expf(m1 - n1) + s1;
+    m0 = n0; m1 = n1;
+  }
+  l0 = quad_sum(l0); l1 = quad_sum(l1);
+  const int i0 = r0 + g, i1 = r0 + g + 8;
+  const int row0 = sRow[i0], row1 = sRow[i1];
+  const float inv0 = row0 >= 0 ? 1.f / l0 : 0.f, inv1 = row1 >= 0 ? 1.f / l1 : 0.f;
+  const size_t prow0 = ((size_t)(b * nh + h) * S + i0) * S, prow1 = ((size_t)(b * nh + h) * S + i1) * S;
+  const bool pair = (S & 1) == 0;          // then every (row, even column) element is 4-byte aligned
+  float out[HD / 8][4];
+#pragma unroll
+  for (int jd = 0; jd < HD / 8; ++jd) { out[jd][0] = 0.f; out[jd][1] = 0.f; out[jd][2] = 0.f; out[jd][3] = 0.f; }
+#pragma unroll 1
+  for (int k0 = 0; k0 < lim; k0 += KB) {
+    float acc[KB / 8][4];
+#pragma unroll
+    for (int j = 0; j < KB / 8; ++j) { acc[j][0] = 0.f; acc[j][1] = 0.f; acc[j][2] = 0.f; acc[j][3] = 0.f; }
+    rows_times_transposed<T, KB, HD>(acc, sQ, sK + k0 * RP, r0, lane, lim - k0);
+    uint32_t pf[KB / 16][4];
+#pragma unroll
+    for (int j = 0; j < KB / 8; ++j) {
+      if (k0 + 8 * j >= lim) continue;
+      const int key = k0 + 8 * j + 2 * t;
+      const int c0 = sCode[key], c1 = sCode[key + 1];
+      const float e00 = c0 != 0 ? __expf((c0 == 1 ? acc[j][0] * scale : -1e30f) - m0) * inv0 : 0.f;
+      const float e01 = c1 != 0 ? __expf((c1 == 1 ? acc[j][1] * scale : -1e30f) - m0) * inv0 : 0.f;
+      const float e10 = c0 != 0 ? __expf((c0 == 1 ? acc[j][2] * scale : -1e30f) - m1) * inv1 : 0.f;
+      const float e11 = c1 != 0 ? __expf((c1 == 1 ? acc[j][3] * scale : -1e30f) - m1) * inv1 : 0.f;
+      // the stored probabilities are the rounded ones, as in the unfused op
+      const uint32_t u0 = Pack<T>::pack(e00, e01), u1 = Pack<T>::pack(e10, e11);
+      store_pair<T>(probs, prow0 + key, u0, row0 >= 0 && key < S, key + 1 < S, pair);
+      store_pair<T>(probs, prow1 + key, u1, row1 >= 0 && key < S, key + 1 < S, pair);
+      float2 q0 = Pack<T>::unpack(u0), q1 = Pack<T>::unpack(u1);
+      if (p > 0.f) {
+        q0.x = keep(seed, stream, (uint32_t)(prow0 + key), p) ? q0.x * inv_keep : 0.f;
+        q0.y = keep(seed, stream, (uint32_t)(prow0 + key + 1), p) ? q0.y * inv_keep : 0.f;
+        q1.x = keep(seed, stream, (uint32_t)(prow1 + key), p) ? q1.x * inv_keep : 0.f;
+        q1.y = keep(seed, stream, (uint32_t)(prow1 + key + 1), p) ? q1.y * inv_keep : 0.f;
+      }
+      pf[j >> 1][(j & 1) * 2 + 0] = Pack<T>::pack(q0.x, q0.y);
+      pf[j >> 1][(j & 1) * 2 + 1] = Pack<T>::pack(q1.x, q1.y);
+    }
+    frag_times_rows<T, KB, HD>(out, pf, sV + k0 * RP, lane, lim - k0);
+  }
+  write_rows<T>(out, ctx + h * HD, H, row0, row1, lane, nullptr);
+}
+
+template <typename T, int SP, int HD>
+__global__ void __launch_bounds__(SP * 2, SP == 128 ? 2 : 1) attention_bwd_blk_kernel(
+    const T* __restrict__ dctx, const T* __restrict__ qkv, const T* __restrict__ bqkv, const T* __restrict__ probs,
+    T* __restrict__ dqkv, int S, int H, int nh, float p, const int* __restrict__ seed_ptr, uint32_t stream,
+    float* __restrict__ bias_acc, const Tok tk, int len_lo) {
+  rb::grid_dep_wait();
+  rb::grid_dep_launch();
+  extern __shared__ __align__(128) uint8_t sm_raw[];
+  constexpr int RP = HD + 8, PB = KB + 8;
+  constexpr int NW = SP / 16;                      // warps
+  constexpr int SLICES = NW / 8;                   // column slices of a dK / dV tile: 4 key tiles x 2 x SLICES = NW tasks
+  constexpr int NJ = HD / 8 / SLICES;
+  T* sQ = reinterpret_cast<T*>(sm_raw);
+  T* sK = sQ + SP * RP;
+  T* sV = sK + SP * RP;
+  T* sDO = sV + SP * RP;
+  T* sDS = sDO + SP * RP;                          // [query][key of the block] dS
+  T* sW = sDS + SP * PB;                           // [query][key of the block] dropped-out probabilities P~
+  float* sBias = reinterpret_cast<float*>(sW + SP * PB);   // [3][HD] column sums of dQ, dK, dV
+  int* sRow = reinterpret_cast<int*>(sBias + 3 * HD);
+  const int h = blockIdx.x, b = blockIdx.y;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int g = lane >> 2, t = lane & 3;
+  const uint32_t seed = p > 0.f ? (uint32_t)(*seed_ptr) : 0u;
+  const float inv_keep = p > 0.f ? 1.f / (1.f - p) : 1.f;
+  const float scale = rsqrtf((float)HD);
+  if (tk.slot != nullptr && b == (int)gridDim.y - 1)
+    for (int w = 0; w < 3; ++w) clear_zero_rows<T>(tk, dqkv, 3 * H, w * H + h * HD, HD);
+  const int len = seq_len(tk, b, S), lim = (len + 15) & ~15;
+  if (len > SP || len <= len_lo) return;
+  if (bias_acc != nullptr)
+    for (int i = threadIdx.x; i < 3 * HD; i += blockDim.x) sBias[i] = 0.f;
+  for (int j = threadIdx.x; j < SP; j += blockDim.x) sRow[j] = j < len ? seq_row(tk, b, S, j) : -1;
+  stage_operands<T, SP, HD, true>(qkv, bqkv, dctx, sQ, sK, sV, sDO, tk, b, h, S, H, len, lim);
+  __syncthreads();
+  const int r0 = warp * 16, i0 = r0 + g, i1 = r0 + g + 8;
+  const bool active = r0 < lim;                    // this warp's 16 query rows exist
+  const int row0 = sRow[i0], row1 = sRow[i1];
+  const size_t prow0 = ((size_t)(b * nh + h) * S + i0) * S, prow1 = ((size_t)(b * nh + h) * S + i1) * S;
+  const bool pair = (S & 1) == 0;
+  uint32_t kept[SP / KB];                          // dropout decisions: bit 4 j + e of block k is element e of tile j
+  float dot0 = 0.f, dot1 = 0.f;
+  if (active) {
+#pragma unroll
+    for (int kb = 0; kb < SP / KB; ++kb) {
+      const int k0 = kb * KB;
+      kept[kb] = 0xffffffffu;
+      if (k0 >= lim) continue;
+      float acc[KB / 8][4];
+#pragma unroll
+      for (int j = 0; j < KB / 8; ++j) { acc[j][0] = 0.f; acc[j][1] = 0.f; acc[j][2] = 0.f; acc[j][3] = 0.f; }
+      rows_times_transposed<T, KB, HD>(acc, sDO, sV + k0 * RP, r0, lane, lim - k0);
+      uint32_t bits = 0u;
+#pragma unroll
+      for (int j = 0; j < KB / 8; ++j) {
+        if (k0 + 8 * j >= lim) continue;
+        const int key = k0 + 8 * j + 2 * t;
+        const float2 pr0 = load_pair<T>(probs, prow0 + key, row0 >= 0 && key < S, key + 1 < S, pair);
+        const float2 pr1 = load_pair<T>(probs, prow1 + key, row1 >= 0 && key < S, key + 1 < S, pair);
+        float m00 = 1.f, m01 = 1.f, m10 = 1.f, m11 = 1.f;
+        if (p > 0.f) {
+          const bool a = keep(seed, stream, (uint32_t)(prow0 + key), p), c = keep(seed, stream, (uint32_t)(prow0 + key + 1), p);
+          const bool d = keep(seed, stream, (uint32_t)(prow1 + key), p), f = keep(seed, stream, (uint32_t)(prow1 + key + 1), p);
+          bits |= ((a ? 1u : 0u) | (c ? 2u : 0u) | (d ? 4u : 0u) | (f ? 8u : 0u)) << (4 * j);
+          m00 = a ? inv_keep : 0.f; m01 = c ? inv_keep : 0.f; m10 = d ? inv_keep : 0.f; m11 = f ? inv_keep : 0.f;
+        }
+        dot0 += acc[j][0] * m00 * pr0.x + acc[j][1] * m01 * pr0.y;
+        dot1 += acc[j][2] * m10 * pr1.x + acc[j][3] * m11 * pr1.y;
+      }
+      if (p > 0.f) kept[kb] = bits;
+    }
+    dot0 = quad_sum(dot0); dot1 = quad_sum(dot1);
+  }
+  float dq[HD / 8][4];
+#pragma unroll
+  for (int jd = 0; jd < HD / 8; ++jd) { dq[jd][0] = 0.f; dq[jd][1] = 0.f; dq[jd][2] = 0.f; dq[jd][3] = 0.f; }
+#pragma unroll
+  for (int kb = 0; kb < SP / KB; ++kb) {
+    const int k0 = kb * KB;
+    if (k0 >= lim) break;                          // the same answer in every thread
+    if (active) {
+      float acc[KB / 8][4];
+#pragma unroll
+      for (int j = 0; j < KB / 8; ++j) { acc[j][0] = 0.f; acc[j][1] = 0.f; acc[j][2] = 0.f; acc[j][3] = 0.f; }
+      rows_times_transposed<T, KB, HD>(acc, sDO, sV + k0 * RP, r0, lane, lim - k0);
+      uint32_t dsf[KB / 16][4];                    // dS as the A operand of dQ += dS K
+#pragma unroll
+      for (int j = 0; j < KB / 8; ++j) {
+        if (k0 + 8 * j >= lim) continue;
+        const int key = k0 + 8 * j + 2 * t;
+        const float2 pr0 = load_pair<T>(probs, prow0 + key, row0 >= 0 && key < S, key + 1 < S, pair);
+        const float2 pr1 = load_pair<T>(probs, prow1 + key, row1 >= 0 && key < S, key + 1 < S, pair);
+        const uint32_t bits = kept[kb] >> (4 * j);
+        const float m00 = (bits & 1u) ? inv_keep : 0.f, m01 = (bits & 2u) ? inv_keep : 0.f;
+        const float m10 = (bits & 4u) ? inv_keep : 0.f, m11 = (bits & 8u) ? inv_keep : 0.f;
+        const uint32_t d0 = Pack<T>::pack(pr0.x * (acc[j][0] * m00 - dot0) * scale, pr0.y * (acc[j][1] * m01 - dot0) * scale);
+        const uint32_t d1 = Pack<T>::pack(pr1.x * (acc[j][2] * m10 - dot1) * scale, pr1.y * (acc[j][3] * m11 - dot1) * scale);
+        const int c = 8 * j + 2 * t;
+        *reinterpret_cast<uint32_t*>(sDS + i0 * PB + c) = d0;
+        *reinterpret_cast<uint32_t*>(sDS + i1 * PB + c) = d1;
+        *reinterpret_cast<uint32_t*>(sW + i0 * PB + c) = Pack<T>::pack(pr0.x * m00, pr0.y * m01);
+        *reinterpret_cast<uint32_t*>(sW + i1 * PB + c) = Pack<T>::pack(pr1.x * m10, pr1.y * m11);
+        dsf[j >> 1][(j & 1) * 2 + 0] = d0;
+        dsf[j >> 1][(j & 1) * 2 + 1] = d1;
+      }
+      frag_times_rows<T, KB, HD>(dq, dsf, sK + k0 * RP, lane, lim - k0);
+    }
+    __syncthreads();
+    {
+      // one 16-key tile of dK (even tasks) or dV (odd ones), or a column slice of it
+      const int kt = (warp >> 1) & 3, which = warp & 1, slice = warp >> 3;
+      const int key0 = k0 + 16 * kt;
+      if (key0 < lim) {
+        float out[NJ][4];
+#pragma unroll
+        for (int jd = 0; jd < NJ; ++jd) { out[jd][0] = 0.f; out[jd][1] = 0.f; out[jd][2] = 0.f; out[jd][3] = 0.f; }
+        const int c0 = slice * NJ * 8;
+        transposed_times_rows<T, SP, HD, NJ>(out, which == 0 ? sDS : sW, PB, 16 * kt, (which == 0 ? sQ : sDO) + c0, lane, lim);
+        write_rows<T>(out, dqkv + (1 + which) * H + h * HD + c0, 3 * H, sRow[key0 + g], sRow[key0 + g + 8], lane,
+                      bias_acc != nullptr ? sBias + (1 + which) * HD + c0 : nullptr);
+      }
+    }
+    __syncthreads();
+  }
+  if (active) write_rows<T>(dq, dqkv + h * HD, 3 * H, row0, row1, lane, bias_acc != nullptr ? sBias : nullptr);
+  if (bias_acc != nullptr) {
+    __syncthreads();
+    float* my_acc = bias_acc + (size_t)((blockIdx.y * gridDim.x + blockIdx.x) % 8) * 3 * H;
+    for (int i = threadIdx.x; i < 3 * HD; i += blockDim.x)
+      atomicAdd(my_acc + (i / HD) * H + h * HD + (i % HD), sBias[i]);
+  }
+}
+
+template <int SP, int HD> constexpr size_t fwd_smem(size_t esz) { return (size_t)3 * SP * (HD + 8) * esz + SP * sizeof(int) + SP; }
+template <int SP, int HD> constexpr size_t bwd_smem(size_t esz) {
+  return (size_t)4 * SP * (HD + 8) * esz + (size_t)2 * SP * ((SP > 64 ? KB : SP) + 8) * esz + 3 * HD * sizeof(float) + SP * sizeof(int);
+}
+
+// One launch of the kernels for sequences of len_lo + 1 .. SP tokens (a CTA whose sequence has another length exits).
+template <typename T, int SP, int HD>
 static int launch_fwd(const void* qkv, const void* bqkv, const int* mask, void* ctx, void* probs, int b, int S, int H,
-                      int nh, float p, const int* seed, unsigned stream_id, const Tok& tk, cudaStream_t st) {
-  auto k = attention_fwd_mma_kernel<T, SP>;
-  constexpr size_t smem = fwd_smem<SP>(sizeof(T));
-  if (smem > 48 * 1024 &&
-      cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return -5;
-  rb::launch_pdl(k, dim3(nh, b), dim3(SP * 2), smem, st, (const T*)qkv, (const T*)bqkv, mask, (T*)ctx, (T*)probs, S, H, nh, p, seed, stream_id, tk);
-  return 0;
+                      int nh, float p, const int* seed, unsigned stream_id, const Tok& tk, int len_lo, cudaStream_t st) {
+  constexpr size_t smem = fwd_smem<SP, HD>(sizeof(T));
+  const auto go = [&](auto k) -> int {
+    if (smem > 48 * 1024 && cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return -5;
+    rb::launch_pdl(k, dim3(nh, b), dim3(SP * 2), smem, st, (const T*)qkv, (const T*)bqkv, mask, (T*)ctx, (T*)probs, S, H, nh, p, seed, stream_id, tk, len_lo);
+    return 0;
+  };
+  if constexpr (SP > 128) return go(attention_fwd_blk_kernel<T, SP, HD>);
+  else return go(attention_fwd_mma_kernel<T, SP, HD>);
 }
 
-template <typename T, int SP>
+template <typename T, int SP, int HD>
 static int launch_bwd(const void* dctx, const void* qkv, const void* bqkv, const void* probs, void* dqkv, int b, int S,
-                      int H, int nh, float p, const int* seed, unsigned stream_id, float* bias_acc, const Tok& tk,
+                      int H, int nh, float p, const int* seed, unsigned stream_id, float* bias_acc, const Tok& tk, int len_lo,
                       cudaStream_t st) {
-  auto k = attention_bwd_mma_kernel<T, SP>;
-  constexpr size_t smem = bwd_smem<SP>(sizeof(T));
-  if (smem > 48 * 1024 &&
-      cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return -5;
-  rb::launch_pdl(k, dim3(nh, b), dim3(SP * 2), smem, st, (const T*)dctx, (const T*)qkv, (const T*)bqkv, (const T*)probs,
-                 (T*)dqkv, S, H, nh, p, seed, stream_id, bias_acc, tk);
-  return 0;
+  constexpr size_t smem = bwd_smem<SP, HD>(sizeof(T));
+  const auto go = [&](auto k) -> int {
+    if (smem > 48 * 1024 && cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return -5;
+    rb::launch_pdl(k, dim3(nh, b), dim3(SP * 2), smem, st, (const T*)dctx, (const T*)qkv, (const T*)bqkv, (const T*)probs,
+                   (T*)dqkv, S, H, nh, p, seed, stream_id, bias_acc, tk, len_lo);
+    return 0;
+  };
+  if constexpr (SP > 64) return go(attention_bwd_blk_kernel<T, SP, HD>);
+  else return go(attention_bwd_mma_kernel<T, SP, HD>);
 }
 
+// Tile sizes by sequence length.  All sequences of a padded batch have length S: one launch of the smallest tile that
+// holds it.  Packed sequences have their own lengths: those of at most half the tile go to the next smaller one in a
+// launch of their own, where twice as many fit an SM.
+#define RB_ATT_LAUNCH(T, HD, FN, S, packed, ...)                                                                    \
+  [&]() -> int {                                                                                                    \
+    if ((S) <= 16) return FN<T, 16, HD>(__VA_ARGS__, 0, st);                                                        \
+    if ((S) <= 32) return FN<T, 32, HD>(__VA_ARGS__, 0, st);                                                        \
+    int rc_ = 0;                                                                                                    \
+    if ((S) <= 64) {                                                                                                \
+      if (packed) rc_ = FN<T, 32, HD>(__VA_ARGS__, 0, st);                                                          \
+      return rc_ ? rc_ : FN<T, 64, HD>(__VA_ARGS__, (packed) ? 32 : 0, st);                                         \
+    }                                                                                                               \
+    if ((S) <= 128) {                                                                                               \
+      if (packed) rc_ = FN<T, 64, HD>(__VA_ARGS__, 0, st);                                                          \
+      return rc_ ? rc_ : FN<T, 128, HD>(__VA_ARGS__, (packed) ? 64 : 0, st);                                        \
+    }                                                                                                               \
+    if constexpr (HD == 64) {                                                                                       \
+      if (packed) rc_ = FN<T, 128, HD>(__VA_ARGS__, 0, st);                                                         \
+      return rc_ ? rc_ : FN<T, 256, HD>(__VA_ARGS__, (packed) ? 128 : 0, st);                                       \
+    }                                                                                                               \
+    return -4;                                                                                                      \
+  }()
 
-// ------------------------------------------------------------------------------------ sequences of 129..512 tokens
+// ------------------------------------------------------------------------------------ sequences of 257..512 tokens
 // Same math and the same fragment routines, blocked: a CTA of 4 warps owns 64 query rows (forward, dQ) or 64 key
 // rows (dK, dV) of one (batch, head) and walks the other dimension in blocks of 128 through shared memory.
 //   forward   two passes over the key blocks: running row maximum / sum first, then probabilities (stored for the
@@ -532,28 +846,6 @@ __device__ __forceinline__ void stage_block(T* dst, const T* __restrict__ src, s
       for (int j = 0; j < 8; ++j) v[j] = 0.f;
     }
     store8(dst + s * RP + d, v);
-  }
-}
-
-// two consecutive elements idx, idx + 1 of a [.., S] row; ok0 / ok1 say which exist; `pair` = 4-byte access allowed
-template <typename T>
-__device__ __forceinline__ float2 load_pair(const T* __restrict__ base, size_t idx, bool ok0, bool ok1, bool pair) {
-  float2 r = make_float2(0.f, 0.f);
-  if (ok0) {
-    if (pair) r = Pack<T>::unpack(*reinterpret_cast<const uint32_t*>(base + idx));
-    else { r.x = to_f(base[idx]); if (ok1) r.y = to_f(base[idx + 1]); }
-  }
-  return r;
-}
-template <typename T>
-__device__ __forceinline__ void store_pair(T* __restrict__ base, size_t idx, uint32_t u, bool ok0, bool ok1, bool pair) {
-  if (ok0) {
-    if (pair) *reinterpret_cast<uint32_t*>(base + idx) = u;
-    else {
-      const T* e = reinterpret_cast<const T*>(&u);
-      base[idx] = e[0];
-      if (ok1) base[idx + 1] = e[1];
-    }
   }
 }
 
@@ -874,18 +1166,24 @@ static int launch_bwd_long(const void* dctx, const void* qkv, const void* bqkv, 
 
 using namespace rb;
 
-// dtype: 1 = bf16, 2 = fp16.  Requires H / nh == 64, 1 <= S <= 128, H % 8 == 0; returns -4 otherwise (callers
-// then use the attention_tc.cu entry points, which also cover head dim 32).  tok_slot / tok_len / tok_meta
-// (all or none): packed tokens, see token_map.cuh.
+// dtype: 1 = bf16, 2 = fp16.  Requires H / nh == 64 or 32, H % 8 == 0, 1 <= S <= 256 (head dim 32: <= 128); returns -4
+// otherwise.  tok_slot / tok_len / tok_meta (all or none): packed tokens, see token_map.cuh.
+static bool mma_args_ok(int dtype, int b, int S, int H, int nh) {
+  if (S < 1 || S > 256 || H % nh || H % 8 || (dtype != RB_BF16 && dtype != RB_F16)) return false;
+  if (H / nh != 64 && !(H / nh == 32 && S <= 128)) return false;
+  return S <= 128 || (long long)b * nh * S * S < (1LL << 32);   // dropout counters are 32-bit element indices
+}
+
 RB_API int rb_attention_fwd_mma(int dtype, const void* qkv, const void* bqkv, const int* mask, void* ctx, void* probs,
                                 int b, int S, int H, int nh, float p, const int* seed, unsigned stream_id,
                                 const int* tok_slot, const int* tok_len, const int* tok_meta, cudaStream_t st) {
-  if (S > 128 || S < 1 || H % nh || H % 8 || H / nh != amma::HD || (dtype != RB_BF16 && dtype != RB_F16)) return -4;
+  if (!mma_args_ok(dtype, b, S, H, nh)) return -4;
   const amma::Tok tk{tok_slot, tok_len, tok_meta};
+  const bool packed = tok_slot != nullptr;
   int rc;
-#define RB_FWD(T, SP) amma::launch_fwd<T, SP>(qkv, bqkv, mask, ctx, probs, b, S, H, nh, p, seed, stream_id, tk, st)
-  if (dtype == RB_BF16) rc = S <= 32 ? RB_FWD(__nv_bfloat16, 32) : S <= 64 ? RB_FWD(__nv_bfloat16, 64) : RB_FWD(__nv_bfloat16, 128);
-  else rc = S <= 32 ? RB_FWD(__half, 32) : S <= 64 ? RB_FWD(__half, 64) : RB_FWD(__half, 128);
+#define RB_FWD(T, HD) RB_ATT_LAUNCH(T, HD, amma::launch_fwd, S, packed, qkv, bqkv, mask, ctx, probs, b, S, H, nh, p, seed, stream_id, tk)
+  if (H / nh == 64) rc = dtype == RB_BF16 ? RB_FWD(__nv_bfloat16, 64) : RB_FWD(__half, 64);
+  else rc = dtype == RB_BF16 ? RB_FWD(__nv_bfloat16, 32) : RB_FWD(__half, 32);
 #undef RB_FWD
   if (rc) return rc;
   RB_LAUNCH_CHECK();
@@ -898,20 +1196,21 @@ RB_API int rb_attention_bwd_mma(int dtype, const void* dctx, const void* qkv, co
                                 void* dqkv, int b, int S, int H, int nh, float p, const int* seed, unsigned stream_id,
                                 float* bias_acc, const int* tok_slot, const int* tok_len, const int* tok_meta,
                                 cudaStream_t st) {
-  if (S > 128 || S < 1 || H % nh || H % 8 || H / nh != amma::HD || (dtype != RB_BF16 && dtype != RB_F16)) return -4;
+  if (!mma_args_ok(dtype, b, S, H, nh)) return -4;
   const amma::Tok tk{tok_slot, tok_len, tok_meta};
+  const bool packed = tok_slot != nullptr;
   int rc;
-#define RB_BWD(T, SP) amma::launch_bwd<T, SP>(dctx, qkv, bqkv, probs, dqkv, b, S, H, nh, p, seed, stream_id, bias_acc, tk, st)
-  if (dtype == RB_BF16) rc = S <= 32 ? RB_BWD(__nv_bfloat16, 32) : S <= 64 ? RB_BWD(__nv_bfloat16, 64) : RB_BWD(__nv_bfloat16, 128);
-  else rc = S <= 32 ? RB_BWD(__half, 32) : S <= 64 ? RB_BWD(__half, 64) : RB_BWD(__half, 128);
+#define RB_BWD(T, HD) RB_ATT_LAUNCH(T, HD, amma::launch_bwd, S, packed, dctx, qkv, bqkv, probs, dqkv, b, S, H, nh, p, seed, stream_id, bias_acc, tk)
+  if (H / nh == 64) rc = dtype == RB_BF16 ? RB_BWD(__nv_bfloat16, 64) : RB_BWD(__half, 64);
+  else rc = dtype == RB_BF16 ? RB_BWD(__nv_bfloat16, 32) : RB_BWD(__half, 32);
 #undef RB_BWD
   if (rc) return rc;
   RB_LAUNCH_CHECK();
   return 0;
 }
 
-// Sequences of 129..512 tokens (same requirements otherwise).  The backward needs ds_ws, a [b, nh, S, S] scratch of
-// the activation dtype (the softmax gradient, written by its first kernel and read by its second); two launches.
+// Sequences of 257..512 tokens, head dim 64 (same requirements otherwise).  The backward needs ds_ws, a [b, nh, S, S]
+// scratch of the activation dtype (the softmax gradient, written by its first kernel and read by its second); two launches.
 static bool long_args_ok(int dtype, int b, int S, int H, int nh) {
   if (S <= 128 || S > 512 || H % nh || H % 8 || H / nh != amma::HD || (dtype != RB_BF16 && dtype != RB_F16)) return false;
   return (long long)b * nh * S * S < (1LL << 32);   // dropout counters are 32-bit element indices

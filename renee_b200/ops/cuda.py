@@ -229,32 +229,35 @@ def embed_ln_bwd(dy, ids, word, pos, gamma, mean, rstd, S, p, rng, stream, pad_i
 
 def attention_packs(dtype, S: int, H: int, nh: int) -> bool:
     """Whether the attention kernels that serve this shape understand packed tokens (those of attention_mma.cu do)."""
-    if dtype == torch.float32 or H // nh != 64 or os.environ.get("RENEE_B200_ATTENTION", "") == "tiles":
+    if dtype == torch.float32 or H // nh not in (32, 64) or os.environ.get("RENEE_B200_ATTENTION", "") == "tiles":
         return False
-    return S <= 128 or (S <= 512 and os.environ.get("RENEE_B200_ATTENTION_LONG", "") != "0")
+    return S <= 128 or (S <= 512 and H // nh == 64 and os.environ.get("RENEE_B200_ATTENTION_LONG", "") != "0")
 
 
 def _attention_fits(qkv, S: int, H: int, nh: int) -> bool:
     """fp32 activations use the CUDA-core kernels, whose backward tiles exceed shared memory for long
     sequences; those shapes are composed from library ops instead (fp32 encoders are a debugging mode)."""
-    if qkv.dtype != torch.float32:
-        return S <= 128
     hd = H // nh
+    if qkv.dtype != torch.float32:
+        return S <= 128 or (S <= 256 and hd == 64 and os.environ.get("RENEE_B200_ATTENTION_LONG", "") != "0"
+                            and _attention_entry("fwd", H, nh).endswith("_mma"))
     return S <= 128 and 2 * S * (S + 1) * 4 + 4 * S * (hd + 2) * 4 <= 227 * 1024
 
 
 def _attention_entry(direction: str, H: int, nh: int) -> str:
-    """16-bit activations: the register-resident kernels for head dim 64 (scores stay in MMA fragments), the
-    shared-memory tile kernels otherwise (head dim 32) or when ``RENEE_B200_ATTENTION=tiles`` asks for them."""
-    if H // nh == 64 and os.environ.get("RENEE_B200_ATTENTION", "") != "tiles":
+    """16-bit activations: the register-resident kernels (scores stay in MMA fragments), or the shared-memory tile
+    kernels when ``RENEE_B200_ATTENTION=tiles`` asks for them."""
+    if H // nh in (32, 64) and os.environ.get("RENEE_B200_ATTENTION", "") != "tiles":
         return f"rb_attention_{direction}_mma"
     return f"rb_attention_{direction}_tc"
 
 
 def _attention_long(qkv, S: int, H: int, nh: int, ws) -> bool:
-    """Sequences of 129..512 tokens, 16-bit activations, head dim 64: the blocked kernels of attention_mma.cu
-    (``RENEE_B200_ATTENTION_LONG=0`` sends these shapes to the composed library ops instead)."""
-    return (qkv.dtype != torch.float32 and 128 < S <= 512 and H // nh == 64 and "ds" in ws
+    """Sequences of 257..512 tokens (129..512 with the tile kernels), 16-bit activations, head dim 64: the streaming
+    kernels of attention_mma.cu (``RENEE_B200_ATTENTION_LONG=0`` sends sequences of more than 128 tokens to the composed
+    library ops instead)."""
+    lo = 256 if _attention_entry("fwd", H, nh).endswith("_mma") else 128
+    return (qkv.dtype != torch.float32 and lo < S <= 512 and H // nh == 64 and "ds" in ws
             and os.environ.get("RENEE_B200_ATTENTION_LONG", "") != "0")
 
 
