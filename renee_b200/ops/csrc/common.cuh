@@ -30,6 +30,23 @@ template <> __device__ __forceinline__ float from_f<float>(float x) { return x; 
 template <> __device__ __forceinline__ __nv_bfloat16 from_f<__nv_bfloat16>(float x) { return __float2bfloat16_rn(x); }
 template <> __device__ __forceinline__ __half from_f<__half>(float x) { return __float2half_rn(x); }
 
+// 8 floats rounded to a 16-bit type, two per conversion instruction
+template <typename T> __device__ __forceinline__ uint4 pack16x8(const float* v) {
+  uint4 raw;
+  uint32_t* w = reinterpret_cast<uint32_t*>(&raw);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    if constexpr (std::is_same<T, __nv_bfloat16>::value) {
+      const __nv_bfloat162 h = __floats2bfloat162_rn(v[2 * i], v[2 * i + 1]);
+      w[i] = *reinterpret_cast<const uint32_t*>(&h);
+    } else {
+      const __half2 h = __floats2half2_rn(v[2 * i], v[2 * i + 1]);
+      w[i] = *reinterpret_cast<const uint32_t*>(&h);
+    }
+  }
+  return raw;
+}
+
 // 8 consecutive elements of T, moved with the widest aligned access available
 template <typename T> struct Vec8 {
   T v[8];
@@ -53,11 +70,7 @@ __device__ __forceinline__ void load8(const T* __restrict__ p, float (&out)[8]) 
 template <typename T>
 __device__ __forceinline__ void store8(T* __restrict__ p, const float (&in)[8]) {
   if constexpr (sizeof(T) == 2) {
-    uint4 raw;
-    T* e = reinterpret_cast<T*>(&raw);
-#pragma unroll
-    for (int i = 0; i < 8; ++i) e[i] = from_f<T>(in[i]);
-    *reinterpret_cast<uint4*>(p) = raw;
+    *reinterpret_cast<uint4*>(p) = pack16x8<T>(in);
   } else {
     *reinterpret_cast<float4*>(p) = make_float4(in[0], in[1], in[2], in[3]);
     *reinterpret_cast<float4*>(p + 4) = make_float4(in[4], in[5], in[6], in[7]);
@@ -96,16 +109,16 @@ template <typename T> __device__ __forceinline__ float round_through(float x) { 
 // fp32 -> fp16 with stochastic rounding: add uniform noise below the 13 mantissa bits fp16 drops, then
 // truncate.  Unbiased for values in fp16's normal range, which keeps updates smaller than half an ulp
 // of W from being lost systematically late in the learning-rate schedule.
-__device__ __forceinline__ __half sr_half(float x, uint32_t rnd) {
-  uint32_t b = __float_as_uint(x);
-  b = (b + (rnd & 0x1FFFu)) & ~0x1FFFu;
-  return __float2half_rz(__uint_as_float(b));
-}
-// The same for either 16-bit type, returned as the fp32 value of the rounded number (bf16 drops 16 bits).
-template <typename T> __device__ __forceinline__ float sr_round(float x, uint32_t rnd) {
-  if (std::is_same<T, __half>::value) return __half2float(sr_half(x, rnd));
-  const uint32_t b = (__float_as_uint(x) + (rnd & 0xFFFFu)) & ~0xFFFFu;
-  return __uint_as_float(b);
+// Two neighbours at once, packed: the low half of rnd is the noise of the first, the high half that of the second (fp16
+// drops 13 bits, bf16 16).  The masking keeps an infinity one; the conversion truncates what lies below fp16's range.
+template <typename T> __device__ __forceinline__ uint32_t sr_pack2(float x, float y, uint32_t rnd) {
+  constexpr uint32_t kNoise = std::is_same<T, __half>::value ? 0x1FFFu : 0xFFFFu;
+  const float a = __uint_as_float((__float_as_uint(x) + (rnd & kNoise)) & ~kNoise);
+  const float b = __uint_as_float((__float_as_uint(y) + ((rnd >> 16) & kNoise)) & ~kNoise);
+  uint32_t r;
+  if (std::is_same<T, __half>::value) asm("cvt.rz.f16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(b), "f"(a));
+  else asm("cvt.rz.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(b), "f"(a));
+  return r;
 }
 
 __device__ __forceinline__ float warp_sum(float v) {
@@ -153,6 +166,52 @@ __device__ __forceinline__ float gelu_grad_f(float z) {
   float e;
   const float cdf = normal_cdf(z, e);
   return fmaf(z * 0.39894228040143268f, e, cdf);
+}
+
+// Two fp32 values per instruction (add / mul / fma .f32x2): IEEE arithmetic, half the issue slots.
+struct F2 { unsigned long long v; };
+__device__ __forceinline__ F2 f2(float a, float b) { F2 r; asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(a), "f"(b)); return r; }
+__device__ __forceinline__ F2 f2(float a) { return f2(a, a); }
+__device__ __forceinline__ void f2_get(F2 x, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(x.v)); }
+__device__ __forceinline__ F2 operator+(F2 a, F2 b) { F2 r; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v)); return r; }
+__device__ __forceinline__ F2 operator*(F2 a, F2 b) { F2 r; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v)); return r; }
+__device__ __forceinline__ F2 f2_fma(F2 a, F2 b, F2 c) {
+  F2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+  return r;
+}
+
+// normal_cdf of two values (the same formula and roundings; the factor 0.5 sits in the coefficients, which is exact)
+__device__ __forceinline__ F2 normal_cdf2(F2 z, F2& e) {
+  float z0, z1;
+  f2_get(z, z0, z1);
+  const F2 ax = f2(fabsf(z0), fabsf(z1)) * f2(0.70710678118654752f);
+  float d0, d1, t0, t1, e0, e1;
+  f2_get(f2_fma(f2(0.3275911f), ax, f2(1.f)), d0, d1);
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(t0) : "f"(d0));
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(t1) : "f"(d1));
+  const F2 t = f2(t0, t1);
+  F2 p = f2(0.5f * 1.061405429f);
+  p = f2_fma(p, t, f2(0.5f * -1.453152027f));
+  p = f2_fma(p, t, f2(0.5f * 1.421413741f));
+  p = f2_fma(p, t, f2(0.5f * -0.284496736f));
+  p = f2_fma(p, t, f2(0.5f * 0.254829592f));
+  f2_get(ax * ax, e0, e1);
+  e0 = __expf(-e0);
+  e1 = __expf(-e1);
+  e = f2(e0, e1);
+  float h0, h1;
+  f2_get(p * t * e, h0, h1);
+  return f2(z0 < 0.f ? h0 : 1.f - h0, z1 < 0.f ? h1 : 1.f - h1);
+}
+__device__ __forceinline__ F2 gelu2(F2 z) {
+  F2 e;
+  return z * normal_cdf2(z, e);
+}
+__device__ __forceinline__ F2 gelu_grad2(F2 z) {
+  F2 e;
+  const F2 cdf = normal_cdf2(z, e);
+  return f2_fma(z * f2(0.39894228040143268f), e, cdf);
 }
 
 // Number of SMs of the current device (queried once per process; all GPUs of a job are alike)
@@ -205,8 +264,11 @@ __device__ __forceinline__ uint32_t mix32(uint32_t seed, uint32_t stream, uint32
   x ^= x >> 15; x *= 0x2C1B3C6Du; x ^= x >> 12; x *= 0x297A2D39u; x ^= x >> 15;
   return x;
 }
+// The rule is (h >> 8) / 2^24 >= p in reals.  Scaling p by 2^24 is exact, so comparing the 24-bit integer with
+// ceil(p 2^24), which the compiler keeps outside the loop, is the same decision without an integer-to-float conversion
+// per element: those run at 16 per clock and SM and bounded the LayerNorm backward and the attention kernels.
 __device__ __forceinline__ bool keep(uint32_t seed, uint32_t stream, uint32_t idx, float p) {
-  return (float)(mix32(seed, stream, idx) >> 8) * (1.0f / 16777216.0f) >= p;
+  return (mix32(seed, stream, idx) >> 8) >= (uint32_t)ceilf(p * 16777216.0f);
 }
 
 }  // namespace rb

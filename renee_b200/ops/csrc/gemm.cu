@@ -117,13 +117,7 @@ struct Params {
 
 constexpr int kColReplicas = 8;   // must equal the replica count of the deferred column reductions (encoder_ops.cu)
 
-template <typename T> __device__ __forceinline__ uint4 pack8(const float* v) {
-  uint4 raw;
-  T* e = reinterpret_cast<T*>(&raw);
-#pragma unroll
-  for (int i = 0; i < 8; ++i) e[i] = from_f<T>(v[i]);
-  return raw;
-}
+template <typename T> __device__ __forceinline__ uint4 pack8(const float* v) { return pack16x8<T>(v); }
 template <typename T> __device__ __forceinline__ void unpack8(const uint4& raw, float* out) {
   const T* e = reinterpret_cast<const T*>(&raw);
 #pragma unroll
@@ -337,8 +331,8 @@ enc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
     int t_local = 0;
     uint32_t in_count = 0;                                // R panels fetched so far (parity of my_in_bar)
     // TOPK: this thread's 8 best (value, column) of its row so far, sorted descending; cur_m = row block they belong to
-    float tv[8];
-    int ti[8];
+    float tv[8] = {};
+    int ti[8] = {};
     int cur_m = -1;
     const auto topk_flush = [&]() {                       // the list of this unit and column group for row block cur_m
       const int frow = cur_m * (BM * NCTA) + (int)rank * BM + r;
@@ -424,10 +418,11 @@ enc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
                   for (int j = 0; j < 8; ++j) b[j] = 0.f;
                 }
 #pragma unroll
-                for (int j = 0; j < 8; ++j) {
-                  o[j] = round_through<T>(a[j] + b[j]);      // the backward pass differentiates at the stored value
-                  a[j] = gelu_f(o[j]);                       // second output, staged after the first has left
-                }
+                for (int j = 0; j < 8; ++j) o[j] = a[j] + b[j];
+                *slot = pack8<T>(o);
+                unpack8<T>(pack8<T>(o), o);                  // the backward pass differentiates at the stored value
+#pragma unroll
+                for (int j = 0; j < 8; j += 2) f2_get(gelu2(f2(o[j], o[j + 1])), a[j], a[j + 1]);   // second output, staged after the first has left
               } else if (EPI == E_BIAS_DROPOUT_RESID) {
                 float b[8], res[8];
                 if (c < p.N) unpack8<T>(__ldg(reinterpret_cast<const uint4*>(reinterpret_cast<const T*>(p.bias) + c)), b);
@@ -448,31 +443,44 @@ enc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
 #pragma unroll
                 for (int j = 0; j < 8; ++j) o[j] = a[j] + res[j];
               } else if (EPI == E_DW_SGD) {
-                // momentum SGD on the tile: m = mo m + (dW + wd w), w -= lr m, with m rounded to 16 bit first
+                // momentum SGD on the tile: m = mo m + (dW + wd w), w -= lr m, with m rounded to 16 bit first.  With one
+                // element at a time and a hash each this was some 40 instructions per element, more than the tile's
+                // bytes take: two per instruction and per hash.
                 uint4* slot2 = reinterpret_cast<uint4*>(pan2 + panel_off(r, chunk));
                 float w[8], mm[8];
                 unpack8<T>(*slot, w);
                 unpack8<T>(*slot2, mm);
-                const float lr = p.hp[HP_LR_XFC];
+                const F2 nlr = f2(-p.hp[HP_LR_XFC]), mo2 = f2(p.mo), wd2 = f2(p.wd);
                 const uint32_t sr_seed = reinterpret_cast<const uint32_t*>(p.hp)[HP_SEED];
                 const uint32_t e = (uint32_t)row * (uint32_t)p.ldW + (uint32_t)c;
 #pragma unroll
-                for (int j = 0; j < 8; ++j) {
-                  mm[j] = round_through<T>(p.mo * mm[j] + (a[j] + p.wd * w[j]));
-                  const float nw = w[j] - lr * mm[j];
-                  o[j] = p.stochastic_round ? sr_round<T>(nw, mix32(sr_seed, 0x5152u, e + j)) : nw;
+                for (int j = 0; j < 8; j += 2)
+                  f2_get(f2_fma(mo2, f2(mm[j], mm[j + 1]), f2_fma(wd2, f2(w[j], w[j + 1]), f2(a[j], a[j + 1]))), mm[j], mm[j + 1]);
+                const uint4 m16 = pack8<T>(mm);
+                unpack8<T>(m16, mm);
+#pragma unroll
+                for (int j = 0; j < 8; j += 2) f2_get(f2_fma(nlr, f2(mm[j], mm[j + 1]), f2(w[j], w[j + 1])), o[j], o[j + 1]);
+                *slot2 = m16;
+                if (p.stochastic_round) {
+                  // one hash per pair of elements: its halves are the noise of the two
+                  uint4 w16;
+                  uint32_t* wp = reinterpret_cast<uint32_t*>(&w16);
+#pragma unroll
+                  for (int j = 0; j < 8; j += 2) wp[j >> 1] = sr_pack2<T>(o[j], o[j + 1], mix32(sr_seed, 0x5152u, (e + j) >> 1));
+                  *slot = w16;
+                } else {
+                  *slot = pack8<T>(o);
                 }
-                *slot2 = pack8<T>(mm);
               } else {   // E_GELU_BWD
                 float f[8];
                 unpack8<T>(*slot, f);
 #pragma unroll
-                for (int j = 0; j < 8; ++j) {
-                  o[j] = round_through<T>(a[j] * gelu_grad_f(f[j]));
-                  a[j] = row < M ? o[j] : 0.f;               // rows past the packed tokens hold what an earlier pass left
-                }
+                for (int j = 0; j < 8; j += 2) f2_get(f2(a[j], a[j + 1]) * gelu_grad2(f2(f[j], f[j + 1])), o[j], o[j + 1]);
+                unpack8<T>(pack8<T>(o), o);
+#pragma unroll
+                for (int j = 0; j < 8; ++j) a[j] = row < M ? o[j] : 0.f;   // rows past the packed tokens hold what an earlier pass left
               }
-              *slot = pack8<T>(o);
+              if (EPI != E_BIAS_GELU && EPI != E_DW_SGD) *slot = pack8<T>(o);
               if (EPI == E_BIAS_GELU) keep2[EPI == E_BIAS_GELU ? chunk : 0] = pack8<T>(a);
             }
             if (EPI == E_GELU_BWD && p.colacc != nullptr) {
