@@ -9,8 +9,8 @@
 // candidates in all (few labels, or logits of -inf) have t = nothing and every list in doubt, which is the same path.
 // So the result is exact for any order of the labels, with a bounded worst case.
 //
-// One CTA per row.  The selection is a binary search for the k-th largest key over keys in shared memory: each of the
-// 32 steps is one conflict-free sweep and one block-wide count, where the radix select it replaces serialised on the
+// One CTA per row.  The selection is a binary search for the k-th largest key: each step is one sweep over the keys and
+// one block-wide count, where the radix select it replaces serialised on the
 // few histogram bins that logits of similar size share (256 rows x 2368 candidates, k = 5: 36 us and 35 us more of
 // library sort and gather launches -> 26 us).  The whole call: 512 rows x 1.3 M labels, k = 100, 9.39 -> 1.51 ms (before:
 // fp32 logits written chunk by chunk and a selection over each chunk); 256 x 131 K, k = 5, 181 -> 126 us.
@@ -51,6 +51,39 @@ __device__ uint32_t kth_key(const uint32_t* key, int n, int kk, int* s_count) {
   return t;
 }
 
+// The same for the candidates alone, with each thread's share of the keys in registers and two bits per step: 16 steps of
+// three counts (13 bits each fit two words), 1 us where 32 sweeps of shared memory took 15 of the kernel's 26 us.
+template <int NPT>
+__device__ uint32_t kth_key_reg(const uint32_t* key, int n, int kk, int* s_count) {
+  uint32_t k[NPT];
+#pragma unroll
+  for (int u = 0; u < NPT; ++u) { const int i = threadIdx.x + u * THREADS; k[u] = i < n ? key[i] : 0u; }
+  uint32_t t = 0u;
+#pragma unroll 1
+  for (int sh = 30; sh >= 0; sh -= 2) {
+    const uint32_t t1 = t | (1u << sh), t2 = t | (2u << sh), t3 = t | (3u << sh);
+    uint32_t c12 = 0u, c3 = 0u;
+#pragma unroll
+    for (int u = 0; u < NPT; ++u) {
+      c12 += (k[u] >= t1 ? 1u : 0u) + (k[u] >= t2 ? 0x10000u : 0u);
+      c3 += k[u] >= t3 ? 1u : 0u;
+    }
+    c12 = __reduce_add_sync(0xffffffffu, c12);
+    c3 = __reduce_add_sync(0xffffffffu, c3);
+    uint2* cnt = reinterpret_cast<uint2*>(s_count) + ((sh >> 1) & 1) * (THREADS / 32);
+    if ((threadIdx.x & 31) == 0) cnt[threadIdx.x >> 5] = make_uint2(c12, c3);
+    __syncthreads();
+    uint32_t s12 = 0u, s3 = 0u;
+#pragma unroll
+    for (int w = 0; w < THREADS / 32; ++w) { const uint2 c = cnt[w]; s12 += c.x; s3 += c.y; }
+    if ((int)s3 >= kk) t = t3;
+    else if ((int)(s12 >> 16) >= kk) t = t2;
+    else if ((int)(s12 & 0xffffu) >= kk) t = t1;
+  }
+  __syncthreads();
+  return t;
+}
+
 // Writes the kk largest entries of the pool to win[0 .. kk), in any order, and 0 behind them.
 __device__ void gather_best(const uint32_t* key, const int* idx, int n, int kk, uint32_t t, unsigned long long* win, int* s_slots) {
   for (int i = threadIdx.x; i < MAX_K; i += THREADS) win[i] = 0ull;
@@ -79,7 +112,7 @@ __global__ void __launch_bounds__(THREADS) topk_select_kernel(const Args a, cons
   uint32_t* key = reinterpret_cast<uint32_t*>(win + MAX_K);                       // [cap]
   int* idx = reinterpret_cast<int*>(key + cap);                                   // [cap]
   uint8_t* doubt = reinterpret_cast<uint8_t*>(idx + cap);                         // [per_row / 8] lists to recompute
-  __shared__ int s_count[2 * (THREADS / 32)];
+  __shared__ __align__(8) int s_count[4 * (THREADS / 32)];
   __shared__ int s_slots[2];
   __shared__ int s_extra, s_any;
   const int row = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -106,7 +139,10 @@ __global__ void __launch_bounds__(THREADS) topk_select_kernel(const Args a, cons
     idx[i] = id;
   }
   __syncthreads();
-  uint32_t t = kth_key(key, a.per_row, a.k, s_count);
+  uint32_t t;
+  if (a.per_row <= 10 * THREADS) t = kth_key_reg<10>(key, a.per_row, a.k, s_count);
+  else if (a.per_row <= 20 * THREADS) t = kth_key_reg<20>(key, a.per_row, a.k, s_count);
+  else t = kth_key(key, a.per_row, a.k, s_count);
   for (int l = tid; l < n_lists; l += THREADS) {
     const bool met = (l % TOPK_GROUPS) * ucols < a.bn && topk_unit_first(l / TOPK_GROUPS, a.units, first, step, a.n_n) >= 0;
     const bool in_doubt = met && (t == 0u || key[l * TOPK_LIST + TOPK_LIST - 1] > t);
