@@ -22,15 +22,14 @@ template <> __device__ __forceinline__ void atomic_add8<float>(float* p, const f
 #pragma unroll
   for (int i = 0; i < 8; ++i) atomicAdd(p + i, v[i]);
 }
+// 16 bytes per reduction instead of 4 (p is 16-byte aligned: rows and columns are multiples of 8 elements)
 template <> __device__ __forceinline__ void atomic_add8<__nv_bfloat16>(__nv_bfloat16* p, const float (&v)[8]) {
-#pragma unroll
-  for (int i = 0; i < 4; ++i)
-    atomicAdd(reinterpret_cast<__nv_bfloat162*>(p) + i, __floats2bfloat162_rn(v[2 * i], v[2 * i + 1]));
+  const uint4 r = pack16x8<__nv_bfloat16>(v);
+  asm volatile("red.global.add.noftz.v4.bf16x2 [%0], {%1, %2, %3, %4};" ::"l"(p), "r"(r.x), "r"(r.y), "r"(r.z), "r"(r.w) : "memory");
 }
 template <> __device__ __forceinline__ void atomic_add8<__half>(__half* p, const float (&v)[8]) {
-#pragma unroll
-  for (int i = 0; i < 4; ++i)
-    atomicAdd(reinterpret_cast<__half2*>(p) + i, __floats2half2_rn(v[2 * i], v[2 * i + 1]));
+  const uint4 r = pack16x8<__half>(v);
+  asm volatile("red.global.add.noftz.v4.f16x2 [%0], {%1, %2, %3, %4};" ::"l"(p), "r"(r.x), "r"(r.y), "r"(r.z), "r"(r.w) : "memory");
 }
 
 // Last-block-done column reduction epilogue.  Every block has already added its partial sums to one of
@@ -712,33 +711,61 @@ __global__ void __launch_bounds__(128) colsum_kernel(const T* __restrict__ x, fl
 }
 
 // ------------------------------------------------------------------------------------ pooling
-// grid = b, block covers H/8 vectors.  Packed tokens: slot gives the row of a token (CLS and attended ones are kept).
+// grid = b.  The block's threads are `slices` sets of H/8 column vectors; for the mean each set walks every slices-th token
+// (one set alone waited for 256 loads one after the other at S = 256: 72 us) and shared memory joins them.  Packed tokens:
+// slot gives the row of a token (CLS and attended ones are kept).
+constexpr int POOL_THREADS = 512;
 template <typename T>
-__global__ void pool_fwd_kernel(const T* __restrict__ h, const int* __restrict__ mask, float* __restrict__ out,
-                                int S, int H, int cls, const int* __restrict__ slot) {
-  const int b = blockIdx.x;
-  for (int col = threadIdx.x * 8; col < H; col += blockDim.x * 8) {
+__global__ void __launch_bounds__(POOL_THREADS) pool_fwd_kernel(const T* __restrict__ h, const int* __restrict__ mask,
+                                                                float* __restrict__ out, int S, int H, int cls,
+                                                                const int* __restrict__ slot) {
+  extern __shared__ __align__(16) float s_acc[];   // [slices][H]
+  __shared__ int s_cnt;
+  const int b = blockIdx.x, nv = H / 8;
+  if (cls) {
+    for (int col = threadIdx.x * 8; col < H; col += blockDim.x * 8) {
+      float acc[8];
+      load8(h + (size_t)(slot != nullptr ? slot[b * S] : b * S) * H + col, acc);
+      store8(out + (size_t)b * H + col, acc);
+    }
+    return;
+  }
+  const int slices = max(1, (int)blockDim.x / nv);
+  if (threadIdx.x == 0) s_cnt = 0;
+  __syncthreads();
+  int n = 0;
+  for (int s = threadIdx.x; s < S; s += blockDim.x) n += mask[b * S + s] != 0 ? 1 : 0;
+  if (n > 0) atomicAdd(&s_cnt, n);
+  __syncthreads();
+  const float inv = 1.f / fmaxf((float)s_cnt, 1e-9f);
+  const int slice = nv <= (int)blockDim.x ? (int)threadIdx.x / nv : 0;
+  for (int v = nv <= (int)blockDim.x ? (int)threadIdx.x % nv : (int)threadIdx.x; v < nv && slice < slices; v += blockDim.x) {
     float acc[8];
 #pragma unroll
     for (int j = 0; j < 8; ++j) acc[j] = 0.f;
-    if (cls) {
-      load8(h + (size_t)(slot != nullptr ? slot[b * S] : b * S) * H + col, acc);
-    } else {
-      float cnt = 0.f;
-      for (int s = 0; s < S; ++s) {
-        if (mask[b * S + s] != 0) {
-          float a[8];
-          load8(h + (size_t)(slot != nullptr ? slot[b * S + s] : b * S + s) * H + col, a);
+#pragma unroll 4
+    for (int s = slice; s < S; s += slices) {
+      if (mask[b * S + s] != 0) {
+        float a[8];
+        load8(h + (size_t)(slot != nullptr ? slot[b * S + s] : b * S + s) * H + v * 8, a);
 #pragma unroll
-          for (int j = 0; j < 8; ++j) acc[j] += a[j];
-          cnt += 1.f;
-        }
+        for (int j = 0; j < 8; ++j) acc[j] += a[j];
       }
-      const float inv = 1.f / fmaxf(cnt, 1e-9f);
+    }
+    if (slices == 1) {
 #pragma unroll
       for (int j = 0; j < 8; ++j) acc[j] *= inv;
+      store8(out + (size_t)b * H + v * 8, acc);
+    } else {
+      store8(s_acc + (size_t)slice * H + v * 8, acc);
     }
-    store8(out + (size_t)b * H + col, acc);
+  }
+  if (slices == 1) return;
+  __syncthreads();
+  for (int c = threadIdx.x; c < H; c += blockDim.x) {
+    float t = 0.f;
+    for (int q = 0; q < slices; ++q) t += s_acc[(size_t)q * H + c];
+    out[(size_t)b * H + c] = t * inv;
   }
 }
 
@@ -975,7 +1002,9 @@ RB_API int rb_colsum(int dtype, const void* x, float* acc, unsigned* counter, vo
 RB_API int rb_pool_fwd(int dtype, const void* h, const int* mask, float* out, int b, int S, int H, int cls,
                        const int* tok_slot, cudaStream_t st) {
   if (H % 8) return -3;
-  DISPATCH_T(dtype, (pool_fwd_kernel<T><<<b, 128, 0, st>>>((const T*)h, mask, out, S, H, cls, tok_slot)));
+  const int nv = H / 8, slices = nv < POOL_THREADS ? POOL_THREADS / nv : 1;
+  const size_t smem = cls || slices == 1 ? 0 : (size_t)slices * H * sizeof(float);     // at most 16 KB
+  DISPATCH_T(dtype, (pool_fwd_kernel<T><<<b, POOL_THREADS, smem, st>>>((const T*)h, mask, out, S, H, cls, tok_slot)));
   RB_LAUNCH_CHECK();
   return 0;
 }
