@@ -140,6 +140,8 @@ class FlatEncoder:
         self._own_mode = "0"
         self._own_supported = False
         self._wgrad_stream = None
+        self._wgrad_group = None
+        self._wgrad_done = [None, None]
         self.pack_tokens = True        # own GEMM path: leave padded tokens out (TokenMap); a comparison may switch it off
         self.rows_hint = 0             # caller's estimate of the kept tokens of the coming batches (tile planning only)
         if self.device.type == "cuda" and act_dtype != torch.float32:
@@ -150,10 +152,9 @@ class FlatEncoder:
             self._own_supported = cu.enc_gemm_supported(self.p16, H, Fd)
             self.own_gemm = self._own_supported and self._own_mode != "auto"
             if self._own_supported and os.environ.get("RENEE_B200_WGRAD_STREAM", "1") != "0":
-                # weight-gradient GEMMs are off the critical path of the backward pass (nothing reads them before
-                # the optimizer): they run on a second stream, where they fill the SMs that the data-gradient
-                # GEMMs' last partial wave of tiles leaves idle (and, at small token counts, the SMs those GEMMs
-                # never use).  Captured into the step's CUDA graph as parallel branches.
+                # weight gradients are off the critical path of the backward pass (nothing reads them before the
+                # optimizer): a layer's launch runs on a second stream, where it fills the SMs that the next layer's
+                # kernels leave idle.  Captured into the step's CUDA graph as parallel branches.
                 self._wgrad_stream = torch.cuda.Stream(device=self.device)
 
     # ------------------------------------------------------------------ parameter views
@@ -228,6 +229,10 @@ class FlatEncoder:
                           emb=e(b, self.out_dims, dtype=torch.float32), tmap=None)
         if self._own_supported and dev.type == "cuda":
             from ..ops import cuda as cu
+            # gradients that the weight-gradient launch of a layer still reads while the next layer is differentiated
+            self._acts["bwd"] = [dict(dpre2=e(T, H), dpre1=e(T, H), df1=e(T, Fd), dqkv=e(T, 3 * H)) for _ in range(2)]
+            if self._wgrad_group is None:
+                self._wgrad_group = cu.WgradGroup([(3 * H, H), (H, H), (Fd, H), (H, Fd)], dev)
             if cu.attention_packs(dt, S, H, nh):
                 self._acts["tmap"] = cu.TokenMap(b, S, dev)
         self._acts_key = key
@@ -356,21 +361,25 @@ class FlatEncoder:
         if on_layer_done is not None:
             on_layer_done(-1)       # embeddings and every vector-shaped gradient are final: the whole buffer is
 
-    def _wgrad(self, dy, x, dW) -> None:
-        """``dW = dy^T x`` on the weight-gradient stream (ordered after everything issued so far on the current one)."""
+    def _wgrad_layer(self, par: int, items) -> None:
+        """The weight gradients of one layer in one launch, on the weight-gradient stream (ordered after everything issued
+        so far on the current one).  Their inputs live in the backward buffers of parity ``par``, which the layer after
+        the next overwrites: :meth:`_wgrad_wait` comes before that."""
         from ..ops import cuda as cu
         side = self._wgrad_stream
         if side is None:
-            cu.linear_wgrad(dy, x, dW, **self._fw["packed"])
+            cu.wgrad_group(items, self._wgrad_group, **self._fw["packed"])
             return
         side.wait_stream(torch.cuda.current_stream())
         with torch.cuda.stream(side):
-            cu.linear_wgrad(dy, x, dW, **self._fw["packed"])
+            cu.wgrad_group(items, self._wgrad_group, **self._fw["packed"])
+            self._wgrad_done[par] = side.record_event()
 
-    def _wgrad_join(self) -> None:
-        """The current stream waits for the weight-gradient GEMMs issued so far (their inputs may be overwritten next)."""
-        if self._wgrad_stream is not None:
-            torch.cuda.current_stream().wait_stream(self._wgrad_stream)
+    def _wgrad_wait(self, par: int) -> None:
+        """The current stream waits for the weight gradients last issued with parity ``par``."""
+        if self._wgrad_done[par] is not None:
+            torch.cuda.current_stream().wait_event(self._wgrad_done[par])
+            self._wgrad_done[par] = None
 
     def _backward(self, d_emb: torch.Tensor, on_layer_done=None) -> None:
         cfg, A, fw = self.cfg, self._acts, self._fw
@@ -395,40 +404,15 @@ class FlatEncoder:
             pre = f"transformer.layer.{l}."
             sb = 8 * (l + 1)
             h_in = L["h_in"]
+            if self.own_gemm:
+                self._backward_layer_fused(l, L, dh, on_layer_done)
+                continue
             # ---- output LN + FFN
             d_pre2, d_f2 = ops.bias_dropout_add_ln_bwd(
                 dh, L["pre2"][:T], self.view(P, pre + "output_layer_norm.weight"), L["mean2"][:T], L["rstd2"][:T],
                 pd, rng, sb + _S_FFN,
                 self.view(G, pre + "output_layer_norm.weight"), self.view(G, pre + "output_layer_norm.bias"),
-                self.view(G, pre + "ffn.lin2.bias"), A["dh_b"][:T], L["f2"][:T], **packed)
-            if self.own_gemm:
-                from ..ops import cuda as cu
-                self._wgrad(d_f2, L["a1"][:T], self.view(G, pre + "ffn.lin2.weight"))
-                df1 = A["df1"][:T]
-                cu.linear_dgrad(d_f2, self.view(P, pre + "ffn.lin2.weight"), df1, "gelu_bwd", pre=L["f1"][:T],
-                                dbias=self.view(G, pre + "ffn.lin1.bias"), **packed)
-                self._wgrad(df1, L["h1"][:T], self.view(G, pre + "ffn.lin1.weight"))
-                dh1 = cu.linear_dgrad(df1, self.view(P, pre + "ffn.lin1.weight"), dh, "add", resid=d_pre2, **packed)
-                if d_f2 is d_pre2:
-                    self._wgrad_join()      # without dropout d_f2 is the shared buffer the next kernel overwrites
-                d_pre1, d_ao = ops.bias_dropout_add_ln_bwd(
-                    dh1, L["pre1"][:T], self.view(P, pre + "sa_layer_norm.weight"), L["mean1"][:T], L["rstd1"][:T],
-                    fw["po"], rng, sb + _S_ATTN,
-                    self.view(G, pre + "sa_layer_norm.weight"), self.view(G, pre + "sa_layer_norm.bias"),
-                    self.view(G, pre + "attention.out_lin.bias"), A["dh_b"][:T], L["ao"][:T], **packed)
-                self._wgrad(d_ao, L["ctx"][:T], self.view(G, pre + "attention.out_lin.weight"))
-                dctx = A["dctx"][:T]
-                cu.linear_dgrad(d_ao, self.view(P, pre + "attention.out_lin.weight"), dctx, **packed)
-                dqkv = A["dqkv"][:T]
-                ops.attention_bwd(dctx, L["qkv"][:T], self._qkv(P, l, "bias"), mask, cfg.n_heads, pa, rng,
-                                  sb + _S_PROBS, L["att"], dqkv, self._qkv(G, l, "bias"), **packed)
-                self._wgrad(dqkv, h_in, self._qkv(G, l, "weight"))
-                cu.linear_dgrad(dqkv, self._qkv(P, l, "weight"), dh, "add", resid=d_pre1, **packed)
-                # the next layer overwrites the shared gradient buffers (dh_b, df1, dqkv) the GEMMs above read
-                self._wgrad_join()
-                if on_layer_done is not None:
-                    on_layer_done(l)
-                continue
+                self.view(G, pre + "ffn.lin2.bias"), A["dh_b"][:T], L["f2"][:T])
             torch.mm(d_f2.t(), L["a1"][:T], out=self.view(G, pre + "ffn.lin2.weight"))
             da1 = A["da1"][:T]
             torch.mm(d_f2, self.view(P, pre + "ffn.lin2.weight"), out=da1)
@@ -461,3 +445,39 @@ class FlatEncoder:
                          self.view(G, "embeddings.word_embeddings.weight"),
                          self.view(G, "embeddings.position_embeddings.weight"),
                          self.view(G, "embeddings.LayerNorm.weight"), self.view(G, "embeddings.LayerNorm.bias"), **packed)
+        self._wgrad_wait(0)
+        self._wgrad_wait(1)
+
+    def _backward_layer_fused(self, l: int, L: dict, dh, on_layer_done) -> None:
+        """One transformer block on the own GEMMs: ``dh`` (gradient of its output) becomes the gradient of its input."""
+        from ..ops import cuda as cu
+        cfg, A, P, G, fw = self.cfg, self._acts, self.p16, self.g, self._fw
+        T, packed, pd, po, rng = fw["b"] * fw["S"], fw["packed"], fw["pd"], fw["po"], fw["rng"]
+        pre, sb, par = f"transformer.layer.{l}.", 8 * (l + 1), l & 1
+        buf = {k: t[:T] for k, t in A["bwd"][par].items()}
+        self._wgrad_wait(par)
+        d_pre2, d_f2 = ops.bias_dropout_add_ln_bwd(
+            dh, L["pre2"][:T], self.view(P, pre + "output_layer_norm.weight"), L["mean2"][:T], L["rstd2"][:T],
+            pd, rng, sb + _S_FFN,
+            self.view(G, pre + "output_layer_norm.weight"), self.view(G, pre + "output_layer_norm.bias"),
+            self.view(G, pre + "ffn.lin2.bias"), buf["dpre2"], L["f2"][:T], **packed)
+        df1 = cu.linear_dgrad(d_f2, self.view(P, pre + "ffn.lin2.weight"), buf["df1"], "gelu_bwd", pre=L["f1"][:T],
+                              dbias=self.view(G, pre + "ffn.lin1.bias"), **packed)
+        dh1 = cu.linear_dgrad(df1, self.view(P, pre + "ffn.lin1.weight"), dh, "add", resid=d_pre2, **packed)
+        d_pre1, d_ao = ops.bias_dropout_add_ln_bwd(
+            dh1, L["pre1"][:T], self.view(P, pre + "sa_layer_norm.weight"), L["mean1"][:T], L["rstd1"][:T],
+            po, rng, sb + _S_ATTN,
+            self.view(G, pre + "sa_layer_norm.weight"), self.view(G, pre + "sa_layer_norm.bias"),
+            self.view(G, pre + "attention.out_lin.bias"), buf["dpre1"], L["ao"][:T], **packed)
+        dctx = cu.linear_dgrad(d_ao, self.view(P, pre + "attention.out_lin.weight"), A["dctx"][:T], **packed)
+        dqkv = buf["dqkv"]
+        ops.attention_bwd(dctx, L["qkv"][:T], self._qkv(P, l, "bias"), fw["mask"], cfg.n_heads, fw["pa"], rng,
+                          sb + _S_PROBS, L["att"], dqkv, self._qkv(G, l, "bias"), **packed)
+        self._wgrad_layer(par, [(df1, L["h1"][:T], self.view(G, pre + "ffn.lin1.weight")),
+                                (d_f2, L["a1"][:T], self.view(G, pre + "ffn.lin2.weight")),
+                                (dqkv, L["h_in"], self._qkv(G, l, "weight")),
+                                (d_ao, L["ctx"][:T], self.view(G, pre + "attention.out_lin.weight"))])
+        cu.linear_dgrad(dqkv, self._qkv(P, l, "weight"), dh, "add", resid=d_pre1, **packed)
+        if on_layer_done is not None:
+            self._wgrad_wait(par)           # the caller may reduce the layer's gradients from here on
+            on_layer_done(l)

@@ -446,6 +446,31 @@ def linear_wgrad(dy, x, dW, bn=0, ncta=0, tmap=None):
     return dW
 
 
+class WgradGroup:
+    """Scratch of :func:`wgrad_group` for one engine: partial tiles (any content) and per-tile counters (zero between
+    launches).  Launches that share it must be ordered."""
+
+    def __init__(self, shapes, device):
+        tiles = sum(((m + 255) // 256) * ((n + 255) // 256) for m, n in shapes)
+        f = lib().rb_wgrad_group_scratch_bytes
+        f.restype = _LL
+        with torch.cuda.device(device):
+            self.scratch = torch.empty(int(f()) // 4, dtype=torch.float32, device=device)
+        self.counters = torch.zeros(2 * tiles, dtype=torch.int32, device=device)
+
+
+def wgrad_group(items, group: WgradGroup, tmap=None):
+    """``dW = dy.T @ x`` for every ``(dy [T, M], x [T, N], dW [M, N])`` of ``items`` (at most four) in one launch."""
+    n, T = len(items), items[0][0].shape[0]
+    dims = (_I * (5 * n))()
+    for i, (dy, x, dW) in enumerate(items):
+        dims[5 * i: 5 * i + 5] = [dy.shape[1], x.shape[1], dy.stride(0), x.stride(0), dW.stride(0)]
+    ws = workspace(items[0][2].device)
+    _call("rb_wgrad_group", _I(DT[items[0][2].dtype]), _I(n), ptr_array([a.data_ptr() for a, _, _ in items]),
+          ptr_array([b.data_ptr() for _, b, _ in items]), ptr_array([c.data_ptr() for _, _, c in items]), dims, _I(T),
+          *_tok(tmap, "meta"), _p(group.scratch), _p(group.counters), _I(group.counters.numel()), _p(ws.status), _stream())
+
+
 def ln_fwd(pre, gamma, beta, eps, y_out, mean, rstd, tmap=None):
     T, H = pre.shape
     _call("rb_ln_fwd", _I(DT[pre.dtype]), _p(pre), _p(gamma), _p(beta), _p(y_out), _p(mean), _p(rstd), _I(T), _I(H),
