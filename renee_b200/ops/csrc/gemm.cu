@@ -139,6 +139,32 @@ __device__ __forceinline__ float warp_colsum32(float (&v)[32], int lane) {
   return v[0];
 }
 
+// First positions of the sorted a[0 .. n) whose values are >= k_lo and >= k_hi, by one warp: each half-warp probes 16 places
+// per step, so ten thousand entries take 4 dependent loads where two binary searches in a row took 28.
+__device__ __forceinline__ void warp_bounds(const int* __restrict__ a, int n, int k_lo, int k_hi, int lane, int& lo, int& hi) {
+  const int i = lane & 15, key = lane < 16 ? k_lo : k_hi;
+  int l = 0, h = n;
+  while (__any_sync(0xffffffffu, l < h)) {
+    const int len = h - l;
+    const bool less = len > 0 && a[l + (int)((long long)len * (i + 1) / 17)] < key;
+    const int c = __popc((__ballot_sync(0xffffffffu, less) >> (lane & 16)) & 0xffffu);      // the probes ascend
+    const int nl = c > 0 ? l + (int)((long long)len * c / 17) + 1 : l;
+    const int nh = c < 16 ? l + (int)((long long)len * (c + 1) / 17) : h;
+    if (len > 0) { l = nl; h = nh; }
+  }
+  lo = __shfl_sync(0xffffffffu, l, 0);
+  hi = __shfl_sync(0xffffffffu, l, 16);
+}
+
+// sigmoid of two logits with one reciprocal: 1 / a = b / (a b).  Below -40 the result is 0 in 16 bits either way, and the
+// bound keeps the product of the denominators finite; a NaN stays one.
+__device__ __forceinline__ void sigmoid2(float x, float y, float& sx, float& sy) {
+  const float dx = 1.f + __expf(-max_nan(x, -40.f)), dy = 1.f + __expf(-max_nan(y, -40.f));
+  const float r = 1.f / (dx * dy);
+  sx = r * dy;
+  sy = r * dx;
+}
+
 // Byte offset of the 16-byte chunk `chunk` (8 columns) of row r inside a 128-byte-swizzled panel.
 __device__ __forceinline__ uint32_t panel_off(int r, int chunk) { return (uint32_t)r * 128u + (uint32_t)((chunk ^ (r & 7)) << 4); }
 
@@ -370,6 +396,10 @@ enc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
       // dropout counters number the padded layout's rows; the word is fetched while the main loop still runs
       int drop_row = row;
       if (EPI == E_BIAS_DROPOUT_RESID && p.tok != nullptr && row < M) drop_row = __ldcg(p.tok + row);
+      // the positives of this CTA's 128 labels: entries pe0 .. pe1 of the label-sorted list, found under the main loop
+      int pe0 = 0, pe1 = 0;
+      if (EPI == E_SIGMOID_POS && p.pos_labels != nullptr && n_pan > 0)
+        warp_bounds(p.pos_labels, *p.nnz_ptr, p.label0 + m0, p.label0 + min(m0 + BM, M), lane, pe0, pe1);
       if (!tc::mbar_wait(tmem_full_bar + buf, use & 1, aborted, p.status, tc::SITE_TMEM_FULL, item)) *s_abort = 1;
       asm volatile("bar.sync 1, %0;" ::"n"(EPI_THREADS) : "memory");
       if (*s_abort) break;                                   // the same answer in every epilogue warp
@@ -409,7 +439,11 @@ enc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
                     if (c + j < p.N) loss += fmaxf(a[j], 0.f) + log1pf(__expf(-fabsf(a[j])));
                 }
 #pragma unroll
-                for (int j = 0; j < 8; ++j) o[j] = (c + j < p.N) ? 1.f / (1.f + __expf(-a[j])) : 0.f;
+                for (int j = 0; j < 8; j += 2) sigmoid2(a[j], a[j + 1], o[j], o[j + 1]);
+                if (c + 8 > p.N) {                       // the columns behind the batch are written as zeros
+#pragma unroll
+                  for (int j = 0; j < 8; ++j) if (c + j >= p.N) o[j] = 0.f;
+                }
               } else if (EPI == E_BIAS_GELU) {
                 float b[8];
                 if (c < p.N) unpack8<T>(__ldg(reinterpret_cast<const uint4*>(reinterpret_cast<const T*>(p.bias) + c)), b);
@@ -493,16 +527,8 @@ enc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
             // subtract 1 at the tile's positives while the tile is still in shared memory: entries of the label-sorted
             // list whose label is one of this CTA's 128 rows and whose batch row is one of the panel's 64 columns
             asm volatile("bar.sync %0, 128;" ::"r"(bar_id) : "memory");      // every row of the panel is written
-            const int nnz = *p.nnz_ptr;
             const int lab_lo = p.label0 + m0;
-            const int lab_hi = p.label0 + min(m0 + BM, M);
-            int lo = 0, hi = nnz;
-            while (lo < hi) { const int mid = (lo + hi) >> 1; if (p.pos_labels[mid] < lab_lo) lo = mid + 1; else hi = mid; }
-            const int e0 = lo;
-            hi = nnz;
-            while (lo < hi) { const int mid = (lo + hi) >> 1; if (p.pos_labels[mid] < lab_hi) lo = mid + 1; else hi = mid; }
-            const int e1 = lo;
-            for (int e = e0 + (int)(threadIdx.x - 64 - 128 * g); e < e1; e += 128) {
+            for (int e = pe0 + (int)(threadIdx.x - 64 - 128 * g); e < pe1; e += 128) {
               const int bcol = p.pos_rows[e] - pcol;
               if (bcol >= 0 && bcol < 64 && pcol + bcol < p.N) {
                 const int prow = p.pos_labels[e] - lab_lo;
