@@ -250,6 +250,11 @@ enc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
     }
   }
   const int n_items = n_m_tiles * p.n_n_tiles * splits;
+  // items of this unit: every n_units-th, or for the logits (few N tiles per M tile) a run of neighbours, so that the
+  // positives of an M tile are looked up once
+  constexpr bool RUNS = EPI == E_SIGMOID_POS;
+  const int per_unit = (n_items + n_units - 1) / n_units;
+  const int it0 = RUNS ? unit * per_unit : unit, it1 = RUNS ? min(n_items, it0 + per_unit) : n_items, its = RUNS ? 1 : n_units;
 
   if (warp == 0 && lane == 0) {
     // ---------------- TMA producer: one continuous stream of (item, k block) stages
@@ -263,7 +268,7 @@ enc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
         if (!wait_flag(p.wait_flags + q, want, p.status, 100 + q)) aborted = true;
       asm volatile("fence.proxy.async;" ::: "memory");
     }
-    for (int item = unit; item < n_items && !aborted; item += n_units) {
+    for (int item = it0; item < it1 && !aborted; item += its) {
       const int tile = item / splits, split = item - tile * splits;
       int mt, nt;
       tile_coords<EPI>(tile, n_m_tiles, p.n_n_tiles, mt, nt);
@@ -310,7 +315,7 @@ enc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
     const uint32_t idesc = tc::make_idesc(FMT, A_MN ? 1 : 0, B_MN ? 1 : 0, BM * NCTA, p.BN);
     int s = 0, t_local = 0;
     uint32_t ph = 0;
-    for (int item = unit; item < n_items && !aborted; item += n_units, ++t_local) {
+    for (int item = it0; item < it1 && !aborted; item += its, ++t_local) {
       const int tile = item / splits, split = item - tile * splits;
       const int kb0 = split * kb_per_split, kb1 = min(kb_total, kb0 + kb_per_split);
       const int buf = t_local & 1;
@@ -369,8 +374,9 @@ enc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
       cv[0] = make_float4(tv[0], tv[1], tv[2], tv[3]); cv[1] = make_float4(tv[4], tv[5], tv[6], tv[7]);
       ci[0] = make_int4(ti[0], ti[1], ti[2], ti[3]); ci[1] = make_int4(ti[4], ti[5], ti[6], ti[7]);
     };
+    int pe0 = 0, pe1 = 0, pos_m = -1;                     // SIGMOID_POS: positives of M tile pos_m
     float loss = 0.f;                                     // SIGMOID_POS: this thread's share of sum softplus(z)
-    for (int item = unit; item < n_items; item += n_units, ++t_local) {
+    for (int item = it0; item < it1; item += its, ++t_local) {
       const int tile = item / splits;
       int mt, nt;
       tile_coords<EPI>(tile, n_m_tiles, p.n_n_tiles, mt, nt);
@@ -397,9 +403,10 @@ enc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
       int drop_row = row;
       if (EPI == E_BIAS_DROPOUT_RESID && p.tok != nullptr && row < M) drop_row = __ldcg(p.tok + row);
       // the positives of this CTA's 128 labels: entries pe0 .. pe1 of the label-sorted list, found under the main loop
-      int pe0 = 0, pe1 = 0;
-      if (EPI == E_SIGMOID_POS && p.pos_labels != nullptr && n_pan > 0)
+      if (EPI == E_SIGMOID_POS && p.pos_labels != nullptr && n_pan > 0 && mt != pos_m) {
+        pos_m = mt;
         warp_bounds(p.pos_labels, *p.nnz_ptr, p.label0 + m0, p.label0 + min(m0 + BM, M), lane, pe0, pe1);
+      }
       if (!tc::mbar_wait(tmem_full_bar + buf, use & 1, aborted, p.status, tc::SITE_TMEM_FULL, item)) *s_abort = 1;
       asm volatile("bar.sync 1, %0;" ::"n"(EPI_THREADS) : "memory");
       if (*s_abort) break;                                   // the same answer in every epilogue warp
