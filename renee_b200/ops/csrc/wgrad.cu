@@ -4,12 +4,15 @@
 // Each of them alone is a poor fit for the chip: at 768 columns they have 9 to 36 tiles of 256 x 256 for 74 SM pairs, so
 // they were split over the tokens, reduced through fp32 atomics in L2 and converted by a last pass -- 29 us per launch,
 // 116 us per layer, at 4900 tokens, where the products take 44 us at the measured cuBLAS rate.  Here the work of all of
-// them is one line of (tile, k block) pairs cut into equal runs, one per pair of SMs ("stream-K"): no partial last wave,
-// and only a tile that a cut falls into is reduced across units.  A unit that holds part of such a tile writes its fp32
+// them is shared out evenly: as many whole tiles per pair of SMs as all pairs get, all walking the tokens in step so that
+// the operands they share come from L2, and before that the left-over tiles, as one line of (tile, k block) pairs cut into
+// equal runs ("stream-K").  (All tiles in one line, without the whole ones: 64 us per layer at 4900 tokens, 140 at 10200;
+// the units then read the operands, 250 MB at 10200 tokens, at unrelated places.)  A tile that a cut falls into is reduced
+// across units.  A unit that holds part of such a tile writes its fp32
 // sums to its own place in a scratch and counts itself; the one that finds all others counted adds their sums to its
 // accumulators, which are still in TMEM, and stores the tile.  Nobody waits for anybody, and the scratch needs no
-// initial value.  Measured: 64 us per layer at 4900 tokens (4 x 29 before); steps 256 x 32 2.74 -> 2.67 ms (the single launches
-// overlapped better with the other stream), 64 x 256 7.06 -> 6.84 ms.
+// initial value.  Measured per layer: 57 us at 4900 tokens
+// (4 x 29 as single split-K launches), 95 at 10200 (164); steps 256 x 32 2.74 -> 2.57 ms, 128 x 128 5.08 -> 4.80 ms.
 //
 // Same structure as gemm.cu: cta_group::2 tiles of 256 x 256 (128 accumulator rows per CTA), warp 0 TMA producer, warp 1
 // MMA issuer, sixteen epilogue warps (a thread owns one row and 64 columns), two accumulators in TMEM, a 7-stage ring that
@@ -71,12 +74,24 @@ __global__ void __launch_bounds__(THREADS, 1) wgrad_group_kernel(const __grid_co
   bool aborted = false;
   grid_dep_wait();
   grid_dep_launch();
-  // this unit's run [x0, x1) of the line of n_tiles * kb (tile, k block) pairs
+  // Work of this unit: a run [x0, x1) of the line of n_cut * kb (tile, k block) pairs of the first n_cut tiles, then every
+  // n_units-th of the other tiles as a whole
   const int rows = p.tok_meta != nullptr ? __ldcg(p.tok_meta + TOK_ROWS) : p.K;
   const int kb = (rows + BK - 1) / BK;
-  const int total = p.n_tiles * kb;
+  const int n_cut = p.n_tiles % n_units;
+  const int total = n_cut * kb;
   const int run = max(min(MIN_RUN, kb), (total + n_units - 1) / n_units);
   const int x0 = min(total, unit * run), x1 = min(total, x0 + run);
+  // The pieces of the run, then the whole tiles: tile, k blocks [k0, k1); x advances along the line, then by whole tiles
+  const int x_end = x1 + (p.n_tiles - n_cut) / n_units;
+  const auto piece = [&](int x, int& tile, int& k0, int& k1) -> int {     // returns the x that follows
+    if (x < x1) {
+      tile = x / kb; k0 = x - tile * kb; k1 = min(kb, k0 + x1 - x);
+      return x + (k1 - k0);
+    }
+    tile = n_cut + (x - x1) * n_units + unit; k0 = 0; k1 = kb;
+    return x + 1;
+  };
   const auto find = [&](int tile, int& m0, int& n0) -> int {
     int i = 0;
     while (i + 1 < p.n_probs && tile >= p.prob[i + 1].first) ++i;
@@ -89,9 +104,9 @@ __global__ void __launch_bounds__(THREADS, 1) wgrad_group_kernel(const __grid_co
   if (warp == 0 && lane == 0) {
     int s = 0;
     uint32_t ph = 0;
-    for (int x = x0; x < x1 && !aborted;) {
-      const int tile = x / kb, k0 = x - tile * kb, k1 = min(kb, k0 + x1 - x);
-      int m0, n0;
+    for (int x = x0; x < x_end && !aborted;) {
+      int tile, k0, k1, m0, n0;
+      x = piece(x, tile, k0, k1);
       const int i = find(tile, m0, n0);
       const int nb = n0 + (int)rank * (BN / 2);
       for (int k = k0; k < k1; ++k, s = (s + 1 == STAGES ? 0 : s + 1), ph ^= (s == 0 ? 1u : 0u)) {
@@ -105,15 +120,15 @@ __global__ void __launch_bounds__(THREADS, 1) wgrad_group_kernel(const __grid_co
         tc::tma_load_2d_pair(sB, &maps.b[i], lbar, nb, k * BK);
         tc::tma_load_2d_pair(sB + 8192, &maps.b[i], lbar, nb + 64, k * BK);
       }
-      x += k1 - k0;
     }
   } else if (warp == 1 && lane == 0 && rank == 0) {
     constexpr int FMT = std::is_same<T, __nv_bfloat16>::value ? 1 : 0;
     const uint32_t idesc = tc::make_idesc(FMT, 1, 1, 2 * BM, BN);
     int s = 0, t_local = 0;
     uint32_t ph = 0;
-    for (int x = x0; x < x1 && !aborted; ++t_local) {
-      const int tile = x / kb, k0 = x - tile * kb, k1 = min(kb, k0 + x1 - x);
+    for (int x = x0; x < x_end && !aborted; ++t_local) {
+      int tile, k0, k1;
+      x = piece(x, tile, k0, k1);
       const int buf = t_local & 1;
       if (!tc::mbar_wait(tmem_empty_bar + buf, (uint32_t)((t_local >> 1) & 1) ^ 1u, aborted, p.status, tc::SITE_TMEM_EMPTY, tile)) break;
       tc::tc_fence_after();
@@ -130,15 +145,13 @@ __global__ void __launch_bounds__(THREADS, 1) wgrad_group_kernel(const __grid_co
       }
       if (aborted) break;
       tc::umma_commit_pair(tmem_full_bar + buf);
-      x += k1 - k0;
     }
   } else if (warp >= 2) {
     const int quarter = warp & 3, g = (warp - 2) >> 2, r = quarter * 32 + lane, et = (int)threadIdx.x - 64;
     int t_local = 0;
-    for (int x = x0; x < x1; ++t_local) {
-      const int tile = x / kb, k0 = x - tile * kb, k1 = min(kb, k0 + x1 - x);
-      x += k1 - k0;
-      int m0, n0;
+    for (int x = x0; x < x_end; ++t_local) {
+      int tile, k0, k1, m0, n0;
+      x = piece(x, tile, k0, k1);
       const Prob& pr = p.prob[find(tile, m0, n0)];
       const int buf = t_local & 1;
       const bool whole = k0 == 0 && k1 == kb;
