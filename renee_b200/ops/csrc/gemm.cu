@@ -582,6 +582,38 @@ enc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
             const float top = max_nan(max_nan(max_nan(m8[0], m8[1]), max_nan(m8[2], m8[3])),
                                       max_nan(max_nan(m8[4], m8[5]), max_nan(m8[6], m8[7])));
             if (top <= tv[7]) continue;
+            if (!__any_sync(__activemask(), tv[7] == -INFINITY)) {
+              // Warm lists: a lane has one or two candidates among its 32 values, but hardly two lanes in the same column.
+              // Every lane steps through its own (bit j of hits), so the warp takes as many insertions as its busiest lane
+              // has candidates, not one per column that any lane has one in (half of them, still, at the 14th fragment).
+              uint32_t hits = 0u;
+#pragma unroll
+              for (int j = 0; j < 32; ++j) hits |= (v[j] <= tv[7] ? 0u : 1u) << j;
+              if (c0 + 32 > p.N) hits &= c0 < p.N ? (1u << (p.N - c0)) - 1u : 0u;
+              while (hits != 0u) {
+                const int j = __ffs(hits) - 1;
+                hits &= hits - 1u;
+                float q16[16], q8[8], q4[4];
+#pragma unroll
+                for (int i = 0; i < 16; ++i) q16[i] = (j & 1) ? v[2 * i + 1] : v[2 * i];
+#pragma unroll
+                for (int i = 0; i < 8; ++i) q8[i] = (j & 2) ? q16[2 * i + 1] : q16[2 * i];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) q4[i] = (j & 4) ? q8[2 * i + 1] : q8[2 * i];
+                const float q0 = (j & 8) ? q4[1] : q4[0], q1 = (j & 8) ? q4[3] : q4[2];
+                const float x = topk_store_value((j & 16) ? q1 : q0);
+                const int col = c0 + j;
+#pragma unroll
+                for (int k = 7; k >= 0; --k) {           // strict: of equal values the lower column stays
+                  const bool up = k > 0 && x > tv[k > 0 ? k - 1 : 0];      // the entry above moves down
+                  const bool here = x > tv[k];
+                  const float nv = up ? tv[k > 0 ? k - 1 : 0] : x;
+                  const int ni = up ? ti[k > 0 ? k - 1 : 0] : col;
+                  if (here) { tv[k] = nv; ti[k] = ni; }
+                }
+              }
+              continue;
+            }
 #pragma unroll
             for (int q = 0; q < 8; ++q) {
               if (m8[q] <= tv[7]) continue;
