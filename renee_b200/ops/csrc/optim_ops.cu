@@ -22,7 +22,22 @@ __global__ void __launch_bounds__(256) grad_check_kernel(const T* __restrict__ g
   if (__any_sync(0xffffffffu, bad) && (threadIdx.x & 31) == 0) hp[HP_FOUND_INF] = 1.0f;
 }
 
-template <typename TG, typename TP>
+// 8 floats in one 256-bit access where the buffer starts on a 32-byte boundary (the flat buffers do), two otherwise.  AdamW is
+// bound by HBM (28 bytes per parameter): 66.4 M parameters 320 -> 301 us (5.8 -> 6.2 TB/s) with the wide accesses.
+template <bool WIDE> __device__ __forceinline__ void load8w(const float* p, float (&v)[8]) {
+  if (WIDE)
+    asm volatile("ld.global.L1::no_allocate.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7]) : "l"(p) : "memory");
+  else load8(p, v);
+}
+template <bool WIDE> __device__ __forceinline__ void store8w(float* p, const float (&v)[8]) {
+  if (WIDE)
+    asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
+                 ::"l"(p), "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7]) : "memory");
+  else store8(p, v);
+}
+
+template <typename TG, typename TP, bool WIDE>
 __global__ void __launch_bounds__(256) adamw_kernel(float* __restrict__ p32, float* __restrict__ m, float* __restrict__ v,
                                                     const TG* __restrict__ g, TP* __restrict__ p16, size_t n_vec,
                                                     size_t n_decay, const float* __restrict__ hp, float beta1, float beta2,
@@ -38,9 +53,9 @@ __global__ void __launch_bounds__(256) adamw_kernel(float* __restrict__ p32, flo
     const size_t e = i * 8;
     float gg[8], pp[8], mm[8], vv[8];
     load8(g + e, gg);
-    load8(p32 + e, pp);
-    load8(m + e, mm);
-    load8(v + e, vv);
+    load8w<WIDE>(p32 + e, pp);
+    load8w<WIDE>(m + e, mm);
+    load8w<WIDE>(v + e, vv);
     const float decay = (e < n_decay) ? 1.f - lr * wd : 1.f;
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
@@ -50,9 +65,9 @@ __global__ void __launch_bounds__(256) adamw_kernel(float* __restrict__ p32, flo
       const float denom = sqrtf(vv[j] * inv_bc2) + eps;
       pp[j] = pp[j] * decay - lr * (mm[j] * inv_bc1) / denom;
     }
-    store8(p32 + e, pp);
-    store8(m + e, mm);
-    store8(v + e, vv);
+    store8w<WIDE>(p32 + e, pp);
+    store8w<WIDE>(m + e, mm);
+    store8w<WIDE>(v + e, vv);
     if (p16 != nullptr) store8(p16 + e, pp);
   }
 }
@@ -102,22 +117,15 @@ RB_API int rb_adamw(int dtype, float* p32, float* m, float* v, const void* g, vo
   if (n % 8 || n_decay % 8) return -3;
   const size_t n_vec = (size_t)n / 8;
   const int blocks = flat_blocks(n_vec);
+  const bool wide = ((reinterpret_cast<uintptr_t>(p32) | reinterpret_cast<uintptr_t>(m) | reinterpret_cast<uintptr_t>(v)) & 31) == 0;
+#define RB_ADAMW(T, W) adamw_kernel<T, T, W><<<blocks, 256, 0, st>>>(p32, m, v, (const T*)g, (T*)p16, n_vec, (size_t)n_decay, hp, beta1, beta2, eps, wd, grad_mult)
   switch (dtype) {
-    case RB_F32:
-      adamw_kernel<float, float><<<blocks, 256, 0, st>>>(p32, m, v, (const float*)g, (float*)p16, n_vec, (size_t)n_decay,
-                                                           hp, beta1, beta2, eps, wd, grad_mult);
-      break;
-    case RB_BF16:
-      adamw_kernel<__nv_bfloat16, __nv_bfloat16><<<blocks, 256, 0, st>>>(p32, m, v, (const __nv_bfloat16*)g,
-                                                                         (__nv_bfloat16*)p16, n_vec, (size_t)n_decay, hp,
-                                                                         beta1, beta2, eps, wd, grad_mult);
-      break;
-    case RB_F16:
-      adamw_kernel<__half, __half><<<blocks, 256, 0, st>>>(p32, m, v, (const __half*)g, (__half*)p16, n_vec,
-                                                           (size_t)n_decay, hp, beta1, beta2, eps, wd, grad_mult);
-      break;
+    case RB_F32: if (wide) RB_ADAMW(float, true); else RB_ADAMW(float, false); break;
+    case RB_BF16: if (wide) RB_ADAMW(__nv_bfloat16, true); else RB_ADAMW(__nv_bfloat16, false); break;
+    case RB_F16: if (wide) RB_ADAMW(__half, true); else RB_ADAMW(__half, false); break;
     default: return -1;
   }
+#undef RB_ADAMW
   RB_LAUNCH_CHECK();
   return 0;
 }
