@@ -196,6 +196,22 @@ __device__ __forceinline__ void write_rows(const float (&out)[NJ][4], T* dst, in
   }
 }
 
+// Elements idx, idx + 1 of a [.., S] row as one packed word, ok0 / ok1 saying which exist (0 for the others); `pair` =
+// 4-byte access allowed.  Issued well before the use: the backward kernels spent most of their time waiting for the stored
+// probabilities one tile after another.
+template <typename T>
+__device__ __forceinline__ uint32_t load_pair_raw(const T* __restrict__ base, size_t idx, bool ok0, bool ok1, bool pair) {
+  uint32_t r = 0u;
+  if (ok0) {
+    if (pair) r = *reinterpret_cast<const uint32_t*>(base + idx);
+    else {
+      r = *reinterpret_cast<const uint16_t*>(base + idx);
+      if (ok1) r |= (uint32_t)*reinterpret_cast<const uint16_t*>(base + idx + 1) << 16;
+    }
+  }
+  return r;
+}
+
 // Stages (q + bq, k + bk, v + bv [, dO]) of one (batch, head) as [SP][RP] tiles; rows of tokens that do not
 // exist are zero, rows >= lim are left alone.
 // The CTA has SP * 2 threads and the tiles SP * HD / 8 segments of 8 columns, so a thread owns the same 8 columns of
@@ -354,7 +370,7 @@ __global__ void __launch_bounds__(SP * 2, SP == 128 ? 2 : 1) attention_fwd_mma_k
 }
 
 template <typename T, int SP, int HD>
-__global__ void __launch_bounds__(SP * 2) attention_bwd_mma_kernel(
+__global__ void __launch_bounds__(SP * 2, SP == 64 ? 4 : 1) attention_bwd_mma_kernel(
     const T* __restrict__ dctx, const T* __restrict__ qkv, const T* __restrict__ bqkv, const T* __restrict__ probs,
     T* __restrict__ dqkv, int S, int H, int nh, float p, const int* __restrict__ seed_ptr, uint32_t stream,
     float* __restrict__ bias_acc, const Tok tk, int len_lo) {
@@ -384,9 +400,19 @@ __global__ void __launch_bounds__(SP * 2) attention_bwd_mma_kernel(
   const int len = seq_len(tk, b, S), lim = (len + 15) & ~15;
   if (len > SP || len <= len_lo) return;       // another launch serves this length
   for (int j = threadIdx.x; j < SP; j += blockDim.x) sRow[j] = j < len ? seq_row(tk, b, S, j) : -1;
+  const int r0 = warp * 16;
+  const int i0 = r0 + g, i1 = r0 + g + 8;
+  const size_t prow0 = ((size_t)(b * nh + h) * S + i0) * S, prow1 = ((size_t)(b * nh + h) * S + i1) * S;
+  const bool pair_load = (S & 1) == 0;
+  uint32_t wf[SP / 8][2];     // the probabilities of rows i0 / i1 (of rows that are no kept token: anything)
+#pragma unroll
+  for (int j = 0; j < SP / 8; ++j) {
+    const int c = 8 * j + 2 * t;
+    wf[j][0] = load_pair_raw<T>(probs, prow0 + c, r0 < lim && 8 * j < lim && i0 < S && c < S, c + 1 < S, pair_load);
+    wf[j][1] = load_pair_raw<T>(probs, prow1 + c, r0 < lim && 8 * j < lim && i1 < S && c < S, c + 1 < S, pair_load);
+  }
   stage_operands<T, SP, HD, true>(qkv, bqkv, dctx, sQ, sK, sV, sDO, tk, b, h, S, H, len, lim);
   __syncthreads();
-  const int r0 = warp * 16;
   const int row0 = sRow[r0 + g], row1 = sRow[r0 + g + 8];
   if (r0 < lim) {
     // dP for this warp's 16 query rows, then dS and P~ in registers
@@ -394,24 +420,14 @@ __global__ void __launch_bounds__(SP * 2) attention_bwd_mma_kernel(
 #pragma unroll
     for (int j = 0; j < SP / 8; ++j) { acc[j][0] = 0.f; acc[j][1] = 0.f; acc[j][2] = 0.f; acc[j][3] = 0.f; }
     rows_times_transposed<T, SP, HD>(acc, sDO, sV, r0, lane, lim);
-    const int i0 = r0 + g, i1 = r0 + g + 8;
-    const size_t prow0 = ((size_t)(b * nh + h) * S + i0) * S, prow1 = ((size_t)(b * nh + h) * S + i1) * S;
-    const bool pair_load = (S & 1) == 0;
-    uint32_t wf[SP / 8][2];   // P~ pairs of rows i0 / i1, later the probabilities' products
     float dot0 = 0.f, dot1 = 0.f;
 #pragma unroll
     for (int j = 0; j < SP / 8; ++j) {
       if (8 * j >= lim) continue;
       const int c = 8 * j + 2 * t;
-      float2 pr0 = make_float2(0.f, 0.f), pr1 = make_float2(0.f, 0.f);
-      if (row0 >= 0 && c < S) {
-        if (pair_load) pr0 = Pack<T>::unpack(*reinterpret_cast<const uint32_t*>(probs + prow0 + c));
-        else { pr0.x = to_f(probs[prow0 + c]); if (c + 1 < S) pr0.y = to_f(probs[prow0 + c + 1]); }
-      }
-      if (row1 >= 0 && c < S) {
-        if (pair_load) pr1 = Pack<T>::unpack(*reinterpret_cast<const uint32_t*>(probs + prow1 + c));
-        else { pr1.x = to_f(probs[prow1 + c]); if (c + 1 < S) pr1.y = to_f(probs[prow1 + c + 1]); }
-      }
+      if (row0 < 0) wf[j][0] = 0u;
+      if (row1 < 0) wf[j][1] = 0u;
+      const float2 pr0 = Pack<T>::unpack(wf[j][0]), pr1 = Pack<T>::unpack(wf[j][1]);
       float m00 = 1.f, m01 = 1.f, m10 = 1.f, m11 = 1.f;
       if (p > 0.f) {
         m00 = keep(seed, stream, (uint32_t)(prow0 + c), p) ? inv_keep : 0.f;
@@ -427,8 +443,6 @@ __global__ void __launch_bounds__(SP * 2) attention_bwd_mma_kernel(
       const uint32_t w0 = Pack<T>::pack(pr0.x * m00, pr0.y * m01), w1 = Pack<T>::pack(pr1.x * m10, pr1.y * m11);
       *reinterpret_cast<uint32_t*>(sW + i0 * PP + c) = w0;
       *reinterpret_cast<uint32_t*>(sW + i1 * PP + c) = w1;
-      wf[j][0] = Pack<T>::pack(pr0.x, pr0.y);   // exact: the probabilities are already T values
-      wf[j][1] = Pack<T>::pack(pr1.x, pr1.y);
     }
     dot0 = quad_sum(dot0); dot1 = quad_sum(dot1);
     uint32_t dsf[SP / 16][4];   // dS as the A operand of dQ = dS K
@@ -670,6 +684,13 @@ __global__ void __launch_bounds__(SP * 2, SP == 128 ? 2 : 1) attention_bwd_blk_k
       const int k0 = kb * KB;
       kept[kb] = 0xffffffffu;
       if (k0 >= lim) continue;
+      uint32_t w0[KB / 8], w1[KB / 8];             // the block's probabilities, on their way during the products
+#pragma unroll
+      for (int j = 0; j < KB / 8; ++j) {
+        const int key = k0 + 8 * j + 2 * t;
+        w0[j] = load_pair_raw<T>(probs, prow0 + key, row0 >= 0 && k0 + 8 * j < lim && key < S, key + 1 < S, pair);
+        w1[j] = load_pair_raw<T>(probs, prow1 + key, row1 >= 0 && k0 + 8 * j < lim && key < S, key + 1 < S, pair);
+      }
       float acc[KB / 8][4];
 #pragma unroll
       for (int j = 0; j < KB / 8; ++j) { acc[j][0] = 0.f; acc[j][1] = 0.f; acc[j][2] = 0.f; acc[j][3] = 0.f; }
@@ -679,8 +700,7 @@ __global__ void __launch_bounds__(SP * 2, SP == 128 ? 2 : 1) attention_bwd_blk_k
       for (int j = 0; j < KB / 8; ++j) {
         if (k0 + 8 * j >= lim) continue;
         const int key = k0 + 8 * j + 2 * t;
-        const float2 pr0 = load_pair<T>(probs, prow0 + key, row0 >= 0 && key < S, key + 1 < S, pair);
-        const float2 pr1 = load_pair<T>(probs, prow1 + key, row1 >= 0 && key < S, key + 1 < S, pair);
+        const float2 pr0 = Pack<T>::unpack(w0[j]), pr1 = Pack<T>::unpack(w1[j]);
         float m00 = 1.f, m01 = 1.f, m10 = 1.f, m11 = 1.f;
         if (p > 0.f) {
           const bool a = keep(seed, stream, (uint32_t)(prow0 + key), p), c = keep(seed, stream, (uint32_t)(prow0 + key + 1), p);
@@ -703,6 +723,13 @@ __global__ void __launch_bounds__(SP * 2, SP == 128 ? 2 : 1) attention_bwd_blk_k
     const int k0 = kb * KB;
     if (k0 >= lim) break;                          // the same answer in every thread
     if (active) {
+      uint32_t w0[KB / 8], w1[KB / 8];             // the block's probabilities, on their way during the products
+#pragma unroll
+      for (int j = 0; j < KB / 8; ++j) {
+        const int key = k0 + 8 * j + 2 * t;
+        w0[j] = load_pair_raw<T>(probs, prow0 + key, row0 >= 0 && k0 + 8 * j < lim && key < S, key + 1 < S, pair);
+        w1[j] = load_pair_raw<T>(probs, prow1 + key, row1 >= 0 && k0 + 8 * j < lim && key < S, key + 1 < S, pair);
+      }
       float acc[KB / 8][4];
 #pragma unroll
       for (int j = 0; j < KB / 8; ++j) { acc[j][0] = 0.f; acc[j][1] = 0.f; acc[j][2] = 0.f; acc[j][3] = 0.f; }
@@ -711,9 +738,7 @@ __global__ void __launch_bounds__(SP * 2, SP == 128 ? 2 : 1) attention_bwd_blk_k
 #pragma unroll
       for (int j = 0; j < KB / 8; ++j) {
         if (k0 + 8 * j >= lim) continue;
-        const int key = k0 + 8 * j + 2 * t;
-        const float2 pr0 = load_pair<T>(probs, prow0 + key, row0 >= 0 && key < S, key + 1 < S, pair);
-        const float2 pr1 = load_pair<T>(probs, prow1 + key, row1 >= 0 && key < S, key + 1 < S, pair);
+        const float2 pr0 = Pack<T>::unpack(w0[j]), pr1 = Pack<T>::unpack(w1[j]);
         const uint32_t bits = kept[kb] >> (4 * j);
         const float m00 = (bits & 1u) ? inv_keep : 0.f, m01 = (bits & 2u) ? inv_keep : 0.f;
         const float m10 = (bits & 4u) ? inv_keep : 0.f, m11 = (bits & 8u) ? inv_keep : 0.f;
