@@ -33,7 +33,8 @@ def lib():
     return _LIB
 
 
-LN_BWD_WARPS = 4     # warps per CTA of the LayerNorm backward kernel (4, 8 or 16; RENEE_B200_LN_BWD_WARPS overrides).  Measured:
+LN_BWD_WARPS = 4     # warps per CTA of the general LayerNorm backward kernel (fp32, or more than 1024 columns; 4, 8 or 16;
+                     # RENEE_B200_LN_BWD_WARPS overrides).  Measured when it still served 16-bit activations:
                      # 8192 x 768 alone 34.9 / 29.2 / 30.6 us with 4 / 8 / 16, but the training step does not gain (3.75 /
                      # 3.74 / 3.73 ms at 8192 tokens) and loses 5 % at 4096 tokens per GPU (2.43 / 2.56 / 2.57 ms)
 
@@ -670,6 +671,9 @@ def topk_rows(Z, n, k, label0, out_val, out_idx):
     _call("rb_topk_rows", _p(Z), _I(ldZ), _I(B), _I(n), _I(k), _I(label0), _p(out_val), _p(out_idx), _stream())
 
 
+TOPK_ROWS = 8192
+
+
 def xfc_topk8(W, X, k):
     """Top-k of every row of ``X Wᵀ`` with the selection fused into the GEMM epilogue: each epilogue thread of the
     persistent tcgen05 GEMM keeps the 8 best entries of its row over all label tiles its CTA visits, so the ``[B, Ls]``
@@ -678,6 +682,9 @@ def xfc_topk8(W, X, k):
     descending, label ids [B, k] int64)``."""
     B, D = X.shape
     Ls = W.shape[0]
+    if B > TOPK_ROWS:                      # bounds the candidates (2368 per row on 148 SMs: 155 MB)
+        parts = [xfc_topk8(W, X[i: i + TOPK_ROWS], k) for i in range(0, B, TOPK_ROWS)]
+        return torch.cat([v for v, _ in parts]), torch.cat([i for _, i in parts])
     plan = (_I * 6)()
     rc = lib().rb_xfc_topk_plan(_I(B), _I(Ls), _I(D), plan)
     if rc != 0:
