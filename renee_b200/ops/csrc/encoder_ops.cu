@@ -325,7 +325,7 @@ __device__ __forceinline__ void smem_add8(float* p, const float (&v)[8]) {
 }
 
 template <typename T, int NV, bool EMBED, int WARPS = 4>
-__global__ void __launch_bounds__(WARPS * 32, WARPS == 4 ? 6 : (WARPS == 8 ? 2 : 1)) ln_bwd_kernel(
+__global__ void __launch_bounds__(WARPS * 32, WARPS == 4 ? (EMBED ? 5 : 6) : (WARPS == 8 ? 2 : 1)) ln_bwd_kernel(
     const T* __restrict__ dy, const T* __restrict__ pre, const int* __restrict__ ids,
     const T* __restrict__ word, const T* __restrict__ pos, const T* __restrict__ gamma,
     const float* __restrict__ mean, const float* __restrict__ rstd,
@@ -358,16 +358,27 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 4 ? 6 : (WARPS == 8 ? 2 :
     const int col = (lane + 32 * i) * 8;
     if (col < H) gam[i] = load_raw8<T>(gamma + col);
   }
+  // EMBED: the next token's packed row and id are on their way while this one is worked on (every load of a token hangs
+  // on them), and a dropout decision is hashed once: 128 x 128 tokens 61 -> 43 us
+  int next_row = -1, next_id = 0;
+  if (EMBED && warp < rows) {
+    next_row = tok != nullptr ? __ldcg(tok + warp) : warp;
+    next_id = ids[warp];
+  }
   for (int row0 = warp; row0 < rows; row0 += total_warps) {
-    const int row = EMBED && tok != nullptr ? __ldcg(tok + row0) : row0;       // row of the stored activations
+    const int row = EMBED ? next_row : row0;                                   // row of the stored activations
+    const int id = EMBED ? next_id : 0;
+    if (EMBED && row0 + total_warps < rows) {
+      next_row = tok != nullptr ? __ldcg(tok + row0 + total_warps) : row0 + total_warps;
+      next_id = ids[row0 + total_warps];
+    }
     if (EMBED && row < 0) continue;
+    uint32_t kept[EMBED ? (NV + 3) / 4 : 1] = {};                              // dropout decisions, bit 8 (i % 4) + j
     const int crow = !EMBED && tok != nullptr && p > 0.f ? __ldcg(tok + row0) : row0;   // row of the dropout counters
     const float mu = mean[row], rs = rstd[row];
     // dy and the LN input stay packed across the two warp reductions
     Raw8<T> rd[NV], rx[NV], rb[NV];
     float s1 = 0.f, s2 = 0.f;
-    int id = 0;
-    if (EMBED) id = ids[row0];
 #pragma unroll
     for (int i = 0; i < NV; ++i) {
       const int col = (lane + 32 * i) * 8;
@@ -395,7 +406,11 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 4 ? 6 : (WARPS == 8 ? 2 :
 #pragma unroll
           for (int j = 0; j < 8; ++j) {
             x[j] += b[j];
-            if (p > 0.f) d[j] = keep(seed, stream, (uint32_t)(crow * H + col + j), p) ? d[j] * inv_keep : 0.f;
+            if (p > 0.f) {
+              const bool on = keep(seed, stream, (uint32_t)(crow * H + col + j), p);
+              if (on) kept[EMBED ? i / 4 : 0] |= 1u << (8 * (i % 4) + j);
+              d[j] = on ? d[j] * inv_keep : 0.f;
+            }
           }
         }
 #pragma unroll
@@ -426,7 +441,7 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 4 ? 6 : (WARPS == 8 ? 2 :
 #pragma unroll
           for (int j = 0; j < 8; ++j) {
             x[j] += b[j];
-            if (p > 0.f) d[j] = keep(seed, stream, (uint32_t)(crow * H + col + j), p) ? d[j] * inv_keep : 0.f;
+            if (p > 0.f) d[j] = (kept[EMBED ? i / 4 : 0] >> (8 * (i % 4) + j)) & 1u ? d[j] * inv_keep : 0.f;
           }
         }
 #pragma unroll
