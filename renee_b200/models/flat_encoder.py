@@ -14,7 +14,7 @@ so this engine is built for CUDA-graph capture instead:
   linear layer is an own tcgen05 GEMM (``ops/csrc/gemm.cu``) whose epilogue carries its element-wise
   neighbours: bias + GELU (storing the pre-activation), bias + dropout + residual (producing the
   LayerNorm input), GELU backward + bias-gradient column sums, the residual-gradient add of the
-  data-gradient GEMMs, and a split-K weight-gradient GEMM.  fp32 activations (CPU, debugging mode) use
+  data-gradient GEMMs; the weight gradients of a layer are one launch (``ops/csrc/wgrad.cu``).  fp32 activations (CPU, debugging mode) use
   library GEMMs and stand-alone element-wise ops;
 * on that path padded tokens are left out: the activations hold packed rows (``ops/csrc/token_map.cuh``), whose number
   the kernels read from the device, so one captured graph serves every batch of its padded shape.  Texts are shorter
@@ -61,8 +61,8 @@ def own_gemm_pays(rows: int, T: int, H: int) -> bool:
     1024 padded tokens all kept 1401 / 1189, 608 kept 1343 / 1190; 2048: 1675 / 1445, 1216 kept 1480 / 1503; 4096: 2131 /
     2125, 2432 kept 1848 / 2120; 6144: 2645 / 2663, 3648 kept 2117 / 2647 -- the own launches cost 1150 + 0.245 per row,
     the library's 880 + 0.30 per padded token.  384 columns (MiniLM) cross at the same places; narrow encoders (128
-    columns, 2 layers: 238 / 256 at 1024 tokens, 378 / 418 at 8192) gain at every size."""
-    return H < 256 or rows < 1.22 * T - 1100
+    columns, 2 layers) are even at 1024 tokens and gain from 2048 on, all kept or not (261 / 272, 4096: 312 / 322)."""
+    return T >= 2048 if H < 256 else rows < 1.22 * T - 1100
 
 
 @dataclass
@@ -234,13 +234,9 @@ class FlatEncoder:
         self._acts = dict(h0=e(T, H), mean0=e(T, dtype=torch.float32), rstd0=e(T, dtype=torch.float32),
                           layers=layers, pooled=e(b, H, dtype=torch.float32),
                           dh=e(T, H), dh_b=e(T, H), dqkv=e(T, 3 * H), dctx=e(T, H), df1=e(T, Fd), da1=e(T, Fd),
-                          emb=e(b, self.out_dims, dtype=torch.float32), tmap=None)
+                          emb=e(b, self.out_dims, dtype=torch.float32), tmap=None, bwd=None)
         if self._own_supported and dev.type == "cuda":
             from ..ops import cuda as cu
-            # gradients that the weight-gradient launch of a layer still reads while the next layer is differentiated
-            self._acts["bwd"] = [dict(dpre2=e(T, H), dpre1=e(T, H), df1=e(T, Fd), dqkv=e(T, 3 * H)) for _ in range(2)]
-            if self._wgrad_group is None:
-                self._wgrad_group = cu.WgradGroup([(3 * H, H), (H, H), (Fd, H), (H, Fd)], dev)
             if cu.attention_packs(dt, S, H, nh):
                 self._acts["tmap"] = cu.TokenMap(b, S, dev)
         self._acts_key = key
@@ -406,6 +402,8 @@ class FlatEncoder:
             d_pool = torch.mm(d_emb, self.bottleneck_weight())
         else:
             d_pool = d_emb
+        if self.own_gemm:
+            self._ensure_backward_buffers()
         dh = A["dh"][:T]
         ops.pool_bwd(d_pool, mask, self.pooling, S, dh.view(b, S, H), **packed)
         for l in reversed(range(cfg.n_layers)):
@@ -456,6 +454,20 @@ class FlatEncoder:
                          self.view(G, "embeddings.LayerNorm.weight"), self.view(G, "embeddings.LayerNorm.bias"), **packed)
         self._wgrad_wait(0)
         self._wgrad_wait(1)
+
+    def _ensure_backward_buffers(self) -> None:
+        """Two sets of the gradients that the weight-gradient launch of a layer still reads while the next layer is
+        differentiated, and that launch's scratch: allocated by the first backward pass on the own GEMMs."""
+        if self._acts["bwd"] is not None:
+            return
+        from ..ops import cuda as cu
+        (b, S), H, Fd = self._acts_key, self.cfg.dim, self.cfg.hidden_dim
+        widths = (("dpre2", H), ("dpre1", H), ("df1", Fd), ("dqkv", 3 * H))
+        sizes = [b * S * n for _, n in widths] * 2
+        flat = guard.empty(sum(sizes), dtype=self.act_dtype, device=self.device, name="encoder.bwd").split(sizes)
+        self._acts["bwd"] = [{k: flat[4 * i + j].view(b * S, n) for j, (k, n) in enumerate(widths)} for i in range(2)]
+        if self._wgrad_group is None:
+            self._wgrad_group = cu.WgradGroup([(3 * H, H), (H, H), (Fd, H), (H, Fd)], self.device)
 
     def _backward_layer_fused(self, l: int, L: dict, dh, on_layer_done) -> None:
         """One transformer block on the own GEMMs: ``dh`` (gradient of its output) becomes the gradient of its input."""

@@ -196,9 +196,9 @@ class TokenMap:
     plan tiles only; 0 = plan for the padded count."""
 
     def __init__(self, b: int, S: int, device):
-        z = lambda n: torch.zeros(n, dtype=torch.int32, device=device)
-        self.tok, self.slot = z(b * S), z(b * S)
-        self.off, self.len, self.cnt, self.meta = z(b), z(b), z(b), z(4)
+        n = b * S
+        z = torch.zeros(2 * n + 3 * b + 4, dtype=torch.int32, device=device)
+        self.tok, self.slot, self.off, self.len, self.cnt, self.meta = z.split([n, n, b, b, b, 4])
         self.rows_hint = 0
 
     def update(self, mask) -> None:
