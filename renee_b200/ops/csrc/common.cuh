@@ -109,12 +109,12 @@ template <typename T> __device__ __forceinline__ float round_through(float x) { 
 // fp32 -> fp16 with stochastic rounding: add uniform noise below the 13 mantissa bits fp16 drops, then
 // truncate.  Unbiased for values in fp16's normal range, which keeps updates smaller than half an ulp
 // of W from being lost systematically late in the learning-rate schedule.
-// Two neighbours at once, packed: the low half of rnd is the noise of the first, the high half that of the second (fp16
-// drops 13 bits, bf16 16).  The masking keeps an infinity one; the conversion truncates what lies below fp16's range.
-template <typename T> __device__ __forceinline__ uint32_t sr_pack2(float x, float y, uint32_t rnd) {
+// Two neighbours at once, packed; rx and ry are the random words of the two (fp16 drops 13 bits, bf16 16).  The masking
+// keeps an infinity one; the conversion truncates what lies below fp16's range.
+template <typename T> __device__ __forceinline__ uint32_t sr_pack2(float x, float y, uint32_t rx, uint32_t ry) {
   constexpr uint32_t kNoise = std::is_same<T, __half>::value ? 0x1FFFu : 0xFFFFu;
-  const float a = __uint_as_float((__float_as_uint(x) + (rnd & kNoise)) & ~kNoise);
-  const float b = __uint_as_float((__float_as_uint(y) + ((rnd >> 16) & kNoise)) & ~kNoise);
+  const float a = __uint_as_float((__float_as_uint(x) + (rx & kNoise)) & ~kNoise);
+  const float b = __uint_as_float((__float_as_uint(y) + (ry & kNoise)) & ~kNoise);
   uint32_t r;
   if (std::is_same<T, __half>::value) asm("cvt.rz.f16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(b), "f"(a));
   else asm("cvt.rz.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(b), "f"(a));

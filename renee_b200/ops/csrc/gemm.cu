@@ -484,9 +484,8 @@ enc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
 #pragma unroll
                 for (int j = 0; j < 8; ++j) o[j] = a[j] + res[j];
               } else if (EPI == E_DW_SGD) {
-                // momentum SGD on the tile: m = mo m + (dW + wd w), w -= lr m, with m rounded to 16 bit first.  With one
-                // element at a time and a hash each this was some 40 instructions per element, more than the tile's
-                // bytes take: two per instruction and per hash.
+                // momentum SGD on the tile: m = mo m + (dW + wd w), w -= lr m, with m rounded to 16 bit first.  One element
+                // at a time this was some 40 instructions per element, more than the tile's bytes take: two per instruction.
                 uint4* slot2 = reinterpret_cast<uint4*>(pan2 + panel_off(r, chunk));
                 float w[8], mm[8];
                 unpack8<T>(*slot, w);
@@ -503,11 +502,11 @@ enc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
                 for (int j = 0; j < 8; j += 2) f2_get(f2_fma(nlr, f2(mm[j], mm[j + 1]), f2(w[j], w[j + 1])), o[j], o[j + 1]);
                 *slot2 = m16;
                 if (p.stochastic_round) {
-                  // one hash per pair of elements: its halves are the noise of the two
-                  uint4 w16;
+                  uint4 w16;                               // every element has a hash of its own number
                   uint32_t* wp = reinterpret_cast<uint32_t*>(&w16);
 #pragma unroll
-                  for (int j = 0; j < 8; j += 2) wp[j >> 1] = sr_pack2<T>(o[j], o[j + 1], mix32(sr_seed, 0x5152u, (e + j) >> 1));
+                  for (int j = 0; j < 8; j += 2)
+                    wp[j >> 1] = sr_pack2<T>(o[j], o[j + 1], mix32(sr_seed, 0x5152u, e + j), mix32(sr_seed, 0x5152u, e + j + 1));
                   *slot = w16;
                 } else {
                   *slot = pack8<T>(o);

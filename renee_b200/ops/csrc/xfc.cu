@@ -590,7 +590,8 @@ xfc_dw_sgd_tma_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
             const float2 ms = __half22float2(m2[j]);
             if (p.stochastic_round) {
               const uint32_t e = (uint32_t)(m0 + r) * (uint32_t)p.ldW + (uint32_t)(n0 + c0 + 8 * j8 + 2 * j);
-              *reinterpret_cast<uint32_t*>(w2 + j) = sr_pack2<__half>(w.x - lr * ms.x, w.y - lr * ms.y, mix32(sr_seed, 0x5152u, e >> 1));
+              *reinterpret_cast<uint32_t*>(w2 + j) = sr_pack2<__half>(w.x - lr * ms.x, w.y - lr * ms.y, mix32(sr_seed, 0x5152u, e),
+                                                                              mix32(sr_seed, 0x5152u, e + 1));
             } else {
               w2[j] = __floats2half2_rn(w.x - lr * ms.x, w.y - lr * ms.y);
             }

@@ -226,11 +226,10 @@ def xfc_dw_sgd(Gt, X, W, M, lr, mo, wd, dW_acc=None, sr_seed=None):
 def stochastic_round_fp16(x: torch.Tensor, seed: int, stream: int = 0x5152) -> torch.Tensor:
     """fp32 -> fp16 with stochastic rounding, the arithmetic of the dW kernel's epilogue (``sr_pack2``): add
     13 uniform random bits below the mantissa bits fp16 keeps, then truncate.  Unbiased in fp16's normal range.
-    The random bits come from the counter-based hash of the number of the pair of neighbouring elements: bits 0..12 for
-    the first, 16..28 for the second."""
+    The random bits come from the counter-based hash of the element index."""
     from .rng import mix32
     idx = torch.arange(x.numel(), dtype=torch.int64, device=x.device)
-    rnd = (mix32(int(seed), stream, idx >> 1) >> (16 * (idx & 1))) & 0x1FFF
+    rnd = mix32(int(seed), stream, idx) & 0x1FFF
     bits = x.float().contiguous().view(torch.int32).view(-1).to(torch.int64) & 0xFFFFFFFF
     bits = ((bits + rnd) & 0xFFFFFFFF) & ~0x1FFF
     bits = torch.where(bits >= 2 ** 31, bits - 2 ** 32, bits).to(torch.int32)
