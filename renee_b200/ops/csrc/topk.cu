@@ -163,7 +163,11 @@ __global__ void __launch_bounds__(THREADS) topk_select_kernel(const Args a, cons
       if (!doubt[l]) continue;
       const int c_lo = (l % TOPK_GROUPS) * ucols, c_hi = min(a.bn, c_lo + ucols);
       for (int tile = topk_unit_first(l / TOPK_GROUPS, a.units, first, step, a.n_n); tile < first + step * a.n_n; tile += a.units) {
-        if (s_extra + TILE_COLS > EXTRA) {                       // make room: keep the k best so far
+        // every thread reads the count between two barriers, so all take the branch (which has barriers of its own) or
+        // none: without the second one a fast warp's first append of this tile could still change what a slow warp reads
+        const bool full = s_extra + TILE_COLS > EXTRA;
+        __syncthreads();
+        if (full) {                                              // make room: keep the k best so far
           t = kth_key(key, cap, a.k, s_count);
           gather_best(key, idx, cap, a.k, t, win, s_slots);
           for (int i = tid; i < cap; i += THREADS) {
