@@ -235,12 +235,15 @@ class FlatEncoder:
                           layers=layers, pooled=e(b, H, dtype=torch.float32),
                           dh=e(T, H), dh_b=e(T, H), dqkv=e(T, 3 * H), dctx=e(T, H), df1=e(T, Fd), da1=e(T, Fd),
                           emb=e(b, self.out_dims, dtype=torch.float32), tmap=None, bwd=None)
-        if self._own_supported and dev.type == "cuda":
+        if self._own_supported and dev.type == "cuda" and self._packs(S):
             from ..ops import cuda as cu
-            if cu.attention_packs(dt, S, H, nh):
-                self._acts["tmap"] = cu.TokenMap(b, S, dev)
+            self._acts["tmap"] = cu.TokenMap(b, S, dev)
         self._acts_key = key
         self.generation += 1      # activation addresses changed: graphs captured over the old ones are stale
+
+    def _packs(self, S: int) -> bool:
+        from ..ops import cuda as cu
+        return cu.attention_packs(self.act_dtype, S, self.cfg.dim, self.cfg.n_heads)
 
     # ------------------------------------------------------------------ forward
     def forward(self, input_ids: torch.Tensor, attention_mask: torch.Tensor, rng, train: bool = True) -> torch.Tensor:
@@ -258,7 +261,8 @@ class FlatEncoder:
         pd = cfg.dropout if train else 0.0
         pa = cfg.attention_dropout if train else 0.0
         po = cfg.attn_output_dropout if train else 0.0
-        tmap = A["tmap"] if self.own_gemm and self.pack_tokens else None
+        # asked again on every pass: the environment may have sent attention to kernels that read the padded layout
+        tmap = A["tmap"] if self.own_gemm and self.pack_tokens and self._packs(S) else None
         packed = {}
         if tmap is not None:
             tmap.rows_hint = min(self.rows_hint, T)

@@ -228,11 +228,23 @@ def embed_ln_bwd(dy, ids, word, pos, gamma, mean, rstd, S, p, rng, stream, pad_i
           _F(p), _p(rng.dev), _U(stream), *_tok(tmap, "slot"), _stream())
 
 
+def _packed_kernels(dtype, S: int, hd: int) -> str | None:
+    """The kernels of attention_mma.cu that serve packed tokens of this shape: "mma", "long" or none."""
+    if dtype == torch.float32 or hd not in (32, 64):
+        return None
+    if S <= 128 or (S <= 256 and hd == 64):
+        return "mma"
+    return "long" if S <= 512 and hd == 64 else None
+
+
 def attention_packs(dtype, S: int, H: int, nh: int) -> bool:
-    """Whether the attention kernels that serve this shape understand packed tokens (those of attention_mma.cu do)."""
-    if dtype == torch.float32 or H // nh not in (32, 64) or os.environ.get("RENEE_B200_ATTENTION", "") == "tiles":
+    """Whether activations of this shape may hold packed tokens: the kernels exist, and the environment does not ask for the
+    padded ones."""
+    if os.environ.get("RENEE_B200_ATTENTION", "") == "tiles":
         return False
-    return S <= 128 or (S <= 512 and H // nh == 64 and os.environ.get("RENEE_B200_ATTENTION_LONG", "") != "0")
+    if S > 128 and os.environ.get("RENEE_B200_ATTENTION_LONG", "") == "0":
+        return False
+    return _packed_kernels(dtype, S, H // nh) is not None
 
 
 def _attention_fits(qkv, S: int, H: int, nh: int) -> bool:
@@ -262,6 +274,24 @@ def _attention_long(qkv, S: int, H: int, nh: int, ws) -> bool:
             and os.environ.get("RENEE_B200_ATTENTION_LONG", "") != "0")
 
 
+def _attention_route(qkv, S: int, H: int, nh: int, ws, direction: str, tmap):
+    """``(entry or "composed", launches)`` of an attention call.  Packed rows go to the kernels that know them whatever the
+    environment says by now (the layout was chosen by the forward pass), and are refused where there are none: every other
+    route would read them as padded ones."""
+    if tmap is not None:
+        kind = _packed_kernels(qkv.dtype, S, H // nh)
+        if kind is None or (kind == "long" and direction == "bwd" and "ds" not in ws):
+            raise KernelError(f"no attention kernel for packed rows: {qkv.dtype}, {S} tokens, head dim {H // nh}")
+        if kind == "mma":
+            return f"rb_attention_{direction}_mma", 1
+        return f"rb_attention_{direction}_long", 1 if direction == "fwd" else 2
+    if _attention_long(qkv, S, H, nh, ws):
+        return f"rb_attention_{direction}_long", 1 if direction == "fwd" else 2
+    if not _attention_fits(qkv, S, H, nh):
+        return "composed", 0
+    return f"rb_attention_{direction}" if qkv.dtype == torch.float32 else _attention_entry(direction, H, nh), 1
+
+
 def _seed_tensor(rng):
     # the device-resident seed as a non-negative int64 scalar: no host read, so the composed path can be captured
     return rng.dev.to(torch.int64).reshape(-1)[0] & 0xFFFFFFFF
@@ -270,50 +300,35 @@ def _seed_tensor(rng):
 def attention_fwd(qkv, bqkv, mask, nh, p, rng, stream, ctx_out, ws, tmap=None):
     b, S = mask.shape
     H = ctx_out.shape[1]
-    if _attention_long(qkv, S, H, nh, ws):
-        _call("rb_attention_fwd_long", _I(DT[qkv.dtype]), _p(qkv), _p(bqkv), _p(mask), _p(ctx_out), _p(ws["probs"]),
-              _I(b), _I(S), _I(H), _I(nh), _F(p), _p(rng.dev), _U(stream), *_tok(tmap, "slot", "len", "meta"), _stream())
-        return
-    if not _attention_fits(qkv, S, H, nh):
+    entry, launches = _attention_route(qkv, S, H, nh, ws, "fwd", tmap)
+    if entry == "composed":
         from . import reference as ref
         ctx, probs = ref.attention_fwd(qkv, bqkv, mask, nh, p, _seed_tensor(rng), stream)
         ctx_out.copy_(ctx)
         ws["probs"][:b].copy_(probs)
         return
-    entry = "rb_attention_fwd" if qkv.dtype == torch.float32 else _attention_entry("fwd", H, nh)
+    maps = _tok(tmap, "slot", "len", "meta") if entry.endswith(("_mma", "_long")) else ()
     _call(entry, _I(DT[qkv.dtype]), _p(qkv), _p(bqkv), _p(mask), _p(ctx_out), _p(ws["probs"]), _I(b), _I(S),
-          _I(H), _I(nh), _F(p), _p(rng.dev), _U(stream),
-          *(_tok(tmap, "slot", "len", "meta") if entry.endswith("_mma") else ()), _stream())
+          _I(H), _I(nh), _F(p), _p(rng.dev), _U(stream), *maps, _stream(), launches=launches)
 
 
 def attention_bwd(dctx, qkv, bqkv, mask, nh, p, rng, stream, ws, dqkv_out, dbqkv_out, tmap=None):
     b, S = mask.shape
     H = dctx.shape[1]
-    if _attention_long(qkv, S, H, nh, ws):
-        acc = _DEFER.slot([dbqkv_out], 3 * H) if _DEFER is not None else None
-        _call("rb_attention_bwd_long", _I(DT[qkv.dtype]), _p(dctx), _p(qkv), _p(bqkv), _p(ws["probs"]), _p(ws["ds"]),
-              _p(dqkv_out), _I(b), _I(S), _I(H), _I(nh), _F(p), _p(rng.dev), _U(stream), _p(acc),
-              *_tok(tmap, "slot", "len", "meta"), _stream(), launches=2)
-        if acc is None:
-            colsum(dqkv_out, dbqkv_out)
-        return
-    if not _attention_fits(qkv, S, H, nh):
+    entry, launches = _attention_route(qkv, S, H, nh, ws, "bwd", tmap)
+    if entry == "composed":
         from . import reference as ref
         d = ref.attention_bwd(dctx, qkv, bqkv, mask, ws["probs"][:b], nh, p, _seed_tensor(rng), stream)
         dqkv_out.copy_(d)
         colsum(dqkv_out, dbqkv_out)
         return
-    if qkv.dtype == torch.float32:
-        _call("rb_attention_bwd", _I(DT[qkv.dtype]), _p(dctx), _p(qkv), _p(bqkv), _p(ws["probs"]), _p(dqkv_out), _I(b),
-              _I(S), _I(H), _I(nh), _F(p), _p(rng.dev), _U(stream), _stream())
-        colsum(dqkv_out, dbqkv_out)
-        return
-    # with a deferred-columns plan active the kernel also accumulates the q/k/v bias gradients
-    acc = _DEFER.slot([dbqkv_out], 3 * H) if _DEFER is not None else None
-    entry = _attention_entry("bwd", H, nh)
-    _call(entry, _I(DT[qkv.dtype]), _p(dctx), _p(qkv), _p(bqkv), _p(ws["probs"]), _p(dqkv_out), _I(b),
-          _I(S), _I(H), _I(nh), _F(p), _p(rng.dev), _U(stream), _p(acc),
-          *(_tok(tmap, "slot", "len", "meta") if entry.endswith("_mma") else ()), _stream())
+    # with a deferred-columns plan active the 16-bit kernels also accumulate the q/k/v bias gradients
+    acc = _DEFER.slot([dbqkv_out], 3 * H) if _DEFER is not None and qkv.dtype != torch.float32 else None
+    long = entry.endswith("_long")
+    maps = _tok(tmap, "slot", "len", "meta") if long or entry.endswith("_mma") else ()
+    _call(entry, _I(DT[qkv.dtype]), _p(dctx), _p(qkv), _p(bqkv), _p(ws["probs"]), *((_p(ws["ds"]),) if long else ()),
+          _p(dqkv_out), _I(b), _I(S), _I(H), _I(nh), _F(p), _p(rng.dev), _U(stream),
+          *(() if qkv.dtype == torch.float32 else (_p(acc),)), *maps, _stream(), launches=launches)
     if acc is None:
         colsum(dqkv_out, dbqkv_out)
 
