@@ -277,13 +277,14 @@ def _attention_long(qkv, S: int, H: int, nh: int, ws) -> bool:
 def _attention_route(qkv, S: int, H: int, nh: int, ws, direction: str, tmap):
     """``(entry or "composed", launches)`` of an attention call.  Packed rows go to the kernels that know them whatever the
     environment says by now (the layout was chosen by the forward pass), and are refused where there are none: every other
-    route would read them as padded ones."""
+    route would read them as padded ones.  Packed batches of 33..256 tokens take two launches, the tile of the padded length
+    and the next smaller one for the short sequences."""
     if tmap is not None:
         kind = _packed_kernels(qkv.dtype, S, H // nh)
         if kind is None or (kind == "long" and direction == "bwd" and "ds" not in ws):
             raise KernelError(f"no attention kernel for packed rows: {qkv.dtype}, {S} tokens, head dim {H // nh}")
         if kind == "mma":
-            return f"rb_attention_{direction}_mma", 1
+            return f"rb_attention_{direction}_mma", 2 if S > 32 else 1
         return f"rb_attention_{direction}_long", 1 if direction == "fwd" else 2
     if _attention_long(qkv, S, H, nh, ws):
         return f"rb_attention_{direction}_long", 1 if direction == "fwd" else 2

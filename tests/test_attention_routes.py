@@ -33,8 +33,8 @@ ENVS = [{}, {"RENEE_B200_ATTENTION": "tiles"}, {"RENEE_B200_ATTENTION_LONG": "0"
 
 @pytest.mark.parametrize("env", ENVS, ids=["default", "tiles", "no_long"])
 @pytest.mark.parametrize("S,hd,dtype,kind,launches", [
-    (1, 64, torch.bfloat16, "mma", (1, 1)), (32, 32, torch.float16, "mma", (1, 1)), (33, 64, torch.float16, "mma", (1, 1)),
-    (128, 32, torch.bfloat16, "mma", (1, 1)), (129, 64, torch.bfloat16, "mma", (1, 1)), (256, 64, torch.float16, "mma", (1, 1)),
+    (1, 64, torch.bfloat16, "mma", (1, 1)), (32, 32, torch.float16, "mma", (1, 1)), (33, 64, torch.float16, "mma", (2, 2)),
+    (128, 32, torch.bfloat16, "mma", (2, 2)), (129, 64, torch.bfloat16, "mma", (2, 2)), (256, 64, torch.float16, "mma", (2, 2)),
     (257, 64, torch.bfloat16, "long", (1, 2)), (512, 64, torch.bfloat16, "long", (1, 2)),
     (129, 32, torch.bfloat16, None, None), (513, 64, torch.bfloat16, None, None), (32, 64, torch.float32, None, None),
     (64, 16, torch.bfloat16, None, None)])
