@@ -382,6 +382,7 @@ enc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
       tile_coords<EPI>(tile, n_m_tiles, p.n_n_tiles, mt, nt);
       if (EPI == E_TOPK && mt != cur_m) {
         topk_flush();
+        __syncwarp();                                      // lanes of rows past M return early
 #pragma unroll
         for (int k = 0; k < 8; ++k) { tv[k] = -INFINITY; ti[k] = -1; }
         cur_m = mt;
@@ -571,6 +572,7 @@ enc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
         {
           for (int cc = 0; u_active && cc < ucols; cc += 32) {
             float v[32];
+            __syncwarp();                                  // the load is warp-wide; lanes leave the body below apart
             tc::tmem_ld32(ttk + cc, v);
             const int c0 = n0 + g * ucols + cc;
             // Most fragments hold nothing for any of the warp's rows once the lists are warm: one maximum over the 32
@@ -580,8 +582,10 @@ enc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
             for (int q = 0; q < 8; ++q) m8[q] = max_nan(max_nan(v[4 * q], v[4 * q + 1]), max_nan(v[4 * q + 2], v[4 * q + 3]));
             const float top = max_nan(max_nan(max_nan(m8[0], m8[1]), max_nan(m8[2], m8[3])),
                                       max_nan(max_nan(m8[4], m8[5]), max_nan(m8[6], m8[7])));
-            if (top <= tv[7]) continue;
-            if (!__any_sync(__activemask(), tv[7] == -INFINITY)) {
+            const bool some = !(top <= tv[7]);
+            const bool cold = __any_sync(0xffffffffu, some && tv[7] == -INFINITY);
+            if (!some) continue;
+            if (!cold) {
               // Warm lists: a lane has one or two candidates among its 32 values, but hardly two lanes in the same column.
               // Every lane steps through its own (bit j of hits), so the warp takes as many insertions as its busiest lane
               // has candidates, not one per column that any lane has one in (half of them, still, at the 14th fragment).
