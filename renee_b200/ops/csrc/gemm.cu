@@ -157,12 +157,18 @@ __device__ __forceinline__ void warp_bounds(const int* __restrict__ a, int n, in
 }
 
 // sigmoid of two logits with one reciprocal: 1 / a = b / (a b).  Below -40 the result is 0 in 16 bits either way, and the
-// bound keeps the product of the denominators finite; a NaN stays one.
+// bound keeps the product of the denominators finite.  A NaN stays one and does not reach its neighbour, whose logit belongs
+// to another row of the batch.
 __device__ __forceinline__ void sigmoid2(float x, float y, float& sx, float& sy) {
-  const float dx = 1.f + __expf(-max_nan(x, -40.f)), dy = 1.f + __expf(-max_nan(y, -40.f));
-  const float r = 1.f / (dx * dy);
-  sx = r * dy;
-  sy = r * dx;
+  const float dx = 1.f + __expf(-max_nan(x, -40.f)), dy = 1.f + __expf(-max_nan(y, -40.f)), d = dx * dy;
+  if (d != d) {
+    sx = 1.f / dx;
+    sy = 1.f / dy;
+  } else {
+    const float r = 1.f / d;
+    sx = r * dy;
+    sy = r * dx;
+  }
 }
 
 // Byte offset of the 16-byte chunk `chunk` (8 columns) of row r inside a 128-byte-swizzled panel.
