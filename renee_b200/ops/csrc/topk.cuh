@@ -35,10 +35,15 @@ __device__ __forceinline__ float max_nan(float a, float b) {
   asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
   return r;
 }
-// A NaN logit ranks above all finite ones, as in torch.topk.  It travels as the largest finite float, which no product
-// of 16-bit operands reaches, and becomes a NaN again in the result.
-__device__ __forceinline__ float topk_store_value(float x) { return x != x ? 3.402823466e38f : x; }
-__device__ __forceinline__ float topk_load_value(float x) { return x == 3.402823466e38f ? __int_as_float(0x7fffffff) : x; }
+// A NaN logit ranks above all others, +inf included, as in torch.topk.  In the lists, where values are compared as floats, a
+// NaN travels as +inf and +inf as the largest finite float, which no product of 16-bit operands reaches; the result has them
+// back.
+__device__ __forceinline__ float topk_store_value(float x) {
+  return x != x ? INFINITY : fminf(x, 3.402823466e38f);
+}
+__device__ __forceinline__ float topk_load_value(float x) {
+  return x == INFINITY ? __int_as_float(0x7fffffff) : (x == 3.402823466e38f ? INFINITY : x);
+}
 
 // fp32 -> unsigned with the same order; 0 is smaller than the key of every stored value
 __device__ __forceinline__ uint32_t order_key(float x) {
