@@ -51,18 +51,13 @@ def _no_decay(name: str) -> bool:
     return any(nd in name for nd in ("bias", "LayerNorm.bias", "LayerNorm.weight"))
 
 
-# Tokens per step and GPU (padded) from which the own GEMMs are always used in "auto" mode.
+# Padded tokens per step and GPU from which the own GEMMs are used in "auto" mode.  The rule looks at nothing but the padded
+# shape: the two paths round differently, and a step must not depend on which batch a run happened to begin with.  Below it
+# the fixed cost per launch of a persistent kernel (TMEM allocation, cluster start-up, a serial K loop on the few SMs the
+# tiles cover) outweighs the fused epilogues where most tokens are kept.  Training steps of 6 DistilBERT layers on one B200,
+# us, own (packed) / library GEMMs: 1024 padded tokens all kept 1401 / 1189, 608 kept 1343 / 1190; 2048: 1675 / 1445, 1216
+# kept 1480 / 1503; 4096: 2131 / 2125, 2432 kept 1848 / 2120; 6144: 2645 / 2663, 3648 kept 2117 / 2647.
 OWN_GEMM_MIN_TOKENS = int(os.environ.get("RENEE_B200_OWN_GEMM_MIN_TOKENS", "8192"))
-
-
-def own_gemm_pays(rows: int, T: int, H: int) -> bool:
-    """Whether the own GEMMs (on the ``rows`` kept tokens) beat library GEMMs and separate element-wise kernels (on all
-    ``T`` padded ones) below OWN_GEMM_MIN_TOKENS.  Training steps of 6 DistilBERT layers on one B200, us, own / library:
-    1024 padded tokens all kept 1401 / 1189, 608 kept 1343 / 1190; 2048: 1675 / 1445, 1216 kept 1480 / 1503; 4096: 2131 /
-    2125, 2432 kept 1848 / 2120; 6144: 2645 / 2663, 3648 kept 2117 / 2647 -- the own launches cost 1150 + 0.245 per row,
-    the library's 880 + 0.30 per padded token.  384 columns (MiniLM) cross at the same places; narrow encoders (128
-    columns, 2 layers) are even at 1024 tokens and gain from 2048 on, all kept or not (261 / 272, 4096: 312 / 322)."""
-    return T >= 2048 if H < 256 else rows < 1.22 * T - 1100
 
 
 @dataclass
@@ -154,8 +149,7 @@ class FlatEncoder:
         if self.device.type == "cuda" and act_dtype != torch.float32:
             from ..ops import cuda as cu
             # RENEE_B200_OWN_GEMM: 1 = the own tcgen05 GEMMs with fused epilogues always, 0 = library GEMMs + separate
-            # element-wise kernels, auto (default) = own from OWN_GEMM_MIN_TOKENS tokens per step and GPU upwards and
-            # where own_gemm_pays
+            # element-wise kernels, auto (default) = own from OWN_GEMM_MIN_TOKENS tokens per step and GPU upwards
             self._own_mode = os.environ.get("RENEE_B200_OWN_GEMM", "auto")
             self._own_supported = cu.enc_gemm_supported(self.p16, H, Fd)
             self.own_gemm = self._own_supported and self._own_mode != "auto"
@@ -255,8 +249,7 @@ class FlatEncoder:
         A = self._acts
         T, H = b * S, cfg.dim
         if self._own_mode == "auto":
-            rows = min(self.rows_hint or T, T)
-            self.own_gemm = self._own_supported and (T >= OWN_GEMM_MIN_TOKENS or own_gemm_pays(rows, T, H))
+            self.own_gemm = self._own_supported and T >= OWN_GEMM_MIN_TOKENS
         P = self.p16
         pd = cfg.dropout if train else 0.0
         pa = cfg.attention_dropout if train else 0.0

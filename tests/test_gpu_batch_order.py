@@ -1,0 +1,44 @@
+"""What a batch gives does not depend on which batch of its shape a trainer met first."""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _trainer(dim, B, S, pooling):
+    from renee_b200.models.encoder import EncoderConfig
+    from renee_b200.parallel.dist import DistContext
+    from renee_b200.train import TrainConfig, XCTrainer
+    from renee_b200.utils.sharding import shard_labels
+    enc = EncoderConfig(dim=dim, n_layers=2, n_heads=dim // 64, hidden_dim=2 * dim, vocab_size=500)
+    cfg = TrainConfig(batch_size=B, epochs=1, maxlen=S, pooling=pooling, fp16xfc=True, noloss=True, dropout=0.5)
+    return XCTrainer(cfg, enc, shard_labels(512, 1), DistContext(device=torch.device("cuda", 0)), steps_per_epoch=4)
+
+
+def _batch(B, S, lens, seed):
+    from renee_b200.data import xcrepo
+    from renee_b200.data.collate import XCCollator
+    from renee_b200.data.synthetic import SyntheticSpec, SyntheticXC
+    from renee_b200.utils.sharding import shard_labels
+    spec = SyntheticSpec(num_labels=512, seq_len=S, len_lo=lens[0], len_hi=lens[1], vocab=500, poisson_lam=2.0, seed=seed)
+    data = xcrepo.InMemoryDataset(*SyntheticXC(spec).rows(np.arange(B)))
+    return XCCollator(shard_labels(512, 1), data, 0, 1, B, True)(np.arange(B))
+
+
+@pytest.mark.parametrize("dim,B,S,pooling", [(256, 128, 32, "mean"), (256, 40, 150, "cls"), (128, 96, 32, "mean"), (256, 256, 32, "mean")])
+def test_first_batch_does_not_choose_the_path(dim, B, S, pooling):
+    short, full, typical = (_batch(B, S, l, k) for k, l in enumerate([(2, 3), (S, S), (S // 4, S)]))
+    outs = []
+    for first in (short, full):
+        tr = _trainer(dim, B, S, pooling)
+        tr.embed_eval(first)
+        own = tr.encoder.own_gemm
+        outs.append([tr.embed_eval(typical) for _ in range(3)][-1])
+        tr.train_step(typical)
+        assert tr.encoder.own_gemm == own
+        outs[-1] = (outs[-1], own)
+    assert outs[0][1] == outs[1][1]
+    assert torch.equal(outs[0][0], outs[1][0])
