@@ -558,7 +558,6 @@ class XCTrainer:
             return self._embed_graphed(batch)
         ids = batch.input_ids.to(dev, non_blocking=True)
         mask = batch.attention_mask.to(dev, non_blocking=True)
-        self._hint_rows(batch)
         emb = self.encoder.forward(ids, mask, self.step_rng, train=False)
         return emb.to(self.xfc.dtype)
 
