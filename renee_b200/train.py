@@ -151,6 +151,8 @@ class XCTrainer:
         self._graph_warm: dict = {}
         self._graph_generation = -1
         self._embed_graphs: dict = {}
+        self._embed_uses: dict = {}         # how often a shape was evaluated
+        self._embed_warm: set = set()       # shapes that have run eagerly on the present activations
         self._embed_generation = -1
         self._pending_loss = None
         self._side_stream = None
@@ -556,43 +558,49 @@ class XCTrainer:
         self._hint_rows(batch)
         if dev.type == "cuda" and self.cfg.cuda_graph and self.act_dtype != torch.float32:
             return self._embed_graphed(batch)
-        ids = batch.input_ids.to(dev, non_blocking=True)
-        mask = batch.attention_mask.to(dev, non_blocking=True)
+        return self._embed_eager(batch)
+
+    def _embed_eager(self, batch: XCBatch) -> torch.Tensor:
+        ids = batch.input_ids.to(self.device, torch.int32, non_blocking=True)
+        mask = batch.attention_mask.to(self.device, torch.int32, non_blocking=True)
         emb = self.encoder.forward(ids, mask, self.step_rng, train=False)
-        return emb.to(self.xfc.dtype)
+        return emb.to(self.xfc.dtype, copy=True)                 # the embedding buffer belongs to the encoder
 
     def _embed_graphed(self, batch: XCBatch) -> torch.Tensor:
         """The evaluation encoder from a CUDA graph: some 45 launches take the host 1.1 ms to issue and the GPU 0.7 ms to
-        run (256 x 32 tokens, DistilBERT).  The first batch of a shape runs eagerly, the second captures; at most
-        ``EMBED_GRAPHS`` shapes are kept (a last partial batch has its own), further ones stay eager."""
+        run (256 x 32 tokens, DistilBERT).  The first batch of a shape runs eagerly, the second captures.  At most
+        ``EMBED_GRAPHS`` shapes are kept (a last partial batch has its own); a further one takes the place of the least used
+        once it has been met more than twice as often, so that shapes of like frequency do not evict one another."""
         enc, shape = self.encoder, tuple(batch.input_ids.shape)
         if self._embed_generation != enc.generation:
-            self._embed_graphs = {}                              # the encoder re-allocated its activations
+            self._embed_graphs, self._embed_warm = {}, set()     # the encoder re-allocated its activations
             self._embed_generation = enc.generation
+        if len(self._embed_uses) >= 1024:
+            self._embed_uses = {k: self._embed_uses[k] for k in self._embed_graphs}
+        uses = self._embed_uses
+        uses[shape] = uses.get(shape, 0) + 1
         st = self._embed_graphs.get(shape)
-        if st is None and len(self._embed_graphs) < EMBED_GRAPHS:
-            st = dict(ids=torch.empty(shape, dtype=torch.int32, device=self.device),
-                      mask=torch.empty(shape, dtype=torch.int32, device=self.device), graph=None, emb=None, seen=0)
+        if st is None and shape in self._embed_warm:
+            rarest = min(self._embed_graphs, key=uses.get) if len(self._embed_graphs) >= EMBED_GRAPHS else None
+            if rarest is None or uses[shape] > 2 * uses[rarest]:
+                torch.cuda.synchronize()                         # the graph that leaves may still be running
+                self._embed_graphs.pop(rarest, None)
+                st = dict(ids=torch.zeros(shape, dtype=torch.int32, device=self.device),
+                          mask=torch.ones(shape, dtype=torch.int32, device=self.device), graph=torch.cuda.CUDAGraph())
+                with torch.cuda.graph(st["graph"], capture_error_mode="thread_local"):
+                    st["emb"] = enc.forward(st["ids"], st["mask"], self.step_rng, train=False)
+                self._embed_graphs[shape] = st
         if st is None:
-            ids = batch.input_ids.to(self.device, torch.int32, non_blocking=True)
-            mask = batch.attention_mask.to(self.device, torch.int32, non_blocking=True)
-            return enc.forward(ids, mask, self.step_rng, train=False).to(self.xfc.dtype, copy=True)
+            emb = self._embed_eager(batch)
+            if self._embed_generation != enc.generation:         # this pass allocated the activations
+                self._embed_graphs, self._embed_warm = {}, set()
+                self._embed_generation = enc.generation
+            self._embed_warm.add(shape)
+            return emb
         st["ids"].copy_(batch.input_ids, non_blocking=True)
         st["mask"].copy_(batch.attention_mask, non_blocking=True)
-        if st["graph"] is None and st["seen"] == 0:
-            st["seen"], st["emb"] = 1, enc.forward(st["ids"], st["mask"], self.step_rng, train=False)
-            if self._embed_generation != enc.generation:         # this pass allocated the activations
-                self._embed_graphs, self._embed_generation = {}, enc.generation
-            self._embed_graphs[shape] = st
-        else:
-            if st["graph"] is None:
-                torch.cuda.synchronize()
-                graph = torch.cuda.CUDAGraph()
-                with torch.cuda.graph(graph, capture_error_mode="thread_local"):
-                    st["emb"] = enc.forward(st["ids"], st["mask"], self.step_rng, train=False)
-                st["graph"] = graph
-            st["graph"].replay()
-        return st["emb"].to(self.xfc.dtype, copy=True)           # the embedding buffer belongs to the encoder
+        st["graph"].replay()
+        return st["emb"].to(self.xfc.dtype, copy=True)
 
     def local_topk(self, X: torch.Tensor, k: int):
         if self.cfg.default_impl:

@@ -42,3 +42,29 @@ def test_first_batch_does_not_choose_the_path(dim, B, S, pooling):
         outs[-1] = (outs[-1], own)
     assert outs[0][1] == outs[1][1]
     assert torch.equal(outs[0][0], outs[1][0])
+
+
+def test_frequent_shapes_take_the_place_of_rare_ones():
+    """The shapes met first do not keep the graphs for good, shapes of like frequency do not evict one another, and every
+    result is the eager one."""
+    from renee_b200.train import EMBED_GRAPHS
+    S, tr = 24, _trainer(128, 40, 24, "mean")
+    batches = {b: _batch(b, S, (2, S), b) for b in range(40, 40 - EMBED_GRAPHS - 3, -1)}
+
+    def ask(b):
+        got = tr.embed_eval(batches[b])
+        want = tr.encoder.forward(batches[b].input_ids.cuda(), batches[b].attention_mask.cuda(), tr.step_rng, train=False)
+        assert torch.equal(got, want.to(got.dtype))
+
+    for _ in range(3):
+        for b in batches:
+            ask(b)
+    first = set(tr._embed_graphs)
+    assert first == {(b, S) for b in list(batches)[:EMBED_GRAPHS]}
+    late = list(batches)[-1]
+    for _ in range(5):
+        ask(late)
+    assert (late, S) in tr._embed_graphs and len(tr._embed_graphs) == EMBED_GRAPHS
+    for b in batches:
+        ask(b)
+    assert len(tr._embed_graphs) == EMBED_GRAPHS
