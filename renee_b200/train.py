@@ -556,7 +556,8 @@ class XCTrainer:
             return e
         b = batch.input_ids.shape[0]
         self._hint_rows(batch)
-        if dev.type == "cuda" and self.cfg.cuda_graph and self.act_dtype != torch.float32:
+        if dev.type == "cuda" and self.cfg.cuda_graph and self.act_dtype != torch.float32 \
+                and not torch.cuda.is_current_stream_capturing():
             return self._embed_graphed(batch)
         return self._embed_eager(batch)
 

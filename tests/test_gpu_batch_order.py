@@ -68,3 +68,20 @@ def test_frequent_shapes_take_the_place_of_rare_ones():
     for b in batches:
         ask(b)
     assert len(tr._embed_graphs) == EMBED_GRAPHS
+
+
+def test_embed_eval_inside_a_callers_graph():
+    """A caller that captures embed_eval into a graph of its own gets the eager launches, also after the shape has a graph."""
+    from types import SimpleNamespace
+    S, tr = 24, _trainer(128, 40, 24, "cls")
+    a, b = (SimpleNamespace(**{n: getattr(x, n).to("cuda", torch.int32) for n in ("input_ids", "attention_mask")})
+            for x in (_batch(40, S, (2, S), 1), _batch(40, S, (2, S), 2)))
+    want = [[tr.embed_eval(x) for _ in range(3)][-1] for x in (a, b)]
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        out = tr.embed_eval(a)
+    for x, w in zip((a, b), want):
+        a.input_ids.copy_(x.input_ids); a.attention_mask.copy_(x.attention_mask)
+        graph.replay()
+        assert torch.equal(out, w)
