@@ -146,14 +146,14 @@ class FlatEncoder:
         self._wgrad_done = [None, None]
         self.pack_tokens = True        # own GEMM path: leave padded tokens out (TokenMap); a comparison may switch it off
         self.rows_hint = 0             # caller's estimate of the kept tokens of the coming batches (tile planning only)
-        if self.device.type == "cuda" and act_dtype != torch.float32:
+        if self.device.type in ("cuda", "meta") and act_dtype != torch.float32:
             from ..ops import cuda as cu
             # RENEE_B200_OWN_GEMM: 1 = the own tcgen05 GEMMs with fused epilogues always, 0 = library GEMMs + separate
             # element-wise kernels, auto (default) = own from OWN_GEMM_MIN_TOKENS tokens per step and GPU upwards
             self._own_mode = os.environ.get("RENEE_B200_OWN_GEMM", "auto")
             self._own_supported = cu.enc_gemm_supported(self.p16, H, Fd)
             self.own_gemm = self._own_supported and self._own_mode != "auto"
-            if self._own_supported and os.environ.get("RENEE_B200_WGRAD_STREAM", "1") != "0":
+            if self._own_supported and self.device.type == "cuda" and os.environ.get("RENEE_B200_WGRAD_STREAM", "1") != "0":
                 # weight gradients are off the critical path of the backward pass (nothing reads them before the
                 # optimizer): a layer's launch runs on a second stream, where it fills the SMs that the next layer's
                 # kernels leave idle.  Captured into the step's CUDA graph as parallel branches.
@@ -218,7 +218,7 @@ class FlatEncoder:
         e = lambda *shape, dtype=dt: guard.empty(*shape, dtype=dtype, device=dev, name=f"encoder.act{guard.registered()}")
         layers = []
         # long sequences: one softmax-gradient scratch serves every layer (it lives within one attention backward)
-        att_ds = (e(b, nh, S, S) if S > 128 and dev.type == "cuda" and dt != torch.float32 else None)
+        att_ds = ops.attention_ds(b, S, nh, dev, dt)
         for _ in range(cfg.n_layers):
             layers.append(dict(qkv=e(T, 3 * H), ctx=e(T, H), ao=e(T, H), pre1=e(T, H), h1=e(T, H),
                                mean1=e(T, dtype=torch.float32), rstd1=e(T, dtype=torch.float32),
@@ -227,13 +227,28 @@ class FlatEncoder:
                                att=ops.attention_workspace(b, S, nh, dev, dt, ds=att_ds)))
         self._acts = dict(h0=e(T, H), mean0=e(T, dtype=torch.float32), rstd0=e(T, dtype=torch.float32),
                           layers=layers, pooled=e(b, H, dtype=torch.float32),
-                          dh=e(T, H), dh_b=e(T, H), dqkv=e(T, 3 * H), dctx=e(T, H), df1=e(T, Fd), da1=e(T, Fd),
-                          emb=e(b, self.out_dims, dtype=torch.float32), tmap=None, bwd=None)
-        if self._own_supported and dev.type == "cuda" and self._packs(S):
+                          dh=e(T, H), dctx=e(T, H), att_ds=att_ds,
+                          emb=e(b, self.out_dims, dtype=torch.float32), tmap=None, own=None, lib=None)
+        if self._own_supported and self._packs(S):
             from ..ops import cuda as cu
             self._acts["tmap"] = cu.TokenMap(b, S, dev)
         self._acts_key = key
         self.generation += 1      # activation addresses changed: graphs captured over the old ones are stale
+
+    def _choose_path(self, T: int) -> None:
+        if self._own_mode == "auto":
+            self.own_gemm = self._own_supported and T >= OWN_GEMM_MIN_TOKENS
+
+    def allocate(self, b: int, S: int, capacity: int = 0) -> None:
+        """Everything that training steps of ``[b, S]`` batches hold (buffers for ``capacity`` >= b rows): what the first
+        forward and backward passes would allocate."""
+        self._alloc(max(b, capacity), S)
+        self._choose_path(b * S)
+        self._ensure_backward_buffers()
+        if self._acts["att_ds"] is not None:
+            from ..ops import cuda as cu
+            if cu.attention_streams(self.act_dtype, S, self.cfg.dim, self.cfg.n_heads):
+                self._acts["att_ds"].get()
 
     def _packs(self, S: int) -> bool:
         from ..ops import cuda as cu
@@ -248,8 +263,7 @@ class FlatEncoder:
         self._alloc(b, S)
         A = self._acts
         T, H = b * S, cfg.dim
-        if self._own_mode == "auto":
-            self.own_gemm = self._own_supported and T >= OWN_GEMM_MIN_TOKENS
+        self._choose_path(T)
         P = self.p16
         pd = cfg.dropout if train else 0.0
         pa = cfg.attention_dropout if train else 0.0
@@ -399,8 +413,7 @@ class FlatEncoder:
             d_pool = torch.mm(d_emb, self.bottleneck_weight())
         else:
             d_pool = d_emb
-        if self.own_gemm:
-            self._ensure_backward_buffers()
+        self._ensure_backward_buffers()
         dh = A["dh"][:T]
         ops.pool_bwd(d_pool, mask, self.pooling, S, dh.view(b, S, H), **packed)
         for l in reversed(range(cfg.n_layers)):
@@ -411,16 +424,17 @@ class FlatEncoder:
             if self.own_gemm:
                 self._backward_layer_fused(l, L, dh, on_layer_done)
                 continue
+            buf = A["lib"][0]
             # ---- output LN + FFN
             d_pre2, d_f2 = ops.bias_dropout_add_ln_bwd(
                 dh, L["pre2"][:T], self.view(P, pre + "output_layer_norm.weight"), L["mean2"][:T], L["rstd2"][:T],
                 pd, rng, sb + _S_FFN,
                 self.view(G, pre + "output_layer_norm.weight"), self.view(G, pre + "output_layer_norm.bias"),
-                self.view(G, pre + "ffn.lin2.bias"), A["dh_b"][:T], L["f2"][:T])
+                self.view(G, pre + "ffn.lin2.bias"), buf["dh_b"][:T], L["f2"][:T])
             torch.mm(d_f2.t(), L["a1"][:T], out=self.view(G, pre + "ffn.lin2.weight"))
-            da1 = A["da1"][:T]
+            da1 = buf["da1"][:T]
             torch.mm(d_f2, self.view(P, pre + "ffn.lin2.weight"), out=da1)
-            df1 = A["df1"][:T]
+            df1 = buf["df1"][:T]
             ops.bias_gelu_bwd(da1, L["f1"][:T], self.view(P, pre + "ffn.lin1.bias"),
                               self.view(G, pre + "ffn.lin1.bias"), df1)
             torch.mm(df1.t(), L["h1"][:T], out=self.view(G, pre + "ffn.lin1.weight"))
@@ -431,11 +445,11 @@ class FlatEncoder:
                 dh1, L["pre1"][:T], self.view(P, pre + "sa_layer_norm.weight"), L["mean1"][:T], L["rstd1"][:T],
                 fw["po"], rng, sb + _S_ATTN,
                 self.view(G, pre + "sa_layer_norm.weight"), self.view(G, pre + "sa_layer_norm.bias"),
-                self.view(G, pre + "attention.out_lin.bias"), A["dh_b"][:T], L["ao"][:T])
+                self.view(G, pre + "attention.out_lin.bias"), buf["dh_b"][:T], L["ao"][:T])
             torch.mm(d_ao.t(), L["ctx"][:T], out=self.view(G, pre + "attention.out_lin.weight"))
             dctx = A["dctx"][:T]
             torch.mm(d_ao, self.view(P, pre + "attention.out_lin.weight"), out=dctx)
-            dqkv = A["dqkv"][:T]
+            dqkv = buf["dqkv"][:T]
             ops.attention_bwd(dctx, L["qkv"][:T], self._qkv(P, l, "bias"), mask, cfg.n_heads, pa, rng,
                               sb + _S_PROBS, L["att"], dqkv, self._qkv(G, l, "bias"))
             torch.mm(dqkv.t(), h_in, out=self._qkv(G, l, "weight"))
@@ -453,17 +467,22 @@ class FlatEncoder:
         self._wgrad_wait(1)
 
     def _ensure_backward_buffers(self) -> None:
-        """Two sets of the gradients that the weight-gradient launch of a layer still reads while the next layer is
-        differentiated, and that launch's scratch: allocated by the first backward pass on the own GEMMs."""
-        if self._acts["bwd"] is not None:
+        """The gradient buffers of one block, allocated by the first backward pass of the path that uses them.  Library path:
+        one set.  Own GEMMs: two sets of the gradients that the weight-gradient launch of a layer still reads while the next
+        layer is differentiated, and that launch's scratch."""
+        which = "own" if self.own_gemm else "lib"
+        if self._acts[which] is not None:
             return
-        from ..ops import cuda as cu
         (b, S), H, Fd = self._acts_key, self.cfg.dim, self.cfg.hidden_dim
-        widths = (("dpre2", H), ("dpre1", H), ("df1", Fd), ("dqkv", 3 * H))
-        sizes = [b * S * n for _, n in widths] * 2
+        widths = (("dpre2", H), ("dpre1", H), ("df1", Fd), ("dqkv", 3 * H)) if self.own_gemm else \
+            (("dh_b", H), ("dqkv", 3 * H), ("df1", Fd), ("da1", Fd))
+        sets = 2 if self.own_gemm else 1
+        sizes = [b * S * n for _, n in widths] * sets
         flat = guard.empty(sum(sizes), dtype=self.act_dtype, device=self.device, name="encoder.bwd").split(sizes)
-        self._acts["bwd"] = [{k: flat[4 * i + j].view(b * S, n) for j, (k, n) in enumerate(widths)} for i in range(2)]
-        if self._wgrad_group is None:
+        self._acts[which] = [{k: flat[len(widths) * i + j].view(b * S, n) for j, (k, n) in enumerate(widths)}
+                             for i in range(sets)]
+        if self.own_gemm and self._wgrad_group is None:
+            from ..ops import cuda as cu
             self._wgrad_group = cu.WgradGroup([(3 * H, H), (H, H), (Fd, H), (H, Fd)], self.device)
 
     def _backward_layer_fused(self, l: int, L: dict, dh, on_layer_done) -> None:
@@ -472,7 +491,7 @@ class FlatEncoder:
         cfg, A, P, G, fw = self.cfg, self._acts, self.p16, self.g, self._fw
         T, packed, pd, po, rng = fw["b"] * fw["S"], fw["packed"], fw["pd"], fw["po"], fw["rng"]
         pre, sb, par = f"transformer.layer.{l}.", 8 * (l + 1), l & 1
-        buf = {k: t[:T] for k, t in A["bwd"][par].items()}
+        buf = {k: t[:T] for k, t in A["own"][par].items()}
         self._wgrad_wait(par)
         d_pre2, d_f2 = ops.bias_dropout_add_ln_bwd(
             dh, L["pre2"][:T], self.view(P, pre + "output_layer_norm.weight"), L["mean2"][:T], L["rstd2"][:T],

@@ -56,13 +56,35 @@ def embed_ln_bwd(dy, ids, word, pos, gamma, mean, rstd, S, p, rng, stream, pad_i
     ref.embed_ln_bwd(dy, ids, word, pos, gamma, mean, rstd, S, p, rng.seed, stream, pad_id, dword, dpos, dgamma, dbeta)
 
 
+class LazyBuffer:
+    """A scratch buffer that is allocated by its first user (``get``) and shared by all holders."""
+
+    def __init__(self, *shape, dtype, device, name):
+        self._make = lambda: guard.empty(*shape, dtype=dtype, device=device, name=name)
+        self._buf = None
+
+    def get(self) -> torch.Tensor:
+        if self._buf is None:
+            self._buf = self._make()
+        return self._buf
+
+
+def attention_ds(b, S, nh, device, dtype):
+    """The softmax-gradient scratch ``[b, nh, S, S]`` of the streaming attention backward (16-bit, 129..512 tokens), or
+    ``None`` where no kernel reads one.  Most shapes up to 256 tokens never do, so it is allocated on first use."""
+    if not (S > 128 and torch.device(device).type in ("cuda", "meta") and dtype != torch.float32):
+        return None
+    return LazyBuffer(b, nh, S, S, dtype=dtype, device=device, name="attention.ds")
+
+
 def attention_workspace(b, S, nh, device, dtype, ds=None):
-    """Buffers the attention forward leaves for its backward: the softmax probabilities.  On CUDA, 16-bit
-    sequences longer than 128 tokens also need a same-shaped scratch for the softmax gradient (``ds``; pass one
-    tensor to share it between layers, it only lives within one backward call)."""
+    """Buffers the attention forward leaves for its backward: the softmax probabilities, and for 16-bit sequences longer
+    than 128 tokens on CUDA :func:`attention_ds` (pass one as ``ds`` to share it between layers, it only lives within one
+    backward call)."""
     ws = {"probs": guard.empty(b, nh, S, S, dtype=dtype, device=device, name="attention.probs")}
-    if S > 128 and torch.device(device).type == "cuda" and dtype != torch.float32:
-        ws["ds"] = ds if ds is not None else guard.empty(b, nh, S, S, dtype=dtype, device=device, name="attention.ds")
+    ds = ds if ds is not None else attention_ds(b, S, nh, device, dtype)
+    if ds is not None:
+        ws["ds"] = ds
     return ws
 
 

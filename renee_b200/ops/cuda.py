@@ -13,6 +13,7 @@ import os
 import torch
 
 from . import build as _build
+from ..utils import guard
 
 _LIB = None
 _LAUNCHES = 0
@@ -197,7 +198,7 @@ class TokenMap:
 
     def __init__(self, b: int, S: int, device):
         n = b * S
-        z = torch.zeros(2 * n + 3 * b + 4, dtype=torch.int32, device=device)
+        z = guard.zeros(2 * n + 3 * b + 4, dtype=torch.int32, device=device, name="encoder.token_map")
         self.tok, self.slot, self.off, self.len, self.cnt, self.meta = z.split([n, n, b, b, b, 4])
         self.rows_hint = 0
 
@@ -265,12 +266,16 @@ def _attention_entry(direction: str, H: int, nh: int) -> str:
     return f"rb_attention_{direction}_tc"
 
 
-def _attention_long(qkv, S: int, H: int, nh: int, ws) -> bool:
+def _scratch(buf):
+    return buf.get() if hasattr(buf, "get") else buf
+
+
+def attention_streams(dtype, S: int, H: int, nh: int) -> bool:
     """Sequences of 257..512 tokens (129..512 with the tile kernels), 16-bit activations, head dim 64: the streaming
     kernels of attention_mma.cu (``RENEE_B200_ATTENTION_LONG=0`` sends sequences of more than 128 tokens to the composed
     library ops instead)."""
     lo = 256 if _attention_entry("fwd", H, nh).endswith("_mma") else 128
-    return (qkv.dtype != torch.float32 and lo < S <= 512 and H // nh == 64 and "ds" in ws
+    return (dtype != torch.float32 and lo < S <= 512 and H // nh == 64
             and os.environ.get("RENEE_B200_ATTENTION_LONG", "") != "0")
 
 
@@ -286,7 +291,7 @@ def _attention_route(qkv, S: int, H: int, nh: int, ws, direction: str, tmap):
         if kind == "mma":
             return f"rb_attention_{direction}_mma", 2 if S > 32 else 1
         return f"rb_attention_{direction}_long", 1 if direction == "fwd" else 2
-    if _attention_long(qkv, S, H, nh, ws):
+    if "ds" in ws and attention_streams(qkv.dtype, S, H, nh):
         return f"rb_attention_{direction}_long", 1 if direction == "fwd" else 2
     if not _attention_fits(qkv, S, H, nh):
         return "composed", 0
@@ -327,7 +332,7 @@ def attention_bwd(dctx, qkv, bqkv, mask, nh, p, rng, stream, ws, dqkv_out, dbqkv
     acc = _DEFER.slot([dbqkv_out], 3 * H) if _DEFER is not None and qkv.dtype != torch.float32 else None
     long = entry.endswith("_long")
     maps = _tok(tmap, "slot", "len", "meta") if long or entry.endswith("_mma") else ()
-    _call(entry, _I(DT[qkv.dtype]), _p(dctx), _p(qkv), _p(bqkv), _p(ws["probs"]), *((_p(ws["ds"]),) if long else ()),
+    _call(entry, _I(DT[qkv.dtype]), _p(dctx), _p(qkv), _p(bqkv), _p(ws["probs"]), *((_p(_scratch(ws["ds"])),) if long else ()),
           _p(dqkv_out), _I(b), _I(S), _I(H), _I(nh), _F(p), _p(rng.dev), _U(stream),
           *(() if qkv.dtype == torch.float32 else (_p(acc),)), *maps, _stream(), launches=launches)
     if acc is None:
@@ -388,8 +393,8 @@ _SK: dict = {}
 
 
 def enc_gemm_supported(t: torch.Tensor, *dims: int) -> bool:
-    """The own GEMMs serve 16-bit CUDA tensors whose feature dimensions are multiples of 64."""
-    return bool(t.is_cuda and t.dtype in (torch.bfloat16, torch.float16) and all(d % 64 == 0 for d in dims)
+    """The own GEMMs serve 16-bit CUDA tensors whose feature dimensions are multiples of 64 (meta: planned for a GPU)."""
+    return bool((t.is_cuda or t.is_meta) and t.dtype in (torch.bfloat16, torch.float16) and all(d % 64 == 0 for d in dims)
                 and os.environ.get("RENEE_B200_OWN_GEMM", "auto") != "0")
 
 
@@ -464,16 +469,22 @@ def linear_wgrad(dy, x, dW, bn=0, ncta=0, tmap=None):
 
 
 class WgradGroup:
-    """Scratch of :func:`wgrad_group` for one engine: partial tiles (any content) and per-tile counters (zero between
-    launches).  Launches that share it must be ordered."""
+    """Scratch of :func:`wgrad_group` for one engine: partial tiles (any content; 39 MB on 148 SMs) and per-tile counters (zero
+    between launches).  Launches that share it must be ordered."""
 
     def __init__(self, shapes, device):
         tiles = sum(((m + 255) // 256) * ((n + 255) // 256) for m, n in shapes)
-        f = lib().rb_wgrad_group_scratch_bytes
-        f.restype = _LL
-        with torch.cuda.device(device):
-            self.scratch = torch.empty(int(f()) // 4, dtype=torch.float32, device=device)
-        self.counters = torch.zeros(2 * tiles, dtype=torch.int32, device=device)
+        self.scratch = guard.empty(_wgrad_scratch_bytes(device) // 4, dtype=torch.float32, device=device, name="encoder.wgrad")
+        self.counters = guard.zeros(2 * tiles, dtype=torch.int32, device=device, name="encoder.wgrad")
+
+
+def _wgrad_scratch_bytes(device) -> int:
+    if torch.device(device).type == "meta":            # size-accounting dry runs: a B200
+        return B200_SMS // 2 * 4 * 128 * 256 * 4
+    f = lib().rb_wgrad_group_scratch_bytes
+    f.restype = _LL
+    with torch.cuda.device(device):
+        return int(f())
 
 
 def wgrad_group(items, group: WgradGroup, tmap=None):
@@ -615,6 +626,7 @@ def xfc_dw_sgd(Gt, ldG, X, W, M, hp_buf, mo, wd, tma_tiles=True, stochastic_roun
           _I(int(tma_tiles)), _I(1 if stochastic_round else 0), _p(ws.status), _stream())
 
 
+B200_SMS = 148
 _SMS: dict = {}
 
 

@@ -42,7 +42,7 @@ def plan(labels: int, gpus: int, global_batch: int, seq: int, enc_cfg=None, fp16
     by_kind: collections.Counter = collections.Counter()
     with guard.enabled_for_test():
         tr = XCTrainer(cfg, enc_cfg, sh, ctx, steps_per_epoch=100)
-        tr.encoder._alloc(b + 1, seq)            # the trainer's staging buffers hold b + 1 rows (ragged final batch)
+        tr.encoder.allocate(b, seq, capacity=b + 1)     # the trainer's staging buffers hold b + 1 rows (ragged final batch)
         tr.xfc.scratch(global_batch)
         for e in guard._registry:
             kind = e.name.rsplit(".", 1)[0] if not e.name.startswith("encoder.act") else "encoder.activations"
@@ -65,6 +65,7 @@ def plan(labels: int, gpus: int, global_batch: int, seq: int, enc_cfg=None, fp16
         "config": {"labels": labels, "gpus": gpus, "global_batch": global_batch, "seq": seq, "labels_per_gpu": ls,
                    "fp16xfc": fp16xfc, "activation_bytes": act_bytes},
         "per_gpu_gb": {k: round(v / 1e9, 3) for k, v in sorted(by_kind.items(), key=lambda kv: -kv[1])},
+        "framework_total_bytes": int(ours),
         "framework_total_gb": round(ours / 1e9, 2),
         "with_allowance_gb": round((ours + OTHER_ALLOWANCE_BYTES) / 1e9, 2),
         "fits_180gb": bool(ours + OTHER_ALLOWANCE_BYTES < HBM_BYTES),
