@@ -403,6 +403,7 @@ class FlatEncoder:
         T, H = b * S, cfg.dim
         P, G = self.p16, self.g
         mask, packed = fw["mask"], fw["packed"]
+        self._wgrad_done = [None, None]      # a pass that ended in an exception may have left an event of its own (or its capture's)
         if self.bottleneck_dims > 0:
             gw = self.view(G, "__bottleneck__.transformer_weight")
             pooled = A["pooled"][:b]

@@ -157,3 +157,46 @@ def test_attention_tile_sizes_against_the_oracle(S, b, nh, hd, dt, p):
         assert rel < 3 * eps, rel
         assert float((got.float() - want).abs().max()) < 16 * eps * float(want.abs().max())
     torch.testing.assert_close(db.float(), d_r.sum(0), rtol=8 * eps, atol=8 * eps * float(d_r.sum(0).abs().max()) + 1e-3)
+
+
+def test_capture_after_a_backward_pass_that_raised(monkeypatch):
+    """A backward pass that ended in a host exception leaves no event behind that a later pass, or its capture, waits for."""
+    from renee_b200.models.encoder import EncoderConfig
+    from renee_b200.ops import StepRNG, cuda as cu
+    cfg = EncoderConfig(dim=128, n_layers=3, n_heads=2, hidden_dim=256, vocab_size=500)
+    enc = _engine(cfg, torch.bfloat16, "mean")
+    gen = torch.Generator().manual_seed(1)
+    mask = _mask("prefix", 8, 32, gen)
+    ids = torch.randint(5, 500, (8, 32), generator=gen, dtype=torch.int32).cuda()
+    d_emb = (torch.randn(8, 128, generator=gen) * 0.1).cuda()
+    rng = StepRNG(7, torch.tensor([7], dtype=torch.int32, device="cuda"))
+
+    def step():
+        enc.forward(ids, mask, rng, train=True)
+        enc.backward(d_emb)
+
+    step()
+    want = enc.g.float().clone()
+    dgrad, n = cu.linear_dgrad, [0]
+
+    def failing(*a, **k):
+        n[0] += 1
+        if n[0] == 5:                        # in the second layer of the pass: the first one's weight gradients are under way
+            raise RuntimeError("stop")
+        return dgrad(*a, **k)
+
+    monkeypatch.setattr(cu, "linear_dgrad", failing)
+    with pytest.raises(RuntimeError, match="stop"):
+        step()
+    monkeypatch.setattr(cu, "linear_dgrad", dgrad)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        step()
+    enc.g.zero_()
+    graph.replay()
+    cu.check_status()
+    for name, slot in enc.slots.items():     # the matrices; the column sums still hold what the failed pass had added
+        if name.startswith("transformer") and name.endswith(("_lin.weight", "lin1.weight", "lin2.weight")):
+            at = slice(slot.offset, slot.offset + slot.numel)
+            assert torch.equal(enc.g[at].float(), want[at]), name
