@@ -13,7 +13,7 @@ def _trainer(dim, B, S, pooling):
     from renee_b200.parallel.dist import DistContext
     from renee_b200.train import TrainConfig, XCTrainer
     from renee_b200.utils.sharding import shard_labels
-    enc = EncoderConfig(dim=dim, n_layers=2, n_heads=dim // 64, hidden_dim=2 * dim, vocab_size=500)
+    enc = EncoderConfig(dim=dim, n_layers=2, n_heads=dim // 64, hidden_dim=2 * dim, vocab_size=2000)
     cfg = TrainConfig(batch_size=B, epochs=1, maxlen=S, pooling=pooling, fp16xfc=True, noloss=True, dropout=0.5)
     return XCTrainer(cfg, enc, shard_labels(512, 1), DistContext(device=torch.device("cuda", 0)), steps_per_epoch=4)
 
@@ -23,7 +23,7 @@ def _batch(B, S, lens, seed):
     from renee_b200.data.collate import XCCollator
     from renee_b200.data.synthetic import SyntheticSpec, SyntheticXC
     from renee_b200.utils.sharding import shard_labels
-    spec = SyntheticSpec(num_labels=512, seq_len=S, len_lo=lens[0], len_hi=lens[1], vocab=500, poisson_lam=2.0, seed=seed)
+    spec = SyntheticSpec(num_labels=512, seq_len=S, len_lo=lens[0], len_hi=lens[1], vocab=2000, poisson_lam=2.0, seed=seed)
     data = xcrepo.InMemoryDataset(*SyntheticXC(spec).rows(np.arange(B)))
     return XCCollator(shard_labels(512, 1), data, 0, 1, B, True)(np.arange(B))
 

@@ -8,7 +8,7 @@ import torch
 
 def _enc(S):
     from renee_b200.models.encoder import EncoderConfig
-    return EncoderConfig(vocab_size=1000, dim=128, n_layers=2, n_heads=2, hidden_dim=256, max_position_embeddings=max(S, 64))
+    return EncoderConfig(vocab_size=2000, dim=128, n_layers=2, n_heads=2, hidden_dim=256, max_position_embeddings=max(S, 64))
 
 
 SHAPES = [(256, 32), (16, 24), (64, 160), (8, 160), (32, 300), (4, 300)]
@@ -47,7 +47,7 @@ def test_plan_is_what_a_trainer_allocates(B, S):
     from renee_b200.utils.sharding import shard_labels
     L = 3000
     want = plan(labels=L, gpus=1, global_batch=B, seq=S, enc_cfg=_enc(S), pooling="mean")["framework_total_bytes"]
-    data = xcrepo.InMemoryDataset(*SyntheticXC(SyntheticSpec(num_labels=L, seq_len=S, len_lo=4, len_hi=S, vocab=1000,
+    data = xcrepo.InMemoryDataset(*SyntheticXC(SyntheticSpec(num_labels=L, seq_len=S, len_lo=4, len_hi=S, vocab=2000,
                                                              poisson_lam=2.0, seed=1)).rows(np.arange(B)))
     batch = XCCollator(shard_labels(L, 1), data, 0, 1, B, True)(np.arange(B))
     cfg = TrainConfig(batch_size=B, epochs=1, seed=0, dropout=0.5, lr1=0.05, lr2=1e-5, warmup=10, wd1=1e-4, noloss=True,
