@@ -243,17 +243,11 @@ enc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
   grid_dep_wait();
   grid_dep_launch();
   // extents of this launch: the host's, or with packed tokens the device's row count (every thread reads the same word)
-  int M = p.M, n_m_tiles = p.n_m_tiles, kb_total = p.kb_total, kb_per_split = p.kb_per_split, splits = p.splits;
-  if (p.tok_meta != nullptr) {
-    const int rows = __ldcg(p.tok_meta + TOK_ROWS);
-    if (LAYOUT == L_TN) {
-      kb_total = (rows + BK - 1) / BK;
-      kb_per_split = (kb_total + splits - 1) / splits;
-      splits = (kb_total + kb_per_split - 1) / kb_per_split;       // no split is empty
-    } else {
-      M = rows;
-      n_m_tiles = (rows + BM * NCTA - 1) / (BM * NCTA);
-    }
+  const int kb_total = p.kb_total, kb_per_split = p.kb_per_split, splits = p.splits;
+  int M = p.M, n_m_tiles = p.n_m_tiles;
+  if (LAYOUT != L_TN && p.tok_meta != nullptr) {
+    M = __ldcg(p.tok_meta + TOK_ROWS);
+    n_m_tiles = (M + BM * NCTA - 1) / (BM * NCTA);
   }
   const int n_items = n_m_tiles * p.n_n_tiles * splits;
   // items of this unit: every n_units-th, or for the logits (few N tiles per M tile) a run of neighbours, so that the
@@ -963,8 +957,8 @@ RB_API int rb_enc_gemm_plan(int layout, int epi, int M, int N, int K, int bn_for
 //   R [M, ldr]: residual (BIAS_DROPOUT_RESID, ADD) or stored pre-activation (GELU_BWD); F [M, ldf]: pre-activation
 //   output (BIAS_GELU).  Layout TN with more than one K-split needs sk_scratch / sk_counters of the sizes
 //   rb_enc_gemm_plan reports (zero on entry, left zero).  bn_forced / ncta_forced: 0 = choose.
-//   tok_meta / tok (nullable): packed tokens (token_map.cuh).  M (NT, NN) or K (TN) is then the capacity in rows and the
-//   kernel takes the row count from tok_meta; plan_rows (0 = the capacity) is the count to plan tiles and splits for.
+//   tok_meta / tok (nullable; layouts NT and NN): packed tokens (token_map.cuh).  M is then the capacity in rows and the
+//   kernel takes the row count from tok_meta; plan_rows (0 = the capacity) is the count to plan tiles for.
 // Returns 0, or -3 for an unsupported shape (the caller then uses the library GEMM).
 RB_API int rb_enc_gemm(int dtype, int layout, int epi, const void* A, const void* B, void* C, int M, int N, int K, int lda,
                        int ldb, int ldc, const void* bias, const void* R, int ldr, void* F, int ldf, float p_drop,
@@ -979,9 +973,8 @@ RB_API int rb_enc_gemm(int dtype, int layout, int epi, const void* A, const void
   if (epi == E_BIAS_GELU && F == nullptr) return -3;
   if (epi == E_BIAS_DROPOUT_RESID && p_drop > 0.f && seed == nullptr) return -3;
   const bool bf16 = dtype == RB_BF16;
-  const bool tn = layout == L_TN;
-  const int pr = plan_rows > 0 ? plan_rows : (tn ? K : M);
-  const Plan pl = make_plan(layout, epi, tn ? M : pr, N, tn ? pr : K, bn_forced, ncta_forced);
+  if (layout == L_TN && tok_meta != nullptr) return -3;
+  const Plan pl = make_plan(layout, epi, plan_rows > 0 ? plan_rows : M, N, K, bn_forced, ncta_forced);
   const int BN = pl.bn, b_rows = BN / pl.ncta;
   Maps m;
   int rc;

@@ -261,9 +261,8 @@ static int launch(const Maps& m, const Params& p, cudaStream_t st) {
 
 using namespace rb;
 
-// Bytes of scratch and words of (zeroed) counters that rb_wgrad_group needs for up to MAX_PROBS problems with n_tiles in all.
+// Bytes of scratch that rb_wgrad_group needs.  It also needs two (zeroed) counter words per 256 x 256 tile of its problems.
 RB_API long long rb_wgrad_group_scratch_bytes(void) { return (long long)(sm_count() / 2) * 4 * (long long)wg::PIECE_FLOATS * 4; }
-RB_API int rb_wgrad_group_max(void) { return wg::MAX_PROBS; }
 
 // dW_i [M_i, ldc_i >= N_i] = A_i [K, lda_i >= M_i]^T B_i [K, ldb_i >= N_i] for i < n.  dims: per problem M, N, lda, ldb, ldc (all
 // multiples of 8); K token rows, or with tok_meta (token_map.cuh) at most K.

@@ -410,7 +410,7 @@ def _enc_gemm(layout, epi, A, B, C, M, N, K, bias=None, R=None, F=None, p=0.0, r
         ncta = int(os.environ.get("RENEE_B200_GEMM_NCTA", "0"))
     if layout == L_TN:
         ncta_o, bn_o, sp_o, words_o, floats_o = _I(0), _I(0), _I(0), _I(0), _LL(0)
-        lib().rb_enc_gemm_plan(_I(layout), _I(epi), _I(M), _I(N), _I(hint or K), _I(bn), _I(ncta), _c.byref(ncta_o), _c.byref(bn_o),
+        lib().rb_enc_gemm_plan(_I(layout), _I(epi), _I(M), _I(N), _I(K), _I(bn), _I(ncta), _c.byref(ncta_o), _c.byref(bn_o),
                                _c.byref(sp_o), _c.byref(floats_o), _c.byref(words_o))
         if sp_o.value > 1:
             key = dev.index if dev.index is not None else torch.cuda.current_device()
@@ -460,11 +460,12 @@ def linear_dgrad(dy, W, out, epi="store", resid=None, pre=None, dbias=None, bn=0
     return out
 
 
-def linear_wgrad(dy, x, dW, bn=0, ncta=0, tmap=None):
-    """``dW = dy.T @ x`` for ``dy [T, N]``, ``x [T, K]``, ``dW [N, K]`` (split over T, reduced in fp32)."""
+def linear_wgrad(dy, x, dW, bn=0, ncta=0):
+    """``dW = dy.T @ x`` for ``dy [T, N]``, ``x [T, K]``, ``dW [N, K]`` (split over T, reduced in fp32): one linear on its own.
+    The engine takes a layer's four at once (:func:`wgrad_group`)."""
     T, N = dy.shape
     K = x.shape[1]
-    _enc_gemm(L_TN, E_SPLITK, dy, x, dW, N, K, T, bn=bn, ncta=ncta, tmap=tmap)
+    _enc_gemm(L_TN, E_SPLITK, dy, x, dW, N, K, T, bn=bn, ncta=ncta)
     return dW
 
 

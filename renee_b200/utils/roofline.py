@@ -92,10 +92,31 @@ def _cases(dev, dt, NS):
             return fn, NS, (Tn * N + N * K + Tn * K) * 2 + extra, 2.0 * Tn * K * N
         return make
 
-    def gemm_wgrad(Tn, N, K):
+    LAYER = ((3 * H, H), (H, H), (F, H), (H, F))       # q/k/v, output projection, FFN1, FFN2
+
+    def packed_map(b, S, len_lo):
+        """The token map of a padded batch with lengths uniform in len_lo..S, and its rows."""
+        lens = torch.randint(len_lo, S + 1, (b,), device=dev)
+        tmap = cu.TokenMap(b, S, dev)
+        tmap.update((torch.arange(S, device=dev)[None] < lens[:, None]).to(torch.int32))
+        tmap.rows_hint = int(lens.sum())
+        return tmap, int(tmap.meta[1])
+
+    def wgrad(Tn, packed=False):
         def make():
-            dy, x, dW = rn(Tn, N, sc=0.1), rn(Tn, K), em(N, K)
-            return (lambda i: cu.linear_wgrad(dy[i], x[i], dW[i])), NS, (Tn * N + Tn * K + N * K) * 2, 2.0 * Tn * K * N
+            tmap, rows = packed_map(Tn // 32, 32, 6) if packed else (None, Tn)
+            group = cu.WgradGroup(LAYER, dev)
+            ops_ = [[(rn(Tn, m, n=1, sc=0.1)[0], rn(Tn, n, n=1)[0], em(m, n, n=1)[0]) for m, n in LAYER] for _ in range(2)]
+            return (lambda i: cu.wgrad_group(ops_[i % 2], group, tmap=tmap)), 2, \
+                sum(rows * (m + n) + m * n for m, n in LAYER) * 2, sum(2.0 * rows * m * n for m, n in LAYER)
+        return make
+
+    def gemm_packed(Tn, K, N):
+        def make():
+            tmap, rows = packed_map(Tn // 32, 32, 6)
+            x, W, out, pre, b = rn(Tn, K), rn(N, K, n=1, sc=0.05)[0], em(Tn, N), em(Tn, N), vec(N)
+            return (lambda i: cu.linear_fwd(x[i], W, out[i], "bias_gelu", bias=b, pre_out=pre[i], tmap=tmap)), NS, \
+                (rows * K + N * K + 2 * rows * N) * 2, 2.0 * rows * K * N
         return make
 
     def lib_mm(Tn, K, N):
@@ -113,12 +134,12 @@ def _cases(dev, dt, NS):
         yield f"gemm dgrad ffn1 add T={Tn}", gemm_dgrad(Tn, F, H, "add")
         yield f"gemm dgrad out-proj store T={Tn}", gemm_dgrad(Tn, H, H, "store")
         yield f"gemm dgrad qkv add T={Tn}", gemm_dgrad(Tn, 3 * H, H, "add")
-        yield f"gemm wgrad ffn2 [768x3072] T={Tn}", gemm_wgrad(Tn, H, F)
-        yield f"gemm wgrad ffn1 [3072x768] T={Tn}", gemm_wgrad(Tn, F, H)
-        yield f"gemm wgrad out-proj [768x768] T={Tn}", gemm_wgrad(Tn, H, H)
-        yield f"gemm wgrad qkv [2304x768] T={Tn}", gemm_wgrad(Tn, 3 * H, H)
+        yield f"wgrad, a layer's four linears in one launch T={Tn}", wgrad(Tn)
         yield f"library mm qkv (cuBLAS, for comparison) T={Tn}", lib_mm(Tn, H, 3 * H)
         yield f"library mm ffn2 (cuBLAS, for comparison) T={Tn}", lib_mm(Tn, F, H)
+
+    yield "gemm fwd ffn1 bias+gelu, packed 256 x 32 (lengths 6..32)", gemm_packed(T, H, F)
+    yield "wgrad, a layer's four linears, packed 256 x 32 (lengths 6..32)", wgrad(T, packed=True)
 
     # ---- encoder element-wise kernels
     def ln_fwd_only():
