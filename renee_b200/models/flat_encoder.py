@@ -18,9 +18,9 @@ so this engine is built for CUDA-graph capture instead:
   library GEMMs and stand-alone element-wise ops;
 * on that path padded tokens are left out: the activations hold packed rows (``ops/csrc/token_map.cuh``), whose number
   the kernels read from the device, so one captured graph serves every batch of its padded shape.  Texts are shorter
-  than the padded length (uniform lengths in the benchmark workloads: 38 to 42 % padding); training steps, padded against
-  packed rows: 256 x 32 tokens 3.90 -> 2.92 ms, 128 x 128 7.41 -> 5.50, 512 x 32 with 1.3 M labels 10.53 -> 8.60,
-  64 x 256 16.58 -> 11.36;
+  than the padded length (uniform lengths in the benchmark workloads: 38 to 42 % padding).  What leaving it out gave when
+  it went in: training steps of 256 x 32 tokens 3.90 -> 2.92 ms, 128 x 128 7.41 -> 5.50, 512 x 32 with 1.3 M labels
+  10.53 -> 8.60, 64 x 256 16.58 -> 11.36;
 * dropout masks are recomputed from a counter-based RNG in the backward pass.
 
 State-dict keys are those of HF DistilBERT (see :mod:`renee_b200.models.encoder`).
@@ -229,9 +229,6 @@ class FlatEncoder:
                           layers=layers, pooled=e(b, H, dtype=torch.float32),
                           dh=e(T, H), dctx=e(T, H), att_ds=att_ds,
                           emb=e(b, self.out_dims, dtype=torch.float32), tmap=None, own=None, lib=None)
-        if self._own_supported and self._packs(S):
-            from ..ops import cuda as cu
-            self._acts["tmap"] = cu.TokenMap(b, S, dev)
         self._acts_key = key
         self.generation += 1      # activation addresses changed: graphs captured over the old ones are stale
 
@@ -244,15 +241,24 @@ class FlatEncoder:
         forward and backward passes would allocate."""
         self._alloc(max(b, capacity), S)
         self._choose_path(b * S)
+        self._token_map(S)
         self._ensure_backward_buffers()
         if self._acts["att_ds"] is not None:
             from ..ops import cuda as cu
             if cu.attention_streams(self.act_dtype, S, self.cfg.dim, self.cfg.n_heads):
                 self._acts["att_ds"].get()
 
-    def _packs(self, S: int) -> bool:
+    def _token_map(self, S: int):
+        """The token map of a pass that packs, made by the first one, or ``None``.  Asked on every pass: the environment may
+        have sent attention to kernels that read the padded layout."""
+        if not (self.own_gemm and self.pack_tokens):
+            return None
         from ..ops import cuda as cu
-        return cu.attention_packs(self.act_dtype, S, self.cfg.dim, self.cfg.n_heads)
+        if not cu.attention_packs(self.act_dtype, S, self.cfg.dim, self.cfg.n_heads):
+            return None
+        if self._acts["tmap"] is None:
+            self._acts["tmap"] = cu.TokenMap(self._acts_key[0], S, self.device)
+        return self._acts["tmap"]
 
     # ------------------------------------------------------------------ forward
     def forward(self, input_ids: torch.Tensor, attention_mask: torch.Tensor, rng, train: bool = True) -> torch.Tensor:
@@ -268,8 +274,7 @@ class FlatEncoder:
         pd = cfg.dropout if train else 0.0
         pa = cfg.attention_dropout if train else 0.0
         po = cfg.attn_output_dropout if train else 0.0
-        # asked again on every pass: the environment may have sent attention to kernels that read the padded layout
-        tmap = A["tmap"] if self.own_gemm and self.pack_tokens and self._packs(S) else None
+        tmap = self._token_map(S)
         packed = {}
         if tmap is not None:
             tmap.rows_hint = min(self.rows_hint, T)

@@ -200,15 +200,20 @@ class TokenMap:
         n = b * S
         z = guard.zeros(2 * n + 3 * b + 4, dtype=torch.int32, device=device, name="encoder.token_map")
         self.tok, self.slot, self.off, self.len, self.cnt, self.meta = z.split([n, n, b, b, b, 4])
+        # every launch of a pass takes some of these: made once, as long as the buffer lives
+        self.pointers = {k: _p(getattr(self, k)) for k in ("tok", "slot", "off", "len", "cnt", "meta")}
         self.rows_hint = 0
 
     def update(self, mask) -> None:
         b, S = mask.shape
-        _call("rb_token_map", _p(mask), _I(b), _I(S), _p(self.off), _p(self.len), _p(self.cnt), _p(self.meta), _stream())
+        _call("rb_token_map", _p(mask), _I(b), _I(S), *_tok(self, "off", "len", "cnt", "meta"), _stream())
+
+
+_NULL = _VP(0)
 
 
 def _tok(tmap, *names):
-    return [_p(None if tmap is None else getattr(tmap, n)) for n in names]
+    return [_NULL if tmap is None else tmap.pointers[n] for n in names]
 
 
 # ----------------------------------------------------------------------------- encoder ops

@@ -15,7 +15,7 @@ def calls(monkeypatch):
 
 
 class _Map:
-    slot = len = meta = torch.zeros(4, dtype=torch.int32)
+    pointers = dict.fromkeys(("slot", "len", "meta"))
 
 
 def _attend(S, hd, dtype, tmap, b=2, nh=2):
