@@ -73,8 +73,11 @@ def _stream():
     return _VP(torch.cuda.current_stream().cuda_stream)
 
 
+_NULL = _VP(0)
+
+
 def _p(t):
-    return _VP(0) if t is None else _VP(t.data_ptr())
+    return _NULL if t is None else _VP(t.data_ptr())
 
 
 def _call(name, *args, launches=1):
@@ -209,11 +212,8 @@ class TokenMap:
         _call("rb_token_map", _p(mask), _I(b), _I(S), *_tok(self, "off", "len", "cnt", "meta"), _stream())
 
 
-_NULL = _VP(0)
-
-
 def _tok(tmap, *names):
-    return [_NULL if tmap is None else tmap.pointers[n] for n in names]
+    return [_NULL] * len(names) if tmap is None else [tmap.pointers[n] for n in names]
 
 
 # ----------------------------------------------------------------------------- encoder ops
