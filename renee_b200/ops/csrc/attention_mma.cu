@@ -4,7 +4,7 @@
 // Same fusion and interface as attention_tc.cu (bias add, scale, key-padding mask, softmax, counter-based
 // attention dropout, head split/merge addressing, q/k/v bias gradients), organised so that the score
 // matrix never touches shared memory:
-//   * one CTA per (batch, head); the padded sequence SP is 32, 64 or 128 and the CTA has SP/16 warps;
+//   * one CTA per (batch, head); the padded sequence SP is 16 to 64 (forward: to 128) and the CTA has SP/16 warps;
 //   * a warp owns 16 query rows.  S = Q K^T (forward) or dP = dO V^T (backward) for those rows is
 //     accumulated in registers by m16n8k16 MMAs fed with ldmatrix, the softmax / softmax-gradient runs on
 //     the accumulator fragments (a row lives in one quad: two shuffles per reduction), and the fragments
@@ -12,8 +12,8 @@
 //   * only dK = dS^T Q and dV = P~^T dO need other warps' rows: dS and P~ go through shared memory once
 //     and each warp then owns 16 key rows.
 // Shared memory per CTA: 3 (forward) or 4 (backward) [SP][72] operand tiles, plus two [SP][SP+8] tiles in
-// the backward: 14 KB / 24 KB at SP = 32, so many CTAs share an SM at short sequences; 55 KB / 143 KB at
-// SP = 128.  At S = 32 a head is a quarter of the 128-row tcgen05 tile, so the warp-level MMA is the
+// the backward: 14 KB / 24 KB at SP = 32, so many CTAs share an SM at short sequences; 28 KB / 56 KB at SP = 64, 55 KB in the
+// forward at SP = 128.  At S = 32 a head is a quarter of the 128-row tcgen05 tile, so the warp-level MMA is the
 // shape that fits this op; the classifier GEMMs, where the FLOPs are, use tcgen05.
 // Reference behaviour: the attention of the HF DistilBERT layers that main.py:225-262 wraps.
 #include <type_traits>
@@ -514,7 +514,8 @@ __device__ __forceinline__ void store_pair(T* __restrict__ base, size_t idx, uin
 }
 
 // ------------------------------------------------------------------------------------ sequences of 65..256 tokens
-// One CTA of SP / 16 warps per (batch, head), SP = 128 or 256, operands staged once.  What keeps the scores in
+// The backward of 65..256 tokens and the forward of 129..256 (up to 128 its score rows still fit in registers): one CTA of
+// SP / 16 warps per (batch, head), SP = 128 or 256, operands staged once.  What keeps the scores in
 // registers at 32..64 tokens does not scale: a warp's 16 x SP score rows and, in the backward, two [SP][SP] tiles in
 // shared memory allowed one CTA of 8 warps per SM at 128 tokens and forced two streaming kernels beyond.  So both passes
 // walk the keys in blocks of KB = 64 over the resident operands: 128 registers per thread, and the dS and P~ tiles shrink
