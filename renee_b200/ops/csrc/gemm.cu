@@ -494,8 +494,8 @@ enc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
               } else if (EPI == E_DW_SGD) {
                 // momentum SGD on the tile: m = mo m + (dW + wd w), w -= lr m, with m rounded to 16 bit first.  One element
                 // at a time this was some 40 instructions per element, more than the tile's bytes take: two per instruction.
-                // The noise of the rounding takes a hash per element, half of what is left (one hash per pair, which gives
-                // other weights for the same seed: step of 512 x 32 tokens and 1.3 M labels 7.90 ms instead of 8.11)
+                // The noise of the rounding takes a hash per element, half of what is left.  1.3 M labels x 768, batch 512:
+                // 2.01 -> 1.76 ms (1.68 with one hash per pair, which gives other weights for the same seed).
                 uint4* slot2 = reinterpret_cast<uint4*>(pan2 + panel_off(r, chunk));
                 float w[8], mm[8];
                 unpack8<T>(*slot, w);
