@@ -484,7 +484,7 @@ class FlatEncoder:
             (("dh_b", H), ("dqkv", 3 * H), ("df1", Fd), ("da1", Fd))
         sets = 2 if self.own_gemm else 1
         sizes = [b * S * n for _, n in widths] * sets
-        flat = guard.empty(sum(sizes), dtype=self.act_dtype, device=self.device, name="encoder.bwd").split(sizes)
+        flat = guard.empty(sum(sizes), dtype=self.act_dtype, device=self.device, name="encoder.activations.bwd").split(sizes)
         self._acts[which] = [{k: flat[len(widths) * i + j].view(b * S, n) for j, (k, n) in enumerate(widths)}
                              for i in range(sets)]
         if self.own_gemm and self._wgrad_group is None:

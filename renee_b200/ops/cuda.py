@@ -201,7 +201,7 @@ class TokenMap:
 
     def __init__(self, b: int, S: int, device):
         n = b * S
-        z = guard.zeros(2 * n + 3 * b + 4, dtype=torch.int32, device=device, name="encoder.token_map")
+        z = guard.zeros(2 * n + 3 * b + 4, dtype=torch.int32, device=device, name="encoder.activations.token_map")
         self.tok, self.slot, self.off, self.len, self.cnt, self.meta = z.split([n, n, b, b, b, 4])
         # every launch of a pass takes some of these: made once, as long as the buffer lives
         self.pointers = {k: _p(getattr(self, k)) for k in ("tok", "slot", "off", "len", "cnt", "meta")}
@@ -480,8 +480,8 @@ class WgradGroup:
 
     def __init__(self, shapes, device):
         tiles = sum(((m + 255) // 256) * ((n + 255) // 256) for m, n in shapes)
-        self.scratch = guard.empty(_wgrad_scratch_bytes(device) // 4, dtype=torch.float32, device=device, name="encoder.wgrad")
-        self.counters = guard.zeros(2 * tiles, dtype=torch.int32, device=device, name="encoder.wgrad")
+        self.scratch = guard.empty(_wgrad_scratch_bytes(device) // 4, dtype=torch.float32, device=device, name="encoder.activations.wgrad")
+        self.counters = guard.zeros(2 * tiles, dtype=torch.int32, device=device, name="encoder.activations.wgrad")
 
 
 def _wgrad_scratch_bytes(device) -> int:
