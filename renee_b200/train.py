@@ -578,6 +578,7 @@ class XCTrainer:
             self._embed_generation = enc.generation
         if len(self._embed_uses) >= 1024:
             self._embed_uses = {k: self._embed_uses[k] for k in self._embed_graphs}
+            self._embed_warm &= set(self._embed_uses)
         uses = self._embed_uses
         uses[shape] = uses.get(shape, 0) + 1
         st = self._embed_graphs.get(shape)
