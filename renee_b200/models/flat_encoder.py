@@ -21,6 +21,9 @@ so this engine is built for CUDA-graph capture instead:
   than the padded length (uniform lengths in the benchmark workloads: 38 to 42 % padding).  What leaving it out gave when
   it went in: training steps of 256 x 32 tokens 3.90 -> 2.92 ms, 128 x 128 7.41 -> 5.50, 512 x 32 with 1.3 M labels
   10.53 -> 8.60, 64 x 256 16.58 -> 11.36;
+* with CLS pooling on that path the last layer goes on with first tokens only behind its attention (``_first_tokens``), as do
+  their gradients up to it: training steps of 256 x 32 tokens 2.58 -> 2.46 ms, 128 x 128 4.60 -> 4.26, 512 x 32 with 1.3 M
+  labels 7.83 -> 7.54; evaluation of 256 x 32 tokens 695 -> 664 us;
 * dropout masks are recomputed from a counter-based RNG in the backward pass.
 
 State-dict keys are those of HF DistilBERT (see :mod:`renee_b200.models.encoder`).
@@ -145,6 +148,7 @@ class FlatEncoder:
         self._wgrad_group = None
         self._wgrad_done = [None, None]
         self.pack_tokens = True        # own GEMM path: leave padded tokens out (TokenMap); a comparison may switch it off
+        self.first_token_layer = True  # packed tokens, CLS pooling: last layer on first tokens only; a comparison may switch it off
         self.rows_hint = 0             # caller's estimate of the kept tokens of the coming batches (tile planning only)
         if self.device.type in ("cuda", "meta") and act_dtype != torch.float32:
             from ..ops import cuda as cu
@@ -260,6 +264,16 @@ class FlatEncoder:
             self._acts["tmap"] = cu.TokenMap(self._acts_key[0], S, self.device)
         return self._acts["tmap"]
 
+    def _first_tokens(self, tmap, S: int):
+        """CLS pooling reads one row per sequence, so behind the attention of the last layer (whose keys and values are all
+        tokens) only first tokens count: its output projection, LayerNorms and FFN, and their gradients, run on ``b`` rows
+        instead of all.  Nothing that is left out reaches the embedding, and the rows' gradients were exact zeros.  For
+        packed tokens with attention kernels that know it, else ``None``."""
+        if tmap is None or self.pooling != "cls" or not self.first_token_layer:
+            return None
+        from ..ops import cuda as cu
+        return tmap.first if cu.attention_first_token(self.act_dtype, S, self.cfg.dim, self.cfg.n_heads) else None
+
     # ------------------------------------------------------------------ forward
     def forward(self, input_ids: torch.Tensor, attention_mask: torch.Tensor, rng, train: bool = True) -> torch.Tensor:
         """ids/mask ``[b, S]`` int32 on the device → pooled embedding ``[b, D]`` fp32 (before the
@@ -280,7 +294,8 @@ class FlatEncoder:
             tmap.rows_hint = min(self.rows_hint, T)
             tmap.update(attention_mask)
             packed = dict(tmap=tmap)
-        self._fw = dict(ids=input_ids, mask=attention_mask, b=b, S=S, pd=pd, pa=pa, po=po, rng=rng, packed=packed)
+        first = self._first_tokens(tmap, S)
+        self._fw = dict(ids=input_ids, mask=attention_mask, b=b, S=S, pd=pd, pa=pa, po=po, rng=rng, packed=packed, first=first)
         h = A["h0"][:T]
         ops.embed_ln_fwd(input_ids, self.view(P, "embeddings.word_embeddings.weight"),
                          self.view(P, "embeddings.position_embeddings.weight"),
@@ -288,7 +303,7 @@ class FlatEncoder:
                          cfg.layer_norm_eps, S, pd, rng, _S_EMB, h, A["mean0"][:T], A["rstd0"][:T],
                          **(dict(mask=attention_mask, **packed) if packed else {}))
         if self.own_gemm:
-            h = self._forward_layers_fused(h, attention_mask, T, pd, pa, po, rng, packed)
+            h = self._forward_layers_fused(h, attention_mask, T, pd, pa, po, rng, packed, first)
         for l, L in enumerate(A["layers"] if not self.own_gemm else ()):
             pre = f"transformer.layer.{l}."
             sb = 8 * (l + 1)
@@ -320,26 +335,37 @@ class FlatEncoder:
             L["h_in"] = h
             h = h2
         pooled = A["pooled"][:b]
-        ops.pool_fwd(h.view(b, S, H), attention_mask, self.pooling, pooled, **packed)
+        if first is not None:
+            ops.pool_fwd(h.view(b, 1, H), attention_mask, self.pooling, pooled)
+        else:
+            ops.pool_fwd(h.view(b, S, H), attention_mask, self.pooling, pooled, **packed)
         if self.bottleneck_dims > 0:
             emb = A["emb"][:b]
             torch.mm(pooled, self.bottleneck_weight().t(), out=emb)   # fp32, master weights
             return emb
         return pooled
 
-    def _forward_layers_fused(self, h, attention_mask, T, pd, pa, po, rng, packed):
+    def _forward_layers_fused(self, h, attention_mask, T, pd, pa, po, rng, packed, first):
         """The transformer blocks on the own GEMMs: 4 GEMMs, 1 attention and 2 LayerNorm launches per layer.  With a
-        token map in ``packed`` the activations hold kept tokens only; the buffers keep their padded capacity."""
+        token map in ``packed`` the activations hold kept tokens only; the buffers keep their padded capacity.  With ``first``
+        the last layer goes on with first tokens only behind its attention (its buffers then hold one row per sequence)."""
         from ..ops import cuda as cu
         cfg, A, P = self.cfg, self._acts, self.p16
         for l, L in enumerate(A["layers"]):
             pre = f"transformer.layer.{l}."
             sb = 8 * (l + 1)
             qkv = L["qkv"][:T]
+            L["h_in"] = h
             cu.linear_fwd(h, self._qkv(P, l, "weight"), qkv, **packed)
+            last = {}
+            if first is not None and l == cfg.n_layers - 1:
+                T = attention_mask.shape[0]
+                last = dict(first=(h, L["ao"][:T]))
             ctx = L["ctx"][:T]
             ops.attention_fwd(qkv, self._qkv(P, l, "bias"), attention_mask, cfg.n_heads, pa, rng, sb + _S_PROBS,
-                              ctx, L["att"], **packed)
+                              ctx, L["att"], **packed, **last)
+            if last:
+                h, packed = L["ao"][:T], dict(tmap=first)
             pre1 = L["pre1"][:T]
             cu.linear_fwd(ctx, self.view(P, pre + "attention.out_lin.weight"), pre1, "bias_dropout_resid",
                           bias=self.view(P, pre + "attention.out_lin.bias"), resid=h, p=po, rng=rng, stream=sb + _S_ATTN,
@@ -357,7 +383,6 @@ class FlatEncoder:
             h2 = L["h2"][:T]
             cu.ln_fwd(pre2, self.view(P, pre + "output_layer_norm.weight"), self.view(P, pre + "output_layer_norm.bias"),
                       cfg.layer_norm_eps, h2, L["mean2"][:T], L["rstd2"][:T], **packed)
-            L["h_in"] = h
             h = h2
         return h
 
@@ -382,18 +407,20 @@ class FlatEncoder:
         if on_layer_done is not None:
             on_layer_done(-1)       # embeddings and every vector-shaped gradient are final: the whole buffer is
 
-    def _wgrad_layer(self, par: int, items) -> None:
-        """The weight gradients of one layer in one launch, on the weight-gradient stream (ordered after everything issued
-        so far on the current one).  Their inputs live in the backward buffers of parity ``par``, which the layer after
+    def _wgrad_layer(self, par: int, *groups) -> None:
+        """The weight gradients of one layer, one launch per ``(items, token map arguments)``, on the weight-gradient stream
+        (ordered after everything issued so far on the current one).  Their inputs live in the backward buffers of parity ``par``, which the layer after
         the next overwrites: :meth:`_wgrad_wait` comes before that."""
         from ..ops import cuda as cu
         side = self._wgrad_stream
         if side is None:
-            cu.wgrad_group(items, self._wgrad_group, **self._fw["packed"])
+            for items, packed in groups:
+                cu.wgrad_group(items, self._wgrad_group, **packed)
             return
         side.wait_stream(torch.cuda.current_stream())
         with torch.cuda.stream(side):
-            cu.wgrad_group(items, self._wgrad_group, **self._fw["packed"])
+            for items, packed in groups:
+                cu.wgrad_group(items, self._wgrad_group, **packed)
             self._wgrad_done[par] = side.record_event()
 
     def _wgrad_wait(self, par: int) -> None:
@@ -421,7 +448,10 @@ class FlatEncoder:
             d_pool = d_emb
         self._ensure_backward_buffers()
         dh = A["dh"][:T]
-        ops.pool_bwd(d_pool, mask, self.pooling, S, dh.view(b, S, H), **packed)
+        if fw["first"] is not None:
+            ops.pool_bwd(d_pool, mask, self.pooling, 1, dh[:b].view(b, 1, H))
+        else:
+            ops.pool_bwd(d_pool, mask, self.pooling, S, dh.view(b, S, H), **packed)
         for l in reversed(range(cfg.n_layers)):
             L = A["layers"][l]
             pre = f"transformer.layer.{l}."
@@ -497,30 +527,42 @@ class FlatEncoder:
         cfg, A, P, G, fw = self.cfg, self._acts, self.p16, self.g, self._fw
         T, packed, pd, po, rng = fw["b"] * fw["S"], fw["packed"], fw["pd"], fw["po"], fw["rng"]
         pre, sb, par = f"transformer.layer.{l}.", 8 * (l + 1), l & 1
-        buf = {k: t[:T] for k, t in A["own"][par].items()}
+        # n rows, numbered by `rows`: all tokens, or first tokens only up to the attention of the last layer
+        n, rows = T, packed
+        if fw["first"] is not None and l == cfg.n_layers - 1:
+            n, rows = fw["b"], dict(tmap=fw["first"])
+        one_row = rows is not packed
+        buf = A["own"][par]
         self._wgrad_wait(par)
         d_pre2, d_f2 = ops.bias_dropout_add_ln_bwd(
-            dh, L["pre2"][:T], self.view(P, pre + "output_layer_norm.weight"), L["mean2"][:T], L["rstd2"][:T],
+            dh[:n], L["pre2"][:n], self.view(P, pre + "output_layer_norm.weight"), L["mean2"][:n], L["rstd2"][:n],
             pd, rng, sb + _S_FFN,
             self.view(G, pre + "output_layer_norm.weight"), self.view(G, pre + "output_layer_norm.bias"),
-            self.view(G, pre + "ffn.lin2.bias"), buf["dpre2"], L["f2"][:T], **packed)
-        df1 = cu.linear_dgrad(d_f2, self.view(P, pre + "ffn.lin2.weight"), buf["df1"], "gelu_bwd", pre=L["f1"][:T],
-                              dbias=self.view(G, pre + "ffn.lin1.bias"), **packed)
-        dh1 = cu.linear_dgrad(df1, self.view(P, pre + "ffn.lin1.weight"), dh, "add", resid=d_pre2, **packed)
+            self.view(G, pre + "ffn.lin2.bias"), buf["dpre2"][:n], L["f2"][:n], **rows)
+        df1 = cu.linear_dgrad(d_f2, self.view(P, pre + "ffn.lin2.weight"), buf["df1"][:n], "gelu_bwd", pre=L["f1"][:n],
+                              dbias=self.view(G, pre + "ffn.lin1.bias"), **rows)
+        dh1 = cu.linear_dgrad(df1, self.view(P, pre + "ffn.lin1.weight"), dh[:n], "add", resid=d_pre2, **rows)
         d_pre1, d_ao = ops.bias_dropout_add_ln_bwd(
-            dh1, L["pre1"][:T], self.view(P, pre + "sa_layer_norm.weight"), L["mean1"][:T], L["rstd1"][:T],
+            dh1, L["pre1"][:n], self.view(P, pre + "sa_layer_norm.weight"), L["mean1"][:n], L["rstd1"][:n],
             po, rng, sb + _S_ATTN,
             self.view(G, pre + "sa_layer_norm.weight"), self.view(G, pre + "sa_layer_norm.bias"),
-            self.view(G, pre + "attention.out_lin.bias"), buf["dpre1"], L["ao"][:T], **packed)
-        dctx = cu.linear_dgrad(d_ao, self.view(P, pre + "attention.out_lin.weight"), A["dctx"][:T], **packed)
-        dqkv = buf["dqkv"]
+            self.view(G, pre + "attention.out_lin.bias"), buf["dpre1"][:n], L["ao"][:n], **rows)
+        dctx = cu.linear_dgrad(d_ao, self.view(P, pre + "attention.out_lin.weight"), A["dctx"][:n], **rows)
+        dqkv = buf["dqkv"][:T]
+        # with one row per sequence the attention kernel lays the residual's gradient out for all tokens (h2 is free by now)
+        resid = L["h2"][:T] if one_row else d_pre1
         ops.attention_bwd(dctx, L["qkv"][:T], self._qkv(P, l, "bias"), fw["mask"], cfg.n_heads, fw["pa"], rng,
-                          sb + _S_PROBS, L["att"], dqkv, self._qkv(G, l, "bias"), **packed)
-        self._wgrad_layer(par, [(df1, L["h1"][:T], self.view(G, pre + "ffn.lin1.weight")),
-                                (d_f2, L["a1"][:T], self.view(G, pre + "ffn.lin2.weight")),
-                                (dqkv, L["h_in"], self._qkv(G, l, "weight")),
-                                (d_ao, L["ctx"][:T], self.view(G, pre + "attention.out_lin.weight"))])
-        cu.linear_dgrad(dqkv, self._qkv(P, l, "weight"), dh, "add", resid=d_pre1, **packed)
+                          sb + _S_PROBS, L["att"], dqkv, self._qkv(G, l, "bias"), **packed,
+                          **(dict(first=(d_pre1, resid)) if one_row else {}))
+        dense = [(df1, L["h1"][:n], self.view(G, pre + "ffn.lin1.weight")),
+                 (d_f2, L["a1"][:n], self.view(G, pre + "ffn.lin2.weight"))]
+        qkv = [(dqkv, L["h_in"], self._qkv(G, l, "weight"))]
+        out = [(d_ao, L["ctx"][:n], self.view(G, pre + "attention.out_lin.weight"))]
+        if one_row:
+            self._wgrad_layer(par, (qkv, packed), (dense + out, {}))
+        else:
+            self._wgrad_layer(par, (dense + qkv + out, packed))
+        cu.linear_dgrad(dqkv, self._qkv(P, l, "weight"), dh, "add", resid=resid, **packed)
         if on_layer_done is not None:
             self._wgrad_wait(par)           # the caller may reduce the layer's gradients from here on
             on_layer_done(l)

@@ -15,6 +15,11 @@
 // the backward: 14 KB / 24 KB at SP = 32, so many CTAs share an SM at short sequences; 28 KB / 56 KB at SP = 64, 55 KB in the
 // forward at SP = 128.  At S = 32 a head is a quarter of the 128-row tcgen05 tile, so the warp-level MMA is the
 // shape that fits this op; the classifier GEMMs, where the FLOPs are, use tcgen05.
+// First-token variant (template parameter CLS): where only the first token of a sequence is read behind a layer (CLS pooling
+// behind the last one), it is the only query.  Its row goes through the same fragments and the same sums as above -- the other
+// 15 rows of its tile are dropped or zero -- so it comes out bit for bit; ctx and dctx then have one row per sequence, the
+// forward also copies the first token's layer input there (the residual of the output projection), and the backward spreads
+// the gradient of that residual over the packed rows (zeros behind the first), where the next GEMM adds it.
 // Reference behaviour: the attention of the HF DistilBERT layers that main.py:225-262 wraps.
 #include <type_traits>
 #include "common.cuh"
@@ -34,6 +39,9 @@ struct Tok {
   const int* len;    // [b] last kept position + 1
   const int* meta;   // row counts
 };
+// First-token variant: forward src = layer input, packed rows of H columns, dst = its first tokens [b, H]; backward src = [b, H]
+// gradient of the residual, dst = packed rows.
+template <typename T> struct FirstTok { const T* src; T* dst; };
 __device__ __forceinline__ int seq_len(const Tok& tk, int b, int S) { return tk.slot != nullptr ? __ldcg(tk.len + b) : S; }
 __device__ __forceinline__ int seq_row(const Tok& tk, int b, int S, int s) {
   return tk.slot != nullptr ? __ldcg(tk.slot + (size_t)b * S + s) : b * S + s;
@@ -216,7 +224,8 @@ __device__ __forceinline__ uint32_t load_pair_raw(const T* __restrict__ base, si
 // exist are zero, rows >= lim are left alone.
 // The CTA has SP * 2 threads and the tiles SP * HD / 8 segments of 8 columns, so a thread owns the same 8 columns of
 // HD / 16 rows: all of its global loads are issued before the first one is used.
-template <typename T, int SP, int HD, bool WITH_DO>
+// CLS: dO has one row per sequence (that of token 0), and only the first 16 queries are staged.
+template <typename T, int SP, int HD, bool WITH_DO, bool CLS = false>
 __device__ __forceinline__ void stage_operands(const T* __restrict__ qkv, const T* __restrict__ bqkv, const T* __restrict__ dctx,
                                                T* sQ, T* sK, T* sV, T* sDO, const Tok& tk, int b, int h, int S, int H, int len,
                                                int lim) {
@@ -233,8 +242,13 @@ __device__ __forceinline__ void stage_operands(const T* __restrict__ qkv, const 
   for (int it = 0; it < NIT; ++it) {
     if (row[it] >= 0) {
       const size_t base = (size_t)row[it] * 3 * H + h * HD + d;
-      rq[it] = load_raw8(qkv + base); rk[it] = load_raw8(qkv + base + H); rv[it] = load_raw8(qkv + base + 2 * H);
-      if constexpr (WITH_DO) rg[it] = load_raw8(dctx + (size_t)row[it] * H + h * HD + d);
+      if (!CLS || s0 + it * ROWS_PER_PASS < 16) rq[it] = load_raw8(qkv + base);
+      rk[it] = load_raw8(qkv + base + H); rv[it] = load_raw8(qkv + base + 2 * H);
+      if constexpr (WITH_DO) {
+        if (!CLS) rg[it] = load_raw8(dctx + (size_t)row[it] * H + h * HD + d);
+        else if (s0 + it * ROWS_PER_PASS == 0) rg[it] = load_raw8(dctx + (size_t)b * H + h * HD + d);
+        else rg[it].v = make_uint4(0u, 0u, 0u, 0u);
+      }
     }
   }
   float bq[8], bk[8], bv[8];
@@ -245,23 +259,47 @@ __device__ __forceinline__ void stage_operands(const T* __restrict__ qkv, const 
     if (s >= lim) continue;
     float q[8], k[8], v[8];
     if (row[it] >= 0) {
-      unpack8(rq[it], q); unpack8(rk[it], k); unpack8(rv[it], v);
+      if (!CLS || s < 16) unpack8(rq[it], q);
+      unpack8(rk[it], k); unpack8(rv[it], v);
 #pragma unroll
-      for (int j = 0; j < 8; ++j) { q[j] += bq[j]; k[j] += bk[j]; v[j] += bv[j]; }
-      if constexpr (WITH_DO) *reinterpret_cast<uint4*>(sDO + s * RP + d) = rg[it].v;
+      for (int j = 0; j < 8; ++j) { if (!CLS || s < 16) q[j] += bq[j]; k[j] += bk[j]; v[j] += bv[j]; }
+      if constexpr (WITH_DO) { if (!CLS || s < 16) *reinterpret_cast<uint4*>(sDO + s * RP + d) = rg[it].v; }
     } else {
 #pragma unroll
       for (int j = 0; j < 8; ++j) { q[j] = 0.f; k[j] = 0.f; v[j] = 0.f; }
-      if constexpr (WITH_DO) *reinterpret_cast<uint4*>(sDO + s * RP + d) = make_uint4(0u, 0u, 0u, 0u);
+      if constexpr (WITH_DO) { if (!CLS || s < 16) *reinterpret_cast<uint4*>(sDO + s * RP + d) = make_uint4(0u, 0u, 0u, 0u); }
     }
-    store8(sQ + s * RP + d, q); store8(sK + s * RP + d, k); store8(sV + s * RP + d, v);
+    if (!CLS || s < 16) store8(sQ + s * RP + d, q);
+    store8(sK + s * RP + d, k); store8(sV + s * RP + d, v);
   }
 }
 
-template <typename T, int SP, int HD>
+// First-token variant, backward: dst rows of the sequence = src row b for token 0, zeros for the others, columns of head h.
+template <typename T, int HD>
+__device__ __forceinline__ void spread_first(const FirstTok<T>& ft, const int* sRow, int len, int b, int h, int H) {
+  constexpr int SEGS = HD / 8;
+  for (int i = threadIdx.x; i < len * SEGS; i += blockDim.x) {
+    const int s = i / SEGS, c = h * HD + (i % SEGS) * 8, row = sRow[s];
+    if (row < 0) continue;
+    *reinterpret_cast<uint4*>(ft.dst + (size_t)row * H + c) =
+        s == 0 ? *reinterpret_cast<const uint4*>(ft.src + (size_t)b * H + c) : make_uint4(0u, 0u, 0u, 0u);
+  }
+}
+// ... and the zero gradient of the queries behind the 16 of the first tile (dst already at the head's first column).
+template <typename T, int HD>
+__device__ __forceinline__ void zero_rest(T* dst, const int* sRow, int len, int ld) {
+  constexpr int SEGS = HD / 8;
+  for (int i = 16 * SEGS + threadIdx.x; i < len * SEGS; i += blockDim.x) {
+    const int row = sRow[i / SEGS];
+    if (row >= 0) *reinterpret_cast<uint4*>(dst + (size_t)row * ld + (i % SEGS) * 8) = make_uint4(0u, 0u, 0u, 0u);
+  }
+}
+
+template <typename T, int SP, int HD, bool CLS>
 __global__ void __launch_bounds__(SP * 2, SP == 128 ? 2 : 1) attention_fwd_mma_kernel(
     const T* __restrict__ qkv, const T* __restrict__ bqkv, const int* __restrict__ mask, T* __restrict__ ctx,
-    T* __restrict__ probs, int S, int H, int nh, float p, const int* __restrict__ seed_ptr, uint32_t stream, const Tok tk, int len_lo) {
+    T* __restrict__ probs, int S, int H, int nh, float p, const int* __restrict__ seed_ptr, uint32_t stream, const Tok tk, int len_lo,
+    const FirstTok<T> ft) {
   rb::grid_dep_wait();        // launched with launch_pdl: nothing above touches global memory
   rb::grid_dep_launch();      // the kernel that follows may start its set-up; it waits for this grid before reading
   extern __shared__ __align__(128) uint8_t sm_raw[];
@@ -277,7 +315,7 @@ __global__ void __launch_bounds__(SP * 2, SP == 128 ? 2 : 1) attention_fwd_mma_k
   const uint32_t seed = p > 0.f ? (uint32_t)(*seed_ptr) : 0u;
   const float inv_keep = p > 0.f ? 1.f / (1.f - p) : 1.f;
   const float scale = rsqrtf((float)HD);
-  if (tk.slot != nullptr && b == (int)gridDim.y - 1) clear_zero_rows<T>(tk, ctx, H, h * HD, HD);
+  if (!CLS && tk.slot != nullptr && b == (int)gridDim.y - 1) clear_zero_rows<T>(tk, ctx, H, h * HD, HD);
   const int len = seq_len(tk, b, S), lim = (len + 15) & ~15;
   if (len > SP || len <= len_lo) return;       // another launch serves this length
   for (int j = threadIdx.x; j < SP; j += blockDim.x) {
@@ -285,10 +323,13 @@ __global__ void __launch_bounds__(SP * 2, SP == 128 ? 2 : 1) attention_fwd_mma_k
     sRow[j] = row;
     sCode[j] = row >= 0 ? (mask[b * S + j] != 0 ? 1 : 2) : 0;
   }
-  stage_operands<T, SP, HD, false>(qkv, bqkv, nullptr, sQ, sK, sV, nullptr, tk, b, h, S, H, len, lim);
+  stage_operands<T, SP, HD, false, CLS>(qkv, bqkv, nullptr, sQ, sK, sV, nullptr, tk, b, h, S, H, len, lim);
   __syncthreads();
   const int r0 = warp * 16;
-  if (r0 >= lim) return;
+  if (r0 >= (CLS ? 16 : lim)) return;
+  if (CLS && lane < HD / 8)
+    *reinterpret_cast<uint4*>(ft.dst + (size_t)b * H + h * HD + 8 * lane) =
+        *reinterpret_cast<const uint4*>(ft.src + (size_t)sRow[0] * H + h * HD + 8 * lane);
   float acc[SP / 8][4];
 #pragma unroll
   for (int j = 0; j < SP / 8; ++j) { acc[j][0] = 0.f; acc[j][1] = 0.f; acc[j][2] = 0.f; acc[j][3] = 0.f; }
@@ -323,7 +364,7 @@ __global__ void __launch_bounds__(SP * 2, SP == 128 ? 2 : 1) attention_fwd_mma_k
   }
   sum0 = quad_sum(sum0); sum1 = quad_sum(sum1);
   const int i0 = r0 + g, i1 = r0 + g + 8;
-  const int row0 = sRow[i0], row1 = sRow[i1];
+  const int row0 = !CLS ? sRow[i0] : (i0 == 0 ? b : -1), row1 = CLS ? -1 : sRow[i1];     // rows of ctx
   const float inv0 = row0 >= 0 ? 1.f / sum0 : 0.f, inv1 = row1 >= 0 ? 1.f / sum1 : 0.f;
   const size_t prow0 = ((size_t)(b * nh + h) * S + i0) * S, prow1 = ((size_t)(b * nh + h) * S + i1) * S;
   const bool pair_store = (S & 1) == 0;   // then every (row, even column) element is 4-byte aligned
@@ -369,11 +410,11 @@ __global__ void __launch_bounds__(SP * 2, SP == 128 ? 2 : 1) attention_fwd_mma_k
   write_rows<T>(out, ctx + h * HD, H, row0, row1, lane, nullptr);
 }
 
-template <typename T, int SP, int HD>
+template <typename T, int SP, int HD, bool CLS>
 __global__ void __launch_bounds__(SP * 2, SP == 64 ? 4 : 1) attention_bwd_mma_kernel(
     const T* __restrict__ dctx, const T* __restrict__ qkv, const T* __restrict__ bqkv, const T* __restrict__ probs,
     T* __restrict__ dqkv, int S, int H, int nh, float p, const int* __restrict__ seed_ptr, uint32_t stream,
-    float* __restrict__ bias_acc, const Tok tk, int len_lo) {
+    float* __restrict__ bias_acc, const Tok tk, int len_lo, const FirstTok<T> ft) {
   rb::grid_dep_wait();
   rb::grid_dep_launch();
   extern __shared__ __align__(128) uint8_t sm_raw[];
@@ -396,7 +437,8 @@ __global__ void __launch_bounds__(SP * 2, SP == 64 ? 4 : 1) attention_bwd_mma_ke
   if (bias_acc != nullptr)
     for (int i = threadIdx.x; i < 3 * HD; i += blockDim.x) sBias[i] = 0.f;
   if (tk.slot != nullptr && b == (int)gridDim.y - 1)
-    for (int w = 0; w < 3; ++w) clear_zero_rows<T>(tk, dqkv, 3 * H, w * H + h * HD, HD);
+    for (int w = 0; w < (CLS ? 4 : 3); ++w)
+      clear_zero_rows<T>(tk, w < 3 ? dqkv : ft.dst, w < 3 ? 3 * H : H, (w < 3 ? w * H : 0) + h * HD, HD);
   const int len = seq_len(tk, b, S), lim = (len + 15) & ~15;
   if (len > SP || len <= len_lo) return;       // another launch serves this length
   for (int j = threadIdx.x; j < SP; j += blockDim.x) sRow[j] = j < len ? seq_row(tk, b, S, j) : -1;
@@ -408,13 +450,18 @@ __global__ void __launch_bounds__(SP * 2, SP == 64 ? 4 : 1) attention_bwd_mma_ke
 #pragma unroll
   for (int j = 0; j < SP / 8; ++j) {
     const int c = 8 * j + 2 * t;
-    wf[j][0] = load_pair_raw<T>(probs, prow0 + c, r0 < lim && 8 * j < lim && i0 < S && c < S, c + 1 < S, pair_load);
-    wf[j][1] = load_pair_raw<T>(probs, prow1 + c, r0 < lim && 8 * j < lim && i1 < S && c < S, c + 1 < S, pair_load);
+    wf[j][0] = load_pair_raw<T>(probs, prow0 + c, r0 < lim && 8 * j < lim && i0 < (CLS ? 1 : S) && c < S, c + 1 < S, pair_load);
+    wf[j][1] = load_pair_raw<T>(probs, prow1 + c, r0 < lim && 8 * j < lim && i1 < (CLS ? 1 : S) && c < S, c + 1 < S, pair_load);
   }
-  stage_operands<T, SP, HD, true>(qkv, bqkv, dctx, sQ, sK, sV, sDO, tk, b, h, S, H, len, lim);
+  stage_operands<T, SP, HD, true, CLS>(qkv, bqkv, dctx, sQ, sK, sV, sDO, tk, b, h, S, H, len, lim);
   __syncthreads();
   const int row0 = sRow[r0 + g], row1 = sRow[r0 + g + 8];
-  if (r0 < lim) {
+  const int qlim = CLS ? 16 : lim;             // queries that have a gradient (CLS: the rows behind the first are zeros)
+  if (CLS) {
+    spread_first<T, HD>(ft, sRow, len, b, h, H);
+    zero_rest<T, HD>(dqkv + h * HD, sRow, len, 3 * H);
+  }
+  if (r0 < qlim) {
     // dP for this warp's 16 query rows, then dS and P~ in registers
     float acc[SP / 8][4];
 #pragma unroll
@@ -471,12 +518,12 @@ __global__ void __launch_bounds__(SP * 2, SP == 64 ? 4 : 1) attention_bwd_mma_ke
     float out[HD / 8][4];
 #pragma unroll
     for (int jd = 0; jd < HD / 8; ++jd) { out[jd][0] = 0.f; out[jd][1] = 0.f; out[jd][2] = 0.f; out[jd][3] = 0.f; }
-    transposed_times_rows<T, SP, HD>(out, sDS, PP, r0, sQ, lane, lim);
+    transposed_times_rows<T, SP, HD>(out, sDS, PP, r0, sQ, lane, qlim);
     write_rows<T>(out, dqkv + H + h * HD, 3 * H, row0, row1, lane,
                   bias_acc != nullptr ? sBias + HD : nullptr);
 #pragma unroll
     for (int jd = 0; jd < HD / 8; ++jd) { out[jd][0] = 0.f; out[jd][1] = 0.f; out[jd][2] = 0.f; out[jd][3] = 0.f; }
-    transposed_times_rows<T, SP, HD>(out, sW, PP, r0, sDO, lane, lim);
+    transposed_times_rows<T, SP, HD>(out, sW, PP, r0, sDO, lane, qlim);
     write_rows<T>(out, dqkv + 2 * H + h * HD, 3 * H, row0, row1, lane,
                   bias_acc != nullptr ? sBias + 2 * HD : nullptr);
   }
@@ -527,11 +574,11 @@ __device__ __forceinline__ void store_pair(T* __restrict__ base, size_t idx, uin
 //             to shared memory, dQ += dS K, then the block's dK = dS^T Q and dV = P~^T dO, spread over all warps.
 constexpr int KB = 64;
 
-template <typename T, int SP, int HD>
+template <typename T, int SP, int HD, bool CLS>
 __global__ void __launch_bounds__(SP * 2, SP == 128 ? 2 : 1) attention_fwd_blk_kernel(
     const T* __restrict__ qkv, const T* __restrict__ bqkv, const int* __restrict__ mask, T* __restrict__ ctx,
     T* __restrict__ probs, int S, int H, int nh, float p, const int* __restrict__ seed_ptr, uint32_t stream, const Tok tk,
-    int len_lo) {
+    int len_lo, const FirstTok<T> ft) {
   rb::grid_dep_wait();
   rb::grid_dep_launch();
   extern __shared__ __align__(128) uint8_t sm_raw[];
@@ -547,7 +594,7 @@ __global__ void __launch_bounds__(SP * 2, SP == 128 ? 2 : 1) attention_fwd_blk_k
   const uint32_t seed = p > 0.f ? (uint32_t)(*seed_ptr) : 0u;
   const float inv_keep = p > 0.f ? 1.f / (1.f - p) : 1.f;
   const float scale = rsqrtf((float)HD);
-  if (tk.slot != nullptr && b == (int)gridDim.y - 1) clear_zero_rows<T>(tk, ctx, H, h * HD, HD);
+  if (!CLS && tk.slot != nullptr && b == (int)gridDim.y - 1) clear_zero_rows<T>(tk, ctx, H, h * HD, HD);
   const int len = seq_len(tk, b, S), lim = (len + 15) & ~15;
   if (len > SP || len <= len_lo) return;
   for (int j = threadIdx.x; j < SP; j += blockDim.x) {
@@ -555,10 +602,13 @@ __global__ void __launch_bounds__(SP * 2, SP == 128 ? 2 : 1) attention_fwd_blk_k
     sRow[j] = row;
     sCode[j] = row >= 0 ? (mask[b * S + j] != 0 ? 1 : 2) : 0;
   }
-  stage_operands<T, SP, HD, false>(qkv, bqkv, nullptr, sQ, sK, sV, nullptr, tk, b, h, S, H, len, lim);
+  stage_operands<T, SP, HD, false, CLS>(qkv, bqkv, nullptr, sQ, sK, sV, nullptr, tk, b, h, S, H, len, lim);
   __syncthreads();
   const int r0 = warp * 16;
-  if (r0 >= lim) return;
+  if (r0 >= (CLS ? 16 : lim)) return;
+  if (CLS && lane < HD / 8)
+    *reinterpret_cast<uint4*>(ft.dst + (size_t)b * H + h * HD + 8 * lane) =
+        *reinterpret_cast<const uint4*>(ft.src + (size_t)sRow[0] * H + h * HD + 8 * lane);
   float m0 = -1e30f, m1 = -1e30f, l0 = 0.f, l1 = 0.f;
 #pragma unroll 1
   for (int k0 = 0; k0 < lim; k0 += KB) {
@@ -595,7 +645,7 @@ __global__ void __launch_bounds__(SP * 2, SP == 128 ? 2 : 1) attention_fwd_blk_k
   }
   l0 = quad_sum(l0); l1 = quad_sum(l1);
   const int i0 = r0 + g, i1 = r0 + g + 8;
-  const int row0 = sRow[i0], row1 = sRow[i1];
+  const int row0 = !CLS ? sRow[i0] : (i0 == 0 ? b : -1), row1 = CLS ? -1 : sRow[i1];     // rows of ctx
   const float inv0 = row0 >= 0 ? 1.f / l0 : 0.f, inv1 = row1 >= 0 ? 1.f / l1 : 0.f;
   const size_t prow0 = ((size_t)(b * nh + h) * S + i0) * S, prow1 = ((size_t)(b * nh + h) * S + i1) * S;
   const bool pair = (S & 1) == 0;          // then every (row, even column) element is 4-byte aligned
@@ -637,11 +687,11 @@ __global__ void __launch_bounds__(SP * 2, SP == 128 ? 2 : 1) attention_fwd_blk_k
   write_rows<T>(out, ctx + h * HD, H, row0, row1, lane, nullptr);
 }
 
-template <typename T, int SP, int HD>
+template <typename T, int SP, int HD, bool CLS>
 __global__ void __launch_bounds__(SP * 2, SP == 128 ? 2 : 1) attention_bwd_blk_kernel(
     const T* __restrict__ dctx, const T* __restrict__ qkv, const T* __restrict__ bqkv, const T* __restrict__ probs,
     T* __restrict__ dqkv, int S, int H, int nh, float p, const int* __restrict__ seed_ptr, uint32_t stream,
-    float* __restrict__ bias_acc, const Tok tk, int len_lo) {
+    float* __restrict__ bias_acc, const Tok tk, int len_lo, const FirstTok<T> ft) {
   rb::grid_dep_wait();
   rb::grid_dep_launch();
   extern __shared__ __align__(128) uint8_t sm_raw[];
@@ -664,17 +714,23 @@ __global__ void __launch_bounds__(SP * 2, SP == 128 ? 2 : 1) attention_bwd_blk_k
   const float inv_keep = p > 0.f ? 1.f / (1.f - p) : 1.f;
   const float scale = rsqrtf((float)HD);
   if (tk.slot != nullptr && b == (int)gridDim.y - 1)
-    for (int w = 0; w < 3; ++w) clear_zero_rows<T>(tk, dqkv, 3 * H, w * H + h * HD, HD);
+    for (int w = 0; w < (CLS ? 4 : 3); ++w)
+      clear_zero_rows<T>(tk, w < 3 ? dqkv : ft.dst, w < 3 ? 3 * H : H, (w < 3 ? w * H : 0) + h * HD, HD);
   const int len = seq_len(tk, b, S), lim = (len + 15) & ~15;
   if (len > SP || len <= len_lo) return;
   if (bias_acc != nullptr)
     for (int i = threadIdx.x; i < 3 * HD; i += blockDim.x) sBias[i] = 0.f;
   for (int j = threadIdx.x; j < SP; j += blockDim.x) sRow[j] = j < len ? seq_row(tk, b, S, j) : -1;
-  stage_operands<T, SP, HD, true>(qkv, bqkv, dctx, sQ, sK, sV, sDO, tk, b, h, S, H, len, lim);
+  stage_operands<T, SP, HD, true, CLS>(qkv, bqkv, dctx, sQ, sK, sV, sDO, tk, b, h, S, H, len, lim);
   __syncthreads();
   const int r0 = warp * 16, i0 = r0 + g, i1 = r0 + g + 8;
-  const bool active = r0 < lim;                    // this warp's 16 query rows exist
+  const int qlim = CLS ? 16 : lim;                 // queries that have a gradient (CLS: the rows behind the first are zeros)
+  const bool active = r0 < qlim;                   // this warp's 16 query rows exist
   const int row0 = sRow[i0], row1 = sRow[i1];
+  if (CLS) {
+    spread_first<T, HD>(ft, sRow, len, b, h, H);
+    zero_rest<T, HD>(dqkv + h * HD, sRow, len, 3 * H);
+  }
   const size_t prow0 = ((size_t)(b * nh + h) * S + i0) * S, prow1 = ((size_t)(b * nh + h) * S + i1) * S;
   const bool pair = (S & 1) == 0;
   uint32_t kept[SP / KB];                          // dropout decisions: bit 4 j + e of block k is element e of tile j
@@ -689,8 +745,8 @@ __global__ void __launch_bounds__(SP * 2, SP == 128 ? 2 : 1) attention_bwd_blk_k
 #pragma unroll
       for (int j = 0; j < KB / 8; ++j) {
         const int key = k0 + 8 * j + 2 * t;
-        w0[j] = load_pair_raw<T>(probs, prow0 + key, row0 >= 0 && k0 + 8 * j < lim && key < S, key + 1 < S, pair);
-        w1[j] = load_pair_raw<T>(probs, prow1 + key, row1 >= 0 && k0 + 8 * j < lim && key < S, key + 1 < S, pair);
+        w0[j] = load_pair_raw<T>(probs, prow0 + key, row0 >= 0 && (!CLS || i0 == 0) && k0 + 8 * j < lim && key < S, key + 1 < S, pair);
+        w1[j] = load_pair_raw<T>(probs, prow1 + key, row1 >= 0 && (!CLS || i1 == 0) && k0 + 8 * j < lim && key < S, key + 1 < S, pair);
       }
       float acc[KB / 8][4];
 #pragma unroll
@@ -728,8 +784,8 @@ __global__ void __launch_bounds__(SP * 2, SP == 128 ? 2 : 1) attention_bwd_blk_k
 #pragma unroll
       for (int j = 0; j < KB / 8; ++j) {
         const int key = k0 + 8 * j + 2 * t;
-        w0[j] = load_pair_raw<T>(probs, prow0 + key, row0 >= 0 && k0 + 8 * j < lim && key < S, key + 1 < S, pair);
-        w1[j] = load_pair_raw<T>(probs, prow1 + key, row1 >= 0 && k0 + 8 * j < lim && key < S, key + 1 < S, pair);
+        w0[j] = load_pair_raw<T>(probs, prow0 + key, row0 >= 0 && (!CLS || i0 == 0) && k0 + 8 * j < lim && key < S, key + 1 < S, pair);
+        w1[j] = load_pair_raw<T>(probs, prow1 + key, row1 >= 0 && (!CLS || i1 == 0) && k0 + 8 * j < lim && key < S, key + 1 < S, pair);
       }
       float acc[KB / 8][4];
 #pragma unroll
@@ -765,7 +821,7 @@ __global__ void __launch_bounds__(SP * 2, SP == 128 ? 2 : 1) attention_bwd_blk_k
 #pragma unroll
         for (int jd = 0; jd < NJ; ++jd) { out[jd][0] = 0.f; out[jd][1] = 0.f; out[jd][2] = 0.f; out[jd][3] = 0.f; }
         const int c0 = slice * NJ * 8;
-        transposed_times_rows<T, SP, HD, NJ>(out, which == 0 ? sDS : sW, PB, 16 * kt, (which == 0 ? sQ : sDO) + c0, lane, lim);
+        transposed_times_rows<T, SP, HD, NJ>(out, which == 0 ? sDS : sW, PB, 16 * kt, (which == 0 ? sQ : sDO) + c0, lane, qlim);
         write_rows<T>(out, dqkv + (1 + which) * H + h * HD + c0, 3 * H, sRow[key0 + g], sRow[key0 + g + 8], lane,
                       bias_acc != nullptr ? sBias + (1 + which) * HD + c0 : nullptr);
       }
@@ -789,30 +845,32 @@ template <int SP, int HD> constexpr size_t bwd_smem(size_t esz) {
 // One launch of the kernels for sequences of len_lo + 1 .. SP tokens (a CTA whose sequence has another length exits).
 template <typename T, int SP, int HD>
 static int launch_fwd(const void* qkv, const void* bqkv, const int* mask, void* ctx, void* probs, int b, int S, int H,
-                      int nh, float p, const int* seed, unsigned stream_id, const Tok& tk, int len_lo, cudaStream_t st) {
+                      int nh, float p, const int* seed, unsigned stream_id, const Tok& tk, const void* first_src, void* first_dst, int len_lo,
+                      cudaStream_t st) {
   constexpr size_t smem = fwd_smem<SP, HD>(sizeof(T));
   const auto go = [&](auto k) -> int {
     if (smem > 48 * 1024 && cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return -5;
-    rb::launch_pdl(k, dim3(nh, b), dim3(SP * 2), smem, st, (const T*)qkv, (const T*)bqkv, mask, (T*)ctx, (T*)probs, S, H, nh, p, seed, stream_id, tk, len_lo);
+    rb::launch_pdl(k, dim3(nh, b), dim3(SP * 2), smem, st, (const T*)qkv, (const T*)bqkv, mask, (T*)ctx, (T*)probs, S, H, nh, p, seed, stream_id, tk, len_lo,
+                   FirstTok<T>{(const T*)first_src, (T*)first_dst});
     return 0;
   };
-  if constexpr (SP > 128) return go(attention_fwd_blk_kernel<T, SP, HD>);
-  else return go(attention_fwd_mma_kernel<T, SP, HD>);
+  if constexpr (SP > 128) return first_dst ? go(attention_fwd_blk_kernel<T, SP, HD, true>) : go(attention_fwd_blk_kernel<T, SP, HD, false>);
+  else return first_dst ? go(attention_fwd_mma_kernel<T, SP, HD, true>) : go(attention_fwd_mma_kernel<T, SP, HD, false>);
 }
 
 template <typename T, int SP, int HD>
 static int launch_bwd(const void* dctx, const void* qkv, const void* bqkv, const void* probs, void* dqkv, int b, int S,
-                      int H, int nh, float p, const int* seed, unsigned stream_id, float* bias_acc, const Tok& tk, int len_lo,
-                      cudaStream_t st) {
+                      int H, int nh, float p, const int* seed, unsigned stream_id, float* bias_acc, const Tok& tk,
+                      const void* first_src, void* first_dst, int len_lo, cudaStream_t st) {
   constexpr size_t smem = bwd_smem<SP, HD>(sizeof(T));
   const auto go = [&](auto k) -> int {
     if (smem > 48 * 1024 && cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return -5;
     rb::launch_pdl(k, dim3(nh, b), dim3(SP * 2), smem, st, (const T*)dctx, (const T*)qkv, (const T*)bqkv, (const T*)probs,
-                   (T*)dqkv, S, H, nh, p, seed, stream_id, bias_acc, tk, len_lo);
+                   (T*)dqkv, S, H, nh, p, seed, stream_id, bias_acc, tk, len_lo, FirstTok<T>{(const T*)first_src, (T*)first_dst});
     return 0;
   };
-  if constexpr (SP > 64) return go(attention_bwd_blk_kernel<T, SP, HD>);
-  else return go(attention_bwd_mma_kernel<T, SP, HD>);
+  if constexpr (SP > 64) return first_dst ? go(attention_bwd_blk_kernel<T, SP, HD, true>) : go(attention_bwd_blk_kernel<T, SP, HD, false>);
+  else return first_dst ? go(attention_bwd_mma_kernel<T, SP, HD, true>) : go(attention_bwd_mma_kernel<T, SP, HD, false>);
 }
 
 // Tile sizes by sequence length.  All sequences of a padded batch have length S: one launch of the smallest tile that
@@ -1200,14 +1258,15 @@ static bool mma_args_ok(int dtype, int b, int S, int H, int nh) {
   return S <= 128 || (long long)b * nh * S * S < (1LL << 32);   // dropout counters are 32-bit element indices
 }
 
-RB_API int rb_attention_fwd_mma(int dtype, const void* qkv, const void* bqkv, const int* mask, void* ctx, void* probs,
-                                int b, int S, int H, int nh, float p, const int* seed, unsigned stream_id,
-                                const int* tok_slot, const int* tok_len, const int* tok_meta, cudaStream_t st) {
+static int attention_fwd_any(int dtype, const void* qkv, const void* bqkv, const int* mask, void* ctx, void* probs,
+                             int b, int S, int H, int nh, float p, const int* seed, unsigned stream_id,
+                             const int* tok_slot, const int* tok_len, const int* tok_meta, const void* first_src,
+                             void* first_dst, cudaStream_t st) {
   if (!mma_args_ok(dtype, b, S, H, nh)) return -4;
   const amma::Tok tk{tok_slot, tok_len, tok_meta};
   const bool packed = tok_slot != nullptr;
   int rc;
-#define RB_FWD(T, HD) RB_ATT_LAUNCH(T, HD, amma::launch_fwd, S, packed, qkv, bqkv, mask, ctx, probs, b, S, H, nh, p, seed, stream_id, tk)
+#define RB_FWD(T, HD) RB_ATT_LAUNCH(T, HD, amma::launch_fwd, S, packed, qkv, bqkv, mask, ctx, probs, b, S, H, nh, p, seed, stream_id, tk, first_src, first_dst)
   if (H / nh == 64) rc = dtype == RB_BF16 ? RB_FWD(__nv_bfloat16, 64) : RB_FWD(__half, 64);
   else rc = dtype == RB_BF16 ? RB_FWD(__nv_bfloat16, 32) : RB_FWD(__half, 32);
 #undef RB_FWD
@@ -1216,23 +1275,59 @@ RB_API int rb_attention_fwd_mma(int dtype, const void* qkv, const void* bqkv, co
   return 0;
 }
 
+RB_API int rb_attention_fwd_mma(int dtype, const void* qkv, const void* bqkv, const int* mask, void* ctx, void* probs,
+                                int b, int S, int H, int nh, float p, const int* seed, unsigned stream_id,
+                                const int* tok_slot, const int* tok_len, const int* tok_meta, cudaStream_t st) {
+  return attention_fwd_any(dtype, qkv, bqkv, mask, ctx, probs, b, S, H, nh, p, seed, stream_id, tok_slot, tok_len, tok_meta,
+                           nullptr, nullptr, st);
+}
+
+// First-token variant, packed rows only: ctx is [b, H], and first_dst [b, H] receives the first tokens' rows of first_src.
+RB_API int rb_attention_fwd_first(int dtype, const void* qkv, const void* bqkv, const int* mask, void* ctx, void* probs,
+                                  int b, int S, int H, int nh, float p, const int* seed, unsigned stream_id,
+                                  const int* tok_slot, const int* tok_len, const int* tok_meta, const void* first_src,
+                                  void* first_dst, cudaStream_t st) {
+  if (tok_slot == nullptr || first_src == nullptr || first_dst == nullptr) return -3;
+  return attention_fwd_any(dtype, qkv, bqkv, mask, ctx, probs, b, S, H, nh, p, seed, stream_id, tok_slot, tok_len, tok_meta,
+                           first_src, first_dst, st);
+}
+
 // bias_acc (nullable): 8 replicas x [3H] fp32; when given, the column sums of dqkv (the q/k/v bias gradients) are
 // accumulated there so that no separate pass over dqkv is needed.
-RB_API int rb_attention_bwd_mma(int dtype, const void* dctx, const void* qkv, const void* bqkv, const void* probs,
-                                void* dqkv, int b, int S, int H, int nh, float p, const int* seed, unsigned stream_id,
-                                float* bias_acc, const int* tok_slot, const int* tok_len, const int* tok_meta,
-                                cudaStream_t st) {
+static int attention_bwd_any(int dtype, const void* dctx, const void* qkv, const void* bqkv, const void* probs,
+                             void* dqkv, int b, int S, int H, int nh, float p, const int* seed, unsigned stream_id,
+                             float* bias_acc, const int* tok_slot, const int* tok_len, const int* tok_meta,
+                             const void* first_src, void* first_dst, cudaStream_t st) {
   if (!mma_args_ok(dtype, b, S, H, nh)) return -4;
   const amma::Tok tk{tok_slot, tok_len, tok_meta};
   const bool packed = tok_slot != nullptr;
   int rc;
-#define RB_BWD(T, HD) RB_ATT_LAUNCH(T, HD, amma::launch_bwd, S, packed, dctx, qkv, bqkv, probs, dqkv, b, S, H, nh, p, seed, stream_id, bias_acc, tk)
+#define RB_BWD(T, HD) RB_ATT_LAUNCH(T, HD, amma::launch_bwd, S, packed, dctx, qkv, bqkv, probs, dqkv, b, S, H, nh, p, seed, stream_id, bias_acc, tk, first_src, first_dst)
   if (H / nh == 64) rc = dtype == RB_BF16 ? RB_BWD(__nv_bfloat16, 64) : RB_BWD(__half, 64);
   else rc = dtype == RB_BF16 ? RB_BWD(__nv_bfloat16, 32) : RB_BWD(__half, 32);
 #undef RB_BWD
   if (rc) return rc;
   RB_LAUNCH_CHECK();
   return 0;
+}
+
+RB_API int rb_attention_bwd_mma(int dtype, const void* dctx, const void* qkv, const void* bqkv, const void* probs,
+                                void* dqkv, int b, int S, int H, int nh, float p, const int* seed, unsigned stream_id,
+                                float* bias_acc, const int* tok_slot, const int* tok_len, const int* tok_meta,
+                                cudaStream_t st) {
+  return attention_bwd_any(dtype, dctx, qkv, bqkv, probs, dqkv, b, S, H, nh, p, seed, stream_id, bias_acc, tok_slot, tok_len,
+                           tok_meta, nullptr, nullptr, st);
+}
+
+// First-token variant, packed rows only: dctx is [b, H]; the packed rows of first_dst receive the rows of first_src [b, H] at
+// the first tokens and zeros elsewhere.
+RB_API int rb_attention_bwd_first(int dtype, const void* dctx, const void* qkv, const void* bqkv, const void* probs,
+                                  void* dqkv, int b, int S, int H, int nh, float p, const int* seed, unsigned stream_id,
+                                  float* bias_acc, const int* tok_slot, const int* tok_len, const int* tok_meta,
+                                  const void* first_src, void* first_dst, cudaStream_t st) {
+  if (tok_slot == nullptr || first_src == nullptr || first_dst == nullptr) return -3;
+  return attention_bwd_any(dtype, dctx, qkv, bqkv, probs, dqkv, b, S, H, nh, p, seed, stream_id, bias_acc, tok_slot, tok_len,
+                           tok_meta, first_src, first_dst, st);
 }
 
 // Sequences of 257..512 tokens, head dim 64 (same requirements otherwise).  The backward needs ds_ws, a [b, nh, S, S]

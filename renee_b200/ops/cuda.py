@@ -201,8 +201,10 @@ class TokenMap:
 
     def __init__(self, b: int, S: int, device):
         n = b * S
-        z = guard.zeros(2 * n + 3 * b + 4, dtype=torch.int32, device=device, name="encoder.activations.token_map")
-        self.tok, self.slot, self.off, self.len, self.cnt, self.meta = z.split([n, n, b, b, b, 4])
+        z = guard.zeros(2 * n + 4 * b + 4, dtype=torch.int32, device=device, name="encoder.activations.token_map")
+        self.tok, self.slot, self.off, self.len, self.cnt, self.meta, first = z.split([n, n, b, b, b, 4, b])
+        torch.arange(0, n, S, dtype=torch.int32, device=device, out=first)
+        self.first = FirstTokens(first)
         # every launch of a pass takes some of these: made once, as long as the buffer lives
         self.pointers = {k: _p(getattr(self, k)) for k in ("tok", "slot", "off", "len", "cnt", "meta")}
         self.rows_hint = 0
@@ -210,6 +212,18 @@ class TokenMap:
     def update(self, mask) -> None:
         b, S = mask.shape
         _call("rb_token_map", _p(mask), _I(b), _I(S), *_tok(self, "off", "len", "cnt", "meta"), _stream())
+
+
+class FirstTokens:
+    """Rows that hold the first token of every sequence, one per sequence: behind the last layer's attention CLS pooling reads
+    nothing else.  Stands where a token map does; the number of rows is the sequences' (known on the host), and ``tok`` numbers
+    their dropout counters in the padded layout."""
+
+    rows_hint = 0
+
+    def __init__(self, tok):
+        self.tok = tok
+        self.pointers = {"tok": _p(tok), "meta": _NULL}
 
 
 def _tok(tmap, *names):
@@ -271,6 +285,11 @@ def _attention_entry(direction: str, H: int, nh: int) -> str:
     return f"rb_attention_{direction}_tc"
 
 
+def attention_first_token(dtype, S: int, H: int, nh: int) -> bool:
+    """Whether the attention kernels of this shape have a first-token variant (packed rows, up to 256 tokens)."""
+    return _packed_kernels(dtype, S, H // nh) == "mma"
+
+
 def _scratch(buf):
     return buf.get() if hasattr(buf, "get") else buf
 
@@ -308,7 +327,9 @@ def _seed_tensor(rng):
     return rng.dev.to(torch.int64).reshape(-1)[0] & 0xFFFFFFFF
 
 
-def attention_fwd(qkv, bqkv, mask, nh, p, rng, stream, ctx_out, ws, tmap=None):
+def attention_fwd(qkv, bqkv, mask, nh, p, rng, stream, ctx_out, ws, tmap=None, first=None):
+    """``first = (h, h_first)``: only the first token of every sequence is a query (:func:`attention_first_token`); ``ctx_out``
+    has one row per sequence, and the rows of ``h`` that belong to those tokens are copied to ``h_first``."""
     b, S = mask.shape
     H = ctx_out.shape[1]
     entry, launches = _attention_route(qkv, S, H, nh, ws, "fwd", tmap)
@@ -318,12 +339,24 @@ def attention_fwd(qkv, bqkv, mask, nh, p, rng, stream, ctx_out, ws, tmap=None):
         ctx_out.copy_(ctx)
         ws["probs"][:b].copy_(probs)
         return
-    maps = _tok(tmap, "slot", "len", "meta") if entry.endswith(("_mma", "_long")) else ()
+    entry, maps = _attention_maps(entry, tmap, first)
     _call(entry, _I(DT[qkv.dtype]), _p(qkv), _p(bqkv), _p(mask), _p(ctx_out), _p(ws["probs"]), _I(b), _I(S),
           _I(H), _I(nh), _F(p), _p(rng.dev), _U(stream), *maps, _stream(), launches=launches)
 
 
-def attention_bwd(dctx, qkv, bqkv, mask, nh, p, rng, stream, ws, dqkv_out, dbqkv_out, tmap=None):
+def _attention_maps(entry: str, tmap, first):
+    """``(entry, trailing arguments)`` of an attention call."""
+    if first is not None and not (tmap is not None and entry.endswith("_mma")):
+        raise KernelError(f"{entry} has no first-token variant")
+    maps = _tok(tmap, "slot", "len", "meta") if entry.endswith(("_mma", "_long")) else []
+    if first is not None:
+        return entry[:-len("mma")] + "first", maps + [_p(t) for t in first]
+    return entry, maps
+
+
+def attention_bwd(dctx, qkv, bqkv, mask, nh, p, rng, stream, ws, dqkv_out, dbqkv_out, tmap=None, first=None):
+    """``first = (d_first, d_rows)``: the first-token variant; ``dctx`` has one row per sequence, and ``d_rows`` (packed rows)
+    receives ``d_first`` at the first tokens and zeros elsewhere."""
     b, S = mask.shape
     H = dctx.shape[1]
     entry, launches = _attention_route(qkv, S, H, nh, ws, "bwd", tmap)
@@ -336,7 +369,7 @@ def attention_bwd(dctx, qkv, bqkv, mask, nh, p, rng, stream, ws, dqkv_out, dbqkv
     # with a deferred-columns plan active the 16-bit kernels also accumulate the q/k/v bias gradients
     acc = _DEFER.slot([dbqkv_out], 3 * H) if _DEFER is not None and qkv.dtype != torch.float32 else None
     long = entry.endswith("_long")
-    maps = _tok(tmap, "slot", "len", "meta") if long or entry.endswith("_mma") else ()
+    entry, maps = _attention_maps(entry, tmap, first)
     _call(entry, _I(DT[qkv.dtype]), _p(dctx), _p(qkv), _p(bqkv), _p(ws["probs"]), *((_p(_scratch(ws["ds"])),) if long else ()),
           _p(dqkv_out), _I(b), _I(S), _I(H), _I(nh), _F(p), _p(rng.dev), _U(stream),
           *(() if qkv.dtype == torch.float32 else (_p(acc),)), *maps, _stream(), launches=launches)
