@@ -215,7 +215,7 @@ enc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
   volatile int* s_abort = reinterpret_cast<volatile int*>(tmem_ptr_smem + 1);
   volatile int* s_last = s_abort + 1;
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = tc::warp_id();
   const int lane = threadIdx.x & 31;
   const uint32_t rank = NCTA == 2 ? tc::cluster_ctarank() : 0u;
   const int unit = NCTA == 2 ? (int)(blockIdx.x >> 1) : (int)blockIdx.x;          // which persistent worker
@@ -264,7 +264,7 @@ enc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
   const int per_unit = (n_items + n_units - 1) / n_units;
   const int it0 = RUNS ? unit * per_unit : unit, it1 = RUNS ? min(n_items, it0 + per_unit) : n_items, its = RUNS ? 1 : n_units;
 
-  if (warp == 0 && lane == 0) {
+  if (warp == 0 && tc::elect_one()) {
     // ---------------- TMA producer: one continuous stream of (item, k block) stages
     int s = 0;
     uint32_t ph = 0;
@@ -318,7 +318,7 @@ enc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
         }
       }
     }
-  } else if (warp == 1 && lane == 0 && rank == 0) {
+  } else if (warp == 1 && rank == 0 && tc::elect_one()) {
     // ---------------- MMA issuer (leader CTA): accumulator (t_local & 1), reused once the epilogue(s) drained it
     const uint32_t idesc = tc::make_idesc(FMT, A_MN ? 1 : 0, B_MN ? 1 : 0, BM * NCTA, p.BN);
     int s = 0, t_local = 0;

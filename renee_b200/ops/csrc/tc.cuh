@@ -16,6 +16,18 @@ constexpr uint64_t kWaitBudgetNs = 1500ull * 1000ull * 1000ull;  // 1.5 s per wa
 // Status words written on a timed-out wait: [0]=code (0 ok), [1]=blockIdx.x, [2]=site, [3]=detail
 enum WaitSite : int { SITE_EMPTY = 1, SITE_FULL = 2, SITE_TMEM_FULL = 3, SITE_PEER_FLAG = 4, SITE_TMEM_EMPTY = 5 };
 
+// One lane of the (converged) warp.  Roles that one thread plays are chosen by this and by a warp number that the compiler knows
+// to be the same in every lane (warp_id), never by `lane == 0`: TMA, MMA and commit instructions take their operands from
+// uniform registers, and in a branch on the lane number the compiler moves each operand there through a loop over the lanes.
+// One k block of a 128 x 128 tile, measured alone: 849 clocks through `lane == 0`, 443 through elect (MMA issue 308 / 270,
+// TMA issue 451 / 286).
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile("{\n .reg .pred P;\n elect.sync _|P, 0xffffffff;\n selp.b32 %0, 1, 0, P;\n}" : "=r"(p));
+  return p != 0;
+}
+__device__ __forceinline__ int warp_id() { return __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0); }
+
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ uint64_t now_ns() {
   uint64_t t;

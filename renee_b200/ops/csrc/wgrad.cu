@@ -55,7 +55,7 @@ __global__ void __launch_bounds__(THREADS, 1) wgrad_group_kernel(const __grid_co
   uint32_t* tmem_ptr_smem = reinterpret_cast<uint32_t*>(tmem_empty_bar + 2);
   volatile int* s_abort = reinterpret_cast<volatile int*>(tmem_ptr_smem + 1);
   volatile int* s_last = s_abort + 1;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = tc::warp_id(), lane = threadIdx.x & 31;
   const uint32_t rank = tc::cluster_ctarank();
   const int unit = (int)(blockIdx.x >> 1), n_units = (int)(gridDim.x >> 1);
   if (threadIdx.x == 0) {
@@ -101,7 +101,7 @@ __global__ void __launch_bounds__(THREADS, 1) wgrad_group_kernel(const __grid_co
     return i;
   };
 
-  if (warp == 0 && lane == 0) {
+  if (warp == 0 && tc::elect_one()) {
     int s = 0;
     uint32_t ph = 0;
     for (int x = x0; x < x_end && !aborted;) {
@@ -121,7 +121,7 @@ __global__ void __launch_bounds__(THREADS, 1) wgrad_group_kernel(const __grid_co
         tc::tma_load_2d_pair(sB + 8192, &maps.b[i], lbar, nb + 64, k * BK);
       }
     }
-  } else if (warp == 1 && lane == 0 && rank == 0) {
+  } else if (warp == 1 && rank == 0 && tc::elect_one()) {
     constexpr int FMT = std::is_same<T, __nv_bfloat16>::value ? 1 : 0;
     const uint32_t idesc = tc::make_idesc(FMT, 1, 1, 2 * BM, BN);
     int s = 0, t_local = 0;
