@@ -29,8 +29,7 @@
 //
 // Structure.  Persistent CTAs walk the work items (tile x K-split).  576 threads: warp 0 TMA producer, warp 1
 // TMEM owner + MMA issuer, warps 2..17 epilogue (four groups of four warps, one TMEM lane quarter per warp, one
-// 64-column panel of the tile per group: the epilogue is bound by instruction latency, not by issue slots, and
-// sixteen warps hide what eight could not).  The shared-memory ring keeps streaming across item boundaries and TMEM
+// 64-column panel of the tile per group).  The shared-memory ring keeps streaming across item boundaries and TMEM
 // holds two accumulators, so the epilogue of item i runs under the main loop of item i + 1.
 //
 // Two tile shapes.  NCTA = 1: a CTA owns a 128 x BN tile.  NCTA = 2 (`cta_group::2`): the two CTAs of a cluster
@@ -44,6 +43,14 @@
 // elements) and written with TMA stores, which clip at the matrix edge; tile-shaped inputs (residual, stored
 // pre-activation) are fetched into the same panels by TMA while the tile's main loop still runs and are updated
 // in place.  Every global access of the epilogue is therefore a full-line bulk copy.
+// A warp owns 32 rows of its group's panel: it fetches, stages and stores them by itself and waits for no other warp.
+// What does not need the accumulator -- the dropout hashes, the bias, the residual's way to registers, the positives of the
+// tile's labels -- is done while the main loop runs; the accumulator comes in fragments of 8 columns, the next one on its way.
+// (With panels shared by four warps, a barrier of all sixteen per tile and these loads behind the accumulator, 4928 tokens:
+// FFN1 bias + GELU 31.8 -> 28.1 us, FFN2 dgrad + GELU backward 33.5 -> 28.5, FFN2 forward + dropout + residual 25.4 -> 21.3,
+// output projection 14.3 -> 11.1; plain products of these shapes take 20.8, 20.8, 19.9 and 9.0.)  What is left of an epilogue
+// in a multi-round launch is shared-memory bandwidth: a 256 x 256 pair tile of K = 768 moves 48 KB per k block and CTA through
+// it for the MMAs and 32 KB for the loads, and two 16-bit outputs another 256 KB.
 //
 // Every wait is bounded (tc.cuh): a protocol error ends with a status word, never with a hang.
 #include <type_traits>
@@ -58,9 +65,12 @@ constexpr int BM = 128;                         // accumulator rows per CTA
 constexpr int BK = 64;
 constexpr int A_BYTES = BM * BK * 2;            // 16 KB
 constexpr int PANEL_BYTES = BM * 64 * 2;        // one staging panel: 128 rows x 64 x 16 bit
+constexpr int SUB_ROWS = 32;                    // a warp's rows of it: it stages, stores and fetches them by itself
+constexpr int SUB_BYTES = SUB_ROWS * 64 * 2;
 constexpr int EGROUPS = 4;                      // epilogue groups of four warps (one per TMEM lane quarter)
 constexpr int N_PANELS = EGROUPS;               // one staging panel per epilogue group
-constexpr int EPI_THREADS = 128 * EGROUPS;
+constexpr int EPI_WARPS = 4 * EGROUPS;
+constexpr int EPI_THREADS = 32 * EPI_WARPS;
 constexpr int THREADS = 64 + EPI_THREADS;       // producer warp, MMA warp, sixteen epilogue warps
 constexpr int ACC_BUFS = 2;
 constexpr int ACC_STRIDE = 256;                 // TMEM columns between the two accumulators
@@ -85,7 +95,7 @@ template <int EPI> struct Cfg {
   static constexpr bool kStaged = staged_epi(EPI);
   static constexpr int kPanels = panel_count(EPI);
   static constexpr int kRing = ring_bytes(EPI);
-  static constexpr int kSmem = kRing + kPanels * PANEL_BYTES + 1024 + 512;
+  static constexpr int kSmem = kRing + kPanels * PANEL_BYTES + 1024 + 512;   // alignment, barriers
 };
 
 struct Params {
@@ -122,21 +132,6 @@ template <typename T> __device__ __forceinline__ void unpack8(const uint4& raw, 
   const T* e = reinterpret_cast<const T*>(&raw);
 #pragma unroll
   for (int i = 0; i < 8; ++i) out[i] = to_f(e[i]);
-}
-
-// Sum over the 32 lanes of v[c] for every c in 0..31: lane L returns the total of column L (31 shuffles).
-__device__ __forceinline__ float warp_colsum32(float (&v)[32], int lane) {
-#pragma unroll
-  for (int n = 16; n >= 1; n >>= 1) {
-    const bool upper = (lane & n) != 0;
-#pragma unroll
-    for (int i = 0; i < n; ++i) {
-      const float send = upper ? v[i] : v[i + n];
-      const float keep_ = upper ? v[i + n] : v[i];
-      v[i] = keep_ + __shfl_xor_sync(0xffffffffu, send, n);
-    }
-  }
-  return v[0];
 }
 
 // First positions of the sorted a[0 .. n) whose values are >= k_lo and >= k_hi, by one warp: each half-warp probes 16 places
@@ -202,7 +197,8 @@ enc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
   constexpr int FMT = std::is_same<T, __nv_bfloat16>::value ? 1 : 0;
   constexpr bool HAS_IN = (EPI == E_BIAS_DROPOUT_RESID || EPI == E_ADD || EPI == E_GELU_BWD || EPI == E_DW_SGD);   // tile-shaped input R
   constexpr bool STAGED = C_::kStaged;                                                           // outputs through panels
-  constexpr uint32_t IN_BYTES = EPI == E_DW_SGD ? 2 * PANEL_BYTES : PANEL_BYTES;
+  constexpr bool HELD_IN = HAS_IN && EPI != E_DW_SGD;      // ... of one tensor: read into registers under the main loop
+  constexpr uint32_t IN_BYTES = EPI == E_DW_SGD ? 2 * SUB_BYTES : SUB_BYTES;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* panels = smem + RING;                           // [N_PANELS][PANEL_BYTES], 1024-byte aligned
@@ -210,8 +206,8 @@ enc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
   uint64_t* empty_bar = full_bar + MAX_STAGES;
   uint64_t* tmem_full_bar = empty_bar + MAX_STAGES;      // [ACC_BUFS]
   uint64_t* tmem_empty_bar = tmem_full_bar + ACC_BUFS;   // [ACC_BUFS]  (used in the leader CTA)
-  uint64_t* in_bar = tmem_empty_bar + ACC_BUFS;          // [N_PANELS]  a group's R panel has landed
-  uint32_t* tmem_ptr_smem = reinterpret_cast<uint32_t*>(in_bar + N_PANELS);
+  uint64_t* in_bar = tmem_empty_bar + ACC_BUFS;          // [EPI_WARPS]  a warp's part of the R panel has landed
+  uint32_t* tmem_ptr_smem = reinterpret_cast<uint32_t*>(in_bar + EPI_WARPS);
   volatile int* s_abort = reinterpret_cast<volatile int*>(tmem_ptr_smem + 1);
   volatile int* s_last = s_abort + 1;
 
@@ -233,7 +229,7 @@ enc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
     if (EPI == E_BIAS_GELU || EPI == E_DW_SGD) tc::prefetch_tmap(&tmF);
     for (int s = 0; s < MAX_STAGES; ++s) { tc::mbar_init(full_bar + s, 1); tc::mbar_init(empty_bar + s, 1); }
     for (int a = 0; a < ACC_BUFS; ++a) { tc::mbar_init(tmem_full_bar + a, 1); tc::mbar_init(tmem_empty_bar + a, 4 * EGROUPS * NCTA); }
-    for (int a = 0; a < N_PANELS; ++a) tc::mbar_init(in_bar + a, 1);
+    for (int a = 0; a < EPI_WARPS; ++a) tc::mbar_init(in_bar + a, 1);
     *s_abort = 0;
     *s_last = 0;
     tc::fence_barrier_init();
@@ -349,21 +345,19 @@ enc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
       if (NCTA == 2) tc::umma_commit_pair(tmem_full_bar + buf); else tc::umma_commit(tmem_full_bar + buf);
     }
   } else if (warp >= 2) {
-    // ---------------- epilogue: group g = (warp - 2) / 4 owns columns [g BN/2, (g + 1) BN/2) of the CTA's 128 rows
+    // ---------------- epilogue: group g = (warp - 2) / 4 owns columns [64 g, 64 g + 64) of the CTA's 128 rows
     const int quarter = warp & 3;
     const int g = (warp - 2) >> 2;
     const int r = quarter * 32 + lane;                    // row of the CTA's accumulator = TMEM lane
     // staged epilogues: group g takes the 64-column panel g of the tile (BN / 64 groups have one, the others idle);
     // the others split the tile's columns into BN / EGROUPS (at least 32) per group
-    const int n_pan = g < (p.BN >> 6) ? 1 : 0;
+    const bool staging = STAGED && g < (p.BN >> 6);
     const int g_col = g * 64;
     const int ucols = p.BN / EGROUPS < 32 ? 32 : p.BN / EGROUPS;
     const bool u_active = g * ucols < p.BN;
-    const int bar_id = 2 + g;                             // named barrier of this group (128 threads)
-    const bool elected = (warp == 2 + 4 * g) && lane == 0;                   // first warp of the group, lane 0
-    uint8_t* pan = panels + g * PANEL_BYTES;              // this group's staging panel
-    uint8_t* pan2 = panels + (N_PANELS + g) * PANEL_BYTES;   // DW_SGD: the momentum panel beside the weight panel
-    uint64_t* my_in_bar = in_bar + g;
+    uint8_t* pan = panels + g * PANEL_BYTES + quarter * SUB_BYTES;              // this warp's 32 rows of the staging panel
+    uint8_t* pan2 = panels + (N_PANELS + g) * PANEL_BYTES + quarter * SUB_BYTES;   // DW_SGD: the momentum beside the weights
+    uint64_t* my_in_bar = in_bar + (warp - 2);
     uint32_t seed = 0u;
     float inv_keep = 1.f;
     if (EPI == E_BIAS_DROPOUT_RESID && p.p > 0.f) { seed = (uint32_t)(*p.seed); inv_keep = 1.f / (1.f - p.p); }
@@ -382,7 +376,9 @@ enc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
       cv[0] = make_float4(tv[0], tv[1], tv[2], tv[3]); cv[1] = make_float4(tv[4], tv[5], tv[6], tv[7]);
       ci[0] = make_int4(ti[0], ti[1], ti[2], ti[3]); ci[1] = make_int4(ti[4], ti[5], ti[6], ti[7]);
     };
-    int pe0 = 0, pe1 = 0, pos_m = -1;                     // SIGMOID_POS: positives of M tile pos_m
+    // SIGMOID_POS: the positives of this warp's 32 labels of M tile pos_m are, of a window of 32 entries of the label-sorted
+    // list that the lanes hold, those in range, and entries pos_more .. pos_end behind it
+    int pos_m = -1, pos_l = -1, pos_c = 0, pos_more = 0, pos_end = 0;
     float loss = 0.f;                                     // SIGMOID_POS: this thread's share of sum softplus(z)
     for (int item = it0; item < it1; item += its, ++t_local) {
       const int tile = item / splits;
@@ -398,182 +394,227 @@ enc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
       const int m0 = mt * (BM * NCTA) + (int)rank * BM;
       const int n0 = nt * p.BN;
       const int row = m0 + r;
+      const int sub0 = m0 + quarter * SUB_ROWS;            // first row of this warp
+      const int pcol = n0 + g_col;                         // first column of this group's panel
       const int buf = t_local & 1;
       const uint32_t use = (uint32_t)(t_local >> 1);
-      if (HAS_IN && elected && n_pan > 0) {
-        // fetch the tile's first R panel while its main loop still runs; the panel is free once the stores
-        // issued from it have read it
-        tc::tma_store_wait_read<0>();
-        tc::mbar_expect_tx(my_in_bar, IN_BYTES);
-        tc::tma_load_2d(pan, &tmR, my_in_bar, n0 + g_col, m0);
-        if (EPI == E_DW_SGD) tc::tma_load_2d(pan2, &tmF, my_in_bar, n0 + g_col, m0);
-      }
-      // dropout counters number the padded layout's rows; the word is fetched while the main loop still runs
-      int drop_row = row;
-      if (EPI == E_BIAS_DROPOUT_RESID && p.tok != nullptr && row < M) drop_row = __ldcg(p.tok + row);
-      // the positives of this CTA's 128 labels: entries pe0 .. pe1 of the label-sorted list, found under the main loop
-      if (EPI == E_SIGMOID_POS && p.pos_labels != nullptr && n_pan > 0 && mt != pos_m) {
-        pos_m = mt;
-        warp_bounds(p.pos_labels, *p.nnz_ptr, p.label0 + m0, p.label0 + min(m0 + BM, M), lane, pe0, pe1);
-      }
-      if (!tc::mbar_wait(tmem_full_bar + buf, use & 1, aborted, p.status, tc::SITE_TMEM_FULL, item)) *s_abort = 1;
-      asm volatile("bar.sync 1, %0;" ::"n"(EPI_THREADS) : "memory");
-      if (*s_abort) break;                                   // the same answer in every epilogue warp
-      tc::tc_fence_after();
-      const uint32_t tbase = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)buf * ACC_STRIDE + (uint32_t)g_col;
-      if (STAGED && n_pan > 0) {
-        {
-          const int pcol = n0 + g_col;                       // first column of this group's panel
+      // Under the main loop: everything that the accumulator is not needed for
+      uint32_t bias2 = 0u;                                 // this lane's two of the panel's 64 bias values
+      uint32_t kept[2] = {0xffffffffu, 0xffffffffu};       // dropout decisions of the 64 columns
+      if (STAGED && staging) {
+        if (tc::elect_one()) {                             // always the same lane: it waits for the stores it issued
+          tc::tma_store_wait_read<0>();                    // the panel is free once the previous store has read it
           if (HAS_IN) {
-            if (!tc::mbar_wait(my_in_bar, in_count & 1, aborted, p.status, tc::SITE_FULL, 2000 + g)) *s_abort = 1;
-            ++in_count;
+            tc::mbar_expect_tx(my_in_bar, IN_BYTES);
+            tc::tma_load_2d(pan, &tmR, my_in_bar, pcol, sub0);
+            if (EPI == E_DW_SGD) tc::tma_load_2d(pan2, &tmF, my_in_bar, pcol, sub0);
+          }
+        }
+        if ((EPI == E_BIAS_GELU || EPI == E_BIAS_DROPOUT_RESID) && pcol + 2 * lane < p.N)
+          bias2 = __ldg(reinterpret_cast<const uint32_t*>(reinterpret_cast<const T*>(p.bias) + pcol) + lane);
+        if (EPI == E_BIAS_DROPOUT_RESID && p.p > 0.f) {
+          // dropout counters number the padded layout's rows
+          const int drop_row = p.tok != nullptr && row < M ? __ldcg(p.tok + row) : row;
+          const uint32_t e0 = (uint32_t)(drop_row * p.N + pcol);
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            uint32_t bits = 0u;
+#pragma unroll 8
+            for (int j = 0; j < 32; ++j) bits |= (keep(seed, p.stream, e0 + 32 * h + j, p.p) ? 1u : 0u) << j;
+            kept[h] = bits;
+          }
+        }
+        if (EPI == E_SIGMOID_POS && p.pos_labels != nullptr && mt != pos_m) {
+          // A unit's tiles ascend, so where positives are sparse the window that one search found serves the next tiles too
+          // (1.3 M labels x 1024 rows, 64-deep: 0.5 positives per 32 labels; with a search of four dependent loads per M tile
+          // the launches took 67 us, without any positives 43)
+          const int k_lo = p.label0 + sub0, k_hi = p.label0 + min(sub0 + SUB_ROWS, M), nnz = *p.nnz_ptr;
+          const bool held = pos_m >= 0 && mt > pos_m && __shfl_sync(0xffffffffu, pos_l, 31) >= k_hi;
+          pos_m = mt;
+          if (!held) {
+            int first;
+            warp_bounds(p.pos_labels, nnz, k_lo, k_hi, lane, first, pos_end);
+            const int e = first + lane;
+            pos_l = e < nnz ? p.pos_labels[e] : 0x7fffffff;
+            pos_c = e < nnz ? p.pos_rows[e] : 0;
+            pos_more = first + 32;
           } else {
-            if (elected) tc::tma_store_wait_read<0>();       // the buffer is free once the previous store has read it
-            asm volatile("bar.sync %0, 128;" ::"r"(bar_id) : "memory");
+            pos_end = 0;                                   // the window reaches past this tile's labels
           }
-          uint4 keep2[EPI == E_BIAS_GELU ? 8 : 1];           // BIAS_GELU: the second output, packed, until the first has left
+        }
+      }
+      bool ok = true;
+      uint4 in_row[HELD_IN ? 8 : 1];                       // the tile-shaped input of this thread's row
+      if (STAGED && staging && HAS_IN) {
+        ok = tc::mbar_wait(my_in_bar, in_count & 1, aborted, p.status, tc::SITE_FULL, 2000 + g);
+        ++in_count;
+        if constexpr (HELD_IN) {
 #pragma unroll
-          for (int hc = 0; hc < 2; ++hc) {                   // two 32-column accumulator fragments per panel
-            float v[32];
-            tc::tmem_ld32(tbase + 32 * hc, v);
+          for (int chunk = 0; chunk < 8; ++chunk) in_row[chunk] = *reinterpret_cast<const uint4*>(pan + panel_off(lane, chunk));
+        }
+      }
+      ok = tc::mbar_wait(tmem_full_bar + buf, use & 1, aborted, p.status, tc::SITE_TMEM_FULL, item) && ok;
+      if constexpr (STAGED) {
+        // a staging warp shares nothing with the others: it ends by itself where a wait has run out
+        if (!__all_sync(0xffffffffu, ok)) break;
+      } else {
+        if (!ok) *s_abort = 1;
+        asm volatile("bar.sync 1, %0;" ::"n"(EPI_THREADS) : "memory");
+        if (*s_abort) break;                               // the same answer in every epilogue warp
+      }
+      tc::tc_fence_after();
+      if (STAGED && staging) {
+        const uint32_t tbase = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)buf * ACC_STRIDE + (uint32_t)g_col;
+        uint4 keep2[EPI == E_BIAS_GELU ? 8 : 1];           // BIAS_GELU: the second output, packed, until the first has left
+        uint32_t frag[2][8];                               // 8 accumulator columns at work, 8 on their way
+        tc::tmem_issue8(tbase, frag[0]);
+        __syncwarp();                                      // lane 0 has seen the panel free (!HAS_IN)
 #pragma unroll
-            for (int j8 = 0; j8 < 4; ++j8) {
-              const int chunk = 4 * hc + j8;
-              const int c = pcol + 8 * chunk;
-              uint4* slot = reinterpret_cast<uint4*>(pan + panel_off(r, chunk));
-              float* a = &v[8 * j8];
-              float o[8];
-              if (EPI == E_STORE) {
+        for (int chunk = 0; chunk < 8; ++chunk) {
+          tc::tmem_wait8(frag[chunk & 1]);
+          if (chunk < 7) tc::tmem_issue8(tbase + 8 * (chunk + 1), frag[(chunk + 1) & 1]);
+          const int c = pcol + 8 * chunk;
+          uint4* slot = reinterpret_cast<uint4*>(pan + panel_off(lane, chunk));
+          float a[8], o[8];
 #pragma unroll
-                for (int j = 0; j < 8; ++j) o[j] = a[j];
-              } else if (EPI == E_SIGMOID_POS) {
-                if (p.loss_acc != nullptr && row < M) {
-                  // sampled loss (dl_base.py:579-583): softplus of every logit here; minus the logits at the positives
-                  // by a separate small kernel
+          for (int j = 0; j < 8; ++j) a[j] = __uint_as_float(frag[chunk & 1][j]);
+          if (EPI == E_STORE) {
 #pragma unroll
-                  for (int j = 0; j < 8; ++j)
-                    if (c + j < p.N) loss += fmaxf(a[j], 0.f) + log1pf(__expf(-fabsf(a[j])));
-                }
-                sigmoid8(a, o);
-                if (c + 8 > p.N) {                       // the columns behind the batch are written as zeros
+            for (int j = 0; j < 8; ++j) o[j] = a[j];
+          } else if (EPI == E_SIGMOID_POS) {
+            if (p.loss_acc != nullptr && row < M) {
+              // sampled loss (dl_base.py:579-583): softplus of every logit here; minus the logits at the positives
+              // by a separate small kernel
 #pragma unroll
-                  for (int j = 0; j < 8; ++j) if (c + j >= p.N) o[j] = 0.f;
-                }
-              } else if (EPI == E_BIAS_GELU) {
-                float b[8];
-                if (c < p.N) unpack8<T>(__ldg(reinterpret_cast<const uint4*>(reinterpret_cast<const T*>(p.bias) + c)), b);
-                else {
-#pragma unroll
-                  for (int j = 0; j < 8; ++j) b[j] = 0.f;
-                }
-#pragma unroll
-                for (int j = 0; j < 8; ++j) o[j] = a[j] + b[j];
-                *slot = pack8<T>(o);
-                unpack8<T>(pack8<T>(o), o);                  // the backward pass differentiates at the stored value
-#pragma unroll
-                for (int j = 0; j < 8; j += 2) f2_get(gelu2(f2(o[j], o[j + 1])), a[j], a[j + 1]);   // second output, staged after the first has left
-              } else if (EPI == E_BIAS_DROPOUT_RESID) {
-                float b[8], res[8];
-                if (c < p.N) unpack8<T>(__ldg(reinterpret_cast<const uint4*>(reinterpret_cast<const T*>(p.bias) + c)), b);
-                else {
-#pragma unroll
-                  for (int j = 0; j < 8; ++j) b[j] = 0.f;
-                }
-                unpack8<T>(*slot, res);
-#pragma unroll
-                for (int j = 0; j < 8; ++j) {
-                  float t = a[j] + b[j];
-                  if (p.p > 0.f) t = keep(seed, p.stream, (uint32_t)(drop_row * p.N + c + j), p.p) ? t * inv_keep : 0.f;
-                  o[j] = res[j] + t;
-                }
-              } else if (EPI == E_ADD) {
-                float res[8];
-                unpack8<T>(*slot, res);
-#pragma unroll
-                for (int j = 0; j < 8; ++j) o[j] = a[j] + res[j];
-              } else if (EPI == E_DW_SGD) {
-                // momentum SGD on the tile: m = mo m + (dW + wd w), w -= lr m, with m rounded to 16 bit first.  One element
-                // at a time this was some 40 instructions per element, more than the tile's bytes take: two per instruction.
-                // The noise of the rounding takes a hash per element, half of what is left.  1.3 M labels x 768, batch 512:
-                // 2.01 -> 1.76 ms (1.68 with one hash per pair, which gives other weights for the same seed).
-                uint4* slot2 = reinterpret_cast<uint4*>(pan2 + panel_off(r, chunk));
-                float w[8], mm[8];
-                unpack8<T>(*slot, w);
-                unpack8<T>(*slot2, mm);
-                const F2 nlr = f2(-p.hp[HP_LR_XFC]), mo2 = f2(p.mo), wd2 = f2(p.wd);
-                const uint32_t sr_seed = reinterpret_cast<const uint32_t*>(p.hp)[HP_SEED];
-                const uint32_t e = (uint32_t)row * (uint32_t)p.ldW + (uint32_t)c;
-#pragma unroll
-                for (int j = 0; j < 8; j += 2)
-                  f2_get(f2_fma(mo2, f2(mm[j], mm[j + 1]), f2_fma(wd2, f2(w[j], w[j + 1]), f2(a[j], a[j + 1]))), mm[j], mm[j + 1]);
-                const uint4 m16 = pack8<T>(mm);
-                unpack8<T>(m16, mm);
-#pragma unroll
-                for (int j = 0; j < 8; j += 2) f2_get(f2_fma(nlr, f2(mm[j], mm[j + 1]), f2(w[j], w[j + 1])), o[j], o[j + 1]);
-                *slot2 = m16;
-                if (p.stochastic_round) {
-                  uint4 w16;                               // every element has a hash of its own number
-                  uint32_t* wp = reinterpret_cast<uint32_t*>(&w16);
-#pragma unroll
-                  for (int j = 0; j < 8; j += 2)
-                    wp[j >> 1] = sr_pack2<T>(o[j], o[j + 1], mix32(sr_seed, 0x5152u, e + j), mix32(sr_seed, 0x5152u, e + j + 1));
-                  *slot = w16;
-                } else {
-                  *slot = pack8<T>(o);
-                }
-              } else {   // E_GELU_BWD
-                float f[8];
-                unpack8<T>(*slot, f);
-#pragma unroll
-                for (int j = 0; j < 8; j += 2) f2_get(f2(a[j], a[j + 1]) * gelu_grad2(f2(f[j], f[j + 1])), o[j], o[j + 1]);
-                unpack8<T>(pack8<T>(o), o);
-#pragma unroll
-                for (int j = 0; j < 8; ++j) a[j] = row < M ? o[j] : 0.f;   // rows past the packed tokens hold what an earlier pass left
-              }
-              if (EPI != E_BIAS_GELU && EPI != E_DW_SGD) *slot = pack8<T>(o);
-              if (EPI == E_BIAS_GELU) keep2[EPI == E_BIAS_GELU ? chunk : 0] = pack8<T>(a);
+              for (int j = 0; j < 8; ++j)
+                if (c + j < p.N) loss += fmaxf(a[j], 0.f) + log1pf(__expf(-fabsf(a[j])));
             }
-            if (EPI == E_GELU_BWD && p.colacc != nullptr) {
-              const float cs = warp_colsum32(v, lane);       // lane L holds the sum of column L of the fragment
-              const int c = pcol + 32 * hc + lane;
-              if (c < p.N) atomicAdd(p.colacc + (size_t)(blockIdx.x % kColReplicas) * p.col_tot + p.col_off + c, cs);
+            sigmoid8(a, o);
+            if (c + 8 > p.N) {                         // the columns behind the batch are written as zeros
+#pragma unroll
+              for (int j = 0; j < 8; ++j) if (c + j >= p.N) o[j] = 0.f;
             }
-          }
-          if (EPI == E_SIGMOID_POS && p.pos_labels != nullptr) {
-            // subtract 1 at the tile's positives while the tile is still in shared memory: entries of the label-sorted
-            // list whose label is one of this CTA's 128 rows and whose batch row is one of the panel's 64 columns
-            asm volatile("bar.sync %0, 128;" ::"r"(bar_id) : "memory");      // every row of the panel is written
-            const int lab_lo = p.label0 + m0;
-            for (int e = pe0 + (int)(threadIdx.x - 64 - 128 * g); e < pe1; e += 128) {
-              const int bcol = p.pos_rows[e] - pcol;
-              if (bcol >= 0 && bcol < 64 && pcol + bcol < p.N) {
-                const int prow = p.pos_labels[e] - lab_lo;
-                T* cell = reinterpret_cast<T*>(pan + panel_off(prow, bcol >> 3)) + (bcol & 7);
-                *cell = from_f<T>(to_f(*cell) - 1.f);      // duplicates are removed by the collator: one writer per cell
+          } else if (EPI == E_BIAS_GELU || EPI == E_BIAS_DROPOUT_RESID) {
+            uint4 braw;
+            braw.x = __shfl_sync(0xffffffffu, bias2, 4 * chunk); braw.y = __shfl_sync(0xffffffffu, bias2, 4 * chunk + 1);
+            braw.z = __shfl_sync(0xffffffffu, bias2, 4 * chunk + 2); braw.w = __shfl_sync(0xffffffffu, bias2, 4 * chunk + 3);
+            float b[8];
+            unpack8<T>(braw, b);
+            if (EPI == E_BIAS_GELU) {
+#pragma unroll
+              for (int j = 0; j < 8; ++j) o[j] = a[j] + b[j];
+              const uint4 f16 = pack8<T>(o);
+              *slot = f16;
+              unpack8<T>(f16, o);                        // the backward pass differentiates at the stored value
+#pragma unroll
+              for (int j = 0; j < 8; j += 2) f2_get(gelu2(f2(o[j], o[j + 1])), a[j], a[j + 1]);
+              keep2[EPI == E_BIAS_GELU ? chunk : 0] = pack8<T>(a);
+            } else {
+              float res[8];
+              unpack8<T>(in_row[HELD_IN ? chunk : 0], res);
+#pragma unroll
+              for (int j = 0; j < 8; ++j) {
+                float t = a[j] + b[j];
+                if (p.p > 0.f) t = (kept[chunk >> 2] >> (8 * (chunk & 3) + j)) & 1u ? t * inv_keep : 0.f;
+                o[j] = res[j] + t;
               }
             }
+          } else if (EPI == E_ADD) {
+            float res[8];
+            unpack8<T>(in_row[HELD_IN ? chunk : 0], res);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) o[j] = a[j] + res[j];
+          } else if (EPI == E_DW_SGD) {
+            // momentum SGD on the tile: m = mo m + (dW + wd w), w -= lr m, with m rounded to 16 bit first.  One element
+            // at a time this was some 40 instructions per element, more than the tile's bytes take: two per instruction.
+            // The noise of the rounding takes a hash per element, half of what is left.  1.3 M labels x 768, batch 512:
+            // 2.01 -> 1.76 ms (1.68 with one hash per pair, which gives other weights for the same seed).
+            uint4* slot2 = reinterpret_cast<uint4*>(pan2 + panel_off(lane, chunk));
+            float w[8], mm[8];
+            unpack8<T>(*slot, w);
+            unpack8<T>(*slot2, mm);
+            const F2 nlr = f2(-p.hp[HP_LR_XFC]), mo2 = f2(p.mo), wd2 = f2(p.wd);
+            const uint32_t sr_seed = reinterpret_cast<const uint32_t*>(p.hp)[HP_SEED];
+            const uint32_t e = (uint32_t)row * (uint32_t)p.ldW + (uint32_t)c;
+#pragma unroll
+            for (int j = 0; j < 8; j += 2)
+              f2_get(f2_fma(mo2, f2(mm[j], mm[j + 1]), f2_fma(wd2, f2(w[j], w[j + 1]), f2(a[j], a[j + 1]))), mm[j], mm[j + 1]);
+            const uint4 m16 = pack8<T>(mm);
+            unpack8<T>(m16, mm);
+#pragma unroll
+            for (int j = 0; j < 8; j += 2) f2_get(f2_fma(nlr, f2(mm[j], mm[j + 1]), f2(w[j], w[j + 1])), o[j], o[j + 1]);
+            *slot2 = m16;
+            if (p.stochastic_round) {
+              uint4 w16;                               // every element has a hash of its own number
+              uint32_t* wp = reinterpret_cast<uint32_t*>(&w16);
+#pragma unroll
+              for (int j = 0; j < 8; j += 2)
+                wp[j >> 1] = sr_pack2<T>(o[j], o[j + 1], mix32(sr_seed, 0x5152u, e + j), mix32(sr_seed, 0x5152u, e + j + 1));
+              *slot = w16;
+            } else {
+              *slot = pack8<T>(o);
+            }
+          } else {   // E_GELU_BWD
+            float f[8];
+            unpack8<T>(in_row[HELD_IN ? chunk : 0], f);
+#pragma unroll
+            for (int j = 0; j < 8; j += 2) f2_get(f2(a[j], a[j + 1]) * gelu_grad2(f2(f[j], f[j + 1])), o[j], o[j + 1]);
           }
-          tc::fence_proxy_async();                 // generic-proxy writes of the panel before the async-proxy store
-          asm volatile("bar.sync %0, 128;" ::"r"(bar_id) : "memory");
-          if (elected) {
-            tc::tma_store_2d(EPI == E_BIAS_GELU ? &tmF : &tmC, pan, pcol, m0);
-            if (EPI == E_DW_SGD) tc::tma_store_2d(&tmF, pan2, pcol, m0);
+          if (EPI != E_BIAS_GELU && EPI != E_DW_SGD) *slot = pack8<T>(o);
+        }
+        if (EPI == E_SIGMOID_POS && p.pos_labels != nullptr) {
+          // subtract 1 at the tile's positives while it is still in shared memory: entries of the label-sorted list whose
+          // label is one of this warp's 32 rows and whose batch row is one of the panel's 64 columns
+          __syncwarp();                                    // every row of the warp's part is written
+          const int lab0 = p.label0 + sub0, n_lab = min(SUB_ROWS, M - sub0);
+          for (int e = pos_more + lane - 32, pl = pos_l, pc = pos_c;;) {
+            const int bcol = pc - pcol, pr = pl - lab0;
+            if (pr >= 0 && pr < n_lab && bcol >= 0 && bcol < 64 && pc < p.N) {
+              T* cell = reinterpret_cast<T*>(pan + panel_off(pr, bcol >> 3)) + (bcol & 7);
+              *cell = from_f<T>(to_f(*cell) - 1.f);        // duplicates are removed by the collator: one writer per cell
+            }
+            e += 32;
+            if (e >= pos_end) break;
+            pl = p.pos_labels[e];
+            pc = p.pos_rows[e];
+          }
+        }
+        tc::fence_proxy_async();                 // generic-proxy writes of the panel before the async-proxy store
+        __syncwarp();
+        if (sub0 < M && tc::elect_one()) {
+          tc::tma_store_2d(EPI == E_BIAS_GELU ? &tmF : &tmC, pan, pcol, sub0);
+          if (EPI == E_DW_SGD) tc::tma_store_2d(&tmF, pan2, pcol, sub0);
+          tc::tma_store_commit();
+        }
+        if (EPI == E_BIAS_GELU) {
+          // second output through the same panel: C = gelu(F), held in registers
+          if (tc::elect_one()) tc::tma_store_wait_read<0>();
+          __syncwarp();
+#pragma unroll
+          for (int chunk = 0; chunk < 8; ++chunk)
+            *reinterpret_cast<uint4*>(pan + panel_off(lane, chunk)) = keep2[EPI == E_BIAS_GELU ? chunk : 0];
+          tc::fence_proxy_async();
+          __syncwarp();
+          if (sub0 < M && tc::elect_one()) {
+            tc::tma_store_2d(&tmC, pan, pcol, sub0);
             tc::tma_store_commit();
           }
-          if (EPI == E_BIAS_GELU) {
-            // second output through the same panel: C = gelu(F), held in the fragment registers
-            if (elected) tc::tma_store_wait_read<0>();
-            asm volatile("bar.sync %0, 128;" ::"r"(bar_id) : "memory");
-#pragma unroll
-            for (int chunk = 0; chunk < 8; ++chunk)
-              *reinterpret_cast<uint4*>(pan + panel_off(r, chunk)) = keep2[EPI == E_BIAS_GELU ? chunk : 0];
-            tc::fence_proxy_async();
-            asm volatile("bar.sync %0, 128;" ::"r"(bar_id) : "memory");
-            if (elected) {
-              tc::tma_store_2d(&tmC, pan, pcol, m0);
-              tc::tma_store_commit();
-            }
+        }
+        if (EPI == E_GELU_BWD && p.colacc != nullptr && sub0 < M && pcol + 2 * lane < p.N) {
+          // bias gradient: each lane adds two columns of the staged (rounded) rows; rows past the packed tokens hold what an
+          // earlier pass left
+          const int n_rows = min(SUB_ROWS, M - sub0);
+          F2 cs = f2(0.f);
+          for (int i = 0; i < n_rows; ++i) {
+            const uint32_t w = *reinterpret_cast<const uint32_t*>(pan + panel_off(i, lane >> 2) + 4 * (lane & 3));
+            const T* e = reinterpret_cast<const T*>(&w);
+            cs = cs + f2(to_f(e[0]), to_f(e[1]));
           }
+          float c0, c1;
+          f2_get(cs, c0, c1);
+          float* at = p.colacc + (size_t)(blockIdx.x % kColReplicas) * p.col_tot + p.col_off + pcol + 2 * lane;
+          atomicAdd(at, c0);
+          atomicAdd(at + 1, c1);
         }
       }
       if (EPI == E_TOPK) {
@@ -735,7 +776,7 @@ enc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
         }
       }
     }
-    if (STAGED && elected) tc::tma_store_wait_read<0>();   // the stores have read shared memory; they complete before the grid does
+    if (STAGED && staging && tc::elect_one()) tc::tma_store_wait_read<0>();   // the stores have read shared memory; they complete before the grid does
     if (EPI == E_SIGMOID_POS && p.loss_acc != nullptr) {
       loss = warp_sum(loss);
       if (lane == 0 && loss != 0.f) atomicAdd(p.loss_acc, loss);
@@ -887,22 +928,38 @@ static int dispatch_enc_gemm(int layout, int epi, const Maps& m, const Params& p
   return -4;
 }
 
-// Tile shape and K-splits from a cost model calibrated on B200 (clocks per CTA):
-//   * a k block costs max(MMA time = 2 BN, operand bytes of the CTA / fetch rate); with every SM busy an SM sustains
-//     about 29 bytes per clock from L2 (the L2-to-SM fabric, about 8 TB/s in total, is the shared limit), with
-//     fewer SMs busy proportionally more, down to a floor of about 3900 clocks of load latency divided by the
-//     number of ring stages (192 KB / stage size: 4 to 8);
-//   * work is spread over the units (SMs, or SM pairs) in rounds;
-//   * about 3000 clocks of start-up per kernel (TMEM allocation, barrier set-up, first load);
-//   * the epilogue of a CTA's last tile is exposed: per 64-column panel about 1200 clocks (store), 2400 (two
-//     outputs), 2800 (a tile-shaped input fetched after the previous panel has left; the first panel's input is
-//     fetched under the main loop);
+// Tile shape and K-splits from a cost model calibrated on B200 (clocks per CTA; grids of 256 x 256 pair tiles down to
+// 128 x 64, K = 64 .. 3072, chained launches):
+//   * a k block costs the largest of MMA time (2.25 BN: shared memory, read by the MMAs and written by the loads, keeps the
+//     tensor pipe from its 2 BN), operand bytes of the CTA over the rate at which an SM receives them (75 bytes per clock
+//     with most SMs busy), and about 290 clocks of issue and barrier traffic;
+//   * work is spread over the units (SMs, or SM pairs) in rounds; a round cannot be shorter than a tile's epilogue, and a
+//     share of the epilogue is added to it (epi_share);
+//   * about 3000 clocks of start-up per kernel (TMEM allocation, barrier set-up, first load), 600 more for pairs;
+//   * the epilogue of a CTA's last tile is exposed: epi_clocks, by 64-column panels;
 //   * a K-split costs about 10000 clocks (partial sums through L2 atomics, the last CTA's conversion pass).
 struct Plan { int ncta, bn, splits, tiles; };
 
 static int g_max_units = 0;
 // Experiments: cap the number of persistent workers (0 = one per SM / SM pair).
 RB_API void rb_enc_gemm_set_max_units(int n) { g_max_units = n; }
+
+static double epi_clocks(int epi, int bn) {
+  const double n = bn / 64.0;
+  switch (epi) {
+    case E_STORE: return 800 + 480 * n;
+    case E_ADD: return 1000 + 560 * n;
+    case E_BIAS_DROPOUT_RESID: return 2500 + 800 * n;
+    case E_BIAS_GELU: return 3000 + 1700 * n;
+    case E_GELU_BWD: return 2800 + 1550 * n;
+    case E_SIGMOID_POS: return 1000 + 1200 * n;
+    case E_DW_SGD: return 1500 + 1500 * n;
+    default: return 800;                       // SPLITK, DX, TOPK
+  }
+}
+// Share of a tile's epilogue that its round is longer than the main loop: shared-memory traffic of the panels, and for the
+// dropout epilogue the hashes of a tile that does not have the epilogue warps to itself.
+static double epi_share(int epi) { return epi == E_BIAS_DROPOUT_RESID ? 0.6 : 0.35; }
 
 static Plan make_plan(int layout, int epi, int M, int N, int K, int bn_forced, int ncta_forced) {
   const int sms = sm_count();
@@ -931,17 +988,13 @@ static Plan make_plan(int layout, int epi, int M, int N, int K, int bn_forced, i
         const long rounds = (items + units - 1) / units;
         const double busy = (double)(items < units ? items : units) * ncta / sms;      // fraction of the SMs at work
         const double bytes = A_BYTES + (double)(bn / ncta) * BK * 2;
-        double t_kb = bytes / (29.0 / (busy > 0.25 ? busy : 0.25));
-        const int stages = (int)(ring_bytes(epi) / bytes) < MAX_STAGES ? (int)(ring_bytes(epi) / bytes) : MAX_STAGES;
-        if (t_kb < 3900.0 / stages) t_kb = 3900.0 / stages;          // load latency over the ring depth
-        if (t_kb < 2.0 * bn) t_kb = 2.0 * bn;
-        const int n_pan = 1;                                         // one staging panel per group and tile
-        double tail;
-        if (epi == E_SPLITK || epi == E_TOPK || epi == E_DX) tail = 800.0 * n_pan;
-        else if (epi == E_STORE) tail = 1200.0 * n_pan;
-        else if (epi == E_BIAS_GELU) tail = 2400.0 * n_pan;
-        else tail = 1200.0 + 2800.0 * (n_pan - 1);
-        const double cost = 3000.0 + rounds * (kb_per * t_kb) + tail + (eff_splits > 1 && epi != E_DX ? 10000.0 : 0.0);
+        double t_kb = bytes / (busy > 0.5 ? 75.0 : 150.0);
+        if (t_kb < 290.0) t_kb = 290.0;
+        if (t_kb < 2.25 * bn) t_kb = 2.25 * bn;
+        const double tail = epi_clocks(epi, bn);
+        double round = kb_per * t_kb + epi_share(epi) * tail;
+        if (round < tail) round = tail;
+        const double cost = 3000.0 + (ncta == 2 ? 600.0 : 0.0) + rounds * round + tail + (eff_splits > 1 && epi != E_DX ? 10000.0 : 0.0);
         if (best_cost < 0 || cost < best_cost) { best_cost = cost; best = Plan{ncta, bn, eff_splits, tiles}; }
       }
     }
@@ -993,13 +1046,13 @@ RB_API int rb_enc_gemm(int dtype, int layout, int epi, const void* A, const void
   if (layout == L_NT) rc = tc::make_tmap_2d(&m.b, B, N, K, ldb, 64, b_rows, bf16);
   else rc = tc::make_tmap_2d(&m.b, B, K, N, ldb, 64, 64, bf16);
   if (rc) return rc;
-  // output / input panels: [128 rows x 64 columns] boxes of the row-major [M, N] matrices
-  rc = tc::make_tmap_2d(&m.c, C, M, N, ldc, 64, BM, bf16);
+  // output / input panels: [32 rows x 64 columns] boxes of the row-major [M, N] matrices, one per epilogue warp
+  rc = tc::make_tmap_2d(&m.c, C, M, N, ldc, 64, SUB_ROWS, bf16);
   if (rc) return rc;
   m.r = m.c;
   m.f = m.c;
-  if (R != nullptr && (rc = tc::make_tmap_2d(&m.r, R, M, N, ldr, 64, BM, bf16)) != 0) return rc;
-  if (F != nullptr && (rc = tc::make_tmap_2d(&m.f, F, M, N, ldf, 64, BM, bf16)) != 0) return rc;
+  if (R != nullptr && (rc = tc::make_tmap_2d(&m.r, R, M, N, ldr, 64, SUB_ROWS, bf16)) != 0) return rc;
+  if (F != nullptr && (rc = tc::make_tmap_2d(&m.f, F, M, N, ldf, 64, SUB_ROWS, bf16)) != 0) return rc;
   Params p{};
   p.M = M; p.N = N; p.BN = BN;
   p.n_m_tiles = (M + BM * pl.ncta - 1) / (BM * pl.ncta); p.n_n_tiles = (N + BN - 1) / BN;
@@ -1107,7 +1160,7 @@ RB_API int rb_xfc_logits_grad_v2(const void* W, int Lc, int D, const void* X, in
   if (rc) return rc;
   rc = tc::make_tmap_2d(&m.b, X, B, D, D, 64, pl.bn / pl.ncta, false);
   if (rc) return rc;
-  rc = tc::make_tmap_2d(&m.c, Gt, Lc, ldG, ldG, 64, BM, false);
+  rc = tc::make_tmap_2d(&m.c, Gt, Lc, ldG, ldG, 64, SUB_ROWS, false);
   if (rc) return rc;
   m.r = m.c; m.f = m.c;
   Params p{};
@@ -1160,10 +1213,10 @@ RB_API int rb_xfc_dw_sgd_v2(const void* Gt, int ldG, const void* X, int B, void*
   if (rc) return rc;
   rc = tc::make_tmap_2d(&m.b, X, B, D, D, 64, 64, false);
   if (rc) return rc;
-  rc = tc::make_tmap_2d(&m.c, W, Lc, D, D, 64, BM, false);
+  rc = tc::make_tmap_2d(&m.c, W, Lc, D, D, 64, SUB_ROWS, false);
   if (rc) return rc;
   m.r = m.c;
-  rc = tc::make_tmap_2d(&m.f, Mom, Lc, D, D, 64, BM, false);
+  rc = tc::make_tmap_2d(&m.f, Mom, Lc, D, D, 64, SUB_ROWS, false);
   if (rc) return rc;
   Params p{};
   p.M = Lc; p.N = D; p.status = status;

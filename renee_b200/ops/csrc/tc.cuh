@@ -163,6 +163,20 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float (&v)[32]) {
   for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
 }
 
+// The same for 8 columns in two steps, so that the next fragment is on its way while one is worked on: the registers hold the
+// values only behind tmem_wait8.
+__device__ __forceinline__ void tmem_issue8(uint32_t taddr, uint32_t (&r)[8]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+               : "r"(taddr)
+               : "memory");
+}
+__device__ __forceinline__ void tmem_wait8(uint32_t (&r)[8]) {
+  asm volatile("tcgen05.wait::ld.sync.aligned;"
+               : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7])
+               :: "memory");
+}
+
 // ---- CTA pairs (cta_group::2): two CTAs of a cluster of two work on one 256-row tile.  CTA rank 0 (the
 // leader) issues the MMAs, which read the A rows and half of the B columns from EACH CTA's shared memory and
 // write 128 accumulator rows into each CTA's TMEM.  No TMA multicast is involved: each CTA loads its own
