@@ -567,16 +567,38 @@ enc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
           // label is one of this warp's 32 rows and whose batch row is one of the panel's 64 columns
           __syncwarp();                                    // every row of the warp's part is written
           const int lab0 = p.label0 + sub0, n_lab = min(SUB_ROWS, M - sub0);
-          for (int e = pos_more + lane - 32, pl = pos_l, pc = pos_c;;) {
-            const int bcol = pc - pcol, pr = pl - lab0;
+          const auto apply = [&](int pl, int pc, uint8_t* part, int col0) {
+            const int bcol = pc - col0, pr = pl - lab0;
             if (pr >= 0 && pr < n_lab && bcol >= 0 && bcol < 64 && pc < p.N) {
-              T* cell = reinterpret_cast<T*>(pan + panel_off(pr, bcol >> 3)) + (bcol & 7);
+              T* cell = reinterpret_cast<T*>(part + panel_off(pr, bcol >> 3)) + (bcol & 7);
               *cell = from_f<T>(to_f(*cell) - 1.f);        // duplicates are removed by the collator: one writer per cell
             }
-            e += 32;
-            if (e >= pos_end) break;
-            pl = p.pos_labels[e];
-            pc = p.pos_rows[e];
+          };
+          apply(pos_l, pos_c, pan, pcol);
+          if (pos_end > pos_more) {
+            // Labels that many rows have (the first 32 of a Zipf-distributed 1.3 M hold 5000 of 21000 positives): the warps of
+            // these 32 rows share the entries out, each applying its own to all panels of the tile, 8 on their way per lane.
+            // Every panel's warp scanning all of them made the launch with those labels take 192 us, where the others take 47.
+            // (The same list, hence the same way here, in each of these warps; a wait that one of them passed cannot run out
+            // in another, as the accumulator stays until all have read it.)
+            const int np = p.BN >> 6;
+            asm volatile("bar.sync %0, %1;" ::"r"(2 + quarter), "r"(32 * np) : "memory");
+            for (int e0 = pos_more + 32 * g + lane; e0 < pos_end; e0 += 256 * np) {
+              int pl[8], pc[8];
+#pragma unroll
+              for (int u = 0; u < 8; ++u) {
+                const int e = e0 + 32 * np * u;
+                pl[u] = e < pos_end ? p.pos_labels[e] : 0x7fffffff;
+                pc[u] = e < pos_end ? p.pos_rows[e] : 0;
+              }
+#pragma unroll
+              for (int u = 0; u < 8; ++u) {
+                const int pg = (pc[u] - n0) >> 6;          // panel of the tile
+                if (pg >= 0 && pg < np) apply(pl[u], pc[u], panels + pg * PANEL_BYTES + quarter * SUB_BYTES, n0 + 64 * pg);
+              }
+            }
+            tc::fence_proxy_async();
+            asm volatile("bar.sync %0, %1;" ::"r"(2 + quarter), "r"(32 * np) : "memory");
           }
         }
         tc::fence_proxy_async();                 // generic-proxy writes of the panel before the async-proxy store
