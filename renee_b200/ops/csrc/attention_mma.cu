@@ -179,29 +179,35 @@ __device__ __forceinline__ void transposed_times_rows(float (&out)[NJ][4], const
 template <typename T, int NJ>
 __device__ __forceinline__ void write_rows(const float (&out)[NJ][4], T* dst, int ld, int row_lo, int row_hi, int lane,
                                            float* col_sums) {
-  const int g = lane >> 2, t = lane & 3;
+  const int t = lane & 3;
   const bool v0 = row_lo >= 0, v1 = row_hi >= 0;
+  float cs[2 * NJ];                                // this lane's columns 8 jd + 2 t + e over its two rows
 #pragma unroll
   for (int jd = 0; jd < NJ; ++jd) {
     const uint32_t lo = Pack<T>::pack(out[jd][0], out[jd][1]);
     const uint32_t hi = Pack<T>::pack(out[jd][2], out[jd][3]);
     if (v0) *reinterpret_cast<uint32_t*>(dst + (size_t)row_lo * ld + 8 * jd + 2 * t) = lo;
     if (v1) *reinterpret_cast<uint32_t*>(dst + (size_t)row_hi * ld + 8 * jd + 2 * t) = hi;
-    if (col_sums != nullptr) {
-      const float2 a = Pack<T>::unpack(lo), b = Pack<T>::unpack(hi);
-      float s0 = (v0 ? a.x : 0.f) + (v1 ? b.x : 0.f);
-      float s1 = (v0 ? a.y : 0.f) + (v1 ? b.y : 0.f);
-#pragma unroll
-      for (int o = 4; o < 32; o <<= 1) {
-        s0 += __shfl_xor_sync(0xffffffffu, s0, o);
-        s1 += __shfl_xor_sync(0xffffffffu, s1, o);
-      }
-      if (g == 0) {
-        atomicAdd(col_sums + 8 * jd + 2 * t, s0);
-        atomicAdd(col_sums + 8 * jd + 2 * t + 1, s1);
-      }
-    }
+    const float2 a = Pack<T>::unpack(lo), b = Pack<T>::unpack(hi);
+    cs[2 * jd] = (v0 ? a.x : 0.f) + (v1 ? b.x : 0.f);
+    cs[2 * jd + 1] = (v0 ? a.y : 0.f) + (v1 ? b.y : 0.f);
   }
+  if (col_sums == nullptr) return;
+  // over the eight lanes of equal t: each step hands half of the columns to the partner lane, 14 shuffles and 2 shared-memory
+  // additions per lane at NJ = 8 instead of 48 and 16
+  int at = 0;
+#pragma unroll
+  for (int o = 16, n = NJ; o >= 4; o >>= 1, n >>= 1) {
+    const bool upper = (lane & o) != 0;
+#pragma unroll
+    for (int i = 0; i < n; ++i) {
+      const float send = upper ? cs[i] : cs[i + n], mine = upper ? cs[i + n] : cs[i];
+      cs[i] = mine + __shfl_xor_sync(0xffffffffu, send, o);
+    }
+    at += upper ? n : 0;
+  }
+#pragma unroll
+  for (int i = 0; i < NJ / 4; ++i) atomicAdd(col_sums + 8 * ((at + i) >> 1) + 2 * t + ((at + i) & 1), cs[i]);
 }
 
 // Elements idx, idx + 1 of a [.., S] row as one packed word, ok0 / ok1 saying which exist (0 for the others); `pair` =
@@ -220,24 +226,43 @@ __device__ __forceinline__ uint32_t load_pair_raw(const T* __restrict__ base, si
   return r;
 }
 
+// Sums of 8 pairs, two per instruction, rounded once
+template <typename T> __device__ __forceinline__ uint4 add16x8(const uint4& a, const uint4& b) {
+  using T2 = typename std::conditional<std::is_same<T, __half>::value, __half2, __nv_bfloat162>::type;
+  uint4 r;
+  const T2 *x = reinterpret_cast<const T2*>(&a), *y = reinterpret_cast<const T2*>(&b);
+  T2* o = reinterpret_cast<T2*>(&r);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) o[i] = __hadd2(x[i], y[i]);
+  return r;
+}
+
 // Stages (q + bq, k + bk, v + bv [, dO]) of one (batch, head) as [SP][RP] tiles; rows of tokens that do not
 // exist are zero, rows >= lim are left alone.
 // The CTA has SP * 2 threads and the tiles SP * HD / 8 segments of 8 columns, so a thread owns the same 8 columns of
 // HD / 16 rows: all of its global loads are issued before the first one is used.
 // CLS: dO has one row per sequence (that of token 0), and only the first 16 queries are staged.
+// The rows of a thread's tokens come from stage_rows.  Up to 32 tokens its loads go out together with that of the sequence's
+// length: one after the other these two and the loads that hang on them were three round trips before the first product
+// (256 x 32 packed, forward / backward with what follows: 15.3 / 40.1 -> 12.7 / 24.8 us).  Longer tiles have the length first,
+// which leaves out the rows behind it.  The bias is added two values per instruction, rounded once as before; the longer
+// forward tiles are the exception, where that came out slower (128 x 128: 66.9 us against 63.0).
+template <int SP, int HD>
+__device__ __forceinline__ void stage_rows(int (&row)[HD / 16], const Tok& tk, int b, int S, int n) {
+  constexpr int SEGS = HD / 8, ROWS_PER_PASS = SP * 2 / SEGS;
+#pragma unroll
+  for (int it = 0; it < HD / 16; ++it) {
+    const int s = (int)threadIdx.x / SEGS + it * ROWS_PER_PASS;
+    row[it] = s < n ? seq_row(tk, b, S, s) : -1;           // of a packed token behind the last kept one: -1 too
+  }
+}
 template <typename T, int SP, int HD, bool WITH_DO, bool CLS = false>
 __device__ __forceinline__ void stage_operands(const T* __restrict__ qkv, const T* __restrict__ bqkv, const T* __restrict__ dctx,
-                                               T* sQ, T* sK, T* sV, T* sDO, const Tok& tk, int b, int h, int S, int H, int len,
+                                               T* sQ, T* sK, T* sV, T* sDO, const int (&row)[HD / 16], int b, int h, int H,
                                                int lim) {
   constexpr int RP = HD + 8, SEGS = HD / 8, ROWS_PER_PASS = SP * 2 / SEGS, NIT = HD / 16;
   const int d = (threadIdx.x % SEGS) * 8, s0 = threadIdx.x / SEGS;
   Raw8<T> rq[NIT], rk[NIT], rv[NIT], rg[NIT];
-  int row[NIT];
-#pragma unroll
-  for (int it = 0; it < NIT; ++it) {
-    const int s = s0 + it * ROWS_PER_PASS;
-    row[it] = s < len ? seq_row(tk, b, S, s) : -1;
-  }
 #pragma unroll
   for (int it = 0; it < NIT; ++it) {
     if (row[it] >= 0) {
@@ -251,26 +276,27 @@ __device__ __forceinline__ void stage_operands(const T* __restrict__ qkv, const 
       }
     }
   }
-  float bq[8], bk[8], bv[8];
-  load8(bqkv + h * HD + d, bq); load8(bqkv + H + h * HD + d, bk); load8(bqkv + 2 * H + h * HD + d, bv);
+  constexpr bool PAIRS = WITH_DO || SP < 64;
+  const Raw8<T> bq = load_raw8(bqkv + h * HD + d), bk = load_raw8(bqkv + H + h * HD + d), bv = load_raw8(bqkv + 2 * H + h * HD + d);
+  const auto sum = [](const Raw8<T>& x, const Raw8<T>& bias) -> uint4 {
+    if constexpr (PAIRS) return add16x8<T>(x.v, bias.v);
+    float a[8], c[8];
+    unpack8(x, a);
+    unpack8(bias, c);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) a[j] += c[j];
+    return pack16x8<T>(a);
+  };
 #pragma unroll
   for (int it = 0; it < NIT; ++it) {
     const int s = s0 + it * ROWS_PER_PASS;
     if (s >= lim) continue;
-    float q[8], k[8], v[8];
-    if (row[it] >= 0) {
-      if (!CLS || s < 16) unpack8(rq[it], q);
-      unpack8(rk[it], k); unpack8(rv[it], v);
-#pragma unroll
-      for (int j = 0; j < 8; ++j) { if (!CLS || s < 16) q[j] += bq[j]; k[j] += bk[j]; v[j] += bv[j]; }
-      if constexpr (WITH_DO) { if (!CLS || s < 16) *reinterpret_cast<uint4*>(sDO + s * RP + d) = rg[it].v; }
-    } else {
-#pragma unroll
-      for (int j = 0; j < 8; ++j) { q[j] = 0.f; k[j] = 0.f; v[j] = 0.f; }
-      if constexpr (WITH_DO) { if (!CLS || s < 16) *reinterpret_cast<uint4*>(sDO + s * RP + d) = make_uint4(0u, 0u, 0u, 0u); }
-    }
-    if (!CLS || s < 16) store8(sQ + s * RP + d, q);
-    store8(sK + s * RP + d, k); store8(sV + s * RP + d, v);
+    const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+    const bool on = row[it] >= 0;
+    if (!CLS || s < 16) *reinterpret_cast<uint4*>(sQ + s * RP + d) = on ? sum(rq[it], bq) : zero;
+    *reinterpret_cast<uint4*>(sK + s * RP + d) = on ? sum(rk[it], bk) : zero;
+    *reinterpret_cast<uint4*>(sV + s * RP + d) = on ? sum(rv[it], bv) : zero;
+    if constexpr (WITH_DO) { if (!CLS || s < 16) *reinterpret_cast<uint4*>(sDO + s * RP + d) = on ? rg[it].v : zero; }
   }
 }
 
@@ -296,7 +322,7 @@ __device__ __forceinline__ void zero_rest(T* dst, const int* sRow, int len, int 
 }
 
 template <typename T, int SP, int HD, bool CLS>
-__global__ void __launch_bounds__(SP * 2, SP == 128 ? 2 : 1) attention_fwd_mma_kernel(
+__global__ void __launch_bounds__(SP * 2, SP == 128 ? 2 : SP == 64 ? 4 : SP == 32 ? 9 : 16) attention_fwd_mma_kernel(
     const T* __restrict__ qkv, const T* __restrict__ bqkv, const int* __restrict__ mask, T* __restrict__ ctx,
     T* __restrict__ probs, int S, int H, int nh, float p, const int* __restrict__ seed_ptr, uint32_t stream, const Tok tk, int len_lo,
     const FirstTok<T> ft) {
@@ -316,14 +342,18 @@ __global__ void __launch_bounds__(SP * 2, SP == 128 ? 2 : 1) attention_fwd_mma_k
   const float inv_keep = p > 0.f ? 1.f / (1.f - p) : 1.f;
   const float scale = rsqrtf((float)HD);
   if (!CLS && tk.slot != nullptr && b == (int)gridDim.y - 1) clear_zero_rows<T>(tk, ctx, H, h * HD, HD);
+  int srow[HD / 16];
+  if constexpr (SP < 64) stage_rows<SP, HD>(srow, tk, b, S, S);
+  const int trow = threadIdx.x < SP && (int)threadIdx.x < S ? seq_row(tk, b, S, threadIdx.x) : -1;    // of token threadIdx.x
+  const int tmask = threadIdx.x < SP && (int)threadIdx.x < S ? mask[b * S + threadIdx.x] : 0;
   const int len = seq_len(tk, b, S), lim = (len + 15) & ~15;
   if (len > SP || len <= len_lo) return;       // another launch serves this length
-  for (int j = threadIdx.x; j < SP; j += blockDim.x) {
-    const int row = j < len ? seq_row(tk, b, S, j) : -1;
-    sRow[j] = row;
-    sCode[j] = row >= 0 ? (mask[b * S + j] != 0 ? 1 : 2) : 0;
+  if constexpr (SP >= 64) stage_rows<SP, HD>(srow, tk, b, S, len);
+  if (threadIdx.x < SP) {
+    sRow[threadIdx.x] = trow;
+    sCode[threadIdx.x] = trow >= 0 ? (tmask != 0 ? 1 : 2) : 0;
   }
-  stage_operands<T, SP, HD, false, CLS>(qkv, bqkv, nullptr, sQ, sK, sV, nullptr, tk, b, h, S, H, len, lim);
+  stage_operands<T, SP, HD, false, CLS>(qkv, bqkv, nullptr, sQ, sK, sV, nullptr, srow, b, h, H, lim);
   __syncthreads();
   const int r0 = warp * 16;
   if (r0 >= (CLS ? 16 : lim)) return;
@@ -366,7 +396,7 @@ __global__ void __launch_bounds__(SP * 2, SP == 128 ? 2 : 1) attention_fwd_mma_k
   const int i0 = r0 + g, i1 = r0 + g + 8;
   const int row0 = !CLS ? sRow[i0] : (i0 == 0 ? b : -1), row1 = CLS ? -1 : sRow[i1];     // rows of ctx
   const float inv0 = row0 >= 0 ? 1.f / sum0 : 0.f, inv1 = row1 >= 0 ? 1.f / sum1 : 0.f;
-  const size_t prow0 = ((size_t)(b * nh + h) * S + i0) * S, prow1 = ((size_t)(b * nh + h) * S + i1) * S;
+  const size_t prow0 = ((size_t)(b * nh + h) * S + i0) * S, prow1 = prow0 + 8 * S;
   const bool pair_store = (S & 1) == 0;   // then every (row, even column) element is 4-byte aligned
   uint32_t pf[SP / 16][4];                // P~ as the A operand of O = P~ V
 #pragma unroll
@@ -411,7 +441,7 @@ __global__ void __launch_bounds__(SP * 2, SP == 128 ? 2 : 1) attention_fwd_mma_k
 }
 
 template <typename T, int SP, int HD, bool CLS>
-__global__ void __launch_bounds__(SP * 2, SP == 64 ? 4 : 1) attention_bwd_mma_kernel(
+__global__ void __launch_bounds__(SP * 2, SP == 64 ? 4 : SP == 32 ? 8 : 16) attention_bwd_mma_kernel(
     const T* __restrict__ dctx, const T* __restrict__ qkv, const T* __restrict__ bqkv, const T* __restrict__ probs,
     T* __restrict__ dqkv, int S, int H, int nh, float p, const int* __restrict__ seed_ptr, uint32_t stream,
     float* __restrict__ bias_acc, const Tok tk, int len_lo, const FirstTok<T> ft) {
@@ -439,9 +469,13 @@ __global__ void __launch_bounds__(SP * 2, SP == 64 ? 4 : 1) attention_bwd_mma_ke
   if (tk.slot != nullptr && b == (int)gridDim.y - 1)
     for (int w = 0; w < (CLS ? 4 : 3); ++w)
       clear_zero_rows<T>(tk, w < 3 ? dqkv : ft.dst, w < 3 ? 3 * H : H, (w < 3 ? w * H : 0) + h * HD, HD);
+  int srow[HD / 16];
+  if constexpr (SP < 64) stage_rows<SP, HD>(srow, tk, b, S, S);
+  const int trow = threadIdx.x < SP && (int)threadIdx.x < S ? seq_row(tk, b, S, threadIdx.x) : -1;    // of token threadIdx.x
   const int len = seq_len(tk, b, S), lim = (len + 15) & ~15;
   if (len > SP || len <= len_lo) return;       // another launch serves this length
-  for (int j = threadIdx.x; j < SP; j += blockDim.x) sRow[j] = j < len ? seq_row(tk, b, S, j) : -1;
+  if constexpr (SP >= 64) stage_rows<SP, HD>(srow, tk, b, S, len);
+  if (threadIdx.x < SP) sRow[threadIdx.x] = trow;
   const int r0 = warp * 16;
   const int i0 = r0 + g, i1 = r0 + g + 8;
   const size_t prow0 = ((size_t)(b * nh + h) * S + i0) * S, prow1 = ((size_t)(b * nh + h) * S + i1) * S;
@@ -453,7 +487,7 @@ __global__ void __launch_bounds__(SP * 2, SP == 64 ? 4 : 1) attention_bwd_mma_ke
     wf[j][0] = load_pair_raw<T>(probs, prow0 + c, r0 < lim && 8 * j < lim && i0 < (CLS ? 1 : S) && c < S, c + 1 < S, pair_load);
     wf[j][1] = load_pair_raw<T>(probs, prow1 + c, r0 < lim && 8 * j < lim && i1 < (CLS ? 1 : S) && c < S, c + 1 < S, pair_load);
   }
-  stage_operands<T, SP, HD, true, CLS>(qkv, bqkv, dctx, sQ, sK, sV, sDO, tk, b, h, S, H, len, lim);
+  stage_operands<T, SP, HD, true, CLS>(qkv, bqkv, dctx, sQ, sK, sV, sDO, srow, b, h, H, lim);
   __syncthreads();
   const int row0 = sRow[r0 + g], row1 = sRow[r0 + g + 8];
   const int qlim = CLS ? 16 : lim;             // queries that have a gradient (CLS: the rows behind the first are zeros)
@@ -595,14 +629,17 @@ __global__ void __launch_bounds__(SP * 2, SP == 128 ? 2 : 1) attention_fwd_blk_k
   const float inv_keep = p > 0.f ? 1.f / (1.f - p) : 1.f;
   const float scale = rsqrtf((float)HD);
   if (!CLS && tk.slot != nullptr && b == (int)gridDim.y - 1) clear_zero_rows<T>(tk, ctx, H, h * HD, HD);
+  int srow[HD / 16];
+  const int trow = threadIdx.x < SP && (int)threadIdx.x < S ? seq_row(tk, b, S, threadIdx.x) : -1;    // of token threadIdx.x
+  const int tmask = threadIdx.x < SP && (int)threadIdx.x < S ? mask[b * S + threadIdx.x] : 0;
   const int len = seq_len(tk, b, S), lim = (len + 15) & ~15;
   if (len > SP || len <= len_lo) return;
-  for (int j = threadIdx.x; j < SP; j += blockDim.x) {
-    const int row = j < len ? seq_row(tk, b, S, j) : -1;
-    sRow[j] = row;
-    sCode[j] = row >= 0 ? (mask[b * S + j] != 0 ? 1 : 2) : 0;
+  stage_rows<SP, HD>(srow, tk, b, S, len);
+  if (threadIdx.x < SP) {
+    sRow[threadIdx.x] = trow;
+    sCode[threadIdx.x] = trow >= 0 ? (tmask != 0 ? 1 : 2) : 0;
   }
-  stage_operands<T, SP, HD, false, CLS>(qkv, bqkv, nullptr, sQ, sK, sV, nullptr, tk, b, h, S, H, len, lim);
+  stage_operands<T, SP, HD, false, CLS>(qkv, bqkv, nullptr, sQ, sK, sV, nullptr, srow, b, h, H, lim);
   __syncthreads();
   const int r0 = warp * 16;
   if (r0 >= (CLS ? 16 : lim)) return;
@@ -716,12 +753,15 @@ __global__ void __launch_bounds__(SP * 2, SP == 128 ? 2 : 1) attention_bwd_blk_k
   if (tk.slot != nullptr && b == (int)gridDim.y - 1)
     for (int w = 0; w < (CLS ? 4 : 3); ++w)
       clear_zero_rows<T>(tk, w < 3 ? dqkv : ft.dst, w < 3 ? 3 * H : H, (w < 3 ? w * H : 0) + h * HD, HD);
+  int srow[HD / 16];
+  const int trow = threadIdx.x < SP && (int)threadIdx.x < S ? seq_row(tk, b, S, threadIdx.x) : -1;    // of token threadIdx.x
   const int len = seq_len(tk, b, S), lim = (len + 15) & ~15;
   if (len > SP || len <= len_lo) return;
+  stage_rows<SP, HD>(srow, tk, b, S, len);
   if (bias_acc != nullptr)
     for (int i = threadIdx.x; i < 3 * HD; i += blockDim.x) sBias[i] = 0.f;
-  for (int j = threadIdx.x; j < SP; j += blockDim.x) sRow[j] = j < len ? seq_row(tk, b, S, j) : -1;
-  stage_operands<T, SP, HD, true, CLS>(qkv, bqkv, dctx, sQ, sK, sV, sDO, tk, b, h, S, H, len, lim);
+  if (threadIdx.x < SP) sRow[threadIdx.x] = trow;
+  stage_operands<T, SP, HD, true, CLS>(qkv, bqkv, dctx, sQ, sK, sV, sDO, srow, b, h, H, lim);
   __syncthreads();
   const int r0 = warp * 16, i0 = r0 + g, i1 = r0 + g + 8;
   const int qlim = CLS ? 16 : lim;                 // queries that have a gradient (CLS: the rows behind the first are zeros)
