@@ -587,6 +587,23 @@ def scaler_update(buf, enabled, growth, backoff, interval):
     _call("rb_scaler_update", _p(buf), _I(1 if enabled else 0), _F(growth), _F(backoff), _I(interval), _stream())
 
 
+# ----------------------------------------------------------------------------- step inputs
+def stage_inputs(pairs, hp_host=None, hp_buf=None, nnz=0, nnz_out=None) -> bool:
+    """Copies every ``(host, device)`` pair of equally shaped contiguous int32 tensors (at most four), the 8 floats ``hp_host`` and
+    the number ``nnz`` to the device in one launch that reads the host memory directly.  Returns ``False``, having done nothing,
+    where a host tensor is not page-locked, contiguous int32 memory: the caller then copies one by one.  The caller keeps the
+    host tensors alive until the launch has run (PyTorch's allocator of page-locked memory knows of copies only)."""
+    for h, d in pairs:
+        if h.is_cuda or h.dtype != torch.int32 or d.dtype != torch.int32 or h.shape != d.shape or not h.is_contiguous() \
+                or not d.is_contiguous() or (h.numel() > 0 and not h.is_pinned()):
+            return False
+    pairs = [(h, d) for h, d in pairs if h.numel() > 0]
+    _call("rb_stage_inputs", _I(len(pairs)), (_VP * 4)(*[h.data_ptr() for h, _ in pairs]),
+          (_VP * 4)(*[d.data_ptr() for _, d in pairs]), (_I * 4)(*[h.numel() for h, _ in pairs]), _p(hp_host), _p(hp_buf),
+          _p(nnz_out), _I(nnz), _stream())
+    return True
+
+
 # ----------------------------------------------------------------------------- classifier step
 def _ld_g(B: int) -> int:
     return (B + 7) // 8 * 8

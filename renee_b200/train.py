@@ -21,6 +21,7 @@ import os
 import random
 import sys
 import time
+from collections import deque
 from dataclasses import dataclass
 
 import numpy as np
@@ -189,6 +190,7 @@ class XCTrainer:
         b, S = cfg.batch_size + 1, cfg.maxlen
         self.max_nnz = 0
         self._rows_hints: dict = {}
+        self._held_inputs: deque = deque()  # (event, host tensors) of launches that read page-locked inputs
         self.buf = dict(
             ids=guard.zeros(b, S, dtype=torch.int32, device=dev, name="step.ids"),
             mask=guard.zeros(b, S, dtype=torch.int32, device=dev, name="step.mask"),
@@ -222,21 +224,38 @@ class XCTrainer:
         seed = self.rng.seed_for_step()
         self.step_rng.set(seed)
         self.hp.set_step(self.xfc_sched.lr(), self.tf_sched.lr(), seed)
-        self.hp.upload()
 
     def _upload(self, batch: XCBatch) -> tuple[int, int]:
         b = batch.input_ids.shape[0]
         nnz = int(batch.pos_rows.numel())
         self._ensure_pos_capacity(nnz)
         bf = self.buf
-        bf["ids"][:b].copy_(batch.input_ids, non_blocking=True)
-        bf["mask"][:b].copy_(batch.attention_mask, non_blocking=True)
-        bf["pos_rows"][:nnz].copy_(batch.pos_rows, non_blocking=True)
-        bf["pos_labels"][:nnz].copy_(batch.pos_labels, non_blocking=True)
-        bf["nnz"].fill_(nnz)
+        pairs = ((batch.input_ids, bf["ids"][:b]), (batch.attention_mask, bf["mask"][:b]),
+                 (batch.pos_rows, bf["pos_rows"][:nnz]), (batch.pos_labels, bf["pos_labels"][:nnz]))
+        if not self._stage(pairs, self.hp.host, self.hp.buf, nnz, bf["nnz"]):
+            self.hp.upload()
+            for host, dev in pairs:
+                dev.copy_(host, non_blocking=True)
+            bf["nnz"].fill_(nnz)
         if batch.uploaded is not None:
             batch.uploaded()            # the loader may refill the batch's staging buffers once these copies are done
         return b, nnz
+
+    def _stage(self, pairs, *scalars) -> bool:
+        """Page-locked inputs in one launch (``ops.cuda.stage_inputs``); ``False`` where they are none.  The host tensors are held
+        until an event behind the launch has passed: their memory could be handed out again before it is read otherwise."""
+        if self.device.type != "cuda":
+            return False
+        from .ops import cuda as cu
+        if not cu.stage_inputs(pairs, *scalars):
+            return False
+        held = self._held_inputs
+        ev = held.popleft()[0] if held and held[0][0].query() else torch.cuda.Event()
+        while held and held[0][0].query():
+            held.popleft()
+        ev.record()
+        held.append((ev, [host for host, _ in pairs]))
+        return True
 
     def _hint_rows(self, batch: XCBatch) -> None:
         """Tells the encoder how many tokens batches of this shape hold, once per shape (the GEMM tiles are planned for it;
@@ -599,8 +618,10 @@ class XCTrainer:
                 self._embed_generation = enc.generation
             self._embed_warm.add(shape)
             return emb
-        st["ids"].copy_(batch.input_ids, non_blocking=True)
-        st["mask"].copy_(batch.attention_mask, non_blocking=True)
+        pairs = ((batch.input_ids, st["ids"]), (batch.attention_mask, st["mask"]))
+        if not self._stage(pairs):
+            for host, dst in pairs:
+                dst.copy_(host, non_blocking=True)
         st["graph"].replay()
         return st["emb"].to(self.xfc.dtype, copy=True)
 
