@@ -475,13 +475,13 @@ class FlatEncoder:
                               self.view(G, pre + "ffn.lin1.bias"), df1)
             torch.mm(df1.t(), L["h1"][:T], out=self.view(G, pre + "ffn.lin1.weight"))
             # dh1 = d_pre2 (residual) + df1 @ W1
-            dh1 = torch.addmm(d_pre2, df1, self.view(P, pre + "ffn.lin1.weight"), out=dh)
+            dh1 = d_pre2.addmm_(df1, self.view(P, pre + "ffn.lin1.weight"))      # in place: no copy of the addend
             # ---- attention LN + attention
             d_pre1, d_ao = ops.bias_dropout_add_ln_bwd(
                 dh1, L["pre1"][:T], self.view(P, pre + "sa_layer_norm.weight"), L["mean1"][:T], L["rstd1"][:T],
                 fw["po"], rng, sb + _S_ATTN,
                 self.view(G, pre + "sa_layer_norm.weight"), self.view(G, pre + "sa_layer_norm.bias"),
-                self.view(G, pre + "attention.out_lin.bias"), buf["dh_b"][:T], L["ao"][:T])
+                self.view(G, pre + "attention.out_lin.bias"), dh, L["ao"][:T])
             torch.mm(d_ao.t(), L["ctx"][:T], out=self.view(G, pre + "attention.out_lin.weight"))
             dctx = A["dctx"][:T]
             torch.mm(d_ao, self.view(P, pre + "attention.out_lin.weight"), out=dctx)
@@ -489,7 +489,7 @@ class FlatEncoder:
             ops.attention_bwd(dctx, L["qkv"][:T], self._qkv(P, l, "bias"), mask, cfg.n_heads, pa, rng,
                               sb + _S_PROBS, L["att"], dqkv, self._qkv(G, l, "bias"))
             torch.mm(dqkv.t(), h_in, out=self._qkv(G, l, "weight"))
-            torch.addmm(d_pre1, dqkv, self._qkv(P, l, "weight"), out=dh)
+            d_pre1.addmm_(dqkv, self._qkv(P, l, "weight"))                       # d_pre1 is dh
             if on_layer_done is not None:
                 on_layer_done(l)
         ops.embed_ln_bwd(dh, fw["ids"], self.view(P, "embeddings.word_embeddings.weight"),
