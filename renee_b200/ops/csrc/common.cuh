@@ -137,37 +137,6 @@ __device__ __forceinline__ void red_add_f32x4(float* p, float a, float b, float 
   asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
 }
 
-// Standard normal CDF Phi(z) = 0.5 erfc(-z / sqrt 2), and e = exp(-z^2 / 2) as a by-product (the GELU
-// gradient needs it for the density).  erfc(|x|) = t (a1 + t (a2 + t (a3 + t (a4 + t a5)))) exp(-x^2) with
-// t = 1 / (1 + p |x|) (Abramowitz & Stegun 7.1.26, |error| <= 1.5e-7): the negative tail comes out of the
-// product directly, without the cancellation of 1 + erf, and the whole thing is 2 special-function
-// instructions and about 12 FMA-pipe ones -- which matters because the GELU kernels are bound by
-// instruction issue rather than by HBM.
-__device__ __forceinline__ float normal_cdf(float z, float& e) {
-  const float ax = fabsf(z) * 0.70710678118654752f;
-  float t;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(t) : "f"(fmaf(0.3275911f, ax, 1.f)));
-  float p = 1.061405429f;
-  p = fmaf(p, t, -1.453152027f);
-  p = fmaf(p, t, 1.421413741f);
-  p = fmaf(p, t, -0.284496736f);
-  p = fmaf(p, t, 0.254829592f);
-  e = __expf(-ax * ax);
-  const float half = 0.5f * p * t * e;
-  return z < 0.f ? half : 1.f - half;
-}
-
-// Exact (erf) GELU and its derivative: gelu(z) = z Phi(z), gelu'(z) = Phi(z) + z phi(z)
-__device__ __forceinline__ float gelu_f(float z) {
-  float e;
-  return z * normal_cdf(z, e);
-}
-__device__ __forceinline__ float gelu_grad_f(float z) {
-  float e;
-  const float cdf = normal_cdf(z, e);
-  return fmaf(z * 0.39894228040143268f, e, cdf);
-}
-
 // Two fp32 values per instruction (add / mul / fma .f32x2): IEEE arithmetic, half the issue slots.
 struct F2 { unsigned long long v; };
 __device__ __forceinline__ F2 f2(float a, float b) { F2 r; asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(a), "f"(b)); return r; }
@@ -181,9 +150,12 @@ __device__ __forceinline__ F2 f2_fma(F2 a, F2 b, F2 c) {
   return r;
 }
 
-// The tail of two values: |z|, -Q(|z|) = -0.5 erfc(|z| / sqrt 2) and e = exp(-z^2 / 2), by the formula above with its factors
-// moved: ax = |z| sqrt(log2(e) / 2), so that the exponential is one instruction, and 0.5 and the sign sit in the coefficients.
-// GELU and its gradient then need no choice between Q and 1 - Q (which was 4 of 25 instructions per pair):
+// Exact (erf) GELU and its derivative for two values, by the tail of the normal distribution: |z|, -Q(|z|) = -0.5 erfc(|z| /
+// sqrt 2) and e = exp(-z^2 / 2).  erfc(x) = t (a1 + t (a2 + t (a3 + t (a4 + t a5)))) exp(-x^2) with t = 1 / (1 + p x)
+// (Abramowitz & Stegun 7.1.26, |error| <= 1.5e-7): the negative tail comes out of the product directly, without the
+// cancellation of 1 + erf.  The factors are moved: ax = |z| sqrt(log2(e) / 2), so that the exponential is one instruction, and
+// 0.5 and the sign sit in the coefficients.  GELU and its gradient then need no choice between Q and 1 - Q (which was 4 of 25
+// instructions per pair; the kernels around them are bound by instruction issue rather than by HBM):
 //   gelu(z) = max(z, 0) - |z| Q      gelu'(z) = [z >= 0] - sign(z) Q + z e / sqrt(2 pi)
 __device__ __forceinline__ F2 normal_tail2(F2 z, F2& az, F2& e) {
   float z0, z1;

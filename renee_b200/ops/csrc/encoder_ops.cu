@@ -652,7 +652,7 @@ __global__ void __launch_bounds__(128) bias_gelu_fwd_kernel(const T* __restrict_
     for (int u = 0; u < 4; ++u)
       if (r + u * gridDim.y < rows) {
 #pragma unroll
-        for (int j = 0; j < 8; ++j) a[u][j] = gelu_f(a[u][j] + b[j]);
+        for (int j = 0; j < 8; j += 2) f2_get(gelu2(f2(a[u][j], a[u][j + 1]) + f2(b[j], b[j + 1])), a[u][j], a[u][j + 1]);
         store8(out + (size_t)(r + u * gridDim.y) * F + col, a[u]);
       }
   }
@@ -665,34 +665,41 @@ __global__ void __launch_bounds__(128) bias_gelu_bwd_kernel(const T* __restrict_
                                                             float* __restrict__ acc, unsigned* __restrict__ counter,
                                                             T* __restrict__ dbias, int rows, int F) {
   const int col = (blockIdx.x * blockDim.x + threadIdx.x) * 8;
-  float b[8], s[8];
-#pragma unroll
-  for (int j = 0; j < 8; ++j) s[j] = 0.f;
   if (col < F) {
+    float b[8];
+    F2 s[4];
     load8(bias + col, b);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) s[j] = f2(0.f);
     for (int r = blockIdx.y; r < rows; r += 2 * gridDim.y) {
-      float a[2][8], g[2][8];
+      Raw8<T> a[2], g[2];
 #pragma unroll
       for (int u = 0; u < 2; ++u) {
         const int rr = r + u * gridDim.y;
-        if (rr < rows) { load8(x + (size_t)rr * F + col, a[u]); load8(da + (size_t)rr * F + col, g[u]); }
+        if (rr < rows) { a[u] = load_raw8<T>(x + (size_t)rr * F + col); g[u] = load_raw8<T>(da + (size_t)rr * F + col); }
       }
 #pragma unroll
       for (int u = 0; u < 2; ++u) {
         const int rr = r + u * gridDim.y;
         if (rr < rows) {
+          float z[8], o[8];
+          unpack8<T>(a[u], z);
+          unpack8<T>(g[u], o);
 #pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            g[u][j] = round_through<T>(g[u][j] * gelu_grad_f(a[u][j] + b[j]));
-            s[j] += g[u][j];
-          }
-          store8(dx + (size_t)rr * F + col, g[u]);
+          for (int j = 0; j < 4; ++j)
+            f2_get(f2(o[2 * j], o[2 * j + 1]) * gelu_grad2(f2(z[2 * j], z[2 * j + 1]) + f2(b[2 * j], b[2 * j + 1])), o[2 * j], o[2 * j + 1]);
+          store8(dx + (size_t)rr * F + col, o);
+#pragma unroll
+          for (int j = 0; j < 4; ++j) s[j] = s[j] + f2(round_through<T>(o[2 * j]), round_through<T>(o[2 * j + 1]));
         }
       }
     }
     float* my_acc = acc_replica(acc, 1, F);
-    red_add_f32x4(my_acc + col, s[0], s[1], s[2], s[3]);
-    red_add_f32x4(my_acc + col + 4, s[4], s[5], s[6], s[7]);
+    float t[8];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) f2_get(s[j], t[2 * j], t[2 * j + 1]);
+    red_add_f32x4(my_acc + col, t[0], t[1], t[2], t[3]);
+    red_add_f32x4(my_acc + col + 4, t[4], t[5], t[6], t[7]);
   }
   if (counter != nullptr) finalize_columns<T>(acc, counter, 1, F, dbias, nullptr, nullptr);
 }
