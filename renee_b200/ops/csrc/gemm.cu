@@ -407,7 +407,20 @@ enc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
           if (HAS_IN) {
             tc::mbar_expect_tx(my_in_bar, IN_BYTES);
             tc::tma_load_2d(pan, &tmR, my_in_bar, pcol, sub0);
-            if (EPI == E_DW_SGD) tc::tma_load_2d(pan2, &tmF, my_in_bar, pcol, sub0);
+            if (EPI == E_DW_SGD) {
+              tc::tma_load_2d(pan2, &tmF, my_in_bar, pcol, sub0);
+              // the next tile's weights and momentum on their way to L2: 1.3 M labels x 768, batch 512, 1680 -> 1661 us; 312330 x
+              // 768, batch 90, 385 -> 375.  (The same for the weights that the logits and top-k products stream made them slower,
+              // 51 -> 63 us at 131072 x 256: their ring already keeps 24 MB on the way.)
+              if (item + its < it1) {
+                const int mt2 = (item + its) / p.n_n_tiles, nt2 = (item + its) - mt2 * p.n_n_tiles;
+                const int row2 = mt2 * (BM * NCTA) + (int)rank * BM + quarter * SUB_ROWS;
+                if (row2 < M) {
+                  tc::tma_prefetch_2d(&tmR, nt2 * p.BN + g_col, row2);
+                  tc::tma_prefetch_2d(&tmF, nt2 * p.BN + g_col, row2);
+                }
+              }
+            }
           }
         }
         if ((EPI == E_BIAS_GELU || EPI == E_BIAS_DROPOUT_RESID) && pcol + 2 * lane < p.N)
