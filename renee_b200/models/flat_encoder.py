@@ -147,6 +147,7 @@ class FlatEncoder:
         self._wgrad_stream = None
         self._wgrad_group = None
         self._wgrad_done = [None, None]
+        self._wgrad_left = None        # (parity, weight gradients that the next layer's launch takes along)
         self.pack_tokens = True        # own GEMM path: leave padded tokens out (TokenMap); a comparison may switch it off
         self.first_token_layer = True  # packed tokens, CLS pooling: last layer on first tokens only; a comparison may switch it off
         self.rows_hint = 0             # caller's estimate of the kept tokens of the coming batches (tile planning only)
@@ -436,6 +437,7 @@ class FlatEncoder:
         P, G = self.p16, self.g
         mask, packed = fw["mask"], fw["packed"]
         self._wgrad_done = [None, None]      # a pass that ended in an exception may have left an event of its own (or its capture's)
+        self._wgrad_left = None
         if self.bottleneck_dims > 0:
             gw = self.view(G, "__bottleneck__.transformer_weight")
             pooled = A["pooled"][:b]
@@ -519,7 +521,7 @@ class FlatEncoder:
                              for i in range(sets)]
         if self.own_gemm and self._wgrad_group is None:
             from ..ops import cuda as cu
-            self._wgrad_group = cu.WgradGroup([(3 * H, H), (H, H), (Fd, H), (H, Fd)], self.device)
+            self._wgrad_group = cu.WgradGroup([(3 * H, H), (H, H), (Fd, H), (H, Fd), (3 * H, H)], self.device)
 
     def _backward_layer_fused(self, l: int, L: dict, dh, on_layer_done) -> None:
         """One transformer block on the own GEMMs: ``dh`` (gradient of its output) becomes the gradient of its input."""
@@ -559,9 +561,18 @@ class FlatEncoder:
         qkv = [(dqkv, L["h_in"], self._qkv(G, l, "weight"))]
         out = [(d_ao, L["ctx"][:n], self.view(G, pre + "attention.out_lin.weight"))]
         if one_row:
-            self._wgrad_layer(par, (qkv, packed), (dense + out, {}))
+            # all tokens behind q/k/v, one row per sequence behind the others: two launches, unless the next layer's can take q/k/v
+            # along (27 tiles on their own are cut into pieces for 74 SM pairs: 32 us at 4900 tokens, 13 in its company)
+            self._wgrad_layer(par, (dense + out, {}))
+            if l > 0 and on_layer_done is None:
+                self._wgrad_left = (par, qkv)
+            else:
+                self._wgrad_layer(par, (qkv, packed))
         else:
-            self._wgrad_layer(par, (dense + qkv + out, packed))
+            left, self._wgrad_left = self._wgrad_left, None
+            self._wgrad_layer(par, (dense + qkv + out + (left[1] if left else []), packed))
+            if left:
+                self._wgrad_done[left[0]] = self._wgrad_done[par]
         cu.linear_dgrad(dqkv, self._qkv(P, l, "weight"), dh, "add", resid=resid, **packed)
         if on_layer_done is not None:
             self._wgrad_wait(par)           # the caller may reduce the layer's gradients from here on

@@ -1029,7 +1029,8 @@ static Plan make_plan(int layout, int epi, int M, int N, int K, int bn_forced, i
         const double tail = epi_clocks(epi, bn);
         double round = kb_per * t_kb + epi_share(epi) * tail;
         if (round < tail) round = tail;
-        const double cost = 3000.0 + (ncta == 2 ? 600.0 : 0.0) + rounds * round + tail + (eff_splits > 1 && epi != E_DX ? 10000.0 : 0.0);
+        double cost = 3000.0 + (ncta == 2 ? 600.0 : 0.0) + rounds * round + tail + (eff_splits > 1 && epi != E_DX ? 10000.0 : 0.0);
+        if (epi == E_TOPK) cost += 120.0 * (items < units ? items : units);      // every unit leaves candidates to select from
         if (best_cost < 0 || cost < best_cost) { best_cost = cost; best = Plan{ncta, bn, eff_splits, tiles}; }
       }
     }

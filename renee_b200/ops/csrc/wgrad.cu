@@ -28,7 +28,7 @@ constexpr int STAGE = BM * BK * 2 + (BN / 2) * BK * 2;    // per CTA: 128 rows o
 constexpr int STAGES = 7;
 constexpr int EPI_WARPS = 16, EPI_THREADS = 32 * EPI_WARPS, THREADS = 64 + EPI_THREADS;
 constexpr int TMEM_COLS = 512;
-constexpr int MAX_PROBS = 4;
+constexpr int MAX_PROBS = 5;                                // a layer's four and one that the layer behind it left over
 constexpr int MIN_RUN = 8;                                 // k blocks per unit at least: bounds the pieces of a tile
 constexpr int SMEM = STAGES * STAGE + 1024 + 512;
 constexpr size_t PIECE_FLOATS = (size_t)BM * BN;           // one CTA's half of a tile

@@ -527,7 +527,7 @@ def _wgrad_scratch_bytes(device) -> int:
 
 
 def wgrad_group(items, group: WgradGroup, tmap=None):
-    """``dW = dy.T @ x`` for every ``(dy [T, M], x [T, N], dW [M, N])`` of ``items`` (at most four) in one launch."""
+    """``dW = dy.T @ x`` for every ``(dy [T, M], x [T, N], dW [M, N])`` of ``items`` (at most five) in one launch."""
     n, T = len(items), items[0][0].shape[0]
     dims = (_I * (5 * n))()
     for i, (dy, x, dW) in enumerate(items):
