@@ -194,7 +194,8 @@ __device__ __forceinline__ F2 gelu_grad2(F2 z) {
   f2_get(z, z0, z1);
   F2 az, e;
   f2_get(normal_tail2(z, az, e), q0, q1);
-  const F2 cdf = f2(z0 < 0.f ? 0.f : 1.f, z1 < 0.f ? 0.f : 1.f) + f2(copysignf(q0, -z0), copysignf(q1, -z1));
+  // the step and the tail's sign by one comparison: by copysign, the derivative at -0 was 1.5
+  const F2 cdf = f2(z0 < 0.f ? 0.f : 1.f, z1 < 0.f ? 0.f : 1.f) + f2(z0 < 0.f ? -q0 : q0, z1 < 0.f ? -q1 : q1);
   return f2_fma(z * f2(0.39894228040143268f), e, cdf);
 }
 
