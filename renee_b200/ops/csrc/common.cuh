@@ -156,11 +156,13 @@ __device__ __forceinline__ F2 f2_fma(F2 a, F2 b, F2 c) {
 // cancellation of 1 + erf.  The factors are moved: ax = |z| sqrt(log2(e) / 2), so that the exponential is one instruction, and
 // 0.5 and the sign sit in the coefficients.  GELU and its gradient then need no choice between Q and 1 - Q (which was 4 of 25
 // instructions per pair; the kernels around them are bound by instruction issue rather than by HBM):
-//   gelu(z) = max(z, 0) - |z| Q      gelu'(z) = [z >= 0] - sign(z) Q + z e / sqrt(2 pi)
+//   gelu(z) = z [z >= 0] - |z| Q      gelu'(z) = [z >= 0] - sign(z) Q + z e / sqrt(2 pi)
+// At the infinities as torch: gelu(inf) = inf; gelu(-inf) and both derivatives are 0 times infinity, a NaN, so that a
+// pre-activation that has overflowed 16 bits is seen behind the FFN whatever its sign (max(z, 0) made a 0 of -inf).
 __device__ __forceinline__ F2 normal_tail2(F2 z, F2& az, F2& e) {
   float z0, z1;
   f2_get(z, z0, z1);
-  // a finite bound, so that an infinite z meets a tail of 0 as 0 (a NaN stays one)
+  // a finite bound, so that |z| Q of an infinite z is 0 (a NaN stays one)
   float a0, a1;
   asm("min.NaN.f32 %0, %1, 0f7F7FFFFF;" : "=f"(a0) : "f"(fabsf(z0)));
   asm("min.NaN.f32 %0, %1, 0f7F7FFFFF;" : "=f"(a1) : "f"(fabsf(z1)));
@@ -187,7 +189,7 @@ __device__ __forceinline__ F2 gelu2(F2 z) {
   f2_get(z, z0, z1);
   F2 az, e;
   const F2 nq = normal_tail2(z, az, e);
-  return f2_fma(az, nq, f2(fmaxf(z0, 0.f), fmaxf(z1, 0.f)));
+  return f2_fma(az, nq, z * f2(z0 < 0.f ? 0.f : 1.f, z1 < 0.f ? 0.f : 1.f));
 }
 __device__ __forceinline__ F2 gelu_grad2(F2 z) {
   float z0, z1, q0, q1;

@@ -59,3 +59,28 @@ def test_derivative_in_the_kernel_of_its_own(dt):
     dx, dbias = torch.empty_like(x), torch.empty_like(bias)
     ops.bias_gelu_bwd(torch.ones_like(x), x, bias, dbias, dx)
     _check(dx.flatten(), _derivative(z).flatten())
+
+
+@pytest.mark.parametrize("ncta", [1, 2])
+@pytest.mark.parametrize("dt", DTYPES)
+def test_gelu_in_the_gemm_epilogue(dt, ncta):
+    from renee_b200.ops import cuda as cu
+    T, K, z = 64, 64, _all_numbers(dt)
+    x, W = torch.zeros(T, K, device="cuda", dtype=dt), torch.zeros(z.numel(), K, device="cuda", dtype=dt)
+    x[:, 0], W[:, 0] = 1.0, z.cuda()
+    act, pre = (torch.empty(T, z.numel(), device="cuda", dtype=dt) for _ in range(2))
+    cu.linear_fwd(x, W, act, "bias_gelu", bias=torch.zeros(z.numel(), device="cuda", dtype=dt), pre_out=pre, ncta=ncta)
+    cu.check_status()
+    # the stored pre-activations are these numbers (fp32 subnormals, which bf16's are, become 0 on the way)
+    stored = torch.where(z.float().abs() < torch.finfo(torch.float32).tiny, 0.0, z.float())
+    assert torch.equal(torch.nan_to_num(pre[0].float().cpu(), 9.0), torch.nan_to_num(stored, 9.0))
+    _check(act[0], torch.nn.functional.gelu(z.double()))
+    assert torch.equal(torch.nan_to_num(act, 9.0), torch.nan_to_num(act[:1].expand(T, -1), 9.0))
+
+
+@pytest.mark.parametrize("dt", DTYPES)
+def test_gelu_in_the_kernel_of_its_own(dt):
+    z = _all_numbers(dt).view(16, 4096)
+    x, out = z.cuda(), torch.empty(16, 4096, device="cuda", dtype=dt)
+    ops.bias_gelu_fwd(x, torch.full((4096,), -0.0, device="cuda", dtype=dt), out)
+    _check(out.flatten(), torch.nn.functional.gelu(z.double()).flatten())
