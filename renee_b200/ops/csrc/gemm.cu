@@ -134,6 +134,11 @@ template <typename T> __device__ __forceinline__ void unpack8(const uint4& raw, 
   for (int i = 0; i < 8; ++i) out[i] = to_f(e[i]);
 }
 
+// The n staging warps of a row quarter come together (barrier 1 is that of all epilogue warps).
+__device__ __forceinline__ void meet_rows(int quarter, int n) {
+  asm volatile("bar.sync %0, %1;" ::"r"(2 + quarter), "r"(32 * n) : "memory");
+}
+
 // First positions of the sorted a[0 .. n) whose values are >= k_lo and >= k_hi, by one warp: each half-warp probes 16 places
 // per step, so ten thousand entries take 4 dependent loads where two binary searches in a row took 28.
 __device__ __forceinline__ void warp_bounds(const int* __restrict__ a, int n, int k_lo, int k_hi, int lane, int& lo, int& hi) {
@@ -468,8 +473,18 @@ enc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
       }
       ok = tc::mbar_wait(tmem_full_bar + buf, use & 1, aborted, p.status, tc::SITE_TMEM_FULL, item) && ok;
       if constexpr (STAGED) {
-        // a staging warp shares nothing with the others: it ends by itself where a wait has run out
-        if (!__all_sync(0xffffffffu, ok)) break;
+        // A staging warp whose wait has run out stores nothing from here on (every later wait of it returns at once).  It leaves by
+        // itself, except from the logits: there the warps of the same 32 rows meet below at barriers without a time limit, and a
+        // neighbour whose wait ended just in time would stand there for ever.  So it still comes to all of them.
+        if (!__all_sync(0xffffffffu, ok)) {
+          if (EPI != E_SIGMOID_POS) break;
+          aborted = true;                                  // in every lane
+          if (staging && p.pos_labels != nullptr && pos_end > pos_more) {
+            meet_rows(quarter, p.BN >> 6);
+            meet_rows(quarter, p.BN >> 6);
+          }
+          continue;
+        }
       } else {
         if (!ok) *s_abort = 1;
         asm volatile("bar.sync 1, %0;" ::"n"(EPI_THREADS) : "memory");
@@ -592,10 +607,9 @@ enc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
             // Labels that many rows have (the first 32 of a Zipf-distributed 1.3 M hold 5000 of 21000 positives): the warps of
             // these 32 rows share the entries out, each applying its own to all panels of the tile, 8 on their way per lane.
             // Every panel's warp scanning all of them made the launch with those labels take 192 us, where the others take 47.
-            // (The same list, hence the same way here, in each of these warps; a wait that one of them passed cannot run out
-            // in another, as the accumulator stays until all have read it.)
+            // (The same list, hence the same two meetings per tile, in each of these warps.)
             const int np = p.BN >> 6;
-            asm volatile("bar.sync %0, %1;" ::"r"(2 + quarter), "r"(32 * np) : "memory");
+            meet_rows(quarter, np);
             for (int e0 = pos_more + 32 * g + lane; e0 < pos_end; e0 += 256 * np) {
               int pl[8], pc[8];
 #pragma unroll
@@ -611,7 +625,7 @@ enc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
               }
             }
             tc::fence_proxy_async();
-            asm volatile("bar.sync %0, %1;" ::"r"(2 + quarter), "r"(32 * np) : "memory");
+            meet_rows(quarter, np);
           }
         }
         tc::fence_proxy_async();                 // generic-proxy writes of the panel before the async-proxy store

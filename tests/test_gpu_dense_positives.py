@@ -30,3 +30,24 @@ def test_logit_gradient_with_heavy_labels(Lc, B, D, heavy):
     err = (Gt[:, :B].float().cpu() - (want - Y.float())).abs()
     assert float(err.max()) < 2.0 ** -10
     assert not Gt[:, B:].any()
+
+
+def test_a_wait_that_runs_out_before_heavy_labels():
+    """A peer whose flag never comes: the launch ends with a status although its warps have meetings ahead, and the next one is right."""
+    from renee_b200.ops import cuda as cu
+    gen = torch.Generator().manual_seed(1)
+    Lc, B, D = 3000, 200, 64
+    W, X = (torch.randn(Lc, D, generator=gen) * 0.05).half(), torch.randn(B, D, generator=gen).half()
+    labels, rows = (torch.rand(Lc, B, generator=gen) < 0.5).nonzero(as_tuple=True)         # 3200 positives per 32 labels
+    Gt = torch.empty(Lc, B, dtype=torch.float16, device="cuda")
+    nnz = torch.tensor([labels.numel()], dtype=torch.int32, device="cuda")
+    flags, step = (torch.full((1,), v, dtype=torch.int32, device="cuda") for v in (0, 1))
+    args = (W.cuda(), X.cuda(), Gt, B, rows.int().cuda(), labels.int().cuda(), nnz, 0)
+    cu.xfc_logits_grad_v2(*args, wait=(flags, 1, step))
+    with pytest.raises(cu.KernelError, match="timed out"):
+        cu.check_status()
+    cu.xfc_logits_grad_v2(*args, wait=(step, 1, step))
+    cu.check_status()
+    want = torch.sigmoid(W.float() @ X.float().t())
+    want[labels, rows] -= 1.0
+    assert float((Gt.float().cpu() - want).abs().max()) < 2.0 ** -10          # two roundings to 16 bits, as above
