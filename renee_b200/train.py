@@ -190,7 +190,7 @@ class XCTrainer:
         b, S = cfg.batch_size + 1, cfg.maxlen
         self.max_nnz = 0
         self._rows_hints: dict = {}
-        self._held_inputs: deque = deque()  # (event, host tensors) of launches that read page-locked inputs
+        self._held_inputs = _HeldInputs()
         self.buf = dict(
             ids=guard.zeros(b, S, dtype=torch.int32, device=dev, name="step.ids"),
             mask=guard.zeros(b, S, dtype=torch.int32, device=dev, name="step.mask"),
@@ -242,19 +242,13 @@ class XCTrainer:
         return b, nnz
 
     def _stage(self, pairs, *scalars) -> bool:
-        """Page-locked inputs in one launch (``ops.cuda.stage_inputs``); ``False`` where they are none.  The host tensors are held
-        until an event behind the launch has passed: their memory could be handed out again before it is read otherwise."""
+        """Page-locked inputs in one launch (``ops.cuda.stage_inputs``); ``False`` where they are none."""
         if self.device.type != "cuda":
             return False
         from .ops import cuda as cu
         if not cu.stage_inputs(pairs, *scalars):
             return False
-        held = self._held_inputs
-        ev = held.popleft()[0] if held and held[0][0].query() else torch.cuda.Event()
-        while held and held[0][0].query():
-            held.popleft()
-        ev.record()
-        held.append((ev, [host for host, _ in pairs]))
+        self._held_inputs.hold([host for host, _ in pairs])
         return True
 
     def _hint_rows(self, batch: XCBatch) -> None:
@@ -630,6 +624,30 @@ class XCTrainer:
             Z = X.float() @ self.model.xfc_weight.float().t()
             return torch.topk(Z, min(k, Z.shape[1]), dim=1)
         return self.xfc.topk(X, k)
+
+
+class _HeldInputs:
+    """Page-locked host tensors that queued launches read, each until an event behind its launch has passed: PyTorch's allocator of
+    page-locked memory knows of copies only and would hand their memory out again before it is read.  The last holder waits: a
+    result may outlive the trainer that queued it."""
+
+    def __init__(self):
+        self._held: deque = deque()         # (event, tensors), oldest first
+
+    def hold(self, tensors) -> None:
+        held, ev = self._held, None
+        while held and held[0][0].query():
+            ev = held.popleft()[0]
+        ev = ev if ev is not None else torch.cuda.Event()
+        ev.record()
+        held.append((ev, tensors))
+
+    def __del__(self):
+        try:
+            for ev, _ in self._held:
+                ev.synchronize()
+        except Exception:                   # the context is gone, and what it read with it
+            pass
 
 
 class _AllGatherRows(torch.autograd.Function):

@@ -68,3 +68,42 @@ def test_steps_from_batches_that_are_dropped_at_once():
     # the steps are the same; the embedding gradients are summed by 16-bit atomics in any order
     for a, b in zip(*out):
         assert float((a.float() - b.float()).norm() / b.float().norm()) < 2.0 ** -9
+
+
+def _trainer(cuda_graph=True, B=12, S=10):
+    from renee_b200.models.encoder import EncoderConfig
+    from renee_b200.parallel.dist import DistContext
+    from renee_b200.train import TrainConfig, XCTrainer
+    from renee_b200.utils.sharding import shard_labels
+    enc = EncoderConfig(dim=128, n_layers=1, n_heads=2, hidden_dim=256, vocab_size=3000)
+    cfg = TrainConfig(batch_size=B, epochs=1, seed=0, dropout=0.5, lr1=0.05, lr2=1e-3, warmup=10, wd1=1e-4, noloss=True,
+                      fp16xfc=True, maxlen=S, pooling="cls", cuda_graph=cuda_graph)
+    return XCTrainer(cfg, enc, shard_labels(700, 1), DistContext(device=torch.device("cuda", 0)), steps_per_epoch=8)
+
+
+def test_an_embedding_outlives_its_trainer():
+    """The trainer and the batch are dropped while the launch that reads the batch is still queued, and their page-locked memory is
+    handed out again at once."""
+    import gc
+    import weakref
+    from types import SimpleNamespace
+    gen = torch.Generator().manual_seed(2)
+    ids, mask = torch.randint(5, 3000, (12, 10), generator=gen, dtype=torch.int32), torch.ones(12, 10, dtype=torch.int32)
+    mask[:, 7:] = 0
+
+    def pinned():
+        return SimpleNamespace(input_ids=ids.clone().pin_memory(), attention_mask=mask.clone().pin_memory())
+    tr = _trainer()
+    for _ in range(3):                                     # eager, captured, staged
+        want = tr.embed_eval(pinned())
+    batch = pinned()
+    torch.cuda.synchronize()
+    torch.cuda._sleep(200_000_000)                         # some 0.1 s
+    got = tr.embed_eval(batch)
+    gone = weakref.ref(tr)
+    del tr, batch
+    gc.collect()
+    assert gone() is None
+    taken = [torch.full((12, 10), 7, dtype=torch.int32).pin_memory() for _ in range(16)]
+    torch.cuda.synchronize()
+    assert torch.equal(got, want) and len(taken) == 16
