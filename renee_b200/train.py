@@ -242,8 +242,9 @@ class XCTrainer:
         return b, nnz
 
     def _stage(self, pairs, *scalars) -> bool:
-        """Page-locked inputs in one launch (``ops.cuda.stage_inputs``); ``False`` where they are none."""
-        if self.device.type != "cuda":
+        """Page-locked inputs in one launch (``ops.cuda.stage_inputs``); ``False`` where they are none, and in a graph of the caller's:
+        it replays copies of the host tensors, which PyTorch keeps track of, and an event recorded there could not be asked."""
+        if self.device.type != "cuda" or torch.cuda.is_current_stream_capturing():
             return False
         from .ops import cuda as cu
         if not cu.stage_inputs(pairs, *scalars):

@@ -107,3 +107,33 @@ def test_an_embedding_outlives_its_trainer():
     taken = [torch.full((12, 10), 7, dtype=torch.int32).pin_memory() for _ in range(16)]
     torch.cuda.synchronize()
     assert torch.equal(got, want) and len(taken) == 16
+
+
+def test_training_step_in_a_graph_of_the_callers():
+    """``cuda_graph=False`` leaves capturing to the caller: a captured step and an eager one behind it, against eager steps."""
+    import numpy as np
+    from renee_b200.data import xcrepo
+    from renee_b200.data.collate import XCCollator
+    from renee_b200.data.synthetic import SyntheticSpec, SyntheticXC
+    from renee_b200.utils.sharding import shard_labels
+    spec = SyntheticSpec(num_labels=700, seq_len=10, len_lo=2, len_hi=10, vocab=3000, poisson_lam=2.0, seed=0)
+    data = xcrepo.InMemoryDataset(*SyntheticXC(spec).rows(np.arange(12)))
+    batch = XCCollator(shard_labels(700, 1), data, 0, 1, 12, True)(np.arange(12)).pin()
+    out = []
+    for capture in (False, True):
+        tr = _trainer(cuda_graph=False)
+        for _ in range(3):
+            tr.train_step(batch)
+        if capture:
+            graph = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(graph):
+                tr.train_step(batch)
+            graph.replay()
+        else:
+            tr.train_step(batch)
+        tr.train_step(batch)
+        torch.cuda.synchronize()
+        out.append((tr.xfc.W.clone(), tr.encoder.p32.clone()))
+    # the steps are the same; the embedding gradients are summed by 16-bit atomics in any order
+    for a, b in zip(*out):
+        assert float((a.float() - b.float()).norm() / b.float().norm()) < 2.0 ** -9
