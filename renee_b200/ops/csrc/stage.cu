@@ -37,6 +37,19 @@ __global__ void __launch_bounds__(256) stage_inputs_kernel(const StageArgs a) {
 
 using namespace rb;
 
+// 1: what was recorded before the event has run; 0: not yet (wait == 0); else minus a CUDA error.  This thread's part in the capture
+// of another thread is relaxed for the call: a query or a wait of this kind ends a capture in the default (global) mode.
+RB_API int rb_event_passed(cudaEvent_t ev, int wait) {
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  cudaError_t e = cudaThreadExchangeStreamCaptureMode(&mode);
+  if (e != cudaSuccess) return -(int)e;
+  e = wait ? cudaEventSynchronize(ev) : cudaEventQuery(ev);
+  const cudaError_t back = cudaThreadExchangeStreamCaptureMode(&mode);
+  if (e == cudaErrorNotReady) { (void)cudaGetLastError(); return back == cudaSuccess ? 0 : -(int)back; }
+  if (e == cudaSuccess) e = back;
+  return e == cudaSuccess ? 1 : -(int)e;
+}
+
 // src[i]: page-locked host memory, n[i] words, i < n_segs <= 4.  hp_host (nullable): STAGE_HP floats, read here; nnz_dst nullable.
 RB_API int rb_stage_inputs(int n_segs, const void* const* src, void* const* dst, const int* n, const float* hp_host, float* hp_dst,
                            int* nnz_dst, int nnz, cudaStream_t st) {

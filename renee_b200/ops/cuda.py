@@ -604,6 +604,15 @@ def stage_inputs(pairs, hp_host=None, hp_buf=None, nnz=0, nnz_out=None) -> bool:
     return True
 
 
+def event_passed(event, wait=False) -> bool:
+    """Whether what was recorded before ``event`` has run; ``wait``: waits for it.  Unlike ``event.query()`` also while another thread
+    captures a graph in the default mode, which forbids every thread of the process such calls and is ended by one."""
+    rc = lib().rb_event_passed(_VP(event.cuda_event), _I(1 if wait else 0))
+    if rc < 0 or rc > 1:
+        raise KernelError(f"rb_event_passed failed with code {rc}")
+    return rc == 1
+
+
 # ----------------------------------------------------------------------------- classifier step
 def _ld_g(B: int) -> int:
     return (B + 7) // 8 * 8

@@ -636,8 +636,9 @@ class _HeldInputs:
         self._held: deque = deque()         # (event, tensors), oldest first
 
     def hold(self, tensors) -> None:
+        from .ops import cuda as cu
         held, ev = self._held, None
-        while held and held[0][0].query():
+        while held and cu.event_passed(held[0][0]):
             ev = held.popleft()[0]
         ev = ev if ev is not None else torch.cuda.Event()
         ev.record()
@@ -645,8 +646,9 @@ class _HeldInputs:
 
     def __del__(self):
         try:
+            from .ops import cuda as cu
             for ev, _ in self._held:
-                ev.synchronize()
+                cu.event_passed(ev, wait=True)
         except Exception:                   # the context is gone, and what it read with it
             pass
 

@@ -137,3 +137,39 @@ def test_training_step_in_a_graph_of_the_callers():
     # the steps are the same; the embedding gradients are summed by 16-bit atomics in any order
     for a, b in zip(*out):
         assert float((a.float() - b.float()).norm() / b.float().norm()) < 2.0 ** -9
+
+
+def test_steps_beside_a_capture_of_another_thread():
+    """A thread that captures in the default mode forbids every thread a query of an event; a step on pinned batches needs none."""
+    import threading
+    import numpy as np
+    from renee_b200.data import xcrepo
+    from renee_b200.data.collate import XCCollator
+    from renee_b200.data.synthetic import SyntheticSpec, SyntheticXC
+    from renee_b200.utils.sharding import shard_labels
+    spec = SyntheticSpec(num_labels=700, seq_len=10, len_lo=2, len_hi=10, vocab=3000, poisson_lam=2.0, seed=0)
+    data = xcrepo.InMemoryDataset(*SyntheticXC(spec).rows(np.arange(12)))
+    batch = XCCollator(shard_labels(700, 1), data, 0, 1, 12, True)(np.arange(12)).pin()
+    tr = _trainer()
+    for _ in range(6):
+        tr.train_step(batch)
+        tr.embed_eval(batch)
+    torch.cuda.synchronize()
+    raised = []
+
+    def steps():
+        try:
+            for _ in range(3):
+                tr.train_step(batch)
+        except Exception as exc:
+            raised.append(exc)
+    x, graph = torch.zeros(8, device="cuda"), torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        x.add_(1.0)
+        thread = threading.Thread(target=steps)
+        thread.start()
+        thread.join()
+    assert not raised
+    graph.replay()
+    torch.cuda.synchronize()
+    assert x.tolist() == [1.0] * 8 and tr.count == 9
