@@ -408,20 +408,18 @@ class FlatEncoder:
         if on_layer_done is not None:
             on_layer_done(-1)       # embeddings and every vector-shaped gradient are final: the whole buffer is
 
-    def _wgrad_layer(self, par: int, *groups) -> None:
-        """The weight gradients of one layer, one launch per ``(items, token map arguments)``, on the weight-gradient stream
-        (ordered after everything issued so far on the current one).  Their inputs live in the backward buffers of parity ``par``, which the layer after
-        the next overwrites: :meth:`_wgrad_wait` comes before that."""
+    def _wgrad_layer(self, par: int, items, packed) -> None:
+        """Weight gradients in one launch, their rows numbered by the token map in ``packed``, on the weight-gradient stream (ordered
+        after everything issued so far on the current one).  Their inputs live in the backward buffers of parity ``par``, which the
+        layer after the next overwrites: :meth:`_wgrad_wait` comes before that."""
         from ..ops import cuda as cu
         side = self._wgrad_stream
         if side is None:
-            for items, packed in groups:
-                cu.wgrad_group(items, self._wgrad_group, **packed)
+            cu.wgrad_group(items, self._wgrad_group, **packed)
             return
         side.wait_stream(torch.cuda.current_stream())
         with torch.cuda.stream(side):
-            for items, packed in groups:
-                cu.wgrad_group(items, self._wgrad_group, **packed)
+            cu.wgrad_group(items, self._wgrad_group, **packed)
             self._wgrad_done[par] = side.record_event()
 
     def _wgrad_wait(self, par: int) -> None:
@@ -563,14 +561,14 @@ class FlatEncoder:
         if one_row:
             # all tokens behind q/k/v, one row per sequence behind the others: two launches, unless the next layer's can take q/k/v
             # along (27 tiles on their own are cut into pieces for 74 SM pairs: 32 us at 4900 tokens, 13 in its company)
-            self._wgrad_layer(par, (dense + out, {}))
+            self._wgrad_layer(par, dense + out, {})
             if l > 0 and on_layer_done is None:
                 self._wgrad_left = (par, qkv)
             else:
-                self._wgrad_layer(par, (qkv, packed))
+                self._wgrad_layer(par, qkv, packed)
         else:
             left, self._wgrad_left = self._wgrad_left, None
-            self._wgrad_layer(par, (dense + qkv + out + (left[1] if left else []), packed))
+            self._wgrad_layer(par, dense + qkv + out + (left[1] if left else []), packed)
             if left:
                 self._wgrad_done[left[0]] = self._wgrad_done[par]
         cu.linear_dgrad(dqkv, self._qkv(P, l, "weight"), dh, "add", resid=resid, **packed)

@@ -45,3 +45,50 @@ def test_first_tokens_only_equals_all_tokens(monkeypatch, S, b, heads, dt, layer
         scale = float(y.abs().max().clamp_min(1e-6))
         tol = 2.0 ** -7 * y.abs() + (3e-2 if name.startswith("embeddings") else 1e-4) * scale
         assert bool(((x - y).abs() <= tol).all()), (name, float((x - y).abs().max()), scale)
+
+
+@pytest.mark.parametrize("S,b,heads,dt", [(16, 9, 8, torch.float16), (33, 70, 4, torch.bfloat16)])
+@pytest.mark.parametrize("layers", [1, 3, 4])
+@pytest.mark.parametrize("side,callback", [(False, True), (True, False), (True, True)])
+def test_weight_gradients_left_to_the_next_launch(monkeypatch, S, b, heads, dt, layers, side, callback):
+    """Weight gradients on a stream of their own, where the backward buffers of two layers take turns, and the caller's callback, which
+    reads a layer's gradients as soon as it is told of them: against one stream without a callback."""
+    from renee_b200.models.encoder import EncoderConfig
+    from renee_b200.models.flat_encoder import FlatEncoder
+    from renee_b200.ops import StepRNG, cuda as cu
+    monkeypatch.setenv("RENEE_B200_OWN_GEMM", "1")
+    cfg = EncoderConfig(dim=256, n_layers=layers, n_heads=heads, hidden_dim=512, vocab_size=2000)
+    gen = torch.Generator().manual_seed(S * 10 + b)
+    mask = (torch.rand(b, S, generator=gen) < 0.6).to(torch.int32).cuda()
+    ids = torch.randint(5, 2000, (b, S), generator=gen, dtype=torch.int32).cuda()
+    d_emb = (torch.randn(b, 256, generator=gen) * 0.1).cuda()
+    rng = StepRNG(7, torch.tensor([7], dtype=torch.int32, device="cuda"))
+    grads = []
+    for on in (False, True):
+        enc = FlatEncoder(cfg, torch.device("cuda", 0), dt, "cls", 0, seed=3)
+        enc._wgrad_stream = torch.cuda.Stream() if on and side else None
+        seen = {}
+
+        def done(l):
+            for name, slot in enc.slots.items():
+                if l >= 0 and name.startswith(f"transformer.layer.{l}.") and len(slot.shape) == 2:
+                    seen[name] = enc.g[slot.offset: slot.offset + slot.numel].clone()
+        for _ in range(2):
+            enc.forward(ids, mask, rng, train=True)
+            assert enc._fw["first"] is not None
+            enc.g.fill_(float("nan"))
+            enc.backward(d_emb, on_layer_done=done if on and callback else None)
+        grads.append(enc.g.float().clone())
+        torch.cuda.synchronize()
+        assert len(seen) == (6 * layers if on and callback else 0)
+        for name, g in seen.items():
+            slot = enc.slots[name]
+            assert torch.equal(g, enc.g[slot.offset: slot.offset + slot.numel]), name
+    cu.check_status()
+    for name, slot in enc.slots.items():
+        x, y = (g[slot.offset: slot.offset + slot.numel] for g in grads)
+        # the products are cut into pieces in other places, whose fp32 sums are rounded once: one ulp, and fp32 noise at the scale
+        # of the largest (embeddings: 16-bit atomics in any order)
+        scale = float(y.abs().max().clamp_min(1e-6))
+        tol = 2.0 ** -7 * y.abs() + (3e-2 if name.startswith("embeddings") else 1e-4) * scale
+        assert bool(((x - y).abs() <= tol).all()), (name, float((x - y).abs().max()), scale)
