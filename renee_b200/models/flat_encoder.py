@@ -55,11 +55,17 @@ def _no_decay(name: str) -> bool:
 
 
 # Padded tokens per step and GPU from which the own GEMMs are used in "auto" mode.  The rule looks at nothing but the padded
-# shape: the two paths round differently, and a step must not depend on which batch a run happened to begin with.  Below it
-# the fixed cost per launch of a persistent kernel (TMEM allocation, cluster start-up, a serial K loop on the few SMs the
-# tiles cover) outweighs the fused epilogues where most tokens are kept.  Training steps of 6 DistilBERT layers on one B200,
-# us, own (packed) / library GEMMs: 1024 padded tokens all kept 1401 / 1189, 608 kept 1343 / 1190; 2048: 1675 / 1445, 1216
-# kept 1480 / 1503; 4096: 2131 / 2125, 2432 kept 1848 / 2120; 6144: 2645 / 2663, 3648 kept 2117 / 2647.
+# shape: the two paths round differently, and a step must not depend on which batch a run happened to begin with.  At small
+# sizes the fixed cost per launch of a persistent kernel (TMEM allocation, cluster start-up, a serial K loop on the few SMs the
+# tiles cover) outweighs the fused epilogues where most tokens are kept.  Training steps with 16384 labels on one B200, us, own
+# (packed) / library GEMMs, all tokens kept; about 60 % kept:
+#   DistilBERT, bf16, CLS, S = 32:   1024 padded tokens 1274 / 1167; 1170 / 1166     2048: 1431 / 1358; 1317 / 1356
+#                                    3072: 1568 / 1578; 1430 / 1572   4096: 1826 / 1912; 1551 / 1963   6144: 2226 / 2536; 1823 / 2491
+#   mean:                            1024: 1298 / 1120; 1180 / 1172   2048: 1486 / 1425; 1352 / 1419   4096: 1954 / 1982; 1615 / 1917
+#   fp16, mean, S = 48:              960: 1288 / 1114; 1233 / 1168    2160: 1520 / 1392; 1462 / 1388   4320: 2072 / 2045; 1733 / 2050
+#   MiniLM (384-wide), bf16, CLS:    1024: 796 / 735; 696 / 682       2048: 884 / 813; 781 / 867       4096: 1035 / 1137; 924 / 1134
+# So with the present kernels the paths cross between 2000 and 4300 tokens even where all are kept.  8192 is where they crossed
+# when the rule was made; steps between have run on the library since, and moving the line changes how they round.
 OWN_GEMM_MIN_TOKENS = int(os.environ.get("RENEE_B200_OWN_GEMM_MIN_TOKENS", "8192"))
 
 

@@ -602,7 +602,8 @@ __device__ __forceinline__ void store_pair(T* __restrict__ base, size_t idx, uin
 // walk the keys in blocks of KB = 64 over the resident operands: 128 registers per thread, and the dS and P~ tiles shrink
 // to [SP][KB] (112 KB per CTA at SP = 128: two per SM; 218 KB at SP = 256).
 // Measured inside the 64 x 256 training step (12 heads, lengths 64..256): streaming kernels 520 (forward) + 842 (dQ) +
-// 304 us (dK, dV) per layer padded; now, packed, 120 and 264 us.  Step 11.36 (packed, streaming kernels) -> 7.50 ms.
+// 304 us (dK, dV) per layer padded; packed, on these, 120 and 210 us (both tiles).  Step 11.36 (packed, streaming kernels) ->
+// 7.50 ms when they went in.
 //   forward   pass 1: running row maximum and sum; pass 2: probabilities (stored for the backward), dropout, O += P~ V
 //   backward  pass 1: row sums of dP * P, keeping the dropout decisions as one bit each; pass 2, per key block: dS and P~
 //             to shared memory, dQ += dS K, then the block's dK = dS^T Q and dV = P~^T dO, spread over all warps.

